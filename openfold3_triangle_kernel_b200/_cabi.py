@@ -53,6 +53,22 @@ ERROR_NAMES = {1: "invalid argument", 2: "unsupported", 3: "CUDA error", 4: "wor
 
 _lock = threading.Lock()
 _lib = None
+_native_module = None
+
+
+def native():
+    """The torch extension module `_native`: the operators' eager host path (checks, allocation, launches and
+    autograd nodes in C++, see csrc/tpf_torch*.cpp)."""
+    global _native_module
+    if _native_module is None:
+        load()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise RuntimeError(f"the extension module _native cannot be loaded ({e}): build it with "
+                               "`python -m openfold3_triangle_kernel_b200.build`") from e
+        _native_module = module
+    return _native_module
 
 
 class TpfError(RuntimeError):

@@ -93,43 +93,13 @@ def is_turbo_attention_supported(q, k, v, res_mask, pair_bias, *, check_device=T
 
 
 # --------------------------------------------------------------------------------------
-# custom ops (flattened batch, padded head dim): the only callers of the C ABI
+# custom ops (flattened batch, padded head dim): what a traced graph (torch.compile, torch.export, fake tensors) holds.
+# An eager call on plain CUDA tensors goes to `_native.attention`, which does the same in one C++ call.
 # --------------------------------------------------------------------------------------
-def _kernel_layout(t):
-    """A [B,O,H,N,D] tensor the TMA descriptors can describe: last dim contiguous,
-    16-byte aligned base and strides.  Anything else is copied once."""
-    ok = t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all((s * 2) % 16 == 0 for s in t.stride()[:-1])
-    return t if ok else t.contiguous()
-
-
-def _prep_mask_bias(mask, bias, n):
-    """mask fp32 [B,O,N] -> row pitch multiple of 4; bias bf16 [G,H,N,N] -> row pitch multiple of 8."""
-    mp = (n + 3) // 4 * 4
-    if mask.dtype != torch.float32 or mp != n or not mask.is_contiguous():
-        m = mask.new_zeros(mask.shape[:-1] + (mp,), dtype=torch.float32)
-        m[..., :n] = mask
-        mask = m
-    bp = (n + 7) // 8 * 8
-    if bias.dtype != torch.bfloat16 or bp != n or not bias.is_contiguous():
-        b = bias.new_zeros(bias.shape[:-1] + (bp,), dtype=torch.bfloat16)
-        b[..., :n] = bias
-        bias = b
-    return mask, mp, bias, bp
-
-
 @torch.library.custom_op("tpf_b200::attn_fwd", mutates_args=())
 def _attn_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, mask: torch.Tensor, bias: torch.Tensor,
               scale: float) -> tuple[torch.Tensor, torch.Tensor]:
-    B, O, H, N, D = q.shape
-    q, k, v = (_kernel_layout(t) for t in (q, k, v))
-    mask_p, mp, bias_p, bp = _prep_mask_bias(mask, bias, N)
-    out = torch.empty((B, O, N, H, D), device=q.device, dtype=torch.bfloat16)
-    lse = torch.empty((B, O, H, N), device=q.device, dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        C.call("tpf_attn_fwd", C.ptr(q), C.ptr(k), C.ptr(v), C.i64_array(q.stride()[:4]),
-               C.i64_array(k.stride()[:4]), C.i64_array(v.stride()[:4]), C.ptr(mask_p), mp, C.ptr(bias_p), bp,
-               bias.shape[0], C.ptr(out), C.ptr(lse), B, O, H, N, D, float(scale), C.current_stream())
-    return out, lse
+    return C.native().attn_fwd(q, k, v, mask, bias, scale)
 
 
 @_attn_fwd.register_fake
@@ -142,23 +112,7 @@ def _(q, k, v, mask, bias, scale):
 def _attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, d_out: torch.Tensor, out: torch.Tensor,
               lse: torch.Tensor, mask: torch.Tensor, bias: torch.Tensor,
               scale: float) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
-    B, O, H, N, D = q.shape
-    G = bias.shape[0]
-    q, k, v = (_kernel_layout(t) for t in (q, k, v))
-    d_out = d_out.contiguous()
-    out = out.contiguous()
-    mask_p, mp, bias_p, bp = _prep_mask_bias(mask, bias, N)
-    dq, dk, dv = (torch.empty((B, O, H, N, D), device=q.device, dtype=torch.bfloat16) for _ in range(3))
-    dbias = torch.empty((G, H, N, N), device=q.device, dtype=torch.float32)
-    delta = torch.empty((B, O, H, N), device=q.device, dtype=torch.float32)
-    ws_bytes = C.load().tpf_attn_bwd_workspace_bytes(B, O, H, N, D, G)
-    ws = torch.empty((max(ws_bytes, 256),), device=q.device, dtype=torch.uint8)
-    with torch.cuda.device(q.device):
-        C.call("tpf_attn_bwd", C.ptr(q), C.ptr(k), C.ptr(v), C.ptr(d_out), C.i64_array(q.stride()[:4]),
-               C.i64_array(k.stride()[:4]), C.i64_array(v.stride()[:4]), C.ptr(out), C.ptr(lse), C.ptr(mask_p), mp,
-               C.ptr(bias_p), bp, G, C.ptr(dq), C.ptr(dk), C.ptr(dv), C.ptr(dbias), C.ptr(delta), C.ptr(ws), ws_bytes,
-               B, O, H, N, D, float(scale), C.current_stream())
-    return dq, dk, dv, dbias
+    return C.native().attn_bwd(q, k, v, d_out, out, lse, mask, bias, scale)
 
 
 @_attn_bwd.register_fake
@@ -196,6 +150,11 @@ def turbo_attention(q, k, v, pair_bias=None, res_mask=None, *, return_lse=False)
     returns the fp32 log-sum-exp ``[*B, O, H, N]`` (``-inf`` for fully masked rows).
     """
     global _INVOCATIONS
+    if not torch.compiler.is_compiling():
+        res = C.native().attention(q, k, v, pair_bias, res_mask, return_lse)
+        if res is not None:
+            _INVOCATIONS += 1
+            return res
     if pair_bias is None:
         raise ValueError("unsupported TurboPairFormer case: pair_bias is required (pass zeros if there is none)")
     if res_mask is None:

@@ -389,6 +389,24 @@ __device__ __forceinline__ float lg2_approx(float x) {
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// Unsigned division by a run-time constant: multiply-high by a rounded-up reciprocal (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", 1994), exact for n < 2^31.  A plain integer division by a
+// run-time value costs several hundred cycles in a lone warp.
+struct FastDiv {
+  uint32_t d, mul, shift;
+  __host__ __device__ static FastDiv make(uint32_t d) {
+    FastDiv f{d, 0u, 0u};
+    if (d > 1) {
+      uint32_t log = 0;
+      while ((1ull << log) < d) ++log;
+      f.mul = (uint32_t)(((1ull << (31 + log)) + d - 1) / d);
+      f.shift = log - 1;
+    }
+    return f;
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return d == 1 ? n : __umulhi(n, mul) >> shift; }
+};
+
 // Programmatic dependent launch: returns once the preceding kernel of the stream has completed and its
 // memory operations are visible (a no-op for a kernel launched without the attribute).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -15,7 +15,11 @@
 // channel-major re-layout that the k-contraction wants are fused into GEMM epilogues.  The
 // a / b / x tensors live channel-major ([B*C][N*N]) so that the k-contraction is a plain batched
 // GEMM in both directions (K-major operands when outgoing, MN-major when incoming).
+#include <cuda_fp16.h>
+
 #include "tpf_gemm_host.cuh"
+#include "tpf_internal.h"
+#include "tpf_pair_rows.cuh"
 
 namespace tpf {
 
@@ -34,9 +38,6 @@ int bmm_bf16(const void* A, int64_t lda, int64_t bsa, int a_mn, const void* B, i
              int64_t k_per_split, int swizzle_bytes, cudaStream_t stream);
 
 typedef __nv_bfloat16 bf16;
-
-__device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xFFFF0000u); }
 
 // =============================================================================================
 // weight packing: fp32 masters -> bf16 W5 [5C,C] = [a_p; a_g; b_p; b_g; g], W5T [C,5C], Wz [C,C], WzT [C,C]
@@ -95,7 +96,8 @@ template <int C>
 __global__ void __launch_bounds__(256) trimul_ln_fwd_kernel(const bf16* __restrict__ z, const float* __restrict__ gamma,
                                                             const float* __restrict__ beta, bf16* __restrict__ zln,
                                                             float* __restrict__ mean, float* __restrict__ rstd,
-                                                            int64_t R) {
+                                                            const PairRows rows, const PairMask pmask,
+                                                            float* __restrict__ mask_out, int64_t R) {
   griddep_wait();
   using L = RowLanes<C>;
   constexpr int G = 4;  // row groups per warp, all loads issued before the first use
@@ -110,13 +112,17 @@ __global__ void __launch_bounds__(256) trimul_ln_fwd_kernel(const bf16* __restri
     b[e] = on ? beta[part * 8 + e] : 0.f;
   }
   uint4 u[G];
-  bool active[G];
+  bool active[G], real[G];  // real: the row exists in the caller's tensor (padding rows come out as zeros)
 #pragma unroll
   for (int r = 0; r < G; ++r) {
     const int64_t row = (warp * G + r) * L::RPW + sub;
     active[r] = on && row < R;
+    const PairPos pos = mask_out != nullptr ? rows.split((uint32_t)(row < R ? row : 0))
+                                            : rows.locate((uint32_t)(row < R ? row : 0));
+    real[r] = active[r] && pos.src >= 0;
     u[r] = make_uint4(0u, 0u, 0u, 0u);
-    if (active[r]) u[r] = *reinterpret_cast<const uint4*>(z + row * C + part * 8);
+    if (real[r]) u[r] = *reinterpret_cast<const uint4*>(z + pos.src * C + part * 8);
+    if (mask_out != nullptr && active[r] && part == 0) mask_out[row] = real[r] ? pmask.load(pos) : 0.f;
   }
 #pragma unroll
   for (int r = 0; r < G; ++r) {
@@ -135,13 +141,15 @@ __global__ void __launch_bounds__(256) trimul_ln_fwd_kernel(const bf16* __restri
     const float var = fmaxf(s2 * (1.f / C) - mu * mu, 0.f);
     const float rs = rsqrtf(var + 1e-5f);
     if (active[r]) {
-      uint4 o;
+      uint4 o = make_uint4(0u, 0u, 0u, 0u);
+      if (real[r]) {
       o.x = pack_bf16x2((x[0] - mu) * rs * g[0] + b[0], (x[1] - mu) * rs * g[1] + b[1]);
       o.y = pack_bf16x2((x[2] - mu) * rs * g[2] + b[2], (x[3] - mu) * rs * g[3] + b[3]);
       o.z = pack_bf16x2((x[4] - mu) * rs * g[4] + b[4], (x[5] - mu) * rs * g[5] + b[5]);
       o.w = pack_bf16x2((x[6] - mu) * rs * g[6] + b[6], (x[7] - mu) * rs * g[7] + b[7]);
+      }
       *reinterpret_cast<uint4*>(zln + row * C + part * 8) = o;
-      if (part == 0) {
+      if (part == 0 && mean != nullptr) {
         mean[row] = mu;
         rstd[row] = rs;
       }
@@ -237,7 +245,7 @@ __global__ void __launch_bounds__(256, 2) trimul_xnorm_fwd_kernel(const bf16* __
         const float y1 = (bf16_hi(fr[i][m]) - mu) * rs * g[i][m].y + bt[i][m].y;
         *reinterpret_cast<uint32_t*>(ys + rr * OUT_PITCH + (32 * i + 8 * m + k2) * 2) = pack_bf16x2(y0, y1);
       }
-    if ((lane & 3) == 0 && r0 + rr < NN) {
+    if (mean != nullptr && (lane & 3) == 0 && r0 + rr < NN) {
       mean[(int64_t)bb * NN + r0 + rr] = mu;
       rstd[(int64_t)bb * NN + r0 + rr] = rs;
     }
@@ -379,11 +387,15 @@ struct EpiProjGate {
   }
 };
 
-// Output projection: out = acc * sigmoid(gate)
+// Output projection: out = acc * sigmoid(gate), and with a residual input sum = res + out.  Rows of the internal
+// (padded) grid are stored at the caller's positions; padding rows are dropped.
 struct EpiOutGate {
   struct Params {
-    bf16* out;        // [R][C]
+    bf16* out;        // caller's rows x C; may be null when `sum` is wanted alone
+    bf16* sum;        // caller's rows x C or null
+    const bf16* res;  // residual input, caller's rows x C (read when sum != null)
     const bf16* gate; // [R][C]
+    PairRows rows;
     int C;
   };
   static constexpr bool kPaired = false;
@@ -411,11 +423,8 @@ struct EpiOutGate {
         ow[4 * i + e] = pack_bf16x2(v[8 * i + 2 * e] * sigmoid_fast(bf16_lo(gw[e])),
                                     v[8 * i + 2 * e + 1] * sigmoid_fast(bf16_hi(gw[e])));
     }
-    const int m_base = m - lane;
-    bf16* blk = p.out + n0;
-    warp_tile_store(reinterpret_cast<uint8_t*>(wsm), lane, ow, [&](int r) -> bf16* {
-      return m_base + r < sh.M ? blk + (int64_t)(m_base + r) * p.C : nullptr;
-    });
+    store_rows_with_residual(reinterpret_cast<uint8_t*>(wsm), lane, ow, p.rows, m - lane, sh.M, p.C, n0, p.out, p.sum,
+                             p.res);
   }
 };
 
@@ -512,30 +521,34 @@ struct EpiGateSplitBwd {
 // backward elementwise stages
 // =============================================================================================
 // d_y = d_out * sigmoid(g);  d_glogit = d_out * out * (1 - sigmoid(g))  -> d_proj5[:, 4C:5C]
+// d_out and out have the caller's rows, the results the internal (padded) rows: zeros where no caller row exists.
 __global__ void __launch_bounds__(256) trimul_out_gate_bwd_kernel(const bf16* __restrict__ d_out,
                                                                   const bf16* __restrict__ out,
                                                                   const bf16* __restrict__ gate, bf16* __restrict__ d_y,
-                                                                  bf16* __restrict__ d_proj5, int64_t R, int C) {
+                                                                  bf16* __restrict__ d_proj5, const PairRows rows,
+                                                                  const FastDiv per_row, int64_t R, int C) {
   griddep_wait();
-  const int64_t n8 = R * C / 8;
-  const int per_row = C / 8;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint4 a = reinterpret_cast<const uint4*>(d_out)[i];
-    const uint4 b = reinterpret_cast<const uint4*>(out)[i];
-    const uint4 g = reinterpret_cast<const uint4*>(gate)[i];
-    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w}, gw[4] = {g.x, g.y, g.z, g.w};
-    uint32_t y[4], l[4];
+  const uint32_t n8 = (uint32_t)(R * C / 8);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += gridDim.x * blockDim.x) {
+    const uint32_t row = per_row.div(i);
+    const int col8 = (int)(i - row * per_row.d);
+    const PairPos pos = rows.locate(row);
+    uint32_t y[4] = {0u, 0u, 0u, 0u}, l[4] = {0u, 0u, 0u, 0u};
+    if (pos.src >= 0) {
+      const uint4 a = *reinterpret_cast<const uint4*>(d_out + pos.src * C + col8 * 8);
+      const uint4 b = *reinterpret_cast<const uint4*>(out + pos.src * C + col8 * 8);
+      const uint4 g = reinterpret_cast<const uint4*>(gate)[i];
+      const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w}, gw[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float s0 = sigmoid_fast(bf16_lo(gw[e])), s1 = sigmoid_fast(bf16_hi(gw[e]));
-      const float d0 = bf16_lo(aw[e]), d1 = bf16_hi(aw[e]);
-      y[e] = pack_bf16x2(d0 * s0, d1 * s1);
-      l[e] = pack_bf16x2(d0 * bf16_lo(bw[e]) * (1.f - s0), d1 * bf16_hi(bw[e]) * (1.f - s1));
+      for (int e = 0; e < 4; ++e) {
+        const float s0 = sigmoid_fast(bf16_lo(gw[e])), s1 = sigmoid_fast(bf16_hi(gw[e]));
+        const float d0 = bf16_lo(aw[e]), d1 = bf16_hi(aw[e]);
+        y[e] = pack_bf16x2(d0 * s0, d1 * s1);
+        l[e] = pack_bf16x2(d0 * bf16_lo(bw[e]) * (1.f - s0), d1 * bf16_hi(bw[e]) * (1.f - s1));
+      }
     }
     reinterpret_cast<uint4*>(d_y)[i] = make_uint4(y[0], y[1], y[2], y[3]);
-    const int64_t row = i / per_row;
-    const int col8 = (int)(i % per_row);
-    *reinterpret_cast<uint4*>(d_proj5 + row * 5 * C + 4 * C + col8 * 8) = make_uint4(l[0], l[1], l[2], l[3]);
+    *reinterpret_cast<uint4*>(d_proj5 + (int64_t)row * 5 * C + 4 * C + col8 * 8) = make_uint4(l[0], l[1], l[2], l[3]);
   }
 }
 
@@ -702,7 +715,8 @@ __global__ void __launch_bounds__(256) trimul_ln_bwd_kernel(const bf16* __restri
                                                             const float* __restrict__ gamma,
                                                             const float* __restrict__ mean,
                                                             const float* __restrict__ rstd, bf16* __restrict__ d_z,
-                                                            float* __restrict__ partials, int64_t R,
+                                                            float* __restrict__ partials, const PairRows rows,
+                                                            const bf16* __restrict__ d_res, int64_t R,
                                                             int rows_per_block) {
   griddep_wait();
   using L = RowLanes<C>;
@@ -721,24 +735,26 @@ __global__ void __launch_bounds__(256) trimul_ln_bwd_kernel(const bf16* __restri
   for (int it0 = warp * L::RPW; it0 < rows_per_block; it0 += G * 8 * L::RPW) {
     uint4 du[G], zu[G];
     float mu[G], rs[G];
+    int64_t src[G];  // the caller's row
     bool active[G];
 #pragma unroll
     for (int r = 0; r < G; ++r) {
       const int it = it0 + r * 8 * L::RPW;
       const int64_t row = row_begin + it + sub;
       active[r] = on && it + sub < rows_per_block && row < R;
+      src[r] = active[r] ? rows.locate((uint32_t)row).src : -1;
+      active[r] = src[r] >= 0;
       du[r] = zu[r] = make_uint4(0u, 0u, 0u, 0u);
       mu[r] = rs[r] = 0.f;
       if (active[r]) {
         du[r] = *reinterpret_cast<const uint4*>(d_zln + row * C + part * 8);
-        zu[r] = *reinterpret_cast<const uint4*>(z + row * C + part * 8);
+        zu[r] = *reinterpret_cast<const uint4*>(z + src[r] * C + part * 8);
         mu[r] = mean[row];
         rs[r] = rstd[row];
       }
     }
 #pragma unroll
     for (int r = 0; r < G; ++r) {
-      const int64_t row = row_begin + it0 + r * 8 * L::RPW + sub;
       float d[8], xh[8];
       unpack8(du[r], d);
       unpack8(zu[r], xh);
@@ -753,11 +769,17 @@ __global__ void __launch_bounds__(256) trimul_ln_bwd_kernel(const bf16* __restri
       const float m1 = slot_sum<C>(a1) * (1.f / C);
       const float m2 = slot_sum<C>(a2) * (1.f / C);
       if (active[r]) {
+        // the gradient that reaches z past the update (residual connection) is added here
+        uint4 ru = make_uint4(0u, 0u, 0u, 0u);
+        if (d_res != nullptr) ru = *reinterpret_cast<const uint4*>(d_res + src[r] * C + part * 8);
+        float res[8];
+        unpack8(ru, res);
         uint32_t o[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          o[e] = pack_bf16x2(rs[r] * (gd[2 * e] - m1 - xh[2 * e] * m2), rs[r] * (gd[2 * e + 1] - m1 - xh[2 * e + 1] * m2));
-        *reinterpret_cast<uint4*>(d_z + row * C + part * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+          o[e] = pack_bf16x2(res[2 * e] + rs[r] * (gd[2 * e] - m1 - xh[2 * e] * m2),
+                             res[2 * e + 1] + rs[r] * (gd[2 * e + 1] - m1 - xh[2 * e + 1] * m2));
+        *reinterpret_cast<uint4*>(d_z + src[r] * C + part * 8) = make_uint4(o[0], o[1], o[2], o[3]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           ag[e] += d[e] * xh[e];
@@ -790,92 +812,74 @@ __global__ void __launch_bounds__(256) trimul_ln_bwd_kernel(const bf16* __restri
   }
 }
 
-// out[j] = fixed-order sum over blocks of partials[blk][j], j < width.  One CTA per 32 columns;
-// warp w adds blocks w, w+32, ... in ascending order, then the 32 warp sums are added in warp order.
-__global__ void __launch_bounds__(1024) trimul_colsum_fold_kernel(const float* __restrict__ partials, int n_blocks,
-                                                                 int width, float* __restrict__ out_a,
-                                                                 float* __restrict__ out_b, int half) {
-  griddep_wait();
-  __shared__ float red[32][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = blockIdx.x * 32 + lane;
-  float s = 0.f;
-  if (j < width) {
-#pragma unroll 4
-    for (int b = warp; b < n_blocks; b += 32) s = __fadd_rn(s, partials[(int64_t)b * width + j]);
-  }
-  red[warp][lane] = s;
-  __syncthreads();
-  if (warp == 0 && j < width) {
-    float t = red[0][lane];
-#pragma unroll
-    for (int w = 1; w < 32; ++w) t = __fadd_rn(t, red[w][lane]);
-    if (j < half) out_a[j] = t;
-    else out_b[j - half] = t;
-  }
-}
-
-// Weight-gradient fold: out_row_block[r][c] = sum over splits (ascending) of part[s][m][c].
-// Rows are routed in blocks of C rows to up to five destinations (W5 = [a_p; a_g; b_p; b_g; g]).
-struct WgradDst {
+// Every fixed-order fold of the backward in one launch: the split-K weight-gradient partials and the per-CTA sums
+// of the two LayerNorm backward kernels.  Each job is tiny (latency bound: a few dependent batches of loads), so what
+// they cost is launches; six of them, folded one after the other, took longer than the sums.
+//   weight gradients: out[r][c] = sum over splits of part[s][m][c], rows routed in blocks of C to up to five
+//                     destinations (W5 = [a_p; a_g; b_p; b_g; g]);
+//   norm gradients:   out[j] = sum over CTAs of partials[blk][j], j < 2C, the halves going to d_gamma and d_beta.
+// A CTA owns 32 output elements; warp g adds its contiguous range of terms in ascending order (a batch of 8 loads is in
+// flight before the first add), then the 8 range sums are added in range order: a fixed summation tree, no atomics.
+struct FoldJob {
+  const float* part;
+  int terms, width;   // width: distance between consecutive terms = number of outputs
+  int C;              // elements per destination row block: C * C (weights) or C (norms)
   float* dst[5];
 };
-__global__ void __launch_bounds__(256) trimul_wgrad_fold_kernel(const float* __restrict__ part, int n_splits, int M,
-                                                                int C, WgradDst d) {
+struct FoldJobs {
+  FoldJob job[4];
+  int first[5];  // first CTA of each job; first[n_jobs] = grid
+  int n_jobs;
+};
+__global__ void __launch_bounds__(256) trimul_fold_kernel(const __grid_constant__ FoldJobs jobs) {
   griddep_wait();
-  // 32 output elements per CTA, 8 warps.  Warp g adds its contiguous range of splits in ascending
-  // order (the loads of a batch of 8 splits are independent, so all are in flight before the first
-  // add), then the 8 range sums are added in range order: a fixed summation tree, no atomics.
   __shared__ float red[8][32];
+  int n = 0;
+  while (n + 1 < jobs.n_jobs && (int)blockIdx.x >= jobs.first[n + 1]) ++n;
+  const FoldJob& jb = jobs.job[n];
   const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i = blockIdx.x * 32 + lane;
-  const int per = (n_splits + 7) / 8;
-  const int k0 = g * per, k1 = min(n_splits, k0 + per);
-  const int64_t stride = (int64_t)M * C;
+  const int i = (blockIdx.x - jobs.first[n]) * 32 + lane;
+  const int per = (jb.terms + 7) / 8;
+  const int k0 = g * per, k1 = min(jb.terms, k0 + per);
   float s = 0.f;
-  if (i < M * C) {
-    const float* src = part + i;
+  if (i < jb.width) {
+    const float* src = jb.part + i;
     int k = k0;
     for (; k + 8 <= k1; k += 8) {
       float v[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = src[(int64_t)(k + u) * stride];
+      for (int u = 0; u < 8; ++u) v[u] = src[(int64_t)(k + u) * jb.width];
 #pragma unroll
       for (int u = 0; u < 8; ++u) s = __fadd_rn(s, v[u]);
     }
-    for (; k < k1; ++k) s = __fadd_rn(s, src[(int64_t)k * stride]);
+    for (; k < k1; ++k) s = __fadd_rn(s, src[(int64_t)k * jb.width]);
   }
   red[g][lane] = s;
   __syncthreads();
-  if (g == 0 && i < M * C) {
+  if (g == 0 && i < jb.width) {
     float t = red[0][lane];
 #pragma unroll
     for (int w = 1; w < 8; ++w) t = __fadd_rn(t, red[w][lane]);
-    const int row = i / C, col = i % C;
-    d.dst[row / C][(row % C) * C + col] = t;
+    const int d = i / jb.C;
+    jb.dst[d][i - d * jb.C] = t;
   }
 }
 
-// First level of the LayerNorm-gradient fold: out[s][j] = fixed-order sum of in[s*256 .. s*256+255][j].
-__global__ void __launch_bounds__(1024) trimul_colsum_stage_kernel(const float* __restrict__ in, int n_in, int width,
-                                                                   float* __restrict__ out) {
-  griddep_wait();
-  __shared__ float red[32][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = blockIdx.x * 32 + lane;
-  const int b0 = blockIdx.y * 256, b1 = min(n_in, b0 + 256);
-  float s = 0.f;
-  if (j < width)
-    for (int b = b0 + warp; b < b1; b += 32) s = __fadd_rn(s, in[(int64_t)b * width + j]);
-  red[warp][lane] = s;
-  __syncthreads();
-  if (warp == 0 && j < width) {
-    float t = red[0][lane];
-#pragma unroll
-    for (int w = 1; w < 32; ++w) t = __fadd_rn(t, red[w][lane]);
-    out[(int64_t)blockIdx.y * width + j] = t;
+struct FoldList {
+  FoldJobs j = {};
+  void add(const float* part, int terms, int width, int C, float* d0, float* d1 = nullptr, float* d2 = nullptr,
+           float* d3 = nullptr, float* d4 = nullptr) {
+    j.job[j.n_jobs] = FoldJob{part, terms, width, C, {d0, d1, d2, d3, d4}};
+    j.first[j.n_jobs + 1] = j.first[j.n_jobs] + (width + 31) / 32;
+    ++j.n_jobs;
   }
-}
+  int launch(cudaStream_t stream) {
+    if (j.n_jobs == 0) return TPF_OK;
+    launch_kernel(trimul_fold_kernel, dim3(j.first[j.n_jobs]), dim3(256), 0, stream, j);
+    TPF_LAUNCH_OK();
+    return TPF_OK;
+  }
+};
 
 // =============================================================================================
 // host orchestration
@@ -885,15 +889,14 @@ struct TrimulPacked {
 };
 static int64_t packed_weight_elems(int64_t C) { return 12 * C * C; }
 
-static int pack_weights(const float* p_in, const float* g_in, const float* p_out, const float* g_out, void* buf,
-                        int C, TrimulPacked* pk, cudaStream_t stream) {
+static TrimulPacked packed_at(void* buf, int64_t C) {
   bf16* base = reinterpret_cast<bf16*>(buf);
-  pk->W5 = base;
-  pk->W5T = base + 5 * C * C;
-  pk->Wz = base + 10 * C * C;
-  pk->WzT = base + 11 * C * C;
-  launch_kernel(trimul_pack_weights_kernel, dim3((5 * C * C + 255) / 256), dim3(256), 0, stream, p_in, g_in, p_out, g_out, pk->W5, pk->W5T,
-                                                                          pk->Wz, pk->WzT, C);
+  return TrimulPacked{base, base + 5 * C * C, base + 10 * C * C, base + 11 * C * C};
+}
+static int pack_weights(const float* p_in, const float* g_in, const float* p_out, const float* g_out,
+                        const TrimulPacked& pk, int C, cudaStream_t stream) {
+  launch_kernel(trimul_pack_weights_kernel, dim3((5 * C * C + 255) / 256), dim3(256), 0, stream, p_in, g_in, p_out,
+                g_out, pk.W5, pk.W5T, pk.Wz, pk.WzT, C);
   TPF_LAUNCH_OK();
   return TPF_OK;
 }
@@ -912,26 +915,29 @@ static int proj_gemm(const bf16* zln, const bf16* W5, int64_t R, int n_cols, con
 }
 
 template <int C>
-static int trimul_fwd_t(const bf16* z, const float* mask, const TrimulPacked& pk, const float* gin, const float* bin,
-                        const float* gout, const float* bout, int incoming, int64_t B, int64_t N, int64_t NN,
-                        int stages, bf16* out, bf16* zln, float* mean_in, float* rstd_in, bf16* a_cm, bf16* b_cm,
-                        bf16* gate, bf16* x_cm, bf16* xln, float* mean_out, float* rstd_out, int* status,
-                        cudaStream_t stream) {
-  // NN = pair rows per batch entry (N*N for a whole pair tensor, N_local*N for a row shard)
-  const int64_t R = B * NN;
+static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPacked& pk, int64_t NN, int stages,
+                        int* status, cudaStream_t stream) {
+  // t.Np: internal extent (a multiple of 8); NN: internal rows per batch entry (Np * Np for a whole pair tensor,
+  // N_local * N for a row shard).
+  const int64_t B = t.B, N = t.Np, R = B * NN;
   using L = RowLanes<C>;
+  const bf16* z = (const bf16*)t.z;
+  bf16 *zln = (bf16*)t.zln, *xln = (bf16*)t.xln, *x_cm = (bf16*)t.x_cm;
+  const PairRows rows = PairRows::make(t.N, t.Np, false);
   int rc = TPF_OK;
   if (stages & 1) {
     const int64_t warps = (R + 4 * L::RPW - 1) / (4 * L::RPW);
     const int64_t blocks = (warps + 7) / 8;
-    launch_kernel(trimul_ln_fwd_kernel<C>, dim3((unsigned)blocks), dim3(256), 0, stream, z, gin, bin, zln, mean_in, rstd_in, R);
+    const PairMask pm{t.mask, t.mask_type, t.mask_stride[0], t.mask_stride[1], t.mask_stride[2]};
+    launch_kernel(trimul_ln_fwd_kernel<C>, dim3((unsigned)blocks), dim3(256), 0, stream, z, t.w.norm_in_w,
+                  t.w.norm_in_b, zln, t.mean_in, t.rstd_in, rows, pm, mask == t.mask_grid ? t.mask_grid : nullptr, R);
     TPF_LAUNCH_OK();
-    EpiProjGate::Params ep{a_cm, b_cm, gate, mask, C, NN};
+    EpiProjGate::Params ep{(bf16*)t.a_cm, (bf16*)t.b_cm, (bf16*)t.gate, mask, C, NN};
     if ((rc = proj_gemm<C, EpiProjGate>(zln, pk.W5, R, 5 * C, ep, status, stream))) return rc;
   }
   if (stages & 2) {
     // k-contraction: batch = B*C problems of N x N x N
-    rc = bmm_bf16(a_cm, N, NN, incoming, b_cm, N, NN, incoming, x_cm, N, NN, 0, N, N, N, B * C, 0, 128, stream);
+    rc = bmm_bf16(t.a_cm, N, NN, t.incoming, t.b_cm, N, NN, t.incoming, x_cm, N, NN, 0, N, N, N, B * C, 0, 128, stream);
     if (rc) return rc;
   }
   if (stages & 4) {
@@ -943,12 +949,13 @@ static int trimul_fwd_t(const bf16* z, const float* mask, const TrimulPacked& pk
       constexpr int smem = 2 * C * (64 * 2 + 16) + 64 * (C * 2 + 16);
       static PerDeviceOnce once;  // per instantiation
       if ((rc = ensure_dynamic_smem(kern, smem, once))) return rc;
-      launch_kernel(kern, dim3(grid), dim3(256), smem, stream, x_cm, gout, bout, xln, mean_out, rstd_out, NN, tiles, (int)(B * tiles));
+      launch_kernel(kern, dim3(grid), dim3(256), smem, stream, x_cm, t.w.norm_out_w, t.w.norm_out_b, xln, t.mean_out,
+                    t.rstd_out, NN, tiles, (int)(B * tiles));
     }
     TPF_LAUNCH_OK();
     using Cfg = GemmCfg<128, C, 128, false, 128, false, 4>;
     GemmShape sh{(int)R, C, C, 1, 0};
-    EpiOutGate::Params ep{out, gate, C};
+    EpiOutGate::Params ep{(bf16*)t.out, (bf16*)t.sum, z, (const bf16*)t.gate, rows, C};
     if ((rc = launch_gemm<Cfg, EpiOutGate>(xln, C, 0, pk.Wz, C, 0, sh, ep, status, stream))) return rc;
   }
   return TPF_OK;
@@ -965,7 +972,7 @@ static void split_plan(int64_t R, int tiles_mn, int* n_splits, int64_t* k_per_sp
 
 struct TrimulBwdWorkspace {
   bf16 *wpack, *d_y, *d_proj5, *d_xln, *dx_cm, *da_cm, *db_cm;  // d_zln aliases d_xln
-  float *part_w5, *part_wz, *part_ln_out, *part_ln_in, *part_lvl2;
+  float *part_w5, *part_wz, *part_ln_out, *part_ln_in;
   int splits_w5, splits_wz, blocks_ln_out, blocks_ln_in, rows_per_block_in;
   int64_t kps_w5, kps_wz;
   int64_t total_bytes;
@@ -997,42 +1004,40 @@ static void plan_bwd_workspace(int64_t B, int64_t NN, int64_t C, char* base, Tri
     const int64_t tiles = B * ((NN + 63) / 64);
     w->blocks_ln_out = (int)(tiles < 2 * sm_count() ? tiles : 2 * sm_count());
   }
-  w->rows_per_block_in = 128;
-  w->blocks_ln_in = (int)((R + 127) / 128);
+  // input-norm backward: at most 8 CTAs per SM, so that few partial rows are left to fold
+  w->rows_per_block_in = (int)(((R + 8 * sm_count() - 1) / (8 * sm_count()) + 127) / 128 * 128);
+  w->blocks_ln_in = (int)((R + w->rows_per_block_in - 1) / w->rows_per_block_in);
   w->part_ln_out = reinterpret_cast<float*>(take((int64_t)w->blocks_ln_out * 2 * C * 4));
   w->part_ln_in = reinterpret_cast<float*>(take((int64_t)w->blocks_ln_in * 2 * C * 4));
-  {
-    const int64_t most = w->blocks_ln_out > w->blocks_ln_in ? w->blocks_ln_out : w->blocks_ln_in;
-    w->part_lvl2 = reinterpret_cast<float*>(take(((most + 255) / 256) * 2 * C * 4));
-  }
   w->total_bytes = off;
 }
 
 template <int C>
-static int trimul_bwd_t(const bf16* d_out, const bf16* z, const float* mask, const float* p_in, const float* g_in,
-                        const float* p_out, const float* g_out, const float* gin, const float* gout, int incoming,
-                        int64_t B, int64_t N, int64_t NN, int stages, bf16* dx_io, bf16* da_io, bf16* db_io,
-                        const bf16* out, const bf16* zln, const float* mean_in,
-                        const float* rstd_in, const bf16* a_cm, const bf16* b_cm, const bf16* gate, const bf16* x_cm,
-                        const bf16* xln, const float* mean_out, const float* rstd_out, bf16* d_z, float* d_p_in,
-                        float* d_g_in, float* d_p_out, float* d_g_out, float* d_gin, float* d_bin, float* d_gout,
-                        float* d_bout, char* workspace, int* status, cudaStream_t stream) {
-  const int64_t R = B * NN;
+static int trimul_bwd_t(const TrimulCall& t, const TrimulGrads& g, const float* mask, const TrimulPacked* packed,
+                        int64_t NN, int stages, bf16* dx_io, bf16* da_io, bf16* db_io, char* workspace, int* status,
+                        cudaStream_t stream) {
+  const int64_t B = t.B, N = t.Np, R = B * NN;
+  const bf16 *z = (const bf16*)t.z, *zln = (const bf16*)t.zln, *xln = (const bf16*)t.xln, *a_cm = (const bf16*)t.a_cm,
+             *b_cm = (const bf16*)t.b_cm, *d_out = (const bf16*)g.d_out;
+  const PairRows rows = PairRows::make(t.N, t.Np, false);
   TrimulBwdWorkspace w;
   plan_bwd_workspace(B, NN, C, workspace, &w);
   if (dx_io) w.dx_cm = dx_io;  // staged (sharded) use: the caller moves these between ranks
   if (da_io) w.da_cm = da_io;
   if (db_io) w.db_cm = db_io;
-  TrimulPacked pk;
+  TrimulPacked pk = packed ? *packed : packed_at(w.wpack, C);
   int rc;
-  if ((rc = pack_weights(p_in, g_in, p_out, g_out, w.wpack, C, &pk, stream))) return rc;
+  if (!packed && (rc = pack_weights(t.w.p_in, t.w.g_in, t.w.p_out, t.w.g_out, pk, C, stream))) return rc;
+  FoldList folds;
 
   if (stages & 1) {
   // 1. output gate: d_y, d_glogit
   {
+    TPF_REQUIRE(R * C / 8 < (1ll << 31), TPF_ERR_INVALID_ARGUMENT, "trimul_bwd: extent too large");
     int blocks = (int)((R * C / 8 + 255) / 256);
     if (blocks > 16 * sm_count()) blocks = 16 * sm_count();
-    launch_kernel(trimul_out_gate_bwd_kernel, dim3(blocks), dim3(256), 0, stream, d_out, out, gate, w.d_y, w.d_proj5, R, C);
+    launch_kernel(trimul_out_gate_bwd_kernel, dim3(blocks), dim3(256), 0, stream, d_out, (const bf16*)t.out,
+                  (const bf16*)t.gate, w.d_y, w.d_proj5, rows, FastDiv::make(C / 8), R, C);
     TPF_LAUNCH_OK();
   }
   // 2. d_xln = d_y Wz ; d_wz = d_y^T xln
@@ -1046,37 +1051,23 @@ static int trimul_bwd_t(const bf16* d_out, const bf16* z, const float* mask, con
   rc = bmm_bf16(w.d_y, C, 0, 1, xln, C, 0, 1, w.part_wz, C, (int64_t)C * C, 1, C, C, R, w.splits_wz, w.kps_wz, 128,
                 stream);
   if (rc) return rc;
-  {
-    WgradDst d;
-    for (int i = 0; i < 5; ++i) d.dst[i] = d_p_out;
-    launch_kernel(trimul_wgrad_fold_kernel, dim3((C * C + 31) / 32), dim3(256), 0, stream, w.part_wz, w.splits_wz, C, C, d);
-    TPF_LAUNCH_OK();
-  }
+  folds.add(w.part_wz, w.splits_wz, C * C, C * C, g.p_out);
   // 3. output norm backward -> d_x (channel-major), d_gamma_out, d_beta_out
   {
     const int tiles = (int)((NN + 63) / 64);
-    {
-      auto kern = trimul_xnorm_bwd_kernel<C>;
-      constexpr int smem = 2 * C * (64 * 2 + 16) + 2 * 64 * (C * 2 + 16);
-      static PerDeviceOnce once;  // per instantiation
-      if ((rc = ensure_dynamic_smem(kern, smem, once))) return rc;
-      launch_kernel(kern, dim3(w.blocks_ln_out), dim3(256), smem, stream, w.d_xln, x_cm, gout, mean_out, rstd_out, w.dx_cm, w.part_ln_out, NN,
-                                                  tiles, (int)(B * tiles));
-    }
+    auto kern = trimul_xnorm_bwd_kernel<C>;
+    constexpr int smem = 2 * C * (64 * 2 + 16) + 2 * 64 * (C * 2 + 16);
+    static PerDeviceOnce once;  // per instantiation
+    if ((rc = ensure_dynamic_smem(kern, smem, once))) return rc;
+    launch_kernel(kern, dim3(w.blocks_ln_out), dim3(256), smem, stream, w.d_xln, (const bf16*)t.x_cm, t.w.norm_out_w,
+                  t.mean_out, t.rstd_out, w.dx_cm, w.part_ln_out, NN, tiles, (int)(B * tiles));
     TPF_LAUNCH_OK();
-    {
-      const int lvl = (w.blocks_ln_out + 255) / 256;
-      launch_kernel(trimul_colsum_stage_kernel, dim3(dim3((2 * C + 31) / 32, lvl)), dim3(1024), 0, stream, w.part_ln_out, w.blocks_ln_out,
-                                                                                    2 * C, w.part_lvl2);
-      TPF_LAUNCH_OK();
-      launch_kernel(trimul_colsum_fold_kernel, dim3((2 * C + 31) / 32), dim3(1024), 0, stream, w.part_lvl2, lvl, 2 * C, d_gout, d_bout, C);
-      TPF_LAUNCH_OK();
-    }
+    folds.add(w.part_ln_out, w.blocks_ln_out, 2 * C, C, g.norm_out_w, g.norm_out_b);
   }
   }
   if (stages & 2) {
   // 4. contraction backward
-  if (!incoming) {
+  if (!t.incoming) {
     // d_a[c,i,k] = sum_j d_x[c,i,j] b[c,j,k] ; d_b[c,j,k] = sum_i d_x[c,i,j] a[c,i,k]
     if ((rc = bmm_bf16(w.dx_cm, N, NN, 0, b_cm, N, NN, 1, w.da_cm, N, NN, 0, N, N, N, B * C, 0, 128, stream))) return rc;
     if ((rc = bmm_bf16(w.dx_cm, N, NN, 1, a_cm, N, NN, 1, w.db_cm, N, NN, 0, N, N, N, B * C, 0, 128, stream))) return rc;
@@ -1105,32 +1096,14 @@ static int trimul_bwd_t(const bf16* d_out, const bf16* z, const float* mask, con
   rc = bmm_bf16(w.d_proj5, 5 * C, 0, 1, zln, C, 0, 1, w.part_w5, C, (int64_t)5 * C * C, 1, 5 * C, C, R, w.splits_w5,
                 w.kps_w5, 128, stream);
   if (rc) return rc;
-  {
-    WgradDst d;
-    d.dst[0] = d_p_in;              // a_p
-    d.dst[1] = d_g_in;              // a_g
-    d.dst[2] = d_p_in + C * C;      // b_p
-    d.dst[3] = d_g_in + C * C;      // b_g
-    d.dst[4] = d_g_out;             // g
-    launch_kernel(trimul_wgrad_fold_kernel, dim3((5 * C * C + 31) / 32), dim3(256), 0, stream, w.part_w5, w.splits_w5, 5 * C, C, d);
-    TPF_LAUNCH_OK();
-  }
+  folds.add(w.part_w5, w.splits_w5, 5 * C * C, C * C, g.p_in, g.g_in, g.p_in + C * C, g.g_in + C * C, g.g_out);
   // 7. input norm backward
-  {
-    launch_kernel(trimul_ln_bwd_kernel<C>, dim3(w.blocks_ln_in), dim3(256), 0, stream, d_zln, z, gin, mean_in, rstd_in, d_z, w.part_ln_in, R,
-                                                                w.rows_per_block_in);
-    TPF_LAUNCH_OK();
-    {
-      const int lvl = (w.blocks_ln_in + 255) / 256;
-      launch_kernel(trimul_colsum_stage_kernel, dim3(dim3((2 * C + 31) / 32, lvl)), dim3(1024), 0, stream, w.part_ln_in, w.blocks_ln_in,
-                                                                                    2 * C, w.part_lvl2);
-      TPF_LAUNCH_OK();
-      launch_kernel(trimul_colsum_fold_kernel, dim3((2 * C + 31) / 32), dim3(1024), 0, stream, w.part_lvl2, lvl, 2 * C, d_gin, d_bin, C);
-      TPF_LAUNCH_OK();
-    }
+  launch_kernel(trimul_ln_bwd_kernel<C>, dim3(w.blocks_ln_in), dim3(256), 0, stream, d_zln, z, t.w.norm_in_w,
+                t.mean_in, t.rstd_in, (bf16*)g.d_z, w.part_ln_in, rows, (const bf16*)g.d_res, R, w.rows_per_block_in);
+  TPF_LAUNCH_OK();
+  folds.add(w.part_ln_in, w.blocks_ln_in, 2 * C, C, g.norm_in_w, g.norm_in_b);
   }
-  }
-  return TPF_OK;
+  return folds.launch(stream);
 }
 
 static int check_trimul_rows(const char* who, int64_t N, int64_t NN, int stages) {
@@ -1160,6 +1133,65 @@ int64_t trimul_bwd_workspace_bytes(int64_t B, int64_t NN, int64_t C) {
   return w.total_bytes;
 }
 
+static int trimul_status(int** status) {
+  static PerDeviceAddress cache;
+  return device_symbol_address(g_trimul_status, cache, reinterpret_cast<void**>(status));
+}
+
+// The kernels' mask: the caller's own when it has the internal layout, else the copy the input norm writes.
+static const float* grid_mask(const TrimulCall& t) {
+  return t.mask_grid ? t.mask_grid : reinterpret_cast<const float*>(t.mask);
+}
+
+static int trimul_fwd_run(const TrimulCall& t, int64_t NN, int stages, bool with_pack, cudaStream_t stream) {
+  int* status = nullptr;
+  int rc = trimul_status(&status);
+  if (rc) return rc;
+  const TrimulPacked pk = packed_at(t.packed, t.C);
+  if (with_pack && (rc = pack_weights(t.w.p_in, t.w.g_in, t.w.p_out, t.w.g_out, pk, (int)t.C, stream))) return rc;
+  switch (t.C) {
+    case 32: return trimul_fwd_t<32>(t, grid_mask(t), pk, NN, stages, status, stream);
+    case 64: return trimul_fwd_t<64>(t, grid_mask(t), pk, NN, stages, status, stream);
+    case 96: return trimul_fwd_t<96>(t, grid_mask(t), pk, NN, stages, status, stream);
+    case 128: return trimul_fwd_t<128>(t, grid_mask(t), pk, NN, stages, status, stream);
+  }
+  return fail(TPF_ERR_UNSUPPORTED, "trimul_fwd: unsupported C");
+}
+
+static int trimul_bwd_run(const TrimulCall& t, const TrimulGrads& g, int64_t NN, int stages, void* dx_io, void* da_io,
+                          void* db_io, void* workspace, cudaStream_t stream) {
+  int* status = nullptr;
+  int rc = trimul_status(&status);
+  if (rc) return rc;
+  TrimulPacked pk = packed_at(t.packed, t.C);
+  const TrimulPacked* packed = t.packed ? &pk : nullptr;
+  bf16 *dx = (bf16*)dx_io, *da = (bf16*)da_io, *db = (bf16*)db_io;
+  char* ws = (char*)workspace;
+  switch (t.C) {
+    case 32: return trimul_bwd_t<32>(t, g, grid_mask(t), packed, NN, stages, dx, da, db, ws, status, stream);
+    case 64: return trimul_bwd_t<64>(t, g, grid_mask(t), packed, NN, stages, dx, da, db, ws, status, stream);
+    case 96: return trimul_bwd_t<96>(t, g, grid_mask(t), packed, NN, stages, dx, da, db, ws, status, stream);
+    case 128: return trimul_bwd_t<128>(t, g, grid_mask(t), packed, NN, stages, dx, da, db, ws, status, stream);
+  }
+  return fail(TPF_ERR_UNSUPPORTED, "trimul_bwd: unsupported C");
+}
+
+int trimul_forward(const TrimulCall& t, cudaStream_t stream) {
+  int rc = check_trimul_shape("trimul_fwd", t.B, t.Np, t.C);
+  if (rc) return rc;
+  return trimul_fwd_run(t, t.Np * t.Np, 7, true, stream);
+}
+
+int trimul_backward(const TrimulCall& t, const TrimulGrads& g, void* workspace, int64_t workspace_bytes,
+                    cudaStream_t stream) {
+  int rc = check_trimul_shape("trimul_bwd", t.B, t.Np, t.C);
+  if (rc) return rc;
+  TPF_REQUIRE(workspace && workspace_bytes >= trimul_bwd_workspace_bytes(t.B, t.Np * t.Np, t.C) &&
+                  (reinterpret_cast<uintptr_t>(workspace) & 255) == 0,
+              TPF_ERR_WORKSPACE, "trimul_bwd: workspace too small or misaligned");
+  return trimul_bwd_run(t, g, t.Np * t.Np, 7, nullptr, nullptr, nullptr, workspace, stream);
+}
+
 int trimul_fwd(const void* z, const float* mask, const float* p_in, const float* g_in, const float* p_out,
                const float* g_out, const float* gin, const float* bin, const float* gout, const float* bout,
                int incoming, int64_t B, int64_t N, int64_t C, void* out, void* zln, float* mean_in, float* rstd_in,
@@ -1174,24 +1206,14 @@ int trimul_fwd(const void* z, const float* mask, const float* p_in, const float*
               TPF_ERR_INVALID_ARGUMENT, "trimul_fwd: null pointer");
   TPF_REQUIRE(workspace && workspace_bytes >= trimul_fwd_workspace_bytes(B, N, C), TPF_ERR_WORKSPACE,
               "trimul_fwd: workspace of %lld bytes required", (long long)trimul_fwd_workspace_bytes(B, N, C));
-  int* status = nullptr;
-  {
-    static PerDeviceAddress cache;
-    if ((rc = device_symbol_address(g_trimul_status, cache, reinterpret_cast<void**>(&status)))) return rc;
-  }
-  TrimulPacked pk;
-  if ((rc = pack_weights(p_in, g_in, p_out, g_out, workspace, (int)C, &pk, stream))) return rc;
-#define TPF_TRIMUL_FWD(CC)                                                                                         \
-  if (C == CC)                                                                                                     \
-    return trimul_fwd_t<CC>((const bf16*)z, mask, pk, gin, bin, gout, bout, incoming, B, N, NN, stages, (bf16*)out, (bf16*)zln, \
-                            mean_in, rstd_in, (bf16*)a_cm, (bf16*)b_cm, (bf16*)gate, (bf16*)x_cm, (bf16*)xln,       \
-                            mean_out, rstd_out, status, stream);
-  TPF_TRIMUL_FWD(32)
-  TPF_TRIMUL_FWD(64)
-  TPF_TRIMUL_FWD(96)
-  TPF_TRIMUL_FWD(128)
-#undef TPF_TRIMUL_FWD
-  return fail(TPF_ERR_UNSUPPORTED, "trimul_fwd: unsupported C");
+  TrimulCall t = {};
+  t.B = B; t.N = N; t.Np = N; t.C = C; t.incoming = incoming;
+  t.z = z; t.mask = mask;
+  t.w = {p_in, g_in, p_out, g_out, gin, bin, gout, bout};
+  t.packed = workspace;
+  t.out = out; t.zln = zln; t.mean_in = mean_in; t.rstd_in = rstd_in; t.a_cm = a_cm; t.b_cm = b_cm; t.gate = gate;
+  t.x_cm = x_cm; t.xln = xln; t.mean_out = mean_out; t.rstd_out = rstd_out;
+  return trimul_fwd_run(t, NN, stages, true, stream);
 }
 
 int trimul_bwd(const void* d_out, const void* z, const float* mask, const float* p_in, const float* g_in,
@@ -1214,25 +1236,17 @@ int trimul_bwd(const void* d_out, const void* z, const float* mask, const float*
                   (reinterpret_cast<uintptr_t>(workspace) & 255) == 0,
               TPF_ERR_WORKSPACE, "trimul_bwd: 256-byte aligned workspace of %lld bytes required",
               (long long)trimul_bwd_workspace_bytes(B, NN, C));
-  int* status = nullptr;
-  {
-    static PerDeviceAddress cache;
-    if ((rc = device_symbol_address(g_trimul_status, cache, reinterpret_cast<void**>(&status)))) return rc;
-  }
-#define TPF_TRIMUL_BWD(CC)                                                                                            \
-  if (C == CC)                                                                                                        \
-    return trimul_bwd_t<CC>((const bf16*)d_out, (const bf16*)z, mask, p_in, g_in, p_out, g_out, gin, gout, incoming,  \
-                            B, N, NN, stages, (bf16*)dx_io, (bf16*)da_io, (bf16*)db_io, (const bf16*)out, (const bf16*)zln, mean_in, rstd_in, (const bf16*)a_cm,            \
-                            (const bf16*)b_cm, (const bf16*)gate, (const bf16*)x_cm, (const bf16*)xln, mean_out,      \
-                            rstd_out, (bf16*)d_z, d_p_in, d_g_in, d_p_out, d_g_out, d_gin, d_bin, d_gout, d_bout,     \
-                            (char*)workspace, status, stream);
-  TPF_TRIMUL_BWD(32)
-  TPF_TRIMUL_BWD(64)
-  TPF_TRIMUL_BWD(96)
-  TPF_TRIMUL_BWD(128)
-#undef TPF_TRIMUL_BWD
-  return fail(TPF_ERR_UNSUPPORTED, "trimul_bwd: unsupported C");
+  TrimulCall t = {};
+  t.B = B; t.N = N; t.Np = N; t.C = C; t.incoming = incoming;
+  t.z = z; t.mask = mask;
+  t.w = {p_in, g_in, p_out, g_out, gin, nullptr, gout, nullptr};
+  t.out = const_cast<void*>(out); t.zln = const_cast<void*>(zln);
+  t.mean_in = const_cast<float*>(mean_in); t.rstd_in = const_cast<float*>(rstd_in);
+  t.a_cm = const_cast<void*>(a_cm); t.b_cm = const_cast<void*>(b_cm); t.gate = const_cast<void*>(gate);
+  t.x_cm = const_cast<void*>(x_cm); t.xln = const_cast<void*>(xln);
+  t.mean_out = const_cast<float*>(mean_out); t.rstd_out = const_cast<float*>(rstd_out);
+  const TrimulGrads g{d_out, nullptr, d_z, d_p_in, d_g_in, d_p_out, d_g_out, d_gin, d_bin, d_gout, d_bout};
+  return trimul_bwd_run(t, g, NN, stages, dx_io, da_io, db_io, workspace, stream);
 }
 
 }  // namespace tpf
-

@@ -29,6 +29,7 @@ Unsupported inputs raise ``ValueError("... unsupported [code]: reason")``.
 from __future__ import annotations
 
 import math
+import operator
 
 import torch
 
@@ -38,6 +39,10 @@ SUPPORTED_CHANNELS = (32, 64, 96, 128)
 _LN_EPS = 1e-5
 _WEIGHT_NAMES = ("norm_in_weight", "norm_in_bias", "p_in_weight", "g_in_weight",
                  "norm_out_weight", "norm_out_bias", "p_out_weight", "g_out_weight")
+_WEIGHT_SET = frozenset(_WEIGHT_NAMES)
+# the order of the custom ops and of `_native.trimul`
+_native_order = operator.itemgetter("p_in_weight", "g_in_weight", "p_out_weight", "g_out_weight", "norm_in_weight",
+                                    "norm_in_bias", "norm_out_weight", "norm_out_bias")
 
 
 class SupportResult(tuple):
@@ -101,34 +106,14 @@ def check_trimul_support(z, direction, mask, weights, *, check_device=True) -> S
 
 
 # --------------------------------------------------------------------------------------
-# custom ops
+# custom ops: what a traced graph (torch.compile, torch.export, fake tensors) holds.  An eager call on plain CUDA
+# tensors goes to `_native.trimul`, which does the same in one C++ call.
 # --------------------------------------------------------------------------------------
-def _f32c(t):
-    return t.detach().to(torch.float32).contiguous()
-
-
 @torch.library.custom_op("tpf_b200::trimul_fwd", mutates_args=())
 def _trimul_fwd(z: torch.Tensor, mask: torch.Tensor, p_in: torch.Tensor, g_in: torch.Tensor, p_out: torch.Tensor,
                 g_out: torch.Tensor, nin_w: torch.Tensor, nin_b: torch.Tensor, nout_w: torch.Tensor,
                 nout_b: torch.Tensor, incoming: bool) -> list[torch.Tensor]:
-    B, N, _, Cc = z.shape
-    R = B * N * N
-    dev = z.device
-    z = z.contiguous()
-    mask = mask.to(torch.float32).contiguous()
-    ws = [_f32c(t) for t in (p_in, g_in, p_out, g_out, nin_w, nin_b, nout_w, nout_b)]
-    bf = lambda *s: torch.empty(s, device=dev, dtype=torch.bfloat16)  # noqa: E731
-    f32 = lambda *s: torch.empty(s, device=dev, dtype=torch.float32)  # noqa: E731
-    out, zln, gate, xln = bf(B, N, N, Cc), bf(R, Cc), bf(R, Cc), bf(R, Cc)
-    a_cm, b_cm, x_cm = bf(B * Cc, N * N), bf(B * Cc, N * N), bf(B * Cc, N * N)
-    mean_in, rstd_in, mean_out, rstd_out = f32(R), f32(R), f32(R), f32(R)
-    nbytes = C.load().tpf_trimul_fwd_workspace_bytes(B, N, Cc)
-    wsb = torch.empty((max(nbytes, 256),), device=dev, dtype=torch.uint8)
-    with torch.cuda.device(dev):
-        C.call("tpf_trimul_fwd", C.ptr(z), C.ptr(mask), *[C.ptr(t) for t in ws], int(incoming), B, N, Cc,
-               C.ptr(out), C.ptr(zln), C.ptr(mean_in), C.ptr(rstd_in), C.ptr(a_cm), C.ptr(b_cm), C.ptr(gate),
-               C.ptr(x_cm), C.ptr(xln), C.ptr(mean_out), C.ptr(rstd_out), C.ptr(wsb), nbytes, C.current_stream())
-    return [out, zln, mean_in, rstd_in, a_cm, b_cm, gate, x_cm, xln, mean_out, rstd_out]
+    return C.native().trimul_fwd(z, mask, [p_in, g_in, p_out, g_out, nin_w, nin_b, nout_w, nout_b], incoming)
 
 
 @_trimul_fwd.register_fake
@@ -147,25 +132,8 @@ def _trimul_bwd(d_out: torch.Tensor, z: torch.Tensor, mask: torch.Tensor, p_in: 
                 out: torch.Tensor, zln: torch.Tensor, mean_in: torch.Tensor, rstd_in: torch.Tensor,
                 a_cm: torch.Tensor, b_cm: torch.Tensor, gate: torch.Tensor, x_cm: torch.Tensor, xln: torch.Tensor,
                 mean_out: torch.Tensor, rstd_out: torch.Tensor) -> list[torch.Tensor]:
-    B, N, _, Cc = z.shape
-    dev = z.device
-    d_out = d_out.to(torch.bfloat16).contiguous()
-    z = z.contiguous()
-    mask = mask.to(torch.float32).contiguous()
-    ws = [_f32c(t) for t in (p_in, g_in, p_out, g_out, nin_w, nout_w)]
-    f32 = lambda *s: torch.empty(s, device=dev, dtype=torch.float32)  # noqa: E731
-    d_z = torch.empty_like(z)
-    d_p_in, d_g_in, d_p_out, d_g_out = f32(2 * Cc, Cc), f32(2 * Cc, Cc), f32(Cc, Cc), f32(Cc, Cc)
-    d_nin_w, d_nin_b, d_nout_w, d_nout_b = f32(Cc), f32(Cc), f32(Cc), f32(Cc)
-    nbytes = C.load().tpf_trimul_bwd_workspace_bytes(B, N, Cc)
-    wsb = torch.empty((max(nbytes, 256),), device=dev, dtype=torch.uint8)
-    with torch.cuda.device(dev):
-        C.call("tpf_trimul_bwd", C.ptr(d_out), C.ptr(z), C.ptr(mask), *[C.ptr(t) for t in ws], int(incoming), B, N,
-               Cc, C.ptr(out), C.ptr(zln), C.ptr(mean_in), C.ptr(rstd_in), C.ptr(a_cm), C.ptr(b_cm), C.ptr(gate),
-               C.ptr(x_cm), C.ptr(xln), C.ptr(mean_out), C.ptr(rstd_out), C.ptr(d_z), C.ptr(d_p_in), C.ptr(d_g_in),
-               C.ptr(d_p_out), C.ptr(d_g_out), C.ptr(d_nin_w), C.ptr(d_nin_b), C.ptr(d_nout_w), C.ptr(d_nout_b),
-               C.ptr(wsb), nbytes, C.current_stream())
-    return [d_z, d_p_in, d_g_in, d_p_out, d_g_out, d_nin_w, d_nin_b, d_nout_w, d_nout_b]
+    return C.native().trimul_bwd(d_out, z, mask, [p_in, g_in, p_out, g_out, nin_w, nout_w], incoming,
+                                 [out, zln, mean_in, rstd_in, a_cm, b_cm, gate, x_cm, xln, mean_out, rstd_out])
 
 
 @_trimul_bwd.register_fake
@@ -246,6 +214,10 @@ def turbo_trimul(z, direction="outgoing", mask=None, *, generator=None, **weight
         mod_weights, direction = _weights_from_module(module)
         mod_weights.update(weights)
         weights = mod_weights
+    if not torch.compiler.is_compiling() and direction in ("outgoing", "incoming") and weights.keys() == _WEIGHT_SET:
+        out = C.native().trimul(z, direction == "incoming", mask, _native_order(weights))
+        if out is not None:
+            return out
     unknown = set(weights) - set(_WEIGHT_NAMES)
     if unknown:
         raise TypeError(f"turbo_trimul got unexpected keyword arguments {sorted(unknown)}")

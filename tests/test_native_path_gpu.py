@@ -1,0 +1,53 @@
+"""The eager C++ route of the operators: ragged lengths without padded copies, operand types and strides, and calls
+without gradients (which keep no intermediates) equal to calls with them."""
+import pytest
+import torch
+
+import openfold3_triangle_kernel_b200 as tk
+from oracle import attention_oracle as ao
+from oracle import trimul_oracle as to
+from oracle.inputs import attention_inputs, trimul_inputs
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a CUDA device")]
+
+
+@pytest.mark.parametrize("direction", ["outgoing", "incoming"])
+@pytest.mark.parametrize("N", [1, 7, 8, 9, 63, 65, 130])
+def test_trimul_any_length(N, direction):
+    t = trimul_inputs(2, N, 64, seed=N, mask_mode="trailing10")
+    d_out = torch.randn(2, N, N, 64, generator=torch.Generator().manual_seed(N)).bfloat16()
+    z = t["z"].cuda().requires_grad_(True)
+    w = {k: v.cuda().requires_grad_(True) for k, v in t["weights"].items()}
+    for mask in (t["mask"].cuda(), t["mask"].cuda().bool(), t["mask"].cuda().half().transpose(1, 2).contiguous().transpose(1, 2)):
+        out = tk.turbo_trimul(z, direction, mask, **w)
+        with torch.no_grad():
+            assert torch.equal(tk.turbo_trimul(z, direction, mask, **w), out)
+    out.backward(d_out.cuda())
+    ref = to.trimul_forward_backward(t["z"], direction, t["mask"], t["weights"], d_out)
+    assert ao.rel_l2(out.detach().cpu(), ref["out"]) <= 1e-2
+    assert ao.rel_l2(z.grad.cpu(), ref["dz"]) <= 2e-2
+    for k in ("p_in_weight", "g_out_weight", "norm_in_bias", "norm_out_weight"):
+        assert ao.rel_l2(w[k].grad.cpu(), ref["d_" + k]) <= 2.5e-2, k
+
+
+@pytest.mark.parametrize("N,D,bias_type,mask_type", [(3, 16, torch.float32, torch.float16), (37, 32, torch.bfloat16, torch.bfloat16),
+                                                     (66, 40, torch.float32, torch.float32), (64, 64, torch.bfloat16, torch.float32)])
+def test_attention_operand_types_and_strides(N, D, bias_type, mask_type):
+    a = attention_inputs(2, N, 2, N, D, seed=N, mask_mode="trailing15")
+    q, k, v = (a[n].cuda().requires_grad_(True) for n in ("q", "k", "v"))
+    base = a["pair_bias"].to(bias_type).cuda().permute(0, 1, 3, 4, 2).contiguous().requires_grad_(True)  # [B,1,N,N,H]
+    bias = base.permute(0, 1, 4, 2, 3)
+    mask = a["res_mask"].to(mask_type).cuda()
+    d_out = torch.randn(2, N, N, 2, D, generator=torch.Generator().manual_seed(N)).bfloat16()
+    out = tk.turbo_attention(q, k, v, pair_bias=bias, res_mask=mask)
+    with torch.no_grad():
+        assert torch.equal(tk.turbo_attention(q, k, v, pair_bias=bias, res_mask=mask), out)
+    out.backward(d_out.cuda())
+    ref = ao.attention_forward_backward(a["q"], a["k"], a["v"], a["pair_bias"], a["res_mask"], d_out)
+    for name, got in (("out", out), ("dq", q.grad), ("dk", k.grad), ("dv", v.grad),
+                      ("dbias", base.grad.permute(0, 1, 4, 2, 3))):
+        assert ao.rel_l2(got.detach().cpu(), ref[name]) <= 1e-2, name
+    # gradients that nobody asked for are not computed; the ones that are do not change
+    q2 = a["q"].cuda().requires_grad_(True)
+    tk.turbo_attention(q2, k.detach(), v.detach(), pair_bias=bias.detach(), res_mask=mask).backward(d_out.cuda())
+    assert torch.equal(q2.grad, q.grad)
