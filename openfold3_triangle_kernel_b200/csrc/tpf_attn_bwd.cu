@@ -23,6 +23,7 @@
 #include <stdlib.h>
 
 #include "tpf_host.cuh"
+#include "tpf_internal.h"
 #include "tpf_ptx.cuh"
 
 namespace tpf {
@@ -81,7 +82,8 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
 // kernel 1: dQ, dK, dV
 // =============================================================================================
 struct AttnBwdParams {
-  __nv_bfloat16 *dq, *dk, *dv;  // [B,O,H,N,D] contiguous
+  __nv_bfloat16 *dq, *dk, *dv;
+  int64_t gb, go, gh, gn;       // their element strides
   const float* lse;             // [B,O,H,N]
   const float* delta;           // [B,O,H,N]
   float* dq_scratch;            // per-CTA [N][D] fp32 when the key axis needs several strips
@@ -435,10 +437,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     };
 
     // One finished 128 x D tile (this thread holds DQ columns of row `row`) -> global memory at `gtile`
-    // (row 0 of the tile; the tile is one contiguous block there).  Staged: every thread drops its piece
-    // into a shared-memory copy of the block, then the 512 compute threads write the block out in
-    // consecutive 16-byte pieces, so each store instruction covers 512 contiguous bytes instead of 32
-    // half-used sectors.  All sixteen compute warps call this together.
+    // (row 0 of the tile; rows are gn elements apart).  Staged: every thread drops its piece
+    // into a shared-memory copy of the tile, then the 512 compute threads write it out in
+    // consecutive 16-byte pieces, so each store instruction covers whole rows (512 contiguous bytes when the
+    // rows are) instead of 32 half-used sectors.  All sixteen compute warps call this together.
     auto store_tile = [&](__nv_bfloat16* gtile, int rows_valid, const float (&v)[DQ], float mul) {
       if constexpr (Cfg::STAGED) {
         uint8_t* stg = smem + Cfg::OFF_STG + stg_slot * Cfg::TILE;
@@ -448,16 +450,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int i = threadIdx.x; i < Cfg::TILE / 16; i += 32 * NCW)
           if ((16 * i) / (2 * D) < rows_valid)
-            *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(gtile) + 16 * i) = *reinterpret_cast<const uint4*>(stg + 16 * i);
+            *reinterpret_cast<uint4*>(gtile + (int64_t)((16 * i) / (2 * D)) * p.gn + ((16 * i) % (2 * D)) / 2) =
+                *reinterpret_cast<const uint4*>(stg + 16 * i);
       } else {
-        if (row < rows_valid) st_cols(gtile + row * D + DQ * part, v, mul);
+        if (row < rows_valid) st_cols(gtile + row * p.gn + DQ * part, v, mul);
       }
     };
 
     // store a finished dQ tile that has been read out of TMEM (or fold it into the per-CTA running sum)
     auto store_dq = [&](int b, int o, int h, int q0, int strip, float (&v)[DQ]) {
       if (p.n_strips == 1) {
-        store_tile(p.dq + ((((int64_t)b * p.O + o) * p.H + h) * p.N + q0) * D, p.N - q0, v, scale);
+        store_tile(p.dq + b * p.gb + o * p.go + h * p.gh + q0 * p.gn, p.N - q0, v, scale);
         return;
       }
       const int q = q0 + row;
@@ -477,7 +480,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           return;
         }
       }
-      st_cols(p.dq + ((((int64_t)b * p.O + o) * p.H + h) * p.N + q) * D + DQ * part, v, scale);
+      st_cols(p.dq + b * p.gb + o * p.go + h * p.gh + q * p.gn + DQ * part, v, scale);
     };
 
     // lse / delta of this thread's query row, loaded one query tile ahead of their first use
@@ -511,7 +514,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         have_prev_strip = false;
         for (int kk = 0; kk < sp_nk; ++kk) {
           const int key0 = (sp_strip * KS + kk) * 128;
-          const int64_t base = ((((int64_t)sp_b * p.O + sp_o) * p.H + sp_h) * p.N + key0) * D;
+          const int64_t base = sp_b * p.gb + sp_o * p.go + sp_h * p.gh + key0 * p.gn;
           float vk1[DQ], vv1[DQ];
           ld_cols(tmem_addr(tmem_base, lane_base, Cfg::TM_DK + kk * D + DQ * part), vk1);
           ld_cols(tmem_addr(tmem_base, lane_base, Cfg::TM_DV + kk * D + DQ * part), vv1);
@@ -990,6 +993,33 @@ __global__ void __launch_bounds__(256) attn_dbias_fold_kernel(const float* __res
   }
 }
 
+// The same sum, written as bf16 rows: row (g, i, j) of `out` (pitch ld) gets the H gradients of pair (i, j), then zeros
+// up to a multiple of 8 columns (they are K columns of the GEMM that follows).
+__global__ void __launch_bounds__(256) attn_dbias_rows_kernel(const float* __restrict__ part,
+                                                              __nv_bfloat16* __restrict__ out, int64_t ld, int H,
+                                                              int64_t NN, int64_t n_rows, int n_chunks) {
+  griddep_wait();
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t g = r / NN, ij = r - g * NN;
+    const int64_t plane = n_rows * H;
+    for (int h0 = 0; h0 < H; h0 += 8) {
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        v[e] = 0.f;
+        if (h0 + e < H) {
+          const float* src = part + (g * H + h0 + e) * NN + ij;
+          float a = src[0];
+          for (int c = 1; c < n_chunks; ++c) a = __fadd_rn(a, src[c * plane]);
+          v[e] = a;
+        }
+      }
+      *reinterpret_cast<uint4*>(out + r * ld + h0) =
+          make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------
@@ -1066,31 +1096,55 @@ int attn_bwd_dqkv(const void* q, const void* k, const void* v, const void* d_out
   }
 
   if (!(stages & 2)) return TPF_OK;
+  AttnCall c = {};
+  c.B = B; c.O = O; c.H = H; c.N = N; c.D = D; c.G = bias_batch;
+  c.scale = scale;
+  c.q = q; c.k = k; c.v = v;
+  for (int i = 0; i < 4; ++i) {
+    c.qs[i] = q_strides[i];
+    c.ks[i] = k_strides[i];
+    c.vs[i] = v_strides[i];
+  }
+  c.mask = mask; c.mask_pitch = mask_pitch;
+  c.bias = bias; c.bias_pitch = bias_pitch;
+  c.lse = const_cast<float*>(lse);
+  c.d_out = d_out;  // [B,O,N,H,D]
+  c.dos[0] = O * N * H * D; c.dos[1] = N * H * D; c.dos[2] = D; c.dos[3] = H * D;
+  c.delta = delta;
+  c.dq = dq; c.dk = dk; c.dv = dv;  // [B,O,H,N,D]
+  c.ds[0] = O * H * N * D; c.ds[1] = H * N * D; c.ds[2] = N * D; c.ds[3] = D;
+  return attn_backward_qkv(c, workspace, workspace_bytes, stream);
+}
+
+int attn_backward_qkv(const AttnCall& c, void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
+  const int64_t B = c.B, O = c.O, H = c.H, N = c.N, D = c.D;
+  const int64_t need = attn_bwd_workspace_bytes(B, O, H, N, D);
+  TPF_REQUIRE(need == 0 || (workspace && workspace_bytes >= need), TPF_ERR_WORKSPACE, "attn_bwd: workspace too small");
   const int swz = 2 * (int)D;
   CUtensorMap tq, tk, tv, tdo, tb, tm;
   int rc;
-  if ((rc = make_qkv_tmap(&tq, q, B, O, H, N, D, q_strides, swz))) return rc;
-  if ((rc = make_qkv_tmap(&tk, k, B, O, H, N, D, k_strides, swz))) return rc;
-  if ((rc = make_qkv_tmap(&tv, v, B, O, H, N, D, v_strides, swz))) return rc;
-  const int64_t do_strides[4] = {O * N * H * D, N * H * D, D, H * D};  // d_out is [B,O,N,H,D]
-  if ((rc = make_qkv_tmap(&tdo, d_out, B, O, H, N, D, do_strides, swz))) return rc;
-  if ((rc = make_bias_tmap(&tb, bias, bias_batch, H, N, bias_pitch))) return rc;
-  if ((rc = make_mask_tmap(&tm, mask, B, O, N, mask_pitch))) return rc;
+  if ((rc = make_qkv_tmap(&tq, c.q, B, O, H, N, D, c.qs, swz))) return rc;
+  if ((rc = make_qkv_tmap(&tk, c.k, B, O, H, N, D, c.ks, swz))) return rc;
+  if ((rc = make_qkv_tmap(&tv, c.v, B, O, H, N, D, c.vs, swz))) return rc;
+  if ((rc = make_qkv_tmap(&tdo, c.d_out, B, O, H, N, D, c.dos, swz))) return rc;
+  if ((rc = make_bias_tmap(&tb, c.bias, c.G, H, N, c.bias_pitch))) return rc;
+  if ((rc = make_mask_tmap(&tm, c.mask, B, O, N, c.mask_pitch))) return rc;
 
   AttnBwdParams p;
-  p.dq = reinterpret_cast<__nv_bfloat16*>(dq);
-  p.dk = reinterpret_cast<__nv_bfloat16*>(dk);
-  p.dv = reinterpret_cast<__nv_bfloat16*>(dv);
-  p.lse = lse;
-  p.delta = delta;
+  p.dq = reinterpret_cast<__nv_bfloat16*>(c.dq);
+  p.dk = reinterpret_cast<__nv_bfloat16*>(c.dk);
+  p.dv = reinterpret_cast<__nv_bfloat16*>(c.dv);
+  p.gb = c.ds[0]; p.go = c.ds[1]; p.gh = c.ds[2]; p.gn = c.ds[3];
+  p.lse = c.lse;
+  p.delta = c.delta;
   p.dq_scratch = reinterpret_cast<float*>(workspace);
   p.B = (int)B; p.O = (int)O; p.H = (int)H; p.N = (int)N;
   p.q_tiles = (int)((N + 127) / 128);
   p.k_tiles = p.q_tiles;
   const int ks = bwd_key_strip(D);
   p.n_strips = (p.k_tiles + ks - 1) / ks;
-  p.bias_broadcast = bias_batch == 1 && B > 1 ? 1 : 0;
-  p.scale = scale;
+  p.bias_broadcast = c.G == 1 && B > 1 ? 1 : 0;
+  p.scale = c.scale;
   p.n_items = (int)(B * O * H);
   int grid = sm_count();
   if (grid > p.n_items) grid = p.n_items;
@@ -1133,6 +1187,12 @@ int64_t attn_dbias_workspace_bytes(int64_t B, int64_t O, int64_t H, int64_t N, i
   return c > 1 ? (int64_t)c * G * H * N * N * 4 : 0;
 }
 
+int64_t attn_dbias_rows_workspace_bytes(int64_t B, int64_t O, int64_t H, int64_t N, int64_t G) {
+  int c, len;
+  dbias_plan(B, O, H, N, G, &c, &len);
+  return (int64_t)c * G * H * N * N * 4;
+}
+
 int attn_bwd_dbias(const void* q, const void* k, const void* v, const void* d_out, const int64_t* q_strides,
                    const int64_t* k_strides, const int64_t* v_strides, const float* lse, const float* delta,
                    const float* mask, int64_t mask_pitch, const void* bias, int64_t bias_pitch, int64_t bias_batch,
@@ -1140,10 +1200,32 @@ int attn_bwd_dbias(const void* q, const void* k, const void* v, const void* d_ou
                    int64_t D, float scale, cudaStream_t stream) {
   TPF_REQUIRE(dbias != nullptr, TPF_ERR_INVALID_ARGUMENT, "attn_bwd: dbias is NULL");
   TPF_REQUIRE_ALIGNED16(dbias, "attn_bwd", "dbias");  // rows are written with float4 stores
-  const int64_t G = bias_batch;
+  AttnCall c = {};
+  c.B = B; c.O = O; c.H = H; c.N = N; c.D = D; c.G = bias_batch;
+  c.scale = scale;
+  c.q = q; c.k = k; c.v = v;
+  for (int i = 0; i < 4; ++i) {
+    c.qs[i] = q_strides[i];
+    c.ks[i] = k_strides[i];
+    c.vs[i] = v_strides[i];
+  }
+  c.mask = mask; c.mask_pitch = mask_pitch;
+  c.bias = bias; c.bias_pitch = bias_pitch;
+  c.lse = const_cast<float*>(lse);
+  c.d_out = d_out;
+  c.dos[0] = O * N * H * D; c.dos[1] = N * H * D; c.dos[2] = D; c.dos[3] = H * D;
+  c.delta = const_cast<float*>(delta);
+  c.dbias = dbias;
+  return attn_backward_bias(c, workspace, workspace_bytes, stream);
+}
+
+int attn_backward_bias(const AttnCall& c, void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
+  const int64_t B = c.B, O = c.O, H = c.H, N = c.N, D = c.D, G = c.G;
   int n_chunks, chunk_len;
   dbias_plan(B, O, H, N, G, &n_chunks, &chunk_len);
-  const int64_t need = attn_dbias_workspace_bytes(B, O, H, N, G);
+  const bool rows = c.dbias == nullptr;  // fp32 planes go to the workspace, bf16 rows come out
+  const int64_t need =
+      rows ? attn_dbias_rows_workspace_bytes(B, O, H, N, G) : attn_dbias_workspace_bytes(B, O, H, N, G);
   TPF_REQUIRE(need == 0 || (workspace && workspace_bytes >= need), TPF_ERR_WORKSPACE,
               "attn_bwd: dBias workspace of %lld bytes required, %lld given", (long long)need,
               (long long)workspace_bytes);
@@ -1152,17 +1234,16 @@ int attn_bwd_dbias(const void* q, const void* k, const void* v, const void* d_ou
   const int swz = 2 * (int)D;
   CUtensorMap tq, tk, tv, tdo, tb, tm;
   int rc;
-  if ((rc = make_qkv_tmap(&tq, q, B, O, H, N, D, q_strides, swz))) return rc;
-  if ((rc = make_qkv_tmap(&tk, k, B, O, H, N, D, k_strides, swz))) return rc;
-  if ((rc = make_qkv_tmap(&tv, v, B, O, H, N, D, v_strides, swz))) return rc;
-  const int64_t do_strides[4] = {O * N * H * D, N * H * D, D, H * D};
-  if ((rc = make_qkv_tmap(&tdo, d_out, B, O, H, N, D, do_strides, swz))) return rc;
-  if ((rc = make_bias_tmap(&tb, bias, bias_batch, H, N, bias_pitch))) return rc;
-  if ((rc = make_mask_tmap(&tm, mask, B, O, N, mask_pitch))) return rc;
+  if ((rc = make_qkv_tmap(&tq, c.q, B, O, H, N, D, c.qs, swz))) return rc;
+  if ((rc = make_qkv_tmap(&tk, c.k, B, O, H, N, D, c.ks, swz))) return rc;
+  if ((rc = make_qkv_tmap(&tv, c.v, B, O, H, N, D, c.vs, swz))) return rc;
+  if ((rc = make_qkv_tmap(&tdo, c.d_out, B, O, H, N, D, c.dos, swz))) return rc;
+  if ((rc = make_bias_tmap(&tb, c.bias, G, H, N, c.bias_pitch))) return rc;
+  if ((rc = make_mask_tmap(&tm, c.mask, B, O, N, c.mask_pitch))) return rc;
   AttnDbiasParams p;
-  p.part = n_chunks > 1 ? reinterpret_cast<float*>(workspace) : dbias;
-  p.lse = lse;
-  p.delta = delta;
+  p.part = n_chunks > 1 || rows ? reinterpret_cast<float*>(workspace) : c.dbias;
+  p.lse = c.lse;
+  p.delta = c.delta;
   p.B = (int)B; p.O = (int)O; p.H = (int)H; p.N = (int)N;
   p.G = (int)G;
   p.planes = (int)((B / G) * O);
@@ -1170,7 +1251,7 @@ int attn_bwd_dbias(const void* q, const void* k, const void* v, const void* d_ou
   p.chunk_len = chunk_len;
   p.q_tiles = (int)((N + 127) / 128);
   p.k_tiles = p.q_tiles;
-  p.scale = scale;
+  p.scale = c.scale;
   const int64_t grid = (int64_t)G * H * p.q_tiles * p.k_tiles * n_chunks;
   TPF_REQUIRE(grid < (1ll << 31), TPF_ERR_INVALID_ARGUMENT, "attn_bwd: dBias grid too large");
   int* status = nullptr;
@@ -1179,11 +1260,15 @@ int attn_bwd_dbias(const void* q, const void* k, const void* v, const void* d_ou
   else if (D == 32) rc = launch_attn_dbias<32>(tq, tk, tv, tdo, tb, tm, p, status, (int)grid, stream);
   else rc = launch_attn_dbias<64>(tq, tk, tv, tdo, tb, tm, p, status, (int)grid, stream);
   if (rc) return rc;
-  if (n_chunks > 1) {
-    const int64_t n = G * H * N * N;
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
-    launch_kernel(attn_dbias_fold_kernel, dim3(blocks), dim3(256), 0, stream, p.part, dbias, n, n_chunks);
+  const int64_t n = rows ? G * N * N : G * H * N * N;
+  int blocks = (int)((n + 255) / 256);
+  if (blocks > 4 * sm_count()) blocks = 4 * sm_count();
+  if (rows) {
+    launch_kernel(attn_dbias_rows_kernel, dim3(blocks), dim3(256), 0, stream, p.part,
+                  reinterpret_cast<__nv_bfloat16*>(c.dbias_rows), c.dbias_ld, (int)H, N * N, n, n_chunks);
+    TPF_LAUNCH_OK();
+  } else if (n_chunks > 1) {
+    launch_kernel(attn_dbias_fold_kernel, dim3(blocks), dim3(256), 0, stream, p.part, c.dbias, n, n_chunks);
     TPF_LAUNCH_OK();
   }
   return TPF_OK;

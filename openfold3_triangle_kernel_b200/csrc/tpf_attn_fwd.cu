@@ -23,6 +23,7 @@
 //  * A tile whose mask row is all zero and that has no ragged key tail (the common case) takes a
 //    code path without the mask add.
 #include "tpf_host.cuh"
+#include "tpf_internal.h"
 #include "tpf_ptx.cuh"
 
 namespace tpf {
@@ -38,8 +39,11 @@ int attn_fwd_status_fetch_and_clear(int* out) {
 }
 
 struct AttnFwdParams {
-  __nv_bfloat16* out;  // [B,O,N,H,D]
-  float* lse;          // [B,O,H,N]
+  __nv_bfloat16* out;
+  int64_t ob, oo, oh, on;   // element strides of out
+  const __nv_bfloat16* gate;  // logits of the output gate, or null
+  int64_t gb, go, gh, gn;
+  float* lse;          // [B,O,H,N] or null
   int B, O, H, N;
   int q_tiles, k_tiles;  // 128-query tiles, 64-key tiles
   int bias_broadcast;    // 1: one bias for all b
@@ -454,28 +458,42 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tc_fence_after();
       const int q = qt * 128 + row;
       const float inv = l_run > 0.f ? __fdividef(1.f, l_run) : 0.f;
-      __nv_bfloat16* orow = p.out + ((((int64_t)b * p.O + o) * p.N + q) * p.H + h) * D;
+      const bool row_ok = q < p.N;
+      __nv_bfloat16* orow = p.out + b * p.ob + o * p.oo + h * p.oh + (int64_t)q * p.on;
+      const __nv_bfloat16* grow = p.gate + b * p.gb + o * p.go + h * p.gh + (int64_t)q * p.gn;
 #pragma unroll
       for (int c = 0; c < D; c += 16) {
         uint32_t ro[16];
         tmem_ld16(t_o + c, ro);
+        uint4 g0 = make_uint4(0u, 0u, 0u, 0u), g1 = g0;
+        if (p.gate != nullptr && row_ok) {
+          g0 = *reinterpret_cast<const uint4*>(grow + c);
+          g1 = *reinterpret_cast<const uint4*>(grow + c + 8);
+        }
         tmem_ld_wait();
-        if (q < p.N) {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(ro[i]) * inv;
+        if (p.gate != nullptr) {
+          const uint32_t gw[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            v[2 * i] *= sigmoid_fast(__uint_as_float(gw[i] << 16));
+            v[2 * i + 1] *= sigmoid_fast(__uint_as_float(gw[i] & 0xFFFF0000u));
+          }
+        }
+        if (row_ok) {
           uint4 pk0, pk1;
-          pk0.x = pack_bf16x2(__uint_as_float(ro[0]) * inv, __uint_as_float(ro[1]) * inv);
-          pk0.y = pack_bf16x2(__uint_as_float(ro[2]) * inv, __uint_as_float(ro[3]) * inv);
-          pk0.z = pack_bf16x2(__uint_as_float(ro[4]) * inv, __uint_as_float(ro[5]) * inv);
-          pk0.w = pack_bf16x2(__uint_as_float(ro[6]) * inv, __uint_as_float(ro[7]) * inv);
-          pk1.x = pack_bf16x2(__uint_as_float(ro[8]) * inv, __uint_as_float(ro[9]) * inv);
-          pk1.y = pack_bf16x2(__uint_as_float(ro[10]) * inv, __uint_as_float(ro[11]) * inv);
-          pk1.z = pack_bf16x2(__uint_as_float(ro[12]) * inv, __uint_as_float(ro[13]) * inv);
-          pk1.w = pack_bf16x2(__uint_as_float(ro[14]) * inv, __uint_as_float(ro[15]) * inv);
+          pk0 = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                           pack_bf16x2(v[6], v[7]));
+          pk1 = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
+                           pack_bf16x2(v[14], v[15]));
           *reinterpret_cast<uint4*>(orow + c) = pk0;
           *reinterpret_cast<uint4*>(orow + c + 8) = pk1;
         }
       }
       tc_fence_before();
-      if (q < p.N)
+      if (row_ok && p.lse != nullptr)
         p.lse[(((int64_t)b * p.O + o) * p.H + h) * p.N + q] = l_run > 0.f ? m_use + log2f(l_run) * kLn2 : -INFINITY;
     }
   }
@@ -539,39 +557,40 @@ int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
   return TPF_OK;
 }
 
-int attn_fwd(const void* q, const void* k, const void* v, const int64_t* q_strides, const int64_t* k_strides,
-             const int64_t* v_strides, const float* mask, int64_t mask_pitch, const void* bias, int64_t bias_pitch,
-             int64_t bias_batch, void* out, float* lse, int64_t B, int64_t O, int64_t H, int64_t N, int64_t D,
-             float scale, cudaStream_t stream) {
-  TPF_REQUIRE(q && k && v && mask && bias && out && lse, TPF_ERR_INVALID_ARGUMENT, "attn_fwd: null pointer");
+int attn_forward(const AttnCall& c, cudaStream_t stream) {
+  const int64_t B = c.B, O = c.O, H = c.H, N = c.N, D = c.D;
+  TPF_REQUIRE(c.q && c.k && c.v && c.mask && c.bias && c.out, TPF_ERR_INVALID_ARGUMENT, "attn_fwd: null pointer");
   TPF_REQUIRE(B > 0 && O > 0 && H > 0 && N > 0, TPF_ERR_INVALID_ARGUMENT, "attn_fwd: B,O,H,N must be positive");
   TPF_REQUIRE(D == 16 || D == 32 || D == 64, TPF_ERR_UNSUPPORTED,
               "attn_fwd: head dim %lld not in {16,32,64} (pad on the host side)", (long long)D);
-  TPF_REQUIRE(bias_batch == 1 || bias_batch == B, TPF_ERR_INVALID_ARGUMENT, "attn_fwd: bias batch must be 1 or B");
-  TPF_REQUIRE(bias_pitch >= N && bias_pitch % 8 == 0, TPF_ERR_INVALID_ARGUMENT,
+  TPF_REQUIRE(c.G == 1 || c.G == B, TPF_ERR_INVALID_ARGUMENT, "attn_fwd: bias batch must be 1 or B");
+  TPF_REQUIRE(c.bias_pitch >= N && c.bias_pitch % 8 == 0, TPF_ERR_INVALID_ARGUMENT,
               "attn_fwd: bias row pitch must be >= N and a multiple of 8 elements");
-  TPF_REQUIRE(mask_pitch >= N && mask_pitch % 4 == 0, TPF_ERR_INVALID_ARGUMENT,
+  TPF_REQUIRE(c.mask_pitch >= N && c.mask_pitch % 4 == 0, TPF_ERR_INVALID_ARGUMENT,
               "attn_fwd: mask row pitch must be >= N and a multiple of 4 elements");
   TPF_REQUIRE(N <= (1 << 24) && B * O * H < (1ll << 31), TPF_ERR_INVALID_ARGUMENT, "attn_fwd: extent too large");
-  TPF_REQUIRE_ALIGNED16(out, "attn_fwd", "out");
-  TPF_REQUIRE((reinterpret_cast<uintptr_t>(lse) & 3) == 0, TPF_ERR_INVALID_ARGUMENT,
+  TPF_REQUIRE_ALIGNED16(c.out, "attn_fwd", "out");
+  TPF_REQUIRE((reinterpret_cast<uintptr_t>(c.lse) & 3) == 0, TPF_ERR_INVALID_ARGUMENT,
               "attn_fwd: lse must be 4-byte aligned");
   const int swz = 2 * (int)D;
   CUtensorMap tq, tk, tv, tb, tm;
   int rc;
-  if ((rc = make_qkv_tmap(&tq, q, B, O, H, N, D, q_strides, swz))) return rc;
-  if ((rc = make_qkv_tmap_rows(&tk, k, B, O, H, N, D, k_strides, swz, 64))) return rc;
-  if ((rc = make_qkv_tmap_rows(&tv, v, B, O, H, N, D, v_strides, swz, 64))) return rc;
-  if ((rc = make_bias_tmap(&tb, bias, bias_batch, H, N, bias_pitch))) return rc;
-  if ((rc = make_mask_tmap_cols(&tm, mask, B, O, N, mask_pitch, 64))) return rc;
+  if ((rc = make_qkv_tmap(&tq, c.q, B, O, H, N, D, c.qs, swz))) return rc;
+  if ((rc = make_qkv_tmap_rows(&tk, c.k, B, O, H, N, D, c.ks, swz, 64))) return rc;
+  if ((rc = make_qkv_tmap_rows(&tv, c.v, B, O, H, N, D, c.vs, swz, 64))) return rc;
+  if ((rc = make_bias_tmap(&tb, c.bias, c.G, H, N, c.bias_pitch))) return rc;
+  if ((rc = make_mask_tmap_cols(&tm, c.mask, B, O, N, c.mask_pitch, 64))) return rc;
   AttnFwdParams p;
-  p.out = reinterpret_cast<__nv_bfloat16*>(out);
-  p.lse = lse;
+  p.out = reinterpret_cast<__nv_bfloat16*>(c.out);
+  p.ob = c.os[0]; p.oo = c.os[1]; p.oh = c.os[2]; p.on = c.os[3];
+  p.gate = reinterpret_cast<const __nv_bfloat16*>(c.gate);
+  p.gb = c.gs[0]; p.go = c.gs[1]; p.gh = c.gs[2]; p.gn = c.gs[3];
+  p.lse = c.lse;
   p.B = (int)B; p.O = (int)O; p.H = (int)H; p.N = (int)N;
   p.q_tiles = (int)((N + 127) / 128);
   p.k_tiles = (int)((N + 63) / 64);
-  p.bias_broadcast = bias_batch == 1 && B > 1 ? 1 : 0;
-  p.scale = scale;
+  p.bias_broadcast = c.G == 1 && B > 1 ? 1 : 0;
+  p.scale = c.scale;
   const int64_t items = B * H * p.q_tiles * O;
   TPF_REQUIRE(items < (1ll << 31), TPF_ERR_INVALID_ARGUMENT, "attn_fwd: too many work items");
   p.n_items = (int)items;
@@ -583,6 +602,28 @@ int attn_fwd(const void* q, const void* k, const void* v, const int64_t* q_strid
   if (D == 16) return launch_attn_fwd<16>(tq, tk, tv, tb, tm, p, status, stream);
   if (D == 32) return launch_attn_fwd<32>(tq, tk, tv, tb, tm, p, status, stream);
   return launch_attn_fwd<64>(tq, tk, tv, tb, tm, p, status, stream);
+}
+
+int attn_fwd(const void* q, const void* k, const void* v, const int64_t* q_strides, const int64_t* k_strides,
+             const int64_t* v_strides, const float* mask, int64_t mask_pitch, const void* bias, int64_t bias_pitch,
+             int64_t bias_batch, void* out, float* lse, int64_t B, int64_t O, int64_t H, int64_t N, int64_t D,
+             float scale, cudaStream_t stream) {
+  TPF_REQUIRE(lse, TPF_ERR_INVALID_ARGUMENT, "attn_fwd: null pointer");
+  AttnCall c = {};
+  c.B = B; c.O = O; c.H = H; c.N = N; c.D = D; c.G = bias_batch;
+  c.scale = scale;
+  c.q = q; c.k = k; c.v = v;
+  for (int i = 0; i < 4; ++i) {
+    c.qs[i] = q_strides[i];
+    c.ks[i] = k_strides[i];
+    c.vs[i] = v_strides[i];
+  }
+  c.mask = mask; c.mask_pitch = mask_pitch;
+  c.bias = bias; c.bias_pitch = bias_pitch;
+  c.out = out;
+  c.os[0] = O * N * H * D; c.os[1] = N * H * D; c.os[2] = D; c.os[3] = H * D;
+  c.lse = lse;
+  return attn_forward(c, stream);
 }
 
 }  // namespace tpf

@@ -40,6 +40,7 @@ int attn_bwd_static_scratch(const void* q, const void* k, const void* v, const v
                             const float* mask, int64_t mask_pitch, const void* bias, int64_t bias_pitch,
                             int64_t bias_batch, void* dq, void* dk, void* dv, float* dbias, float* delta, int64_t B,
                             int64_t O, int64_t H, int64_t N, int64_t D, float scale, cudaStream_t stream);
+int pair_attn_status_fetch_and_clear(int* out);
 int selftest_status_fetch_and_clear(int* out);
 int selftest_bounded_wait(unsigned int* report, cudaStream_t stream);
 
@@ -81,6 +82,8 @@ int tpf_device_status(int* status) {
   if ((rc = tpf::attn_bwd_status_fetch_and_clear(&v))) return rc;
   total |= v;
   if ((rc = tpf::trimul_status_fetch_and_clear(&v))) return rc;
+  total |= v;
+  if ((rc = tpf::pair_attn_status_fetch_and_clear(&v))) return rc;
   total |= v;
   if ((rc = tpf::selftest_status_fetch_and_clear(&v))) return rc;
   total |= v;

@@ -64,40 +64,52 @@ struct PairMask {
   }
 };
 
+// Address of column n0 of internal row `row` in the caller's [.., C] tensor; nullptr: no such row.
+__device__ __forceinline__ __nv_bfloat16* row_address(__nv_bfloat16* base, const PairRows& rows, int row, int M, int C,
+                                                      int n0) {
+  if (row >= M) return nullptr;
+  int64_t src = row;
+  if (!rows.identity) src = rows.split((uint32_t)row).src;
+  return src < 0 ? nullptr : base + src * C + n0;
+}
+
+// A warp's 32 rows x 64 bytes in the arrangement of warp_tile_store: access i covers rows 8 i .. 8 i + 7.
+__device__ __forceinline__ void load_rows(const __nv_bfloat16* base, const PairRows& rows, int m_base, int M, int C,
+                                          int n0, int lane, uint4 (&u)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat16* src =
+        row_address(const_cast<__nv_bfloat16*>(base), rows, m_base + 8 * i + (lane >> 2), M, C, n0);
+    u[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (src != nullptr) u[i] = *reinterpret_cast<const uint4*>(src + 8 * (lane & 3));
+  }
+}
+
+__device__ __forceinline__ uint4 add_bf16x8(const uint4& x, const uint4& y) {
+  const uint32_t a[4] = {x.x, x.y, x.z, x.w}, b[4] = {y.x, y.y, y.z, y.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(bf16_lo(a[e]) + bf16_lo(b[e]), bf16_hi(a[e]) + bf16_hi(b[e]));
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // Stores a warp's 32 x 32 bf16 block (lane = row, packed column pairs) of internal rows m_base.. at the caller's rows:
-// `out` receives the block, `sum` the block added to `res` (the block is rounded to bf16 first, as a separate add would
-// see it).  Staged through the warp's 2 KB tile so that one access covers 8 rows x 64 contiguous bytes.
-__device__ __forceinline__ void store_rows_with_residual(uint8_t* tile, int lane, const uint32_t (&pk)[16],
-                                                         const PairRows& rows, int m_base, int M, int C, int n0,
-                                                         __nv_bfloat16* out, __nv_bfloat16* sum,
-                                                         const __nv_bfloat16* res) {
+// `out` (may be null) receives the block, `sum` the block added to the residual `r` (from load_rows).  The block is
+// rounded to bf16 first, as a separate add would see it.
+__device__ __forceinline__ void store_rows_added(uint8_t* tile, int lane, const uint32_t (&pk)[16], const PairRows& rows,
+                                                 int m_base, int M, int C, int n0, __nv_bfloat16* out,
+                                                 __nv_bfloat16* sum, const uint4 (&r)[4]) {
   warp_tile_put(tile, lane, pk);
-  int64_t off[4];
-  uint4 r4[4];
+  __syncwarp();
   const int piece = lane & 3;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int row = m_base + 8 * i + (lane >> 2);
-    off[i] = -1;
-    if (row < M) {
-      const int64_t src = rows.locate((uint32_t)row).src;
-      if (src >= 0) off[i] = src * C + n0 + 8 * piece;
-    }
-    if (sum != nullptr && off[i] >= 0) r4[i] = *reinterpret_cast<const uint4*>(res + off[i]);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (off[i] < 0) continue;
-    const uint4 u = warp_tile_get(tile, 8 * i + (lane >> 2), piece);
-    if (out != nullptr) *reinterpret_cast<uint4*>(out + off[i]) = u;
-    if (sum != nullptr) {
-      const uint32_t a[4] = {u.x, u.y, u.z, u.w}, b[4] = {r4[i].x, r4[i].y, r4[i].z, r4[i].w};
-      uint32_t o[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(bf16_lo(a[e]) + bf16_lo(b[e]), bf16_hi(a[e]) + bf16_hi(b[e]));
-      *reinterpret_cast<uint4*>(sum + off[i]) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
+    const int rr = 8 * i + (lane >> 2);
+    __nv_bfloat16* dst = row_address(sum, rows, m_base + rr, M, C, n0);
+    if (dst == nullptr) continue;
+    const uint4 u = warp_tile_get(tile, rr, piece);
+    if (out != nullptr) *reinterpret_cast<uint4*>(out + (dst - sum) + 8 * piece) = u;
+    *reinterpret_cast<uint4*>(dst + 8 * piece) = add_bf16x8(u, r[i]);
   }
   __syncwarp();
 }

@@ -17,6 +17,7 @@ struct PrepParams {
   __nv_bfloat16* bias_dst;     // [G,H,N,bias_pitch]
   float* mask_dst;             // [B,O,mask_pitch]
   int H, N, O, bias_pitch, mask_pitch;
+  float mask_add, mask_mul;    // mask value = (source + add) * mul
   int64_t bias_groups, mask_groups;  // 8-element / 4-element pieces
   int bias_blocks;
 };
@@ -24,6 +25,7 @@ struct PrepParams {
 __device__ __forceinline__ float prep_load(const PrepSource& s, int64_t off) {
   if (s.type == kPrepF32) return reinterpret_cast<const float*>(s.src)[off];
   if (s.type == kPrepBF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(s.src)[off]);
+  if (s.type == kPrepBool) return reinterpret_cast<const uint8_t*>(s.src)[off] ? 1.f : 0.f;
   return __half2float(reinterpret_cast<const __half*>(s.src)[off]);
 }
 
@@ -56,14 +58,18 @@ __global__ void __launch_bounds__(256) attn_prep_kernel(const PrepParams p) {
     const int64_t base = (r / p.O) * p.mask.stride[0] + (r % p.O) * p.mask.stride[1];
     float o[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) o[e] = j0 + e < p.N ? prep_load(p.mask, base + (j0 + e) * p.mask.stride[2]) : 0.f;
+    for (int e = 0; e < 4; ++e)
+      o[e] = j0 + e < p.N ? (prep_load(p.mask, base + (j0 + e) * p.mask.stride[2]) + p.mask_add) * p.mask_mul : 0.f;
     reinterpret_cast<float4*>(p.mask_dst)[i] = make_float4(o[0], o[1], o[2], o[3]);
   }
 }
 
 int attn_prep(const PrepSource& bias, int64_t G, int64_t H, void* bias_dst, int64_t bias_pitch, const PrepSource& mask,
-              int64_t B, int64_t O, float* mask_dst, int64_t mask_pitch, int64_t N, cudaStream_t stream) {
+              int64_t B, int64_t O, float* mask_dst, int64_t mask_pitch, int64_t N, cudaStream_t stream, float mask_add,
+              float mask_mul) {
   PrepParams p = {};
+  p.mask_add = mask_add;
+  p.mask_mul = mask_mul;
   p.bias = bias;
   p.mask = mask;
   p.bias_dst = reinterpret_cast<__nv_bfloat16*>(bias_dst);

@@ -43,5 +43,6 @@ PYBIND11_MODULE(_native, m) {
   m.def("attn_bwd", &tpf_torch::attn_bwd);
   m.def("trimul", &tpf_torch::py_trimul);
   m.def("trimul_fwd", &tpf_torch::trimul_fwd);
+  m.def("pair_block", &tpf_torch::py_pair_block);
   m.def("trimul_bwd", &tpf_torch::trimul_bwd);
 }

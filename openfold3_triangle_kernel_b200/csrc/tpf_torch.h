@@ -70,4 +70,8 @@ std::vector<Tensor> trimul_fwd(const Tensor& z, const Tensor& mask, std::vector<
 std::vector<Tensor> trimul_bwd(const Tensor& d_out, const Tensor& z, const Tensor& mask, std::vector<Tensor> w,
                                bool incoming, std::vector<Tensor> saved);
 
+// ---- pair-stack block (tpf_torch_block.cpp) -------------------------------------------------
+py::object py_pair_block(py::handle z, py::handle mask, py::tuple tri_out, py::tuple tri_in, py::tuple start,
+                         py::tuple end, int64_t heads);
+
 }  // namespace tpf_torch

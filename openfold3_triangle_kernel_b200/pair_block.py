@@ -3,9 +3,11 @@ axially over the GPUs of one node.
 
 Mirrors ``PairBlock.forward`` (openfold3/core/model/latent/base_blocks.py:433-534, dropout inactive,
 pair transition excluded) and ``TriangleAttention.forward``
-(openfold3/core/model/layers/triangular_attention.py:245-409): the LayerNorm and the bias-free
-q/k/v/g/o/bias Linears around the attention operator run as plain bf16 torch ops; the two hot
-operators are :func:`turbo_trimul` and :func:`turbo_attention` (or their axial variants).
+(openfold3/core/model/layers/triangular_attention.py:245-409).  On one GPU the block is one C++ call
+(csrc/tpf_torch_block.cpp) whose kernels contain the LayerNorms, the bias-free q/k/v/g/o/bias Linears, the
+gates and the residual adds (csrc/tpf_pair_attn.cu, csrc/tpf_trimul.cu).  The sharded block, and shapes that
+call does not cover, compose :func:`turbo_trimul` and :func:`turbo_attention` (or their axial variants) with
+plain bf16 torch ops.
 
 Sharded layout (``group`` given): ``z`` is row-sharded ``[B, N/P, N, C]``.  TriMul uses
 :func:`dap.axial_trimul`; starting-node attention shards its outer rows and all-gathers the
@@ -14,13 +16,18 @@ transpose of the sharded pair tensor, and is transposed back afterwards.
 """
 from __future__ import annotations
 
+import operator
+
 import torch
 import torch.distributed as dist
 import torch.nn.functional as F
 
+from . import _cabi as C
 from . import dap
 from .attention import turbo_attention
-from .trimul import turbo_trimul
+from .trimul import native_weight_order, turbo_trimul
+
+_attention_order = operator.itemgetter("ln_w", "ln_b", "w_z", "w_q", "w_k", "w_v", "w_g", "w_o")
 
 
 class _GatherRows(torch.autograd.Function):
@@ -91,6 +98,15 @@ def pair_stack_block(z, mask, params, heads, group=None, trimul_backend=None, at
     ``synthetic.block_params`` (fp32 masters).  ``trimul_backend`` / ``attention_fn`` replace the
     CUDA stage back end of :func:`dap.axial_trimul` and :func:`turbo_attention` in the sharded
     path (used to test the collectives on CPU ranks); the defaults are the B200 operators."""
+    if group is None and not torch.compiler.is_compiling():
+        # one C++ call with fused kernels (residual adds, gates and projections inside); None: a shape, type or
+        # context it does not cover (head dims other than 16 and 32, tensor subclasses, ...), composed below
+        out = C.native().pair_block(z, mask, native_weight_order(params["tri_mul_out"]),
+                                    native_weight_order(params["tri_mul_in"]),
+                                    _attention_order(params["tri_att_start"]),
+                                    _attention_order(params["tri_att_end"]), heads)
+        if out is not None:
+            return out
     if group is None:
         z = z + turbo_trimul(z, "outgoing", mask, **params["tri_mul_out"])
         z = z + turbo_trimul(z, "incoming", mask, **params["tri_mul_in"])

@@ -41,7 +41,7 @@ _WEIGHT_NAMES = ("norm_in_weight", "norm_in_bias", "p_in_weight", "g_in_weight",
                  "norm_out_weight", "norm_out_bias", "p_out_weight", "g_out_weight")
 _WEIGHT_SET = frozenset(_WEIGHT_NAMES)
 # the order of the custom ops and of `_native.trimul`
-_native_order = operator.itemgetter("p_in_weight", "g_in_weight", "p_out_weight", "g_out_weight", "norm_in_weight",
+native_weight_order = operator.itemgetter("p_in_weight", "g_in_weight", "p_out_weight", "g_out_weight", "norm_in_weight",
                                     "norm_in_bias", "norm_out_weight", "norm_out_bias")
 
 
@@ -215,7 +215,7 @@ def turbo_trimul(z, direction="outgoing", mask=None, *, generator=None, **weight
         mod_weights.update(weights)
         weights = mod_weights
     if not torch.compiler.is_compiling() and direction in ("outgoing", "incoming") and weights.keys() == _WEIGHT_SET:
-        out = C.native().trimul(z, direction == "incoming", mask, _native_order(weights))
+        out = C.native().trimul(z, direction == "incoming", mask, native_weight_order(weights))
         if out is not None:
             return out
     unknown = set(weights) - set(_WEIGHT_NAMES)

@@ -51,3 +51,36 @@ def test_attention_operand_types_and_strides(N, D, bias_type, mask_type):
     q2 = a["q"].cuda().requires_grad_(True)
     tk.turbo_attention(q2, k.detach(), v.detach(), pair_bias=bias.detach(), res_mask=mask).backward(d_out.cuda())
     assert torch.equal(q2.grad, q.grad)
+
+
+@pytest.mark.parametrize("N,C,H,D", [(1, 64, 4, 16), (9, 128, 4, 32), (65, 32, 2, 16), (130, 96, 3, 32), (40, 64, 8, 16)])
+def test_pair_block_any_length(N, C, H, D):
+    from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
+    from oracle.pair_block_oracle import block_params, pair_block_forward
+    g = torch.Generator().manual_seed(N)
+    z = torch.randn(2, N, N, C, generator=g).bfloat16()
+    mask = torch.ones(2, N, N)
+    if N > 4:
+        mask[0, N - 3:] = 0
+        mask[0, :, N - 3:] = 0
+    d_out = torch.randn(2, N, N, C, generator=g).bfloat16() * mask.unsqueeze(-1).bfloat16()
+    params = block_params(C, H, D, seed=N)
+    zr = z.double().requires_grad_(True)
+    pr = {k: {n: t.double().requires_grad_(True) for n, t in v.items()} for k, v in params.items()}
+    ref = pair_block_forward(zr, mask, pr, H, dtype=torch.float64)
+    ref.backward(d_out.double())
+    pd = {k: {n: t.cuda().requires_grad_(True) for n, t in v.items()} for k, v in params.items()}
+    zz = z.cuda().requires_grad_(True)
+    out = pair_stack_block(zz, mask.cuda(), pd, H)
+    with torch.no_grad():
+        assert torch.equal(pair_stack_block(zz, mask.cuda().bool(), pd, H), out)
+    out.backward(d_out.cuda())
+    valid = mask.bool().unsqueeze(-1)
+    pick = lambda t: torch.where(valid, t.detach().cpu().double(), 0.0)  # noqa: E731
+    assert ao.rel_l2(pick(out), pick(ref)) <= 1e-2
+    assert ao.rel_l2(pick(zz.grad), pick(zr.grad)) <= 2e-2
+    for k, v in pd.items():
+        for n, t in v.items():
+            want = pr[k][n].grad
+            if want.norm() > 1e-6 * N:   # N = 1: a softmax over one key has no gradient in q, k and the bias
+                assert ao.rel_l2(t.grad.cpu(), want) <= 4e-2, (k, n)
