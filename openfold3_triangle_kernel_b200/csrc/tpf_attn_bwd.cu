@@ -235,7 +235,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   if (warp == Cfg::WARP_TMA) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    {
+      const uint32_t el = elect_one();
       int q_s = 0, kv_s = 0, b_s = 0;
       uint32_t q_ph = 1, kv_ph = 1, b_ph = 1;
       BwdWalk w;
@@ -248,9 +249,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         if (w.first_kk()) {
           mbar_wait(&q_empty[q_s], q_ph, wctx);
-          mbar_expect_tx(&q_full[q_s], 2 * Cfg::TILE);
-          tma_load_5d(smem + Cfg::OFF_Q + q_s * Cfg::TILE, &tmQ, &q_full[q_s], 0, w.qt * 128, h, o, b);
-          tma_load_5d(smem + Cfg::OFF_DO + q_s * Cfg::TILE, &tmDO, &q_full[q_s], 0, w.qt * 128, h, o, b);
+          mbar_expect_tx(el, &q_full[q_s], 2 * Cfg::TILE);
+          tma_load_5d(el, smem + Cfg::OFF_Q + q_s * Cfg::TILE, &tmQ, &q_full[q_s], 0, w.qt * 128, h, o, b);
+          tma_load_5d(el, smem + Cfg::OFF_DO + q_s * Cfg::TILE, &tmDO, &q_full[q_s], 0, w.qt * 128, h, o, b);
           if (++q_s == NQ) {
             q_s = 0;
             q_ph ^= 1;
@@ -258,19 +259,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         const int kt = w.kt();
         mbar_wait(&kv_empty[kv_s], kv_ph, wctx);
-        mbar_expect_tx(&kv_full[kv_s], 2 * Cfg::TILE + 512);
-        tma_load_5d(smem + Cfg::OFF_K + kv_s * Cfg::TILE, &tmK, &kv_full[kv_s], 0, kt * 128, h, o, b);
-        tma_load_5d(smem + Cfg::OFF_V + kv_s * Cfg::TILE, &tmV, &kv_full[kv_s], 0, kt * 128, h, o, b);
-        tma_load_3d(smem + Cfg::OFF_MASK + kv_s * 512, &tmMask, &kv_full[kv_s], kt * 128, o, b);
+        mbar_expect_tx(el, &kv_full[kv_s], 2 * Cfg::TILE + 512);
+        tma_load_5d(el, smem + Cfg::OFF_K + kv_s * Cfg::TILE, &tmK, &kv_full[kv_s], 0, kt * 128, h, o, b);
+        tma_load_5d(el, smem + Cfg::OFF_V + kv_s * Cfg::TILE, &tmV, &kv_full[kv_s], 0, kt * 128, h, o, b);
+        tma_load_3d(el, smem + Cfg::OFF_MASK + kv_s * 512, &tmMask, &kv_full[kv_s], kt * 128, o, b);
         if (++kv_s == NKV) {
           kv_s = 0;
           kv_ph ^= 1;
         }
         const int bb = p.bias_broadcast ? 0 : b;
         mbar_wait(&b_empty[b_s], b_ph, wctx);
-        mbar_expect_tx(&b_full[b_s], Cfg::BIAS_STAGE);
-        tma_load_4d(smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], kt * 128, w.qt * 128, h, bb);
-        tma_load_4d(smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE + 16384, &tmBias, &b_full[b_s], kt * 128 + 64,
+        mbar_expect_tx(el, &b_full[b_s], Cfg::BIAS_STAGE);
+        tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], kt * 128, w.qt * 128, h, bb);
+        tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE + 16384, &tmBias, &b_full[b_s], kt * 128 + 64,
                     w.qt * 128, h, bb);
         if (++b_s == NB) {
           b_s = 0;
@@ -280,7 +281,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == Cfg::WARP_MMA) {
     // ------------------------------------------------------------------ UMMA issuer
-    if (lane == 0) {
+    {
+      const uint32_t el = elect_one();
       constexpr uint32_t idesc_sd = make_idesc_bf16(128, 128, false, false);  // S, dP
       constexpr uint32_t idesc_kv = make_idesc_bf16(128, D, true, true);      // dV, dK
       constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, false, true);     // dQ
@@ -318,11 +320,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint64_t qo = aq_s * kTile16, ko = akv_s * kTile16;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
-          umma_ss(tmem_base + Cfg::TM_S, dq_k + qo + 2 * ks, dk_k + ko + 2 * ks, idesc_sd, ks != 0);
+          umma_ss(el, tmem_base + Cfg::TM_S, dq_k + qo + 2 * ks, dk_k + ko + 2 * ks, idesc_sd, ks != 0);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
-          umma_ss(tmem_base + Cfg::TM_DP, ddo_k + qo + 2 * ks, dv_k + ko + 2 * ks, idesc_sd, ks != 0);
-        umma_commit(sdp_full);
+          umma_ss(el, tmem_base + Cfg::TM_DP, ddo_k + qo + 2 * ks, dv_k + ko + 2 * ks, idesc_sd, ks != 0);
+        umma_commit(el, sdp_full);
         if (++akv_s == NKV) {
           akv_s = 0;
           akv_ph ^= 1;
@@ -354,25 +356,25 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // dV(kt) (+)= P^T dO ; dK(kt) (+)= dS^T Q   (16 queries per step)
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_ss(tmem_base + Cfg::TM_DV + wb.kk * D, dp_mn + (uint64_t)(ks * 128), ddo_mn + qo + (uint64_t)(ks * Cfg::SWZ),
+          umma_ss(el, tmem_base + Cfg::TM_DV + wb.kk * D, dp_mn + (uint64_t)(ks * 128), ddo_mn + qo + (uint64_t)(ks * Cfg::SWZ),
                   idesc_kv, (ks != 0) ? 1u : acc_kv);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_ss(tmem_base + Cfg::TM_DK + wb.kk * D, dds_mn + (uint64_t)(ks * 128), dq_mn + qo + (uint64_t)(ks * Cfg::SWZ),
+          umma_ss(el, tmem_base + Cfg::TM_DK + wb.kk * D, dds_mn + (uint64_t)(ks * 128), dq_mn + qo + (uint64_t)(ks * Cfg::SWZ),
                   idesc_kv, (ks != 0) ? 1u : acc_kv);
         // dQ(qt) (+)= dS K   (16 keys per step)
         const uint32_t acc_q = wb.first_kk() ? 0u : 1u;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_ss(tmem_base + Cfg::TM_DQ, dds_k + (uint64_t)((ks >> 2) * 1024 + (ks & 3) * 2),
+          umma_ss(el, tmem_base + Cfg::TM_DQ, dds_k + (uint64_t)((ks >> 2) * 1024 + (ks & 3) * 2),
                   dk_mn + ko + (uint64_t)(ks * Cfg::SWZ), idesc_dq, (ks != 0) ? 1u : acc_q);
-        umma_commit(pds_free);
-        umma_commit(&kv_empty[bkv_s]);
+        umma_commit(el, pds_free);
+        umma_commit(el, &kv_empty[bkv_s]);
         if (++bkv_s == NKV) bkv_s = 0;
         const bool last_kk = wb.last_kk();
         const bool strip_done = last_kk && wb.last_qt();
         if (last_kk) {
-          umma_commit(&q_empty[bq_s]);
+          umma_commit(el, &q_empty[bq_s]);
           if (++bq_s == NQ) bq_s = 0;
         }
         (void)strip_done;  // the compute warps learn of a finished strip from pds_free of its last tile
@@ -774,23 +776,24 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == WARP_TMA) {
-    if (lane == 0) {
-      mbar_expect_tx(bias_full, 32768);
-      tma_load_4d(bias_stage, &tmBias, bias_full, kt * 128, qt * 128, h, g);
-      tma_load_4d(bias_stage + 16384, &tmBias, bias_full, kt * 128 + 64, qt * 128, h, g);
+    {
+      const uint32_t el = elect_one();
+      mbar_expect_tx(el, bias_full, 32768);
+      tma_load_4d(el, bias_stage, &tmBias, bias_full, kt * 128, qt * 128, h, g);
+      tma_load_4d(el, bias_stage + 16384, &tmBias, bias_full, kt * 128 + 64, qt * 128, h, g);
       int s = 0;
       uint32_t ph = 1;
       for (int pl = pl0; pl < pl1; ++pl) {
         const int b = g * b_per_g + pl / p.O, o = pl % p.O;
         if (pl - pl0 == NST - 1) mbar_wait(bias_done, 0, wctx);  // first use of the buffer the bias was staged in
         mbar_wait(&empty[s], ph, wctx);
-        mbar_expect_tx(&full[s], 4 * Cfg::TILE + 512);
+        mbar_expect_tx(el, &full[s], 4 * Cfg::TILE + 512);
         uint8_t* st = smem + Cfg::OFF_ST + s * Cfg::STAGE;
-        tma_load_5d(st, &tmQ, &full[s], 0, qt * 128, h, o, b);
-        tma_load_5d(st + Cfg::TILE, &tmDO, &full[s], 0, qt * 128, h, o, b);
-        tma_load_5d(st + 2 * Cfg::TILE, &tmK, &full[s], 0, kt * 128, h, o, b);
-        tma_load_5d(st + 3 * Cfg::TILE, &tmV, &full[s], 0, kt * 128, h, o, b);
-        tma_load_3d(st + 4 * Cfg::TILE, &tmMask, &full[s], kt * 128, o, b);
+        tma_load_5d(el, st, &tmQ, &full[s], 0, qt * 128, h, o, b);
+        tma_load_5d(el, st + Cfg::TILE, &tmDO, &full[s], 0, qt * 128, h, o, b);
+        tma_load_5d(el, st + 2 * Cfg::TILE, &tmK, &full[s], 0, kt * 128, h, o, b);
+        tma_load_5d(el, st + 3 * Cfg::TILE, &tmV, &full[s], 0, kt * 128, h, o, b);
+        tma_load_3d(el, st + 4 * Cfg::TILE, &tmMask, &full[s], kt * 128, o, b);
         if (++s == NST) {
           s = 0;
           ph ^= 1;
@@ -798,7 +801,8 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
     }
   } else if (warp == WARP_MMA) {
-    if (lane == 0) {
+    {
+      const uint32_t el = elect_one();
       constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, false);
       constexpr uint32_t swz = swizzle_mode_for_bytes(Cfg::SWZ);
       int s = 0, buf = 0;
@@ -810,14 +814,14 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         const uint32_t st = smem_u32(smem + Cfg::OFF_ST + s * Cfg::STAGE);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
-          umma_ss(tmem_base + buf * 256, make_smem_desc(st + ks * 32, 16, 8 * Cfg::SWZ, swz),
+          umma_ss(el, tmem_base + buf * 256, make_smem_desc(st + ks * 32, 16, 8 * Cfg::SWZ, swz),
                   make_smem_desc(st + 2 * Cfg::TILE + ks * 32, 16, 8 * Cfg::SWZ, swz), idesc, ks != 0);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
-          umma_ss(tmem_base + buf * 256 + 128, make_smem_desc(st + Cfg::TILE + ks * 32, 16, 8 * Cfg::SWZ, swz),
+          umma_ss(el, tmem_base + buf * 256 + 128, make_smem_desc(st + Cfg::TILE + ks * 32, 16, 8 * Cfg::SWZ, swz),
                   make_smem_desc(st + 3 * Cfg::TILE + ks * 32, 16, 8 * Cfg::SWZ, swz), idesc, ks != 0);
-        umma_commit(&sdp_full[buf]);
-        umma_commit(&empty[s]);
+        umma_commit(el, &sdp_full[buf]);
+        umma_commit(el, &empty[s]);
         buf ^= 1;
         if (++s == NST) {
           s = 0;

@@ -185,7 +185,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // Ring order K(0) V(0) K(1) V(1) ...: a K slot is free again once its Q K^T has run (early in the
     // tile), a V slot once its P V has run (end of the tile), so three slots keep K one tile and V
     // two tiles ahead.  The mask row of a tile arrives on the barrier of its K tile.
-    if (lane == 0) {
+    {
+      const uint32_t el = elect_one();
       uint32_t q_ph = 1;
       int kv_s = 0, b_s = 0, m_s = 0;
       uint32_t kv_ph = 1, b_ph = 1;
@@ -196,28 +197,28 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int bb = p.bias_broadcast ? 0 : b;
         mbar_wait(q_empty, q_ph, wctx);
         q_ph ^= 1;
-        mbar_expect_tx(q_full, Cfg::Q_TILE);
-        tma_load_5d(smem + Cfg::OFF_Q, &tmQ, q_full, 0, qt * 128, h, o, b);
+        mbar_expect_tx(el, q_full, Cfg::Q_TILE);
+        tma_load_5d(el, smem + Cfg::OFF_Q, &tmQ, q_full, 0, qt * 128, h, o, b);
         for (int j = 0; j < KT; ++j) {
           mbar_wait(&kv_empty[kv_s], kv_ph, wctx);
-          mbar_expect_tx(&kv_full[kv_s], Cfg::KV_TILE + 256);
-          tma_load_5d(smem + Cfg::OFF_KV + kv_s * Cfg::KV_TILE, &tmK, &kv_full[kv_s], 0, j * KEYS, h, o, b);
-          tma_load_3d(smem + Cfg::OFF_MASK + m_s * 256, &tmMask, &kv_full[kv_s], j * KEYS, o, b);
+          mbar_expect_tx(el, &kv_full[kv_s], Cfg::KV_TILE + 256);
+          tma_load_5d(el, smem + Cfg::OFF_KV + kv_s * Cfg::KV_TILE, &tmK, &kv_full[kv_s], 0, j * KEYS, h, o, b);
+          tma_load_3d(el, smem + Cfg::OFF_MASK + m_s * 256, &tmMask, &kv_full[kv_s], j * KEYS, o, b);
           m_s = (m_s + 1) & (NMASK - 1);
           if (++kv_s == NKV) {
             kv_s = 0;
             kv_ph ^= 1;
           }
           mbar_wait(&b_empty[b_s], b_ph, wctx);
-          mbar_expect_tx(&b_full[b_s], Cfg::BIAS_STAGE);
-          tma_load_4d(smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], j * KEYS, qt * 128, h, bb);
+          mbar_expect_tx(el, &b_full[b_s], Cfg::BIAS_STAGE);
+          tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], j * KEYS, qt * 128, h, bb);
           if (++b_s == NB) {
             b_s = 0;
             b_ph ^= 1;
           }
           mbar_wait(&kv_empty[kv_s], kv_ph, wctx);
-          mbar_expect_tx(&kv_full[kv_s], Cfg::KV_TILE);
-          tma_load_5d(smem + Cfg::OFF_KV + kv_s * Cfg::KV_TILE, &tmV, &kv_full[kv_s], 0, j * KEYS, h, o, b);
+          mbar_expect_tx(el, &kv_full[kv_s], Cfg::KV_TILE);
+          tma_load_5d(el, smem + Cfg::OFF_KV + kv_s * Cfg::KV_TILE, &tmV, &kv_full[kv_s], 0, j * KEYS, h, o, b);
           if (++kv_s == NKV) {
             kv_s = 0;
             kv_ph ^= 1;
@@ -227,7 +228,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == Cfg::WARP_MMA) {
     // ------------------------------------------------------------------ UMMA issuer
-    if (lane == 0) {
+    {
+      const uint32_t el = elect_one();
       constexpr uint32_t idesc_qk = make_idesc_bf16(128, KEYS, false, false);
       constexpr uint32_t idesc_pv = make_idesc_bf16(128, D, false, true);
       constexpr uint32_t swz = swizzle_mode_for_bytes(Cfg::SWZ);
@@ -255,10 +257,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint64_t kd = k_desc0 + (uint64_t)((k_s * Cfg::KV_TILE) >> 4);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
-          umma_ss(tmem_base + Cfg::TM_S, q_desc0 + 2 * ks, kd + 2 * ks, idesc_qk, ks != 0);
-        umma_commit(s_full);
-        umma_commit(&kv_empty[k_s]);
-        if (last) umma_commit(q_empty);
+          umma_ss(el, tmem_base + Cfg::TM_S, q_desc0 + 2 * ks, kd + 2 * ks, idesc_qk, ks != 0);
+        umma_commit(el, s_full);
+        umma_commit(el, &kv_empty[k_s]);
+        if (last) umma_commit(el, q_empty);
         advance2(k_s, k_ph);
       };
 
@@ -286,10 +288,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const uint64_t vd = v_desc0 + (uint64_t)((v_s * Cfg::KV_TILE) >> 4);
 #pragma unroll
           for (int ks = 0; ks < KEYS / 16; ++ks)  // 16 keys per step; A = P from TMEM (8 columns of bf16 pairs)
-            umma_ts(tmem_base + Cfg::TM_O, tmem_base + Cfg::TM_P + 8 * ks, vd + (uint64_t)(ks * Cfg::SWZ), idesc_pv,
+            umma_ts(el, tmem_base + Cfg::TM_O, tmem_base + Cfg::TM_P + 8 * ks, vd + (uint64_t)(ks * Cfg::SWZ), idesc_pv,
                     (ks | j) != 0);
-          umma_commit(pv_done);
-          umma_commit(&kv_empty[v_s]);
+          umma_commit(el, pv_done);
+          umma_commit(el, &kv_empty[v_s]);
           advance2(v_s, v_ph);
         }
       }

@@ -3,8 +3,9 @@
 //   D[b][m][n] = sum_k A[b][m][k] * B[b][n][k]        (bf16 x bf16 -> fp32 in TMEM)
 //
 // One CTA per SM walks a static list of (batch, m-tile, n-tile) output tiles.
-//   warp 0      : TMA producer  (one elected lane) - STAGES-deep smem ring
-//   warp 1      : UMMA issuer   (one elected lane) - accumulators double-buffered in TMEM
+//   warp 0      : TMA producer - STAGES-deep smem ring
+//   warp 1      : UMMA issuer - accumulators double-buffered in TMEM
+//   (both run converged and issue through one elected lane, see elect_one)
 //   warps 2..   : epilogue      (8 or 16 warps: two or four per 32 TMEM lanes = rows; they
 //                               interleave 32-column chunks)
 // Either operand may be K-major (k contiguous in memory) or MN-major (m / n
@@ -253,24 +254,25 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    {
+      const uint32_t el = elect_one();
       // one k-block of an operand tile -> dst (the swizzled canonical layout the UMMA descriptors describe)
       auto load_a = [&](uint8_t* dst, uint64_t* bar, int k0, int m0, int bc) {
         if constexpr (!Cfg::A_MN) {
-          tma_load_3d(dst, &tmA, bar, k0, m0, bc);
+          tma_load_3d(el, dst, &tmA, bar, k0, m0, bc);
         } else {
 #pragma unroll
           for (int c = 0; c < Cfg::BM / Cfg::CHUNK_A; ++c)
-            tma_load_3d(dst + c * Cfg::BK * Cfg::SWZ_A, &tmA, bar, m0 + c * Cfg::CHUNK_A, k0, bc);
+            tma_load_3d(el, dst + c * Cfg::BK * Cfg::SWZ_A, &tmA, bar, m0 + c * Cfg::CHUNK_A, k0, bc);
         }
       };
       auto load_b = [&](uint8_t* dst, uint64_t* bar, int k0, int n0, int bc) {
         if constexpr (!Cfg::B_MN) {
-          tma_load_3d(dst, &tmB, bar, k0, n0, bc);
+          tma_load_3d(el, dst, &tmB, bar, k0, n0, bc);
         } else {
 #pragma unroll
           for (int c = 0; c < Cfg::BN / Cfg::CHUNK_B; ++c)
-            tma_load_3d(dst + c * Cfg::BK * Cfg::SWZ_B, &tmB, bar, n0 + c * Cfg::CHUNK_B, k0, bc);
+            tma_load_3d(el, dst + c * Cfg::BK * Cfg::SWZ_B, &tmB, bar, n0 + c * Cfg::CHUNK_B, k0, bc);
         }
       };
       int s = 0;
@@ -289,7 +291,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               free_ph ^= 1;
             }
             cur_key = key;
-            mbar_expect_tx(st_full, kb_count * (Cfg::STAT == 1 ? Cfg::A_BYTES : Cfg::B_BYTES));
+            mbar_expect_tx(el, st_full, kb_count * (Cfg::STAT == 1 ? Cfg::A_BYTES : Cfg::B_BYTES));
             for (int kb = 0; kb < kb_count; ++kb) {
               if constexpr (Cfg::STAT == 1) load_a(st_buf + kb * Cfg::A_BYTES, st_full, kbase + kb * Cfg::BK, m0, bc);
               else load_b(st_buf + kb * Cfg::B_BYTES, st_full, kbase + kb * Cfg::BK, n0, bc);
@@ -298,7 +300,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         for (int kb = 0; kb < kb_count; ++kb) {
           mbar_wait(&empty[s], ph, wctx);
-          mbar_expect_tx(&full[s], Cfg::STAGE_BYTES);
+          mbar_expect_tx(el, &full[s], Cfg::STAGE_BYTES);
           const int k0 = kbase + kb * Cfg::BK;
           uint8_t* stage = ring + s * Cfg::STAGE_BYTES;
           if constexpr (Cfg::STAT != 1) load_a(stage, &full[s], k0, m0, bc);
@@ -311,7 +313,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t el = elect_one();
       constexpr uint32_t idesc = make_idesc_bf16(Cfg::BM, Cfg::BN, Cfg::A_MN, Cfg::B_MN);
       constexpr uint32_t sw_a = swizzle_mode_for_bytes(Cfg::SWZ_A);
       constexpr uint32_t sw_b = swizzle_mode_for_bytes(Cfg::SWZ_B);
@@ -328,15 +331,6 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int cur_key = -1;
       uint32_t stat_ph = 0;
       TileWalk<Cfg> w = walk;
-      // A barrier probe by this thread takes a few hundred cycles to answer even when the phase completed long
-      // ago (its shared-memory operations queue behind the epilogue warps'), so every barrier is probed one step
-      // early: the answer arrives while the UMMAs of the step before are being issued, and the blocking wait is
-      // only the fallback.
-      bool full_ready = false, acc_ready = false;
-      if (w.count > 0) {
-        acc_ready = mbar_test_wait(&tempty[0], 1);
-        full_ready = mbar_test_wait(&full[0], 0);
-      }
       for (int i = 0; i < w.count; ++i) {
         const int n0 = w.n0(), key = w.key();
         if constexpr (Cfg::STAT != 0) {
@@ -346,13 +340,13 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             cur_key = key;
           }
         }
-        if (!acc_ready) mbar_wait(&tempty[acc], acc_ph, wctx);
+        mbar_wait(&tempty[acc], acc_ph, wctx);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_STRIDE;
         bool swap = false;
         if constexpr (kCanSwap) swap = Epi::swapped(ep, n0);
         for (int kb = 0; kb < kb_count; ++kb) {
-          if (!full_ready) mbar_wait(&full[s], ph, wctx);
+          mbar_wait(&full[s], ph, wctx);
           tc_fence_after();
           // descriptors = a base descriptor + (byte offset >> 4) in the start-address field (no carry out of it:
           // shared memory is far smaller than the field's range)
@@ -360,43 +354,34 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const uint32_t b_off = Cfg::STAT == 2 ? kb * Cfg::B_BYTES : Cfg::STAT_BYTES + s * Cfg::STAGE_BYTES + Cfg::STAGE_A;
           const uint64_t ad0 = a_desc0 + (a_off >> 4);
           const uint64_t bd0 = b_desc0 + (b_off >> 4);
-          // probed while the UMMAs go out: the stage after this one (it may belong to the next tile) and the
-          // accumulator the next tile will use
-          const int sn = s + 1 == Cfg::STAGES ? 0 : s + 1;
-          const uint32_t phn = s + 1 == Cfg::STAGES ? ph ^ 1 : ph;
-          const uint32_t acc_phn = acc == 1 ? acc_ph ^ 1 : acc_ph;
           constexpr int A_STEP = Cfg::A_MN ? (16 * Cfg::SWZ_A >> 4) : 2;
           constexpr int B_STEP = Cfg::B_MN ? (16 * Cfg::SWZ_B >> 4) : 2;
-          uint32_t probes = 0;
           bool swapped_now = false;
           if constexpr (kCanSwap) swapped_now = swap;
-          if constexpr (Cfg::BK != 64) {
-            // narrow swizzle modes (small K): fewer UMMAs per k-block, plain issue, blocking waits
-#pragma unroll
-            for (int j = 0; j < Cfg::BK / 16; ++j)
-              umma_ss(d_tmem, ad0 + j * A_STEP, bd0 + j * B_STEP, idesc, (kb | j) != 0 ? 1u : 0u);
-            umma_commit(&empty[s]);
-          } else if (swapped_now) {
+          if (swapped_now) {
             // Operand roles exchanged: the two 128-row halves of the B tile are the M operands of two UMMAs
             // that share the A tile as their N operand.  Accumulator lane = row of the B tile (an output
             // column of the problem), accumulator column = row of the A tile; the first half's product sits
             // in columns [0, BM), the second half's in [BN / 2, BN / 2 + BM).
             constexpr uint32_t idesc_sw = make_idesc_bf16(128, Cfg::BM, false, false);
-            probes = umma_ss_x4x2_probed<2, (128 * Cfg::SWZ_B >> 4)>(d_tmem, d_tmem + Cfg::BN / 2, bd0, ad0, idesc_sw,
-                                                                    kb != 0 ? 1u : 0u, &empty[s], &full[sn], phn,
-                                                                    &tempty[acc ^ 1], acc_phn);
+#pragma unroll
+            for (int j = 0; j < Cfg::BK / 16; ++j) {
+              umma_ss(el, d_tmem, bd0 + j * B_STEP, ad0 + j * A_STEP, idesc_sw, (kb | j) != 0 ? 1u : 0u);
+              umma_ss(el, d_tmem + Cfg::BN / 2, bd0 + (128 * Cfg::SWZ_B >> 4) + j * B_STEP, ad0 + j * A_STEP, idesc_sw,
+                      (kb | j) != 0 ? 1u : 0u);
+            }
           } else {
-            probes = umma_ss_x4_probed<A_STEP, B_STEP>(d_tmem, ad0, bd0, idesc, kb != 0 ? 1u : 0u, &empty[s], &full[sn],
-                                                       phn, &tempty[acc ^ 1], acc_phn);
+#pragma unroll
+            for (int j = 0; j < Cfg::BK / 16; ++j)
+              umma_ss(el, d_tmem, ad0 + j * A_STEP, bd0 + j * B_STEP, idesc, (kb | j) != 0 ? 1u : 0u);
           }
-          full_ready = (kb + 1 < kb_count || i + 1 < w.count) && (probes & 1u);
-          if (kb + 1 == kb_count) acc_ready = i + 1 < w.count && (probes & 2u);
+          umma_commit(el, &empty[s]);
           if (++s == Cfg::STAGES) {
             s = 0;
             ph ^= 1;
           }
         }
-        umma_commit(&tfull[acc]);
+        umma_commit(el, &tfull[acc]);
         if (++acc == 2) {
           acc = 0;
           acc_ph ^= 1;
@@ -404,7 +389,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         w.next();
         if constexpr (Cfg::STAT != 0) {
           // end of a run: the buffer may be overwritten once everything issued so far has completed
-          if (i + 1 == w.count || w.key() != cur_key) umma_commit(st_free);
+          if (i + 1 == w.count || w.key() != cur_key) umma_commit(el, st_free);
         }
       }
     }
