@@ -1172,16 +1172,25 @@ int launch_attn_dbias(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   return TPF_OK;
 }
 
-// How the outer planes of one dBias tile are split into independent chunks.
+// How the outer planes of one dBias tile are split into independent chunks: the split with the shortest schedule, i.e.
+// waves of CTAs (one per SM) times planes per CTA, plus about three planes' time for a CTA's start and its partial
+// plane.  With one chunk whenever there are more tiles than SMs (N = 1021: 256 tiles) the last wave left half the
+// machine idle.
 static void dbias_plan(int64_t B, int64_t O, int64_t H, int64_t N, int64_t G, int* n_chunks, int* chunk_len) {
   const int64_t tiles = G * H * ((N + 127) / 128) * ((N + 127) / 128);
   const int64_t planes = (B / G) * O;
-  int64_t c = sm_count() / tiles;
-  if (c < 1) c = 1;
-  if (c > planes) c = planes;
-  const int64_t len = (planes + c - 1) / c;
-  c = (planes + len - 1) / len;
-  *n_chunks = (int)c;
+  const int64_t sms = sm_count();
+  int64_t best = 0, best_cost = 0;
+  for (int64_t c = 1; c <= planes && (c == 1 || tiles * c <= 8 * sms); ++c) {
+    const int64_t len = (planes + c - 1) / c;
+    const int64_t cost = (tiles * c + sms - 1) / sms * (len + 3);
+    if (best == 0 || cost < best_cost) {
+      best = c;
+      best_cost = cost;
+    }
+  }
+  const int64_t len = (planes + best - 1) / best;
+  *n_chunks = (int)((planes + len - 1) / len);
   *chunk_len = (int)len;
 }
 

@@ -8,20 +8,26 @@
 // same math and rounding points (fp32 running max / sum, probabilities rounded to bf16 for P V,
 // fully masked rows give out = 0 and lse = -inf), different machine mapping:
 //
-//  * A work item is one (b, o, h, 128-query tile); a CTA walks its items and, inside an item, the
-//    64-key tiles.  CTAs are small (6 warps, about 55 KB of shared memory, 128 TMEM columns and about
-//    70 registers per thread at D <= 32) so that FOUR of them are resident per SM: the latency of a
-//    barrier hand-off, a TMA load or an MMA of one CTA is covered by the arithmetic of the others, and
-//    the FMA / ALU work (bias add, maximum) of one overlaps the MUFU work (exponentials) of another.
-//  * warps 0-3: softmax warps, one thread per query row (= TMEM lane).  warp 4: TMA producer.
-//    warp 5: UMMA issuer.
-//  * Q K^T runs on tcgen05 with S in TMEM.  The softmax warps walk a tile 16 columns at a time straight
-//    from TMEM (one pass: bias add, running maximum, exponentials, row sum).  The bf16 probabilities go
-//    back to TMEM (not to shared memory) and P V is issued with its A operand in TMEM; O accumulates
-//    in TMEM across key tiles.  The reference maximum of a row is raised - and the row's partial
-//    results rescaled - only when a chunk exceeds it by more than a fixed gap.
-//  * A tile whose mask row is all zero and that has no ragged key tail (the common case) takes a
-//    code path without the mask add.
+//  * A work item is one (b, o, h, 128-query tile); a CTA walks its items and, inside an item, the 64-key tiles.
+//    Three CTAs (two at D = 64) of five warps share an SM: four softmax warps with one thread per query row
+//    (= TMEM lane), and one warp that issues every TMA load and UMMA.
+//  * A softmax thread holds the 64 logits of its row in registers: one pass of TMEM loads (after which Q K^T of a later
+//    tile may use the buffer), bias add, maximum, exponentials, row sum.  What bounds the kernel is the length of that
+//    instruction stream (about 440 instructions per tile and warp against 64 exponentials; the MUFU pipe is half busy)
+//    so it carries no bookkeeping: S and P are double-buffered, and the issuing warp needs no "empty" barriers (see
+//    there).  The bf16 probabilities overwrite their S buffer in TMEM and P V takes them as its A operand; O accumulates
+//    in TMEM across key tiles.
+//  * The reference maximum of a row is raised - and the row's partial results rescaled - only when a tile exceeds
+//    it by more than a fixed gap.
+//  * The finished row of an item is normalised, gated and stored under the next item's first tile, when its last P V
+//    has long completed.
+//  * Items are numbered with the query tile fastest: CTAs running at the same time share K and V of an outer row (and
+//    each bias strip stays in L2 anyway).  With the outer row fastest K and V came from DRAM once per query tile.
+//  * A tile whose mask row is all zero and that has no ragged key tail (the common case) skips the mask add; warps
+//    whose 32 query rows lie beyond N, and the second half of a key tile with at most 32 keys, are skipped.
+//
+// Measured (B200, H = 4, D = 32, cold L2): N = 384 119 us (142 us before: four CTAs of six warps, 16 logits at a time,
+// roles issued by one lane), N = 768 789 us (977), N = 1021 1.82 ms (2.27); D = 64, N = 257 86 us (127).
 #include "tpf_host.cuh"
 #include "tpf_internal.h"
 #include "tpf_ptx.cuh"
@@ -55,82 +61,64 @@ template <int D_>
 struct AttnFwdCfg {
   static constexpr int D = D_;
   static constexpr int KEYS = 64;                // keys per tile
-  static constexpr int CTAS_PER_SM = D <= 32 ? 4 : 2;
+  static constexpr int CTAS_PER_SM = D <= 32 ? 3 : 2;
   static constexpr int SWZ = 2 * D;              // bytes per smem row of a Q/K/V tile
   static constexpr int Q_TILE = 128 * D * 2;
   static constexpr int KV_TILE = KEYS * D * 2;
-  static constexpr int NB = 2;                   // bias stages
-  static constexpr int NKV = 3;                  // slots of the shared K / V ring (K0 V0 K1 V1 ...)
-  static constexpr int NMASK = 4;                // mask-row slots (256 B each)
+  static constexpr int NS = 3;                   // K / mask slots
+  static constexpr int NB = 2;                   // bias / V slots
   static constexpr int BIAS_STAGE = 128 * KEYS * 2;
   static constexpr int OFF_BIAS = 0;
-  static constexpr int OFF_Q = OFF_BIAS + NB * BIAS_STAGE;
-  static constexpr int OFF_KV = OFF_Q + Q_TILE;                  // [NKV]
-  static constexpr int OFF_MASK = OFF_KV + NKV * KV_TILE;        // [NMASK] x 256 B
-  static constexpr int OFF_BAR = OFF_MASK + NMASK * 256;
-  static constexpr int N_BAR = 2 * NB + 2 + 2 * NKV + 4;
-  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
-  static constexpr int TM_S = 0;      // logits, fp32, 64 columns
-  static constexpr int TM_P = 64;     // probabilities, bf16 pairs, 32 columns
-  static constexpr int TM_O = 96;     // output accumulator, fp32, D columns
-  static constexpr int TMEM_COLS = TM_O + D <= 128 ? 128 : 256;
-  static constexpr int THREADS = 192;            // 4 softmax warps, TMA warp, UMMA warp
-  static constexpr int WARP_TMA = 4, WARP_MMA = 5;
+  static constexpr int OFF_Q = OFF_BIAS + NB * BIAS_STAGE;       // [2]
+  static constexpr int OFF_K = OFF_Q + 2 * Q_TILE;               // [NS]
+  static constexpr int OFF_V = OFF_K + NS * KV_TILE;             // [NB]
+  static constexpr int OFF_MASK = OFF_V + NB * KV_TILE;          // [NS] x 256 B
+  static constexpr int OFF_BAR = OFF_MASK + NS * 256;
+  static constexpr int N_BAR = NB + 2 + NS + 6;
+  static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 32 + 1024;
+  // two S buffers (fp32, 64 columns); the bf16 probabilities of a tile overwrite the first 32 columns of its S buffer
+  static constexpr int S_COLS = 128;
+  static constexpr int O_COLS = D <= 32 ? 32 : 64;
+  static constexpr int THREADS = 160;            // 4 softmax warps, one warp that issues TMA loads and UMMAs
+  static constexpr int WARP_MMA = 4;
   static_assert(D == 16 || D == 32 || D == 64, "head dim lanes");
-  static_assert(TMEM_COLS * CTAS_PER_SM <= 512, "TMEM budget");
+  static_assert((S_COLS + O_COLS) * CTAS_PER_SM <= 512, "TMEM budget");
   static_assert((SMEM_BYTES + 1024) * CTAS_PER_SM <= 233472, "shared memory budget");
   static_assert(KV_TILE % 1024 == 0 && Q_TILE % 1024 == 0, "tile buffers keep 1024-byte alignment");
 };
 
-// Softmax is done in ONE pass over each 64-key tile, 16 columns at a time straight out of TMEM, so a
-// thread holds 16 logits at a time instead of a whole row segment (about 70 registers per thread,
-// which is what lets four CTAs share an SM).  The exponentials of a chunk use the row's current
-// reference maximum m; a chunk whose own maximum exceeds m by more than kGap first raises m and
-// rescales what the row has accumulated so far (its sum, the part of P already stored for this tile,
-// and O).  Every exponent argument is therefore bounded by kGap and the result does not depend on
-// how often m was raised: lse = m + log(sum) at the end.
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, Cfg::CTAS_PER_SM)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmBias,
                 const __grid_constant__ CUtensorMap tmMask, const AttnFwdParams p, int* __restrict__ status) {
   griddep_wait();
-  constexpr int D = Cfg::D, NKV = Cfg::NKV, NB = Cfg::NB, NMASK = Cfg::NMASK, KEYS = Cfg::KEYS;
+  constexpr int D = Cfg::D, NS = Cfg::NS, NB = Cfg::NB, KEYS = Cfg::KEYS;
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   uint64_t* b_full = bars;                  // [NB]
-  uint64_t* b_empty = b_full + NB;          // [NB]
-  uint64_t* q_full = b_empty + NB;
-  uint64_t* q_empty = q_full + 1;
-  uint64_t* kv_full = q_empty + 1;          // [NKV]
-  uint64_t* kv_empty = kv_full + NKV;       // [NKV]
-  uint64_t* s_full = kv_empty + NKV;
-  uint64_t* s_free = s_full + 1;
-  uint64_t* p_ready = s_free + 1;
-  uint64_t* pv_done = p_ready + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::N_BAR);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* q_full = b_full + NB;           // [2]
+  uint64_t* k_full = q_full + 2;            // [NS]
+  uint64_t* s_full = k_full + NS;          // [2]
+  uint64_t* p_ready = s_full + 2;           // [2]
+  uint64_t* pv_done = p_ready + 2;          // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::N_BAR);  // S, O
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
   const WaitCtx wctx{abort_flag, status};
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NB; ++s) {
-      mbar_init(&b_full[s], 1);
-      mbar_init(&b_empty[s], 4);
+    for (int s = 0; s < NB; ++s) mbar_init(&b_full[s], 1);
+    for (int s = 0; s < NS; ++s) mbar_init(&k_full[s], 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&q_full[s], 1);
+      mbar_init(&s_full[s], 1);
+      mbar_init(&p_ready[s], 4);
+      mbar_init(&pv_done[s], 1);
     }
-    mbar_init(q_full, 1);
-    mbar_init(q_empty, 1);
-    for (int s = 0; s < NKV; ++s) {
-      mbar_init(&kv_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
-    }
-    mbar_init(s_full, 1);
-    mbar_init(s_free, 4);
-    mbar_init(p_ready, 4);
-    mbar_init(pv_done, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
@@ -140,39 +128,40 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tma_prefetch_desc(&tmMask);
   }
   if (warp == Cfg::WARP_MMA) {
-    tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+    tmem_alloc(tmem_slot, Cfg::S_COLS);
+    tmem_alloc(tmem_slot + 1, Cfg::O_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_s = tmem_slot[0], tmem_o = tmem_slot[1];
 
   const int KT = p.k_tiles;
 
-  // item -> (b, h, qt, o); o fastest so that CTAs running at the same time read the same bias strip.
+  // item -> (b, h, o, qt), the query tile fastest.
   // The coordinates are a mixed-radix counter advanced by the grid size: the divisions happen once, not per
   // item (an integer division by a run-time value costs a warp several hundred cycles on its critical path).
   struct ItemWalk {
-    int o, qt, h, b;      // current item
-    int so, sq, sh, sb;   // the step, decomposed
-    int O, Q, H;
+    int qt, o, h, b;      // current item
+    int sq, so, sh, sb;   // the step, decomposed
+    int Q, O, H;
     __device__ void init(int item, int step, int O_, int Q_, int H_) {
       O = O_; Q = Q_; H = H_;
-      o = item % O; int r = item / O;
-      qt = r % Q; r /= Q;
+      qt = item % Q; int r = item / Q;
+      o = r % O; r /= O;
       h = r % H; b = r / H;
-      so = step % O; r = step / O;
-      sq = r % Q; r /= Q;
+      sq = step % Q; r = step / Q;
+      so = r % O; r /= O;
       sh = r % H; sb = r / H;
     }
     __device__ __forceinline__ void next() {
-      o += so;
-      int c = o >= O ? 1 : 0;
-      o -= c * O;
-      qt += sq + c;
-      c = qt >= Q ? 1 : 0;
+      qt += sq;
+      int c = qt >= Q ? 1 : 0;
       qt -= c * Q;
+      o += so + c;
+      c = o >= O ? 1 : 0;
+      o -= c * O;
       h += sh + c;
       c = h >= H ? 1 : 0;
       h -= c * H;
@@ -180,297 +169,146 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   };
 
-  if (warp == Cfg::WARP_TMA) {
-    // ------------------------------------------------------------------ TMA producer
-    // Ring order K(0) V(0) K(1) V(1) ...: a K slot is free again once its Q K^T has run (early in the
-    // tile), a V slot once its P V has run (end of the tile), so three slots keep K one tile and V
-    // two tiles ahead.  The mask row of a tile arrives on the barrier of its K tile.
-    {
-      const uint32_t el = elect_one();
-      uint32_t q_ph = 1;
-      int kv_s = 0, b_s = 0, m_s = 0;
-      uint32_t kv_ph = 1, b_ph = 1;
-      ItemWalk iw;
-      iw.init(blockIdx.x, gridDim.x, p.O, p.q_tiles, p.H);
-      for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, iw.next()) {
-        const int b = iw.b, h = iw.h, qt = iw.qt, o = iw.o;
-        const int bb = p.bias_broadcast ? 0 : b;
-        mbar_wait(q_empty, q_ph, wctx);
-        q_ph ^= 1;
-        mbar_expect_tx(el, q_full, Cfg::Q_TILE);
-        tma_load_5d(el, smem + Cfg::OFF_Q, &tmQ, q_full, 0, qt * 128, h, o, b);
-        for (int j = 0; j < KT; ++j) {
-          mbar_wait(&kv_empty[kv_s], kv_ph, wctx);
-          mbar_expect_tx(el, &kv_full[kv_s], Cfg::KV_TILE + 256);
-          tma_load_5d(el, smem + Cfg::OFF_KV + kv_s * Cfg::KV_TILE, &tmK, &kv_full[kv_s], 0, j * KEYS, h, o, b);
-          tma_load_3d(el, smem + Cfg::OFF_MASK + m_s * 256, &tmMask, &kv_full[kv_s], j * KEYS, o, b);
-          m_s = (m_s + 1) & (NMASK - 1);
-          if (++kv_s == NKV) {
-            kv_s = 0;
-            kv_ph ^= 1;
-          }
-          mbar_wait(&b_empty[b_s], b_ph, wctx);
-          mbar_expect_tx(el, &b_full[b_s], Cfg::BIAS_STAGE);
-          tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], j * KEYS, qt * 128, h, bb);
-          if (++b_s == NB) {
-            b_s = 0;
-            b_ph ^= 1;
-          }
-          mbar_wait(&kv_empty[kv_s], kv_ph, wctx);
-          mbar_expect_tx(el, &kv_full[kv_s], Cfg::KV_TILE);
-          tma_load_5d(el, smem + Cfg::OFF_KV + kv_s * Cfg::KV_TILE, &tmV, &kv_full[kv_s], 0, j * KEYS, h, o, b);
-          if (++kv_s == NKV) {
-            kv_s = 0;
-            kv_ph ^= 1;
-          }
-        }
-      }
-    }
-  } else if (warp == Cfg::WARP_MMA) {
-    // ------------------------------------------------------------------ UMMA issuer
+  if (warp == Cfg::WARP_MMA) {
+    // ------------------------------------------------------------------ TMA loads and UMMAs
+    // One thread issues both.  p_ready(t) says that the softmax warps have read S, bias and mask of tile t, and the
+    // completion of P V (t) that every buffer of tile t is free: no "empty" barriers are needed.  Q K^T runs two tiles
+    // ahead of P V (its S buffer is free once P V (t), whose P lies in it, is done), K / mask loads run three
+    // tiles ahead, bias and V loads two.
     {
       const uint32_t el = elect_one();
       constexpr uint32_t idesc_qk = make_idesc_bf16(128, KEYS, false, false);
       constexpr uint32_t idesc_pv = make_idesc_bf16(128, D, false, true);
       constexpr uint32_t swz = swizzle_mode_for_bytes(Cfg::SWZ);
-      uint32_t q_ph = 0, sfree_ph = 1, pready_ph = 0;
-      // ring positions of the next K tile and the next V tile (K and V alternate in the ring)
-      int k_s = 0, v_s = 1;
-      uint32_t k_ph = 0, v_ph = 0;
       const uint64_t q_desc0 = make_smem_desc(smem_u32(smem + Cfg::OFF_Q), 16, 8 * Cfg::SWZ, swz);
-      const uint64_t k_desc0 = make_smem_desc(smem_u32(smem + Cfg::OFF_KV), 16, 8 * Cfg::SWZ, swz);
-      const uint64_t v_desc0 = make_smem_desc(smem_u32(smem + Cfg::OFF_KV), KEYS * Cfg::SWZ, 8 * Cfg::SWZ, swz);
-      auto advance2 = [&](int& s, uint32_t& ph) {
-        s += 2;
-        if (s >= NKV) {
-          s -= NKV;
-          ph ^= 1;
+      const uint64_t k_desc0 = make_smem_desc(smem_u32(smem + Cfg::OFF_K), 16, 8 * Cfg::SWZ, swz);
+      const uint64_t v_desc0 = make_smem_desc(smem_u32(smem + Cfg::OFF_V), KEYS * Cfg::SWZ, 8 * Cfg::SWZ, swz);
+      const int my_items = (p.n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+      const int tiles = my_items * KT;
+
+      // K / mask stream (and Q, at an item's first tile)
+      ItemWalk kw;
+      kw.init(blockIdx.x, gridDim.x, p.O, p.q_tiles, p.H);
+      int kj = 0, k_s = 0, kq = 0;
+      auto load_k = [&]() {
+        if (kj == 0) {
+          mbar_expect_tx(el, &q_full[kq], Cfg::Q_TILE);
+          tma_load_5d(el, smem + Cfg::OFF_Q + kq * Cfg::Q_TILE, &tmQ, &q_full[kq], 0, kw.qt * 128, kw.h, kw.o, kw.b);
+          kq ^= 1;
+        }
+        mbar_expect_tx(el, &k_full[k_s], Cfg::KV_TILE + 256);
+        tma_load_5d(el, smem + Cfg::OFF_K + k_s * Cfg::KV_TILE, &tmK, &k_full[k_s], 0, kj * KEYS, kw.h, kw.o, kw.b);
+        tma_load_3d(el, smem + Cfg::OFF_MASK + k_s * 256, &tmMask, &k_full[k_s], kj * KEYS, kw.o, kw.b);
+        if (++k_s == NS) k_s = 0;
+        if (++kj == KT) {
+          kj = 0;
+          kw.next();
         }
       };
-
-      auto issue_qk = [&](bool last) {
-        // s_free: the softmax warps have read the whole previous S tile
-        mbar_wait2(&kv_full[k_s], k_ph, s_free, sfree_ph, wctx);
-        sfree_ph ^= 1;
-        tc_fence_after();
-        // descriptors differ from the hoisted ones only in the start-address field (bits 0-13, in 16-byte units)
-        const uint64_t kd = k_desc0 + (uint64_t)((k_s * Cfg::KV_TILE) >> 4);
+      // bias / V stream
+      ItemWalk bw;
+      bw.init(blockIdx.x, gridDim.x, p.O, p.q_tiles, p.H);
+      int bj = 0, b_s = 0;
+      auto load_bv = [&]() {
+        mbar_expect_tx(el, &b_full[b_s], Cfg::BIAS_STAGE + Cfg::KV_TILE);
+        tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], bj * KEYS, bw.qt * 128, bw.h,
+                    p.bias_broadcast ? 0 : bw.b);
+        tma_load_5d(el, smem + Cfg::OFF_V + b_s * Cfg::KV_TILE, &tmV, &b_full[b_s], 0, bj * KEYS, bw.h, bw.o, bw.b);
+        b_s ^= 1;
+        if (++bj == KT) {
+          bj = 0;
+          bw.next();
+        }
+      };
+      // Q K^T stream
+      int qj = 0, q_s = 0, qk_s = 0, qk_buf = 0;
+      uint32_t q_ph = 0, qk_ph = 0;
+      auto issue_qk = [&]() {
+        if (qj == 0) mbar_wait2(&q_full[q_s], q_ph, &k_full[qk_s], qk_ph, wctx);
+        else mbar_wait(&k_full[qk_s], qk_ph, wctx);
+        const uint64_t qd = q_desc0 + (uint64_t)((q_s * Cfg::Q_TILE) >> 4);
+        const uint64_t kd = k_desc0 + (uint64_t)((qk_s * Cfg::KV_TILE) >> 4);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
-          umma_ss(el, tmem_base + Cfg::TM_S, q_desc0 + 2 * ks, kd + 2 * ks, idesc_qk, ks != 0);
-        umma_commit(el, s_full);
-        umma_commit(el, &kv_empty[k_s]);
-        if (last) umma_commit(el, q_empty);
-        advance2(k_s, k_ph);
+          umma_ss(el, tmem_s + 64 * qk_buf, qd + 2 * ks, kd + 2 * ks, idesc_qk, ks != 0);
+        umma_commit(el, &s_full[qk_buf]);
+        qk_buf ^= 1;
+        if (++qk_s == NS) {
+          qk_s = 0;
+          qk_ph ^= 1;
+        }
+        if (++qj == KT) {
+          qj = 0;
+          q_s ^= 1;
+          if (q_s == 0) q_ph ^= 1;
+        }
       };
 
-      bool first = true;
-      for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
-        if (first) {
-          mbar_wait(q_full, q_ph, wctx);
-          q_ph ^= 1;
-          issue_qk(KT == 1);
-          first = false;
-        }
-        const bool more_items = item + (int)gridDim.x < p.n_items;
-        for (int j = 0; j < KT; ++j) {
-          // Q K^T of the next tile (of this item or of the next one) as soon as S has been read
-          if (j + 1 < KT) {
-            issue_qk(j + 2 == KT);
-          } else if (more_items) {
-            mbar_wait(q_full, q_ph, wctx);
-            q_ph ^= 1;
-            issue_qk(KT == 1);
-          }
-          mbar_wait2(p_ready, pready_ph, &kv_full[v_s], v_ph, wctx);
-          pready_ph ^= 1;
-          tc_fence_after();
-          const uint64_t vd = v_desc0 + (uint64_t)((v_s * Cfg::KV_TILE) >> 4);
+      load_k();
+      load_bv();
+      if (tiles > 1) {
+        load_k();
+        load_bv();
+      }
+      if (tiles > 2) load_k();
+      issue_qk();
+      if (tiles > 1) issue_qk();
+      int j = 0;
+      for (int t = 0; t < tiles; ++t) {
+        const int buf = t & 1;
+        const uint32_t ph = (t >> 1) & 1;
+        mbar_wait(&p_ready[buf], ph, wctx);
+        tc_fence_after();
+        const uint64_t vd = v_desc0 + (uint64_t)((buf * Cfg::KV_TILE) >> 4);
+        // 16 keys per step; A = P from TMEM (8 columns of bf16 pairs).  A tail of at most 32 keys has no P beyond them.
+        const bool half = j + 1 == KT && p.N - j * KEYS <= 32;
 #pragma unroll
-          for (int ks = 0; ks < KEYS / 16; ++ks)  // 16 keys per step; A = P from TMEM (8 columns of bf16 pairs)
-            umma_ts(el, tmem_base + Cfg::TM_O, tmem_base + Cfg::TM_P + 8 * ks, vd + (uint64_t)(ks * Cfg::SWZ), idesc_pv,
-                    (ks | j) != 0);
-          umma_commit(el, pv_done);
-          umma_commit(el, &kv_empty[v_s]);
-          advance2(v_s, v_ph);
+        for (int ks = 0; ks < KEYS / 16; ++ks)
+          if (ks < 2 || !half)
+            umma_ts(el, tmem_o, tmem_s + 64 * buf + 8 * ks, vd + (uint64_t)(ks * Cfg::SWZ), idesc_pv, (ks | j) != 0);
+        umma_commit(el, &pv_done[buf]);
+        if (++j == KT) j = 0;
+        if (t + 2 < tiles) {
+          mbar_wait(&pv_done[buf], ph, wctx);
+          tc_fence_after();
+          issue_qk();
+          load_bv();
+          if (t + 3 < tiles) load_k();
         }
       }
     }
   } else {
     // ------------------------------------------------------------------ softmax warps: one thread per query row
     const int row = 32 * warp + lane;  // query row inside the tile == TMEM lane
-    const uint32_t t_s = tmem_addr(tmem_base, 32 * warp, Cfg::TM_S);
-    const uint32_t t_p = tmem_addr(tmem_base, 32 * warp, Cfg::TM_P);
-    const uint32_t t_o = tmem_addr(tmem_base, 32 * warp, Cfg::TM_O);
+    const uint32_t t_s = tmem_addr(tmem_s, 32 * warp, 0);
+    const uint32_t t_o = tmem_addr(tmem_o, 32 * warp, 0);
     constexpr float kLog2e = 1.4426950408889634f;
     constexpr float kLn2 = 0.6931471805599453f;
     constexpr float kGap = 12.0f;  // largest exponent (natural units) a probability may have relative to m
     const uint64_t scale2 = f2_pack(p.scale, p.scale);
     const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
 
-    uint32_t sfull_ph = 0, pv_ph = 0, b_ph = 0;
-    int b_s = 0, m_s = 0;
-
-    ItemWalk iw;
-    iw.init(blockIdx.x, gridDim.x, p.O, p.q_tiles, p.H);
-    for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, iw.next()) {
-      const int b = iw.b, h = iw.h, qt = iw.qt, o = iw.o;
-      float m_use = -INFINITY, l_run = 0.f;
-
-      for (int j = 0; j < KT; ++j) {
-        // s_full completes after Q K^T of this tile, hence after the K tile and the mask row that
-        // arrives on the same barrier have landed
-        mbar_wait(s_full, sfull_ph, wctx);
-        sfull_ph ^= 1;
-        const float* mask_row = reinterpret_cast<const float*>(smem + Cfg::OFF_MASK + m_s * 256);
-        m_s = (m_s + 1) & (NMASK - 1);
-        const bool tail = (j + 1) * KEYS > p.N;
-        const float2 mprobe = *reinterpret_cast<const float2*>(mask_row + 2 * lane);
-        const bool general = tail || __any_sync(0xffffffffu, (mprobe.x != 0.f) || (mprobe.y != 0.f));
-        const uint8_t* bias_row = smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE + row * 128;
-        if (j > 0) {
-          // P V of the previous tile must be complete before P is overwritten or O is rescaled (it was
-          // issued a whole tile ago)
-          mbar_wait2(&b_full[b_s], b_ph, pv_done, pv_ph, wctx);
-          pv_ph ^= 1;
-        } else {
-          mbar_wait(&b_full[b_s], b_ph, wctx);
-        }
-        tc_fence_after();
-        float neg_m = (m_use == -INFINITY) ? 0.f : -m_use * kLog2e;
-        uint64_t rs2 = 0ull;  // packed partial row sum of this tile
-
-#pragma unroll
-        for (int c = 0; c < KEYS / 16; ++c) {  // 16 key columns per step
-          uint32_t raw[16];
-          tmem_ld16(t_s + 16 * c, raw);
-          const uint4 bv0 = *reinterpret_cast<const uint4*>(bias_row + (((2 * c) ^ (row & 7)) << 4));
-          const uint4 bv1 = *reinterpret_cast<const uint4*>(bias_row + (((2 * c + 1) ^ (row & 7)) << 4));
-          tmem_ld_wait();
-          if (c == KEYS / 16 - 1) {
-            // the whole S tile and bias tile have been read: the next Q K^T / bias load may overwrite them
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-              mbar_arrive(s_free);
-              mbar_arrive(&b_empty[b_s]);
-            }
-          }
-          const uint32_t bw[8] = {bv0.x, bv0.y, bv0.z, bv0.w, bv1.x, bv1.y, bv1.z, bv1.w};
-          uint64_t v2[8];
-          float cmax0 = -INFINITY, cmax1 = -INFINITY;
-          if (!general) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const uint64_t b2 = f2_pack_bits(bw[e] << 16, bw[e] & 0xFFFF0000u);
-              v2[e] = f2_fma(f2_pack_bits(raw[2 * e], raw[2 * e + 1]), scale2, b2);
-              float v0, v1;
-              f2_unpack(v2[e], v0, v1);
-              if (e & 1) cmax1 = max3(cmax1, v0, v1);
-              else cmax0 = max3(cmax0, v0, v1);
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const uint64_t b2 = f2_pack_bits(bw[e] << 16, bw[e] & 0xFFFF0000u);
-              const float2 mk = *reinterpret_cast<const float2*>(mask_row + 16 * c + 2 * e);
-              float v0, v1;
-              f2_unpack(f2_add(f2_fma(f2_pack_bits(raw[2 * e], raw[2 * e + 1]), scale2, b2), f2_pack(mk.x, mk.y)), v0,
-                        v1);
-              if (tail) {
-                const int k0 = j * KEYS + 16 * c + 2 * e;
-                if (k0 >= p.N) v0 = -INFINITY;
-                if (k0 + 1 >= p.N) v1 = -INFINITY;
-              }
-              v2[e] = f2_pack(v0, v1);
-              if (e & 1) cmax1 = max3(cmax1, v0, v1);
-              else cmax0 = max3(cmax0, v0, v1);
-            }
-          }
-          const float cmax = fmaxf(cmax0, cmax1);
-          if (__any_sync(0xffffffffu, cmax > m_use + kGap)) {
-            // Raise the reference maximum of the rows that need it (f = 1 for the others) and rescale what
-            // those rows have accumulated.  Runs for the first finite chunk of every row and then only
-            // when the logits of a row grow by more than kGap.
-            const bool grow = cmax > m_use + kGap;
-            const float f = grow ? ex2_approx((m_use - cmax) * kLog2e) : 1.f;  // m_use = -inf gives 0; nothing accumulated then
-            if (grow) m_use = cmax;
-            neg_m = (m_use == -INFINITY) ? 0.f : -m_use * kLog2e;
-            l_run *= f;
-            {
-              float r0, r1;
-              f2_unpack(rs2, r0, r1);
-              rs2 = f2_pack(r0 * f, r1 * f);
-            }
-            if (c > 0) tmem_st_wait();
-#pragma unroll
-            for (int cc = 0; cc < KEYS / 16; ++cc) {
-              if (cc < c) {  // part of P already stored for this tile
-                uint32_t pr[8];
-                tmem_ld8(t_p + 8 * cc, pr);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                  pr[i] = pack_bf16x2(__uint_as_float(pr[i] << 16) * f, __uint_as_float(pr[i] & 0xFFFF0000u) * f);
-                tmem_st8(t_p + 8 * cc, pr);
-              }
-            }
-            if (j > 0) {
-#pragma unroll
-              for (int cc = 0; cc < D; cc += 8) {
-                uint32_t ro[8];
-                tmem_ld8(t_o + cc, ro);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 8; ++i) ro[i] = __float_as_uint(__uint_as_float(ro[i]) * f);
-                tmem_st8(t_o + cc, ro);
-              }
-            }
-          }
-          const uint64_t neg_m2 = f2_pack(neg_m, neg_m);
-          uint32_t pk[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            float a0, a1;
-            f2_unpack(f2_fma(v2[e], log2e2, neg_m2), a0, a1);
-            const float e0 = ex2_approx(a0), e1 = ex2_approx(a1);
-            rs2 = f2_add(rs2, f2_pack(e0, e1));
-            pk[e] = pack_bf16x2(e0, e1);
-          }
-          tmem_st8(t_p + 8 * c, pk);
-        }
-        {
-          float r0, r1;
-          f2_unpack(rs2, r0, r1);
-          l_run += r0 + r1;
-        }
-        if (++b_s == NB) {
-          b_s = 0;
-          b_ph ^= 1;
-        }
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(p_ready);
-      }
-
-      // last tile's P V, then the accumulated output row
-      mbar_wait(pv_done, pv_ph, wctx);
-      pv_ph ^= 1;
+    int m_s = 0;
+    int t = 0;  // tiles done by this CTA: tile t uses S / P buffer t & 1 for the (t >> 1)-th time
+    bool pend = false;
+    int f_q = 0, f_b = 0, f_o = 0, f_h = 0;
+    float f_m = 0.f, f_l = 0.f;
+    // normalise, gate and store the output row of the item whose last P V was tile t - 1
+    auto finish_item = [&]() {
+      mbar_wait(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, wctx);
       tc_fence_after();
-      const int q = qt * 128 + row;
-      const float inv = l_run > 0.f ? __fdividef(1.f, l_run) : 0.f;
-      const bool row_ok = q < p.N;
-      __nv_bfloat16* orow = p.out + b * p.ob + o * p.oo + h * p.oh + (int64_t)q * p.on;
-      const __nv_bfloat16* grow = p.gate + b * p.gb + o * p.go + h * p.gh + (int64_t)q * p.gn;
+      const float inv = f_l > 0.f ? __fdividef(1.f, f_l) : 0.f;
+      const bool f_ok = f_q < p.N;
+      __nv_bfloat16* f_out = p.out + f_b * p.ob + f_o * p.oo + f_h * p.oh + (int64_t)f_q * p.on;
+      const __nv_bfloat16* f_gate = p.gate + f_b * p.gb + f_o * p.go + f_h * p.gh + (int64_t)f_q * p.gn;
 #pragma unroll
       for (int c = 0; c < D; c += 16) {
         uint32_t ro[16];
         tmem_ld16(t_o + c, ro);
         uint4 g0 = make_uint4(0u, 0u, 0u, 0u), g1 = g0;
-        if (p.gate != nullptr && row_ok) {
-          g0 = *reinterpret_cast<const uint4*>(grow + c);
-          g1 = *reinterpret_cast<const uint4*>(grow + c + 8);
+        if (p.gate != nullptr && f_ok) {
+          g0 = *reinterpret_cast<const uint4*>(f_gate + c);
+          g1 = *reinterpret_cast<const uint4*>(f_gate + c + 8);
         }
         tmem_ld_wait();
         float v[16];
@@ -484,27 +322,149 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             v[2 * i + 1] *= sigmoid_fast(__uint_as_float(gw[i] & 0xFFFF0000u));
           }
         }
-        if (row_ok) {
-          uint4 pk0, pk1;
-          pk0 = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
-                           pack_bf16x2(v[6], v[7]));
-          pk1 = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]), pack_bf16x2(v[12], v[13]),
-                           pack_bf16x2(v[14], v[15]));
-          *reinterpret_cast<uint4*>(orow + c) = pk0;
-          *reinterpret_cast<uint4*>(orow + c + 8) = pk1;
+        if (f_ok) {
+          *reinterpret_cast<uint4*>(f_out + c) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]),
+                                                            pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+          *reinterpret_cast<uint4*>(f_out + c + 8) = make_uint4(pack_bf16x2(v[8], v[9]), pack_bf16x2(v[10], v[11]),
+                                                                pack_bf16x2(v[12], v[13]), pack_bf16x2(v[14], v[15]));
         }
       }
-      tc_fence_before();
-      if (row_ok && p.lse != nullptr)
-        p.lse[(((int64_t)b * p.O + o) * p.H + h) * p.N + q] = l_run > 0.f ? m_use + log2f(l_run) * kLn2 : -INFINITY;
+      if (f_ok && p.lse != nullptr)
+        p.lse[(((int64_t)f_b * p.O + f_o) * p.H + f_h) * p.N + f_q] = f_l > 0.f ? f_m + log2f(f_l) * kLn2 : -INFINITY;
+    };
+
+    ItemWalk iw;
+    iw.init(blockIdx.x, gridDim.x, p.O, p.q_tiles, p.H);
+    for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, iw.next()) {
+      float m_use = -INFINITY, l_run = 0.f;
+      const bool live = iw.qt * 128 + 32 * warp < p.N;  // a warp without query rows only keeps the barriers going
+      for (int j = 0; j < KT; ++j, ++t) {
+        const int buf = t & 1;
+        const uint32_t ph = (t >> 1) & 1;
+        // s_full completes after Q K^T of this tile, hence after the K tile and the mask row that
+        // arrives on the same barrier have landed
+        mbar_wait2(&s_full[buf], ph, &b_full[buf], ph, wctx);
+        tc_fence_after();
+        if (!live) {
+          if (++m_s == NS) m_s = 0;
+          if (pend) {
+            finish_item();
+            pend = false;
+            tc_fence_before();
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_ready[buf]);
+          continue;
+        }
+        uint32_t raw[64];  // this row's logits
+        tmem_ld32(t_s + 64 * buf, *reinterpret_cast<uint32_t(*)[32]>(raw));
+        tmem_ld32(t_s + 64 * buf + 32, *reinterpret_cast<uint32_t(*)[32]>(raw + 32));
+        const float* mask_row = reinterpret_cast<const float*>(smem + Cfg::OFF_MASK + m_s * 256);
+        const int n_keys = p.N - j * KEYS;
+        const float2 mprobe = *reinterpret_cast<const float2*>(mask_row + 2 * lane);
+        const bool general = n_keys < KEYS || __any_sync(0xffffffffu, (mprobe.x != 0.f) || (mprobe.y != 0.f));
+        const uint8_t* bias_row = smem + Cfg::OFF_BIAS + buf * Cfg::BIAS_STAGE + row * 128;
+        tmem_ld_wait();
+        if (++m_s == NS) m_s = 0;
+        float cm0 = -INFINITY, cm1 = -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (u == 4 && n_keys <= 32) break;
+          const uint4 bv = *reinterpret_cast<const uint4*>(bias_row + ((u ^ (row & 7)) << 4));
+          const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = 8 * u + 2 * e;
+            float v0, v1;
+            f2_unpack(f2_fma(f2_pack_bits(raw[i], raw[i + 1]), scale2, f2_pack_bits(bw[e] << 16, bw[e] & 0xFFFF0000u)), v0, v1);
+            raw[i] = __float_as_uint(v0);
+            raw[i + 1] = __float_as_uint(v1);
+          }
+        }
+        if (general) {
+#pragma unroll
+          for (int u = 0; u < 16; ++u) {
+            if (u == 8 && n_keys <= 32) break;
+            const float4 mk = *reinterpret_cast<const float4*>(mask_row + 4 * u);
+            const float m4[4] = {mk.x, mk.y, mk.z, mk.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float v = __uint_as_float(raw[4 * u + e]) + m4[e];
+              raw[4 * u + e] = __float_as_uint(4 * u + e < n_keys ? v : -INFINITY);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 64; i += 4) {
+          if (i == 32 && n_keys <= 32) break;
+          cm0 = max3(cm0, __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]));
+          cm1 = max3(cm1, __uint_as_float(raw[i + 2]), __uint_as_float(raw[i + 3]));
+        }
+        const float cmax = fmaxf(cm0, cm1);
+        if (__any_sync(0xffffffffu, cmax > m_use + kGap)) {
+          // Raise the reference maximum of the rows that need it (f = 1 for the others) and rescale what
+          // those rows have accumulated.  Runs for the first finite tile of every row and then only
+          // when the logits of a row grow by more than kGap.
+          const bool grow = cmax > m_use + kGap;
+          const float f = grow ? ex2_approx((m_use - cmax) * kLog2e) : 1.f;  // m_use = -inf gives 0; nothing accumulated then
+          if (grow) m_use = cmax;
+          l_run *= f;
+          if (j > 0) {
+            mbar_wait(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, wctx);
+            tc_fence_after();
+#pragma unroll 1
+            for (int cc = 0; cc < D; cc += 8) {
+              uint32_t ro[8];
+              tmem_ld8(t_o + cc, ro);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 8; ++i) ro[i] = __float_as_uint(__uint_as_float(ro[i]) * f);
+              tmem_st8(t_o + cc, ro);
+            }
+          }
+        }
+        const float neg_m = (m_use == -INFINITY) ? 0.f : -m_use * kLog2e;
+        const uint64_t neg_m2 = f2_pack(neg_m, neg_m);
+        uint64_t rs2a = 0ull, rs2b = 0ull;  // packed partial row sums of this tile
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (c == 2 && n_keys <= 32) break;
+          uint32_t pk[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            float a0, a1;
+            f2_unpack(f2_fma(f2_pack_bits(raw[16 * c + 2 * e], raw[16 * c + 2 * e + 1]), log2e2, neg_m2), a0, a1);
+            const float e0 = ex2_approx(a0), e1 = ex2_approx(a1);
+            if (e & 1) rs2b = f2_add(rs2b, f2_pack(e0, e1));
+            else rs2a = f2_add(rs2a, f2_pack(e0, e1));
+            pk[e] = pack_bf16x2(e0, e1);
+          }
+          tmem_st8(t_s + 64 * buf + 8 * c, pk);
+        }
+        float r0, r1;
+        f2_unpack(f2_add(rs2a, rs2b), r0, r1);
+        l_run += r0 + r1;
+        // the previous item's row leaves before this item's first P V overwrites the accumulator
+        if (j == 0 && pend) finish_item();
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_ready[buf]);
+      }
+      pend = live;
+      f_q = iw.qt * 128 + row; f_b = iw.b; f_o = iw.o; f_h = iw.h;
+      f_m = m_use;
+      f_l = l_run;
     }
+    if (pend) finish_item();
   }
 
   tc_fence_before();
   __syncthreads();
   if (warp == Cfg::WARP_MMA) {
     __syncwarp();
-    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    tmem_dealloc(tmem_s, Cfg::S_COLS);
+    tmem_dealloc(tmem_o, Cfg::O_COLS);
   }
 }
 
