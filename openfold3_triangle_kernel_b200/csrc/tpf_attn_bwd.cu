@@ -92,6 +92,7 @@ struct AttnBwdParams {
   int bias_broadcast;
   float scale;
   int n_items;
+  FastDiv div_h, div_o;
 };
 
 template <int D_>
@@ -114,11 +115,7 @@ struct AttnBwdCfg {
   static constexpr int OFF_K = OFF_DO + NQ * TILE;       // [NKV]
   static constexpr int OFF_V = OFF_K + NKV * TILE;       // [NKV]
   static constexpr int OFF_MASK = OFF_V + NKV * TILE;    // [NKV] x 512
-  // two staging tiles through which finished dQ / dK / dV tiles leave as whole, contiguous 128 x D blocks
-  // (only where shared memory has room for them; otherwise every thread stores its own piece)
-  static constexpr int OFF_STG = OFF_MASK + NKV * 512;
-  static constexpr bool STAGED = OFF_STG + 2 * TILE + 1024 + 256 <= 232448 - 1024;
-  static constexpr int OFF_BAR = OFF_STG + (STAGED ? 2 * TILE : 0);
+  static constexpr int OFF_BAR = OFF_MASK + NKV * 512;
   static constexpr int N_BAR = 2 * NB + 2 * NQ + 2 * NKV + 6;
   static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
   static constexpr int TM_S = 0, TM_DP = 128, TM_DQ = 256, TM_DK = 320, TM_DV = 320 + KS * D;
@@ -227,10 +224,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t tmem_base = *tmem_slot;
 
   auto decode = [&](int item, int& b, int& o, int& h) {
-    h = item % p.H;
-    const int r = item / p.H;
-    o = r % p.O;
-    b = r / p.O;
+    const int r = (int)p.div_h.div((uint32_t)item);
+    h = item - r * p.H;
+    b = (int)p.div_o.div((uint32_t)r);
+    o = r - b * p.O;
   };
 
   if (warp == Cfg::WARP_TMA) {
@@ -403,9 +400,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float neg_lse2 = -INFINITY, delta = 0.f;
     bool have_prev_dq = false;     // a finished dQ tile waits in TMEM
     bool have_prev_strip = false;  // the dK / dV accumulators of a finished strip wait in TMEM
-    int prev_q0 = 0, prev_b = 0, prev_o = 0, prev_h = 0, prev_strip = 0;
-    int sp_b = 0, sp_o = 0, sp_h = 0, sp_strip = 0, sp_nk = 0;
-    int stg_slot = 0;
+    int64_t prev_off = 0;          // their plane's offset in dq / dk / dv
+    int prev_q0 = 0, prev_strip = 0;
 
     // read DQ consecutive accumulator columns of this thread's row
     auto ld_cols = [&](uint32_t taddr, float (&v)[DQ]) {
@@ -426,63 +422,47 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
     };
-    auto st_cols = [&](__nv_bfloat16* dst, const float (&v)[DQ], float mul) {
-      if constexpr (DQ == 4) {
-        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0] * mul, v[1] * mul), pack_bf16x2(v[2] * mul, v[3] * mul));
+    // Finished tiles leave straight from registers, 16 bytes (8 at D = 16) of a row per thread: the stores are not waited
+    // for.  (Collecting a tile in shared memory first, so that a store instruction covers whole lines, put 500 cycles of
+    // barriers and copies per tile, 7 tiles per plane, on the path between two UMMA batches.)  dQ, which is finished
+    // most often, is only packed before the hand-over of P / dS and stored after it.
+    constexpr int PQ = DQ / 2;  // packed words per thread
+    auto pack_cols = [&](const float (&v)[DQ], float mul, uint32_t (&w)[PQ]) {
+#pragma unroll
+      for (int i = 0; i < PQ; ++i) w[i] = pack_bf16x2(v[2 * i] * mul, v[2 * i + 1] * mul);
+    };
+    auto store_packed = [&](__nv_bfloat16* dst, const uint32_t (&w)[PQ]) {
+      if constexpr (PQ == 2) {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
       } else {
 #pragma unroll
-        for (int c = 0; c < DQ; c += 8)
-          *reinterpret_cast<uint4*>(dst + c) =
-              make_uint4(pack_bf16x2(v[c] * mul, v[c + 1] * mul), pack_bf16x2(v[c + 2] * mul, v[c + 3] * mul),
-                         pack_bf16x2(v[c + 4] * mul, v[c + 5] * mul), pack_bf16x2(v[c + 6] * mul, v[c + 7] * mul));
+        for (int i = 0; i < PQ; i += 4) *reinterpret_cast<uint4*>(dst + 2 * i) = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
       }
     };
+    uint32_t dqw[PQ];
+    bool out_dq = false;  // a packed dQ tile waits in registers
 
-    // One finished 128 x D tile (this thread holds DQ columns of row `row`) -> global memory at `gtile`
-    // (row 0 of the tile; rows are gn elements apart).  Staged: every thread drops its piece
-    // into a shared-memory copy of the tile, then the 512 compute threads write it out in
-    // consecutive 16-byte pieces, so each store instruction covers whole rows (512 contiguous bytes when the
-    // rows are) instead of 32 half-used sectors.  All sixteen compute warps call this together.
-    auto store_tile = [&](__nv_bfloat16* gtile, int rows_valid, const float (&v)[DQ], float mul) {
-      if constexpr (Cfg::STAGED) {
-        uint8_t* stg = smem + Cfg::OFF_STG + stg_slot * Cfg::TILE;
-        stg_slot ^= 1;
-        st_cols(reinterpret_cast<__nv_bfloat16*>(stg) + row * D + DQ * part, v, mul);
-        named_barrier_sync(1, 32 * NCW);
-#pragma unroll
-        for (int i = threadIdx.x; i < Cfg::TILE / 16; i += 32 * NCW)
-          if ((16 * i) / (2 * D) < rows_valid)
-            *reinterpret_cast<uint4*>(gtile + (int64_t)((16 * i) / (2 * D)) * p.gn + ((16 * i) % (2 * D)) / 2) =
-                *reinterpret_cast<const uint4*>(stg + 16 * i);
-      } else {
-        if (row < rows_valid) st_cols(gtile + row * p.gn + DQ * part, v, mul);
-      }
-    };
-
-    // store a finished dQ tile that has been read out of TMEM (or fold it into the per-CTA running sum)
-    auto store_dq = [&](int b, int o, int h, int q0, int strip, float (&v)[DQ]) {
-      if (p.n_strips == 1) {
-        store_tile(p.dq + b * p.gb + o * p.go + h * p.gh + q0 * p.gn, p.N - q0, v, scale);
-        return;
-      }
-      const int q = q0 + row;
-      if (q >= p.N) return;
+    // a finished dQ tile that has been read out of TMEM: packed, or folded into the per-CTA running sum
+    auto take_dq = [&](float (&v)[DQ]) {
       if (p.n_strips > 1) {
-        float* sc = p.dq_scratch + ((int64_t)blockIdx.x * p.N + q) * D + DQ * part;
-        if (strip > 0) {
+        const int q = prev_q0 + row;
+        if (q < p.N) {
+          float* sc = p.dq_scratch + ((int64_t)blockIdx.x * p.N + q) * D + DQ * part;
+          if (prev_strip > 0) {
 #pragma unroll
-          for (int c = 0; c < DQ; c += 4) {
-            const float4 o4 = *reinterpret_cast<const float4*>(sc + c);
-            v[c] += o4.x; v[c + 1] += o4.y; v[c + 2] += o4.z; v[c + 3] += o4.w;
+            for (int c = 0; c < DQ; c += 4) {
+              const float4 o4 = *reinterpret_cast<const float4*>(sc + c);
+              v[c] += o4.x; v[c + 1] += o4.y; v[c + 2] += o4.z; v[c + 3] += o4.w;
+            }
+          }
+          if (prev_strip + 1 < p.n_strips) {
+#pragma unroll
+            for (int c = 0; c < DQ; c += 4) *reinterpret_cast<float4*>(sc + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
           }
         }
-        if (strip + 1 < p.n_strips) {
-#pragma unroll
-          for (int c = 0; c < DQ; c += 4) *reinterpret_cast<float4*>(sc + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
-          return;
-        }
       }
-      st_cols(p.dq + b * p.gb + o * p.go + h * p.gh + q * p.gn + DQ * part, v, scale);
+      out_dq = prev_strip + 1 == p.n_strips;
+      pack_cols(v, scale, dqw);
     };
 
     // lse / delta of this thread's query row, loaded one query tile ahead of their first use
@@ -502,32 +482,47 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     };
 
-    // Reads finished accumulators out of TMEM and sends them on their way: the dQ tile of a finished query
-    // tile and, after the last tile of a strip, the strip's dK / dV tiles (then the UMMA issuer may start the
-    // next strip in those columns).  Called by all compute warps once the UMMAs of the previous tile are done.
-    auto drain_finished = [&]() {
+    // Reads finished accumulators out of TMEM: the dQ tile of a finished query tile and, after the last tile of a
+    // strip, the strip's dK / dV tiles, which are stored at once (then the UMMA issuer may start the next strip in those columns).  Called by
+    // all compute warps once the UMMAs of the previous tile are done.
+    auto take_finished = [&]() {
       if (have_prev_dq) {
         float dqv[DQ];
         ld_cols(t_dq, dqv);
         have_prev_dq = false;
-        store_dq(prev_b, prev_o, prev_h, prev_q0, prev_strip, dqv);
+        take_dq(dqv);
       }
       if (have_prev_strip) {
         have_prev_strip = false;
-        for (int kk = 0; kk < sp_nk; ++kk) {
-          const int key0 = (sp_strip * KS + kk) * 128;
-          const int64_t base = sp_b * p.gb + sp_o * p.go + sp_h * p.gh + key0 * p.gn;
-          float vk1[DQ], vv1[DQ];
-          ld_cols(tmem_addr(tmem_base, lane_base, Cfg::TM_DK + kk * D + DQ * part), vk1);
-          ld_cols(tmem_addr(tmem_base, lane_base, Cfg::TM_DV + kk * D + DQ * part), vv1);
-          store_tile(p.dk + base, p.N - key0, vk1, scale);
-          store_tile(p.dv + base, p.N - key0, vv1, 1.f);
+        __nv_bfloat16* dk = p.dk + prev_off + (prev_strip * KS * 128 + row) * p.gn + DQ * part;
+        __nv_bfloat16* dv = p.dv + (dk - p.dk);
+#pragma unroll
+        for (int kk = 0; kk < KS; ++kk) {
+          if (prev_strip * KS + kk < p.k_tiles) {
+            float vk[DQ], vv[DQ];
+            ld_cols(tmem_addr(tmem_base, lane_base, Cfg::TM_DK + kk * D + DQ * part), vk);
+            ld_cols(tmem_addr(tmem_base, lane_base, Cfg::TM_DV + kk * D + DQ * part), vv);
+            if ((prev_strip * KS + kk) * 128 + row < p.N) {
+              uint32_t w[PQ];
+              pack_cols(vk, scale, w);
+              store_packed(dk + kk * 128 * p.gn, w);
+              pack_cols(vv, 1.f, w);
+              store_packed(dv + kk * 128 * p.gn, w);
+            }
+          }
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(dkv_free);
       } else {
         tc_fence_before();
+      }
+    };
+    auto store_finished = [&]() {
+      if (out_dq) {
+        out_dq = false;
+        const int q = prev_q0 + row;
+        if (q < p.N) store_packed(p.dq + prev_off + q * p.gn + DQ * part, dqw);
       }
     };
 
@@ -546,8 +541,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         neg_lse2 = (l_pref == -INFINITY) ? -INFINITY : -l_pref * kLog2e;
         delta = d_pref;
         BwdWalk nx = w;
-        const int sl = w.strip_len();
-        for (int t = 0; t < sl; ++t) nx.next();
+        nx.kk = w.strip_len() - 1;
+        nx.next();
         prefetch_row_scalars(nx);
       }
       const uint64_t nlse2 = f2_pack(neg_lse2, neg_lse2);
@@ -623,9 +618,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_wait(pds_free, pdsfree_ph, wctx);
       pdsfree_ph ^= 1;
       tc_fence_after();
-      // the same completion covers the last tile of a strip: its dQ and the strip's dK / dV leave now,
+      // the same completion covers the last tile of a strip: its dQ and the strip's dK / dV are read out now,
       // before this tile's P / dS release the UMMAs that would overwrite them
-      drain_finished();
+      take_finished();
       {
         uint8_t* p_row = smem + Cfg::OFF_P + half_off;
         uint8_t* ds_row = smem + Cfg::OFF_DS + half_off;
@@ -639,14 +634,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(pds_ready);
+      store_finished();
 
       if (w.last_kk()) {
         have_prev_dq = true;
-        prev_b = b; prev_o = o; prev_h = h; prev_q0 = w.qt * 128; prev_strip = w.strip;
-      }
-      if (w.last_kk() && w.last_qt()) {
-        have_prev_strip = true;
-        sp_b = b; sp_o = o; sp_h = h; sp_strip = w.strip; sp_nk = w.strip_len();
+        prev_off = b * p.gb + o * p.go + h * p.gh;
+        prev_q0 = w.qt * 128;
+        prev_strip = w.strip;
+        have_prev_strip = w.last_qt();
       }
     }
     // the last tile of this CTA: wait for its UMMAs, then the same drain
@@ -654,7 +649,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_wait(pds_free, pdsfree_ph, wctx);
       pdsfree_ph ^= 1;
       tc_fence_after();
-      drain_finished();
+      take_finished();
+      store_finished();
     }
   }
 
@@ -1150,6 +1146,8 @@ int attn_backward_qkv(const AttnCall& c, void* workspace, int64_t workspace_byte
   p.bias_broadcast = c.G == 1 && B > 1 ? 1 : 0;
   p.scale = c.scale;
   p.n_items = (int)(B * O * H);
+  p.div_h = FastDiv::make((uint32_t)H);
+  p.div_o = FastDiv::make((uint32_t)O);
   int grid = sm_count();
   if (grid > p.n_items) grid = p.n_items;
   int* status = nullptr;

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const bf16* __restrict__ d_
   for (int e = 0; e < 8; ++e) ag[e] = ab[e] = 0.f;
   constexpr int G = 4;  // row groups in flight per warp: all their loads are issued before the first use
   for (int it0 = warp * L::RPW; it0 < rows_per_block; it0 += G * 8 * L::RPW) {
-    uint4 du[G], zu[G];
+    uint4 du[G], zu[G], ru[G];  // ru: the gradient that reaches z past the update (residual connection)
     float mu[G], rs[G];
     int64_t src[G];  // the caller's row
     bool active[G];
@@ -140,11 +140,12 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const bf16* __restrict__ d_
       active[r] = on && it + sub < rows_per_block && row < R;
       src[r] = active[r] ? rows.locate((uint32_t)row).src : -1;
       active[r] = src[r] >= 0;
-      du[r] = zu[r] = make_uint4(0u, 0u, 0u, 0u);
+      du[r] = zu[r] = ru[r] = make_uint4(0u, 0u, 0u, 0u);
       mu[r] = rs[r] = 0.f;
       if (active[r]) {
         du[r] = *reinterpret_cast<const uint4*>(d_zln + row * C + part * 8);
         zu[r] = *reinterpret_cast<const uint4*>(z + src[r] * C + part * 8);
+        if (d_res != nullptr) ru[r] = *reinterpret_cast<const uint4*>(d_res + src[r] * C + part * 8);
         mu[r] = mean[row];
         rs[r] = rstd[row];
       }
@@ -165,11 +166,8 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const bf16* __restrict__ d_
       const float m1 = slot_sum<C>(a1) * (1.f / C);
       const float m2 = slot_sum<C>(a2) * (1.f / C);
       if (active[r]) {
-        // the gradient that reaches z past the update (residual connection) is added here
-        uint4 ru = make_uint4(0u, 0u, 0u, 0u);
-        if (d_res != nullptr) ru = *reinterpret_cast<const uint4*>(d_res + src[r] * C + part * 8);
         float res[8];
-        unpack8(ru, res);
+        unpack8(ru[r], res);
         uint32_t o[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e)

@@ -414,12 +414,13 @@ int64_t pair_attn_bwd_workspace_bytes(int64_t B, int64_t N, int64_t C, int64_t H
   return w.total;
 }
 
-template <int D, int BN>
+template <int D>
 static int gate_bwd(const PairAttnCall& t, const void* d_out, const PairAttnBwdWorkspace& w, const AttnPacked& pk,
                     int* status, cudaStream_t stream) {
   const int64_t R = t.B * t.N * t.N, HD = t.H * D, P = proj_cols(t.H, D);
-  // the epilogue keeps gate logits and gated outputs of the next tile in flight: one 32-column chunk per warp
-  using Cfg = GemmCfg<128, BN, 128, false, 128, false, 4, (BN > 64 ? 16 : 8)>;
+  // the epilogue keeps gate logits and gated outputs of the next tile in flight: one 32-column chunk per warp (see the
+  // output projection of the multiplicative update)
+  using Cfg = GemmCfg<128, 64, 128, false, 128, false, 4>;
   using Epi = EpiGateBwd<D>;
   typename Epi::Params ep{(const bf16*)t.qkvg + 3 * t.H * R * D, (const bf16*)t.og, w.d_o, R * D, w.d_rows + 3 * HD, P,
                           w.delta, t.ending, (int)t.H, (int)t.N, (int)HD, PairRows::make(t.N, t.N, false)};
@@ -459,10 +460,7 @@ int pair_attn_backward(const PairAttnCall& t, const PairAttnGrads& g, void* work
   const AttnPacked pk = attn_packed_at(t.packed, C, H, D);
   FoldList folds;
   // 1. d_og = d_out Wo -> d_o, d_g, delta
-  if (D == 16) rc = HD <= 64 ? gate_bwd<16, 64>(t, g.d_out, w, pk, status, stream)
-                             : gate_bwd<16, 128>(t, g.d_out, w, pk, status, stream);
-  else rc = HD <= 64 ? gate_bwd<32, 64>(t, g.d_out, w, pk, status, stream)
-                     : gate_bwd<32, 128>(t, g.d_out, w, pk, status, stream);
+  rc = D == 16 ? gate_bwd<16>(t, g.d_out, w, pk, status, stream) : gate_bwd<32>(t, g.d_out, w, pk, status, stream);
   if (rc) return rc;
   // 2. d_wo = d_out^T og
   rc = bmm_bf16(g.d_out, C, 0, 1, t.og, HD, 0, 1, w.part_wo, HD, C * HD, 1, C, HD, R, w.splits_wo, w.kps_wo, 128, stream);

@@ -695,12 +695,16 @@ static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPack
                     t.rstd_out, NN, tiles, (int)(B * tiles));
     }
     TPF_LAUNCH_OK();
-    using Cfg = GemmCfg<128, C, 128, false, 128, false, 4>;
     GemmShape sh{(int)R, C, C, 1, 0};
     if (t.sum) {
+      // The residual doubles the operands the epilogue keeps in flight: narrow tiles, so that a warp has one 32-column
+      // chunk and 165 registers for it (wider tiles with two chunks, or with 16 warps of 96 registers, spill).  The
+      // activations are read once more per tile column, from L2.
+      using Cfg = GemmCfg<128, (C % 64 == 0 ? 64 : 32), 128, false, 128, false, 4>;
       typename EpiOutGate<true>::Params ep{(bf16*)t.out, (bf16*)t.sum, z, (const bf16*)t.gate, rows, C};
       rc = launch_gemm<Cfg, EpiOutGate<true>>(xln, C, 0, pk.Wz, C, 0, sh, ep, status, stream);
     } else {
+      using Cfg = GemmCfg<128, C, 128, false, 128, false, 4>;
       typename EpiOutGate<false>::Params ep{(bf16*)t.out, nullptr, nullptr, (const bf16*)t.gate, rows, C};
       rc = launch_gemm<Cfg, EpiOutGate<false>>(xln, C, 0, pk.Wz, C, 0, sh, ep, status, stream);
     }
