@@ -23,7 +23,8 @@ int bmm_dispatch(const void* A, int64_t lda, int64_t bsa, const void* B, int64_t
   constexpr int kStages = (196608 / (256 * kBK * 2)) > 8 ? 8 : (196608 / (256 * kBK * 2));
   using Cfg = GemmCfg<128, 128, SWZ, A_MN, SWZ, B_MN, kStages>;
   using Epi = EpiStore<OutT>;
-  typename Epi::Params ep{reinterpret_cast<OutT*>(D), ldd, bsd};
+  typename Epi::Params ep;
+  if (int rc = epi_store_params<OutT>(&ep, reinterpret_cast<OutT*>(D), ldd, bsd, sh)) return rc;
   return launch_gemm<Cfg, Epi>(A, lda, bsa, B, ldb, bsb, sh, ep, status, stream);
 }
 

@@ -22,6 +22,29 @@ inline int make_operand_tmap(CUtensorMap* tm, const void* base, bool mn_major, i
   return make_tmap_bf16(tm, base, 3, dims, strides, box, swz);
 }
 
+// Tensor map of a bf16 output [batch][rows][cols] for warp_tile_store_tma: 32 x 32 boxes, 64-byte swizzle.
+inline int make_store_tmap(CUtensorMap* tm, const void* base, int64_t cols, int64_t rows, int64_t ld, int64_t batch,
+                           int64_t batch_stride) {
+  uint64_t dims[3] = {(uint64_t)cols, (uint64_t)rows, (uint64_t)batch};
+  uint64_t strides[2] = {(uint64_t)ld * 2, (uint64_t)(batch_stride ? batch_stride : 8) * 2};
+  uint32_t box[3] = {32, 32, 1};
+  return make_tmap_bf16(tm, base, 3, dims, strides, box, 64);
+}
+// Parameters of EpiStore; bf16 outputs with 16-byte aligned rows get a tensor map.
+template <typename OutT>
+inline int epi_store_params(typename EpiStore<OutT>::Params* ep, OutT* D, int64_t ldd, int64_t batch_stride,
+                            const GemmShape& sh) {
+  *ep = {};
+  ep->D = D;
+  ep->ldd = ldd;
+  ep->batch_stride = batch_stride;
+  if (sizeof(OutT) == 2 && ldd % 8 == 0 && batch_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(D) & 15) == 0) {
+    ep->has_map = 1;
+    return make_store_tmap(&ep->map, D, sh.N, sh.M, ldd, sh.batch, batch_stride);
+  }
+  return TPF_OK;
+}
+
 template <class Cfg, class Epi>
 int launch_gemm(const void* A, int64_t lda, int64_t bsa, const void* B, int64_t ldb, int64_t bsb,
                 const GemmShape& sh, const typename Epi::Params& ep, int* status, cudaStream_t stream,

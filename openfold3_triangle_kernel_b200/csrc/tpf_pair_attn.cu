@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(256) pair_attn_pack_kernel(const PairAttnWeigh
 // Joint projection: column chunks of q, k, v, g go to [plane][row][D]; the bias chunk to [b][h][i][j].
 struct EpiQkvg {
   struct Params {
+    CUtensorMap map;       // D = 32: stores [4H][R][D]
     bf16* planes;
     int64_t plane_stride;  // R * D
     int log_d, D;
@@ -93,17 +94,21 @@ struct EpiQkvg {
   };
   static constexpr bool kPaired = false;
   static constexpr bool kStaged = false;
-  static constexpr int kSmemPerWarp = 2048;
+  static constexpr int kSmemPerWarp = kTmaTiles;
   struct Pre {};
   __device__ static __forceinline__ void prefetch(const Params&, const GemmShape&, int, int, int, int, Pre&) {}
   __device__ static __forceinline__ void apply(const Params& p, const GemmShape& sh, int, int m, int n0,
-                                               const float (&v)[32], float* wsm, int lane, const Pre&) {
+                                               const float (&v)[32], float* wsm, int lane, const Pre&, int& buf) {
     const int m_base = m - lane;
     if (n0 < p.HD4) {
       uint32_t pk[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
       uint8_t* tile = reinterpret_cast<uint8_t*>(wsm);
+      if (p.D == 32) {
+        if (m_base < sh.M) warp_tile_store_tma(tile, buf, lane, pk, &p.map, 0, m_base, n0 >> 5);
+        return;
+      }
       warp_tile_put(tile, lane, pk);
       __syncwarp();
       const int piece = lane & 3, col = n0 + 8 * piece;
@@ -146,7 +151,7 @@ struct EpiResidual {
     load_rows(p.res, p.rows, m - lane, sh.M, p.C, n0, lane, pre.r);
   }
   __device__ static __forceinline__ void apply(const Params& p, const GemmShape& sh, int, int m, int n0,
-                                               const float (&v)[32], float* wsm, int lane, const Pre& pre) {
+                                               const float (&v)[32], float* wsm, int lane, const Pre& pre, int&) {
     uint32_t pk[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
@@ -160,6 +165,7 @@ struct EpiResidual {
 template <int D>
 struct EpiGateBwd {
   struct Params {
+    CUtensorMap map_o, map_g;  // stores: d_o planes (D = 32), the row matrix's gate columns
     const bf16* gate;      // gate-logit planes [H][R][D]
     const bf16* og;        // [R][HD]
     bf16* d_o;             // planes [H][R][D]
@@ -172,7 +178,7 @@ struct EpiGateBwd {
   };
   static constexpr bool kPaired = false;
   static constexpr bool kStaged = false;
-  static constexpr int kSmemPerWarp = 2048;
+  static constexpr int kSmemPerWarp = kTmaTiles;
   struct Pre {
     uint4 g[4], o[4];
   };
@@ -188,7 +194,7 @@ struct EpiGateBwd {
     }
   }
   __device__ static __forceinline__ void apply(const Params& p, const GemmShape& sh, int, int m, int n0,
-                                               const float (&v)[32], float* wsm, int lane, const Pre& pre) {
+                                               const float (&v)[32], float* wsm, int lane, const Pre& pre, int& buf) {
     uint32_t po[16], pg[16];
     float sum[2] = {0.f, 0.f};
 #pragma unroll
@@ -214,22 +220,26 @@ struct EpiGateBwd {
       if (D == 16) dst[p.N] = sum[1];
     }
     const int m_base = m - lane;
+    if (m_base >= sh.M) return;
     uint8_t* tile = reinterpret_cast<uint8_t*>(wsm);
-    warp_tile_put(tile, lane, po);
-    __syncwarp();
-    const int piece = lane & 3, col = n0 + 8 * piece;
-    bf16* dst = p.d_o + (int64_t)(col / D) * p.plane_stride + col % D;
+    if constexpr (D == 32) {
+      warp_tile_store_tma(tile, buf, lane, po, &p.map_o, 0, m_base, n0 / D);
+    } else {
+      bulk_wait_read<0>();
+      __syncwarp();
+      warp_tile_put(tile, lane, po);
+      __syncwarp();
+      const int piece = lane & 3, col = n0 + 8 * piece;
+      bf16* dst = p.d_o + (int64_t)(col / D) * p.plane_stride + col % D;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = 8 * i + (lane >> 2);
-      if (m_base + r < sh.M)
-        *reinterpret_cast<uint4*>(dst + (int64_t)(m_base + r) * D) = warp_tile_get(tile, r, piece);
+      for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2);
+        if (m_base + r < sh.M)
+          *reinterpret_cast<uint4*>(dst + (int64_t)(m_base + r) * D) = warp_tile_get(tile, r, piece);
+      }
+      __syncwarp();
     }
-    __syncwarp();
-    bf16* blk = p.d_rows + n0;
-    warp_tile_store(tile, lane, pg, [&](int r) -> bf16* {
-      return m_base + r < sh.M ? blk + (int64_t)(m_base + r) * p.ld : nullptr;
-    });
+    warp_tile_store_tma(tile, buf, lane, pg, &p.map_g, n0, m_base, 0);
   }
 };
 
@@ -343,8 +353,9 @@ int pair_attn_forward(const PairAttnCall& t, cudaStream_t stream) {
   {
     int log_d = 0;
     while ((1 << log_d) < t.D) ++log_d;
-    EpiQkvg::Params ep{(bf16*)t.qkvg, R * t.D, log_d, (int)t.D, (int)(4 * HD), (bf16*)t.bias, (int)t.H, (int)t.N,
+    EpiQkvg::Params ep{{}, (bf16*)t.qkvg, R * t.D, log_d, (int)t.D, (int)(4 * HD), (bf16*)t.bias, (int)t.H, (int)t.N,
                        (t.N + 7) / 8 * 8, PairRows::make(t.N, t.N, false)};
+    if (t.D == 32 && (rc = make_store_tmap(&ep.map, t.qkvg, t.D, R, t.D, 4 * t.H, R * t.D))) return rc;
     GemmShape sh{(int)R, (int)P, (int)C, 1, 0};
     // 4 HD + H columns in as few, as full tiles as possible: 3 x 192 at H * D = 128, 3 x 96 at 64.  The weight tile
     // stays in shared memory while the rows stream past (see GemmCfg).
@@ -422,8 +433,10 @@ static int gate_bwd(const PairAttnCall& t, const void* d_out, const PairAttnBwdW
   // output projection of the multiplicative update)
   using Cfg = GemmCfg<128, 64, 128, false, 128, false, 4>;
   using Epi = EpiGateBwd<D>;
-  typename Epi::Params ep{(const bf16*)t.qkvg + 3 * t.H * R * D, (const bf16*)t.og, w.d_o, R * D, w.d_rows + 3 * HD, P,
+  typename Epi::Params ep{{}, {}, (const bf16*)t.qkvg + 3 * t.H * R * D, (const bf16*)t.og, w.d_o, R * D, w.d_rows + 3 * HD, P,
                           w.delta, t.ending, (int)t.H, (int)t.N, (int)HD, PairRows::make(t.N, t.N, false)};
+  int rc = D == 32 ? make_store_tmap(&ep.map_o, w.d_o, D, R, D, t.H, R * D) : TPF_OK;
+  if (rc || (rc = make_store_tmap(&ep.map_g, w.d_rows + 3 * HD, HD, R, P, 1, 0))) return rc;
   GemmShape sh{(int)R, (int)HD, (int)t.C, 1, 0};
   return launch_gemm<Cfg, Epi>(d_out, t.C, 0, pk.WoT, t.C, 0, sh, ep, status, stream);
 }
@@ -436,7 +449,8 @@ static int norm_bwd(const PairAttnCall& t, const PairAttnGrads& g, const PairAtt
     using Cfg = GemmCfg<128, C, 128, false, 128, false, 6>;
     using Epi = EpiStore<bf16>;
     GemmShape sh{(int)R, C, (int)P, 1, 0};
-    typename Epi::Params ep{w.d_x, C, 0};
+    typename Epi::Params ep;
+    if (int rc = epi_store_params<bf16>(&ep, w.d_x, C, 0, sh)) return rc;
     if (int rc = launch_gemm<Cfg, Epi>(w.d_rows, P, 0, pk.WT, P, 0, sh, ep, status, stream)) return rc;
   }
   launch_kernel(ln_bwd_kernel<C>, dim3(w.blocks_ln), dim3(256), 0, stream, (const bf16*)w.d_x, (const bf16*)t.z,

@@ -205,6 +205,24 @@ __device__ __forceinline__ void tma_load_5d(uint32_t elected, void* dst, const C
       : "memory");
 }
 
+// TMA tile stores (shared memory -> global).  Every lane that wrote the tile calls fence_async_smem() first; one lane
+// issues the store and its group, and waits: bulk_wait_read<N>: all but the N newest groups have read their shared
+// memory; bulk_wait_all: everything is written.
+__device__ __forceinline__ void tma_store_3d(uint32_t elected, const CUtensorMap* map, const void* src, int c0, int c1,
+                                             int c2) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];\n\t"
+      "@q cp.async.bulk.commit_group;\n\t}"
+      ::"l"(map), "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(elected)
+      : "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------
 // TMEM allocation (one full warp executes these)
 // ----------------------------------------------------------------------------

@@ -196,6 +196,7 @@ __device__ __forceinline__ void split_row(int row, int64_t NN, int M, int& bb, i
 
 struct EpiProjGate {
   struct Params {
+    CUtensorMap map_a, map_b, map_gate;  // stores: [B][C][NN], [R][C]
     bf16* a_cm;        // [B*C][NN]
     bf16* b_cm;        // [B*C][NN]
     bf16* gate;        // [R][C] raw gate logits
@@ -205,7 +206,7 @@ struct EpiProjGate {
   };
   static constexpr bool kPaired = true;
   static constexpr bool kStaged = false;
-  static constexpr int kSmemPerWarp = 32 * 33 * 4;
+  static constexpr int kSmemPerWarp = 4608;  // two staging tiles and a mask row, or one 32 x 33 float block
   struct Pre {
     float mk;  // pair mask: of this lane's row, or (exchanged tile) of row `lane` of the warp's 32-row chunk
   };
@@ -221,17 +222,18 @@ struct EpiProjGate {
   }
   __device__ static __forceinline__ void apply2(const Params& p, const GemmShape& sh, int, int m0, int rit, int n0,
                                                 int c0, const float (&v0)[32], const float (&v1)[32], float* wsm,
-                                                int lane, bool swap, const Pre& pre) {
+                                                int lane, bool swap, const Pre& pre, int& buf) {
     const int which = tile_kind(n0, p.C);
     if (swap) {
       // lane = channel `rit`; v0[i] / v1[i] = projection / gate logit of pair row m0 + c0 + i
-      wsm[lane] = pre.mk;
+      float* msm = wsm + kTmaTiles / 4;
+      msm[lane] = pre.mk;
       __syncwarp();
       const uint64_t half2 = f2_pack(0.5f, 0.5f);
       uint32_t ow[16];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const float4 mk = reinterpret_cast<const float4*>(wsm)[q];  // same address in every lane: one broadcast
+        const float4 mk = reinterpret_cast<const float4*>(msm)[q];  // same address in every lane: one broadcast
         const float mks[4] = {mk.x, mk.y, mk.z, mk.w};
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -244,17 +246,15 @@ struct EpiProjGate {
           ow[2 * q + e] = pack_bf16x2(a0, a1);
         }
       }
-      __syncwarp();  // the mask row has been read: the scratch becomes the staging tile
       // Rows (and the sharded row count) are multiples of 64, so the 32-row chunk lies inside one batch entry
-      // and is inside M as a whole or not at all.  A lane's 64 bytes go out through the staging tile so that one
-      // store instruction covers 8 channels x 64 contiguous bytes instead of 32 channels x 16 bytes.
+      // and is inside M as a whole or not at all.
       const int r0 = m0 + c0;
       int bb, rr;
       split_row(r0, p.NN, sh.M, bb, rr);
-      bf16* blk = (which == 0 ? p.a_cm : p.b_cm) + ((int64_t)bb * p.C + (rit - lane)) * p.NN + rr;  // channel of lane 0
-      const bool ok = r0 < sh.M;
-      warp_tile_store(reinterpret_cast<uint8_t*>(wsm), lane, ow,
-                      [&](int r) -> bf16* { return ok ? blk + (int64_t)r * p.NN : nullptr; });
+      if (r0 < sh.M)
+        warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, ow, which == 0 ? &p.map_a : &p.map_b, rr, rit - lane,
+                            bb);
+      __syncwarp();  // the mask row has been read
       return;
     }
     const int m = m0 + rit;
@@ -263,15 +263,15 @@ struct EpiProjGate {
       uint32_t pk[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(v0[2 * i], v0[2 * i + 1]);
-      bf16* blk = p.gate + c0;
-      warp_tile_store(reinterpret_cast<uint8_t*>(wsm), lane, pk, [&](int r) -> bf16* {
-        return m_base + r < sh.M ? blk + (int64_t)(m_base + r) * p.C : nullptr;
-      });
+      if (m_base < sh.M)
+        warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk, &p.map_gate, c0, m_base, 0);
       return;
     }
     // a / b tile with lane = pair row (C < 128): each lane owns one row of the accumulator tile, which would
     // make 2-byte scattered stores; the 32x32 block is transposed through a per-warp smem tile so that each
     // lane writes 8 consecutive rows of four channels (4 x 16 bytes).
+    bulk_wait_read<0>();  // the block shares its memory with the gate tiles' staging buffers
+    __syncwarp();
     const float mk = pre.mk;
 #pragma unroll
     for (int i = 0; i < 32; ++i) wsm[lane * 33 + i] = v0[i] * sigmoid_fast(v1[i]) * mk;
@@ -302,6 +302,7 @@ struct EpiProjGate {
 template <bool RES>
 struct EpiOutGate {
   struct Params {
+    CUtensorMap map_out;  // !RES, identity rows: out leaves by TMA
     bf16* out;        // caller's rows x C; may be null when `sum` is wanted alone
     bf16* sum;        // RES: caller's rows x C
     const bf16* res;  // RES: residual input, caller's rows x C
@@ -311,7 +312,7 @@ struct EpiOutGate {
   };
   static constexpr bool kPaired = false;
   static constexpr bool kStaged = false;
-  static constexpr int kSmemPerWarp = 2048;
+  static constexpr int kSmemPerWarp = kTmaTiles;
   struct Pre {
     uint4 g[4];            // 32 gate logits of this lane's row
     uint4 r[RES ? 4 : 1];  // residual, in the arrangement of the stores (8 rows x 64 bytes per access)
@@ -325,7 +326,7 @@ struct EpiOutGate {
     for (int i = 0; i < 4; ++i) pre.g[i] = g[i];
   }
   __device__ static __forceinline__ void apply(const Params& p, const GemmShape& sh, int, int m, int n0,
-                                               const float (&v)[32], float* wsm, int lane, const Pre& pre) {
+                                               const float (&v)[32], float* wsm, int lane, const Pre& pre, int& buf) {
     uint32_t ow[16];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -339,7 +340,9 @@ struct EpiOutGate {
     uint8_t* tile = reinterpret_cast<uint8_t*>(wsm);
     if constexpr (RES)
       store_rows_added(tile, lane, ow, p.rows, m - lane, sh.M, p.C, n0, p.out, p.sum, pre.r);
-    else
+    else if (p.rows.identity) {
+      if (m - lane < sh.M) warp_tile_store_tma(tile, buf, lane, ow, &p.map_out, n0, m - lane, 0);
+    } else
       warp_tile_store(tile, lane, ow, [&](int r) { return row_address(p.out, p.rows, m - lane + r, sh.M, p.C, n0); });
   }
 };
@@ -347,6 +350,7 @@ struct EpiOutGate {
 // Backward of the gated projections: recomputed (p, g) pair + incoming d_a / d_b -> d_proj5[:, 0:4C]
 struct EpiGateSplitBwd {
   struct Params {
+    CUtensorMap map_d;  // stores: d_proj5 [R][5C]
     const bf16* da_cm;  // [B*C][NN]
     const bf16* db_cm;
     const float* mask;  // [R]
@@ -356,7 +360,7 @@ struct EpiGateSplitBwd {
   };
   static constexpr bool kPaired = true;
   static constexpr bool kStaged = true;
-  static constexpr int kSmemPerWarp = 32 * 33 * 4;
+  static constexpr int kSmemPerWarp = 4608;  // a 32 x 33 float block, then two staging tiles
   struct Pre {
     uint4 d[4];  // incoming gradient, channel-major: d[g] = 8 consecutive rows of channel 8*g + lane/4
     float mk;    // pair mask of this lane's row
@@ -384,6 +388,8 @@ struct EpiGateSplitBwd {
   // The prefetched channel-major block is transposed through smem so that afterwards lane = row finds
   // its 32 channels at wsm[lane * 33 ..].
   __device__ static __forceinline__ void stage(const Pre& pre, float* wsm, int lane) {
+    bulk_wait_read<0>();  // the staging tiles of the previous chunk lie in the same memory
+    __syncwarp();
     float* col = wsm + (8 * (lane & 3)) * 33 + (lane >> 2);
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -399,7 +405,7 @@ struct EpiGateSplitBwd {
   }
   __device__ static __forceinline__ void apply2(const Params& p, const GemmShape& sh, int, int m0, int rit, int n0,
                                                 int c0, const float (&v0)[32], const float (&v1)[32], float* wsm,
-                                                int lane, bool, const Pre& pre) {
+                                                int lane, bool, const Pre& pre, int& buf) {
     const int which = tile_kind(n0, p.C);  // 0: a, 1: b
     const int m = m0 + rit;
     // d = incoming gradient * mask; t = tanh(g / 2): sigmoid s = 0.5 + 0.5 t, s (1 - s) = 0.25 - 0.25 t^2.
@@ -423,13 +429,10 @@ struct EpiGateSplitBwd {
     }
     __syncwarp();  // the transposed gradient block has been consumed: its smem is reused as staging tiles
     const int m_base = m - lane;
-    bf16* dp = p.d_proj5 + which * 2 * p.C + c0;  // d_p block of row 0
-    warp_tile_store(reinterpret_cast<uint8_t*>(wsm), lane, pk0, [&](int r) -> bf16* {
-      return m_base + r < sh.M ? dp + (int64_t)(m_base + r) * 5 * p.C : nullptr;
-    });
-    warp_tile_store(reinterpret_cast<uint8_t*>(wsm) + 2048, lane, pk1, [&](int r) -> bf16* {
-      return m_base + r < sh.M ? dp + p.C + (int64_t)(m_base + r) * 5 * p.C : nullptr;  // d_g: C columns further
-    });
+    if (m_base >= sh.M) return;
+    const int col = which * 2 * p.C + c0;  // d_p; d_g lies C columns further
+    warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk0, &p.map_d, col, m_base, 0);
+    warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk1, &p.map_d, col + p.C, m_base, 0);
   }
 };
 
@@ -648,12 +651,12 @@ static int pack_weights(const float* p_in, const float* g_in, const float* p_out
 template <int C, class Epi>
 static int proj_gemm(const bf16* zln, const bf16* W5, int64_t R, int n_cols, const typename Epi::Params& ep,
                      int* status, cudaStream_t stream) {
-  // The gated epilogues are latency-bound: at C = 128 (four 32-column chunk pairs per tile) 16
+  // The gated epilogues are latency-bound: at C = 128 and 96 (four, three 32-column chunk pairs per tile) 16
   // epilogue warps keep one chunk pair each in flight; narrower tiles have work for 8 only.
   // The weight tile (2C rows x C) stays in shared memory while the CTA walks a contiguous range of row
   // tiles; only the activations stream.  CTAs j, j + n/3, j + 2n/3 walk the same rows for the a, b and
   // gate tiles at about the same time, so the activations come from DRAM once and from L2 twice.
-  using Cfg = GemmCfg<128, 2 * C, 128, false, 128, false, 4, (C == 128 ? 16 : 8), 2, (C + 63) / 64>;
+  using Cfg = GemmCfg<128, 2 * C, 128, false, 128, false, 4, (C >= 96 ? 16 : 8), 2, (C + 63) / 64>;
   GemmShape sh{(int)R, n_cols, C, 1, 0};
   return launch_gemm<Cfg, Epi>(zln, C, 0, W5, C, 0, sh, ep, status, stream);
 }
@@ -674,7 +677,11 @@ static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPack
                   dim3(ln_fwd_blocks<C>(R)), dim3(256), 0, stream, z, t.w.norm_in_w, t.w.norm_in_b, zln, t.mean_in,
                   t.rstd_in, rows, pm, t.mask_grid, R);
     TPF_LAUNCH_OK();
-    EpiProjGate::Params ep{(bf16*)t.a_cm, (bf16*)t.b_cm, (bf16*)t.gate, mask, C, NN};
+    EpiProjGate::Params ep{{}, {}, {}, (bf16*)t.a_cm, (bf16*)t.b_cm, (bf16*)t.gate, mask, C, NN};
+    if ((rc = make_store_tmap(&ep.map_a, t.a_cm, NN, C, NN, B, C * NN)) ||
+        (rc = make_store_tmap(&ep.map_b, t.b_cm, NN, C, NN, B, C * NN)) ||
+        (rc = make_store_tmap(&ep.map_gate, t.gate, C, R, C, 1, 0)))
+      return rc;
     if ((rc = proj_gemm<C, EpiProjGate>(zln, pk.W5, R, 5 * C, ep, status, stream))) return rc;
   }
   if (stages & 2) {
@@ -701,11 +708,12 @@ static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPack
       // chunk and 165 registers for it (wider tiles with two chunks, or with 16 warps of 96 registers, spill).  The
       // activations are read once more per tile column, from L2.
       using Cfg = GemmCfg<128, (C % 64 == 0 ? 64 : 32), 128, false, 128, false, 4>;
-      typename EpiOutGate<true>::Params ep{(bf16*)t.out, (bf16*)t.sum, z, (const bf16*)t.gate, rows, C};
+      typename EpiOutGate<true>::Params ep{{}, (bf16*)t.out, (bf16*)t.sum, z, (const bf16*)t.gate, rows, C};
       rc = launch_gemm<Cfg, EpiOutGate<true>>(xln, C, 0, pk.Wz, C, 0, sh, ep, status, stream);
     } else {
       using Cfg = GemmCfg<128, C, 128, false, 128, false, 4>;
-      typename EpiOutGate<false>::Params ep{(bf16*)t.out, nullptr, nullptr, (const bf16*)t.gate, rows, C};
+      typename EpiOutGate<false>::Params ep{{}, (bf16*)t.out, nullptr, nullptr, (const bf16*)t.gate, rows, C};
+      if (rows.identity && (rc = make_store_tmap(&ep.map_out, t.out, C, R, C, 1, 0))) return rc;
       rc = launch_gemm<Cfg, EpiOutGate<false>>(xln, C, 0, pk.Wz, C, 0, sh, ep, status, stream);
     }
     if (rc) return rc;
@@ -796,7 +804,8 @@ static int trimul_bwd_t(const TrimulCall& t, const TrimulGrads& g, const float* 
     using Cfg = GemmCfg<128, 128, 128, false, 128, false, 4>;
     using Epi = EpiStore<bf16>;
     GemmShape sh{(int)R, C, C, 1, 0};
-    typename Epi::Params ep{w.d_xln, C, 0};
+    typename Epi::Params ep;
+    if ((rc = epi_store_params<bf16>(&ep, w.d_xln, C, 0, sh))) return rc;
     if ((rc = launch_gemm<Cfg, Epi>(w.d_y, C, 0, pk.WzT, C, 0, sh, ep, status, stream))) return rc;
   }
   rc = bmm_bf16(w.d_y, C, 0, 1, xln, C, 0, 1, w.part_wz, C, (int64_t)C * C, 1, C, C, R, w.splits_wz, w.kps_wz, 128,
@@ -831,7 +840,8 @@ static int trimul_bwd_t(const TrimulCall& t, const TrimulGrads& g, const float* 
   if (stages & 4) {
   // 5. gated projections backward (recompute p, g) -> d_proj5[:, 0:4C]
   {
-    EpiGateSplitBwd::Params ep{w.da_cm, w.db_cm, mask, w.d_proj5, C, NN};
+    EpiGateSplitBwd::Params ep{{}, w.da_cm, w.db_cm, mask, w.d_proj5, C, NN};
+    if ((rc = make_store_tmap(&ep.map_d, w.d_proj5, 5 * C, R, 5 * C, 1, 0))) return rc;
     if ((rc = proj_gemm<C, EpiGateSplitBwd>(zln, pk.W5, R, 4 * C, ep, status, stream))) return rc;
   }
   // 6. d_zln = d_proj5 W5 ; dW5 = d_proj5^T zln
@@ -841,7 +851,8 @@ static int trimul_bwd_t(const TrimulCall& t, const TrimulGrads& g, const float* 
     using Cfg = GemmCfg<128, 128, 128, false, 128, false, 6>;
     using Epi = EpiStore<bf16>;
     GemmShape sh{(int)R, C, 5 * C, 1, 0};
-    typename Epi::Params ep{d_zln, C, 0};
+    typename Epi::Params ep;
+    if ((rc = epi_store_params<bf16>(&ep, d_zln, C, 0, sh))) return rc;
     if ((rc = launch_gemm<Cfg, Epi>(w.d_proj5, 5 * C, 0, pk.W5T, 5 * C, 0, sh, ep, status, stream))) return rc;
   }
   rc = bmm_bf16(w.d_proj5, 5 * C, 0, 1, zln, C, 0, 1, w.part_w5, C, (int64_t)5 * C * C, 1, 5 * C, C, R, w.splits_w5,
