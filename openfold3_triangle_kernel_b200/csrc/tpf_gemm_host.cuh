@@ -45,6 +45,14 @@ inline int epi_store_params(typename EpiStore<OutT>::Params* ep, OutT* D, int64_
   return TPF_OK;
 }
 
+// B resident in every CTA, or one tile column of it per CTA (GemmCfg::STAT 3 or 2) for R rows and nt tile columns?
+// Compared by the longest sequence of tiles a CTA gets: with few rows the second divides the work better.  At (nearly)
+// equal lengths the first wins, by its single read of A.
+inline bool resident_pays(int64_t R, int64_t nt) {
+  const int64_t mt = (R + 127) / 128, sms = sm_count();
+  return 8 * nt * ((mt + sms - 1) / sms) <= 9 * ((mt * nt + sms - 1) / sms);
+}
+
 template <class Cfg, class Epi>
 int launch_gemm(const void* A, int64_t lda, int64_t bsa, const void* B, int64_t ldb, int64_t bsb,
                 const GemmShape& sh, const typename Epi::Params& ep, int* status, cudaStream_t stream,
@@ -53,7 +61,7 @@ int launch_gemm(const void* A, int64_t lda, int64_t bsa, const void* B, int64_t 
   const int64_t tensor_batch = sh.k_per_split > 0 ? 1 : sh.batch;
   int rc = make_operand_tmap(&tmA, A, Cfg::A_MN, sh.M, sh.K, lda, tensor_batch, bsa, Cfg::SWZ_A, Cfg::BM, Cfg::BK);
   if (rc) return rc;
-  rc = make_operand_tmap(&tmB, B, Cfg::B_MN, sh.N, sh.K, ldb, tensor_batch, bsb, Cfg::SWZ_B, Cfg::BN, Cfg::BK);
+  rc = make_operand_tmap(&tmB, B, Cfg::B_MN, sh.N, sh.K, ldb, tensor_batch, bsb, Cfg::SWZ_B, Cfg::B_BOX, Cfg::BK);
   if (rc) return rc;
   auto kern = gemm_umma_kernel<Cfg, Epi>;
   constexpr int smem_bytes = Cfg::SMEM_BYTES + Cfg::EPI_WARPS * Epi::kSmemPerWarp;
@@ -64,14 +72,17 @@ int launch_gemm(const void* A, int64_t lda, int64_t bsa, const void* B, int64_t 
   const int tiles = sh.batch * mt * nt;
   int grid = sm_count();
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  if (grid > tiles) grid = tiles;
+  if (grid > (Cfg::RESIDENT ? mt : tiles)) grid = Cfg::RESIDENT ? mt : tiles;
   if (grid < 1) return TPF_OK;
   if constexpr (Cfg::STAT != 0) {
     const int k_len = sh.k_per_split > 0 ? sh.k_per_split : sh.K;
     TPF_REQUIRE(k_len <= Cfg::STAT_KB * Cfg::BK, TPF_ERR_UNSUPPORTED,
                 "gemm: K = %d exceeds the stationary operand buffer (%d)", k_len, Cfg::STAT_KB * Cfg::BK);
-    const int per = (tiles + grid - 1) / grid;  // contiguous tiles per CTA; CTAs that would get none are not launched
-    grid = (tiles + per - 1) / per;
+    if constexpr (Cfg::RESIDENT) {
+      TPF_REQUIRE(sh.batch == 1 && sh.N <= Cfg::B_ROWS, TPF_ERR_UNSUPPORTED, "gemm: B does not fit as a whole");
+    }
+    const int per = Cfg::RESIDENT ? 1 : (tiles + grid - 1) / grid;  // contiguous tiles per CTA; CTAs that would get none are not launched
+    if (!Cfg::RESIDENT) grid = (tiles + per - 1) / per;
   }
   launch_kernel(kern, dim3(grid), dim3(Cfg::THREADS), smem_bytes, stream, tmA, tmB, sh, ep, status);
   TPF_LAUNCH_OK();

@@ -357,9 +357,12 @@ int pair_attn_forward(const PairAttnCall& t, cudaStream_t stream) {
                        (t.N + 7) / 8 * 8, PairRows::make(t.N, t.N, false)};
     if (t.D == 32 && (rc = make_store_tmap(&ep.map, t.qkvg, t.D, R, t.D, 4 * t.H, R * t.D))) return rc;
     GemmShape sh{(int)R, (int)P, (int)C, 1, 0};
-    // 4 HD + H columns in as few, as full tiles as possible: 3 x 192 at H * D = 128, 3 x 96 at 64.  The weight tile
-    // stays in shared memory while the rows stream past (see GemmCfg).
-    if (HD <= 64) {
+    // 4 HD + H columns in as few, as full tiles as possible: 3 x 192 at H * D = 128, 3 x 96 at 64.  The weights, or as
+    // much of them as a tile needs, stay in shared memory while the rows stream past (see GemmCfg).
+    if (P > 272 && P <= 544 && resident_pays(R, 3)) {
+      using Cfg = GemmCfg<128, 192, 128, false, 128, false, 3, 8, 3, 2, 544>;
+      rc = launch_gemm<Cfg, EpiQkvg>(t.x, C, 0, pk.W, C, 0, sh, ep, status, stream);
+    } else if (HD <= 64) {
       using Cfg = GemmCfg<128, 96, 128, false, 128, false, 4, 8, 2, 2>;
       rc = launch_gemm<Cfg, EpiQkvg>(t.x, C, 0, pk.W, C, 0, sh, ep, status, stream);
     } else {

@@ -189,6 +189,14 @@ __device__ __forceinline__ void tma_load_3d(uint32_t elected, void* dst, const C
       ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(elected)
       : "memory");
 }
+// Brings a tile into L2 only.
+__device__ __forceinline__ void tma_prefetch_3d(uint32_t elected, const CUtensorMap* map, int c0, int c1, int c2) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
+      "@q cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];\n\t}"
+      ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(elected)
+      : "memory");
+}
 __device__ __forceinline__ void tma_load_4d(uint32_t elected, void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %7, 0;\n\t"

@@ -194,19 +194,25 @@ __device__ __forceinline__ void split_row(int row, int64_t NN, int M, int& bb, i
   }
 }
 
+struct ProjGateParams {
+  CUtensorMap map_a, map_b, map_gate;  // stores: [B][C][NN], [R][C]
+  bf16* a_cm;        // [B*C][NN]
+  bf16* b_cm;        // [B*C][NN]
+  bf16* gate;        // [R][C] raw gate logits
+  const float* mask; // [R]
+  int C;
+  int64_t NN;
+};
+// COMPACT (C = 128 with 16 warps and all weights in shared memory): one staging tile per warp, the warps' mask rows
+// behind the last of them.
+template <bool COMPACT>
 struct EpiProjGate {
-  struct Params {
-    CUtensorMap map_a, map_b, map_gate;  // stores: [B][C][NN], [R][C]
-    bf16* a_cm;        // [B*C][NN]
-    bf16* b_cm;        // [B*C][NN]
-    bf16* gate;        // [R][C] raw gate logits
-    const float* mask; // [R]
-    int C;
-    int64_t NN;
-  };
+  using Params = ProjGateParams;
   static constexpr bool kPaired = true;
   static constexpr bool kStaged = false;
-  static constexpr int kSmemPerWarp = 4608;  // two staging tiles and a mask row, or one 32 x 33 float block
+  static constexpr int kSmemPerWarp = COMPACT ? 2048 + 128 : 4608;  // staging and a mask row, or one 32 x 33 float block
+  static constexpr int kStagePitch = COMPACT ? 2048 : 4608;         // from warp to warp
+  static constexpr int kBufs = COMPACT ? 1 : 2;
   struct Pre {
     float mk;  // pair mask: of this lane's row, or (exchanged tile) of row `lane` of the warp's 32-row chunk
   };
@@ -226,7 +232,8 @@ struct EpiProjGate {
     const int which = tile_kind(n0, p.C);
     if (swap) {
       // lane = channel `rit`; v0[i] / v1[i] = projection / gate logit of pair row m0 + c0 + i
-      float* msm = wsm + kTmaTiles / 4;
+      const int ew = (threadIdx.x >> 5) - 2;
+      float* msm = COMPACT ? wsm + (16 - ew) * 512 + ew * 32 : wsm + kTmaTiles / 4;
       msm[lane] = pre.mk;
       __syncwarp();
       const uint64_t half2 = f2_pack(0.5f, 0.5f);
@@ -252,7 +259,7 @@ struct EpiProjGate {
       int bb, rr;
       split_row(r0, p.NN, sh.M, bb, rr);
       if (r0 < sh.M)
-        warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, ow, which == 0 ? &p.map_a : &p.map_b, rr, rit - lane,
+        warp_tile_store_tma<kBufs>(reinterpret_cast<uint8_t*>(wsm), buf, lane, ow, which == 0 ? &p.map_a : &p.map_b, rr, rit - lane,
                             bb);
       __syncwarp();  // the mask row has been read
       return;
@@ -264,9 +271,10 @@ struct EpiProjGate {
 #pragma unroll
       for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(v0[2 * i], v0[2 * i + 1]);
       if (m_base < sh.M)
-        warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk, &p.map_gate, c0, m_base, 0);
+        warp_tile_store_tma<kBufs>(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk, &p.map_gate, c0, m_base, 0);
       return;
     }
+    if constexpr (COMPACT) return;  // C = 128: both other tiles are exchanged
     // a / b tile with lane = pair row (C < 128): each lane owns one row of the accumulator tile, which would
     // make 2-byte scattered stores; the 32x32 block is transposed through a per-warp smem tile so that each
     // lane writes 8 consecutive rows of four channels (4 x 16 bytes).
@@ -360,7 +368,7 @@ struct EpiGateSplitBwd {
   };
   static constexpr bool kPaired = true;
   static constexpr bool kStaged = true;
-  static constexpr int kSmemPerWarp = 4608;  // a 32 x 33 float block, then two staging tiles
+  static constexpr int kSmemPerWarp = kTmaTiles;  // a 32 x 34 bf16 block, then two staging tiles
   struct Pre {
     uint4 d[4];  // incoming gradient, channel-major: d[g] = 8 consecutive rows of channel 8*g + lane/4
     float mk;    // pair mask of this lane's row
@@ -386,19 +394,19 @@ struct EpiGateSplitBwd {
     pre.mk = (m < sh.M) ? p.mask[m] : 0.f;
   }
   // The prefetched channel-major block is transposed through smem so that afterwards lane = row finds
-  // its 32 channels at wsm[lane * 33 ..].
+  // its 32 channels in the 34 bf16 from lane * 34 on (17 words a row: no bank conflicts either way).
   __device__ static __forceinline__ void stage(const Pre& pre, float* wsm, int lane) {
     bulk_wait_read<0>();  // the staging tiles of the previous chunk lie in the same memory
     __syncwarp();
-    float* col = wsm + (8 * (lane & 3)) * 33 + (lane >> 2);
+    uint16_t* col = reinterpret_cast<uint16_t*>(wsm) + (8 * (lane & 3)) * 34 + (lane >> 2);
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       const uint4 u = pre.d[g];
       const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        col[(2 * e) * 33 + 8 * g] = bf16_lo(w[e]);
-        col[(2 * e + 1) * 33 + 8 * g] = bf16_hi(w[e]);
+        col[(2 * e) * 34 + 8 * g] = (uint16_t)w[e];
+        col[(2 * e + 1) * 34 + 8 * g] = (uint16_t)(w[e] >> 16);
       }
     }
     __syncwarp();
@@ -413,10 +421,12 @@ struct EpiGateSplitBwd {
     // only the packed results stay live.
     const uint64_t mk2 = f2_pack(pre.mk, pre.mk);
     const uint64_t half2 = f2_pack(0.5f, 0.5f), quarter2 = f2_pack(0.25f, 0.25f), nquarter2 = f2_pack(-0.25f, -0.25f);
+    const uint32_t* drow = reinterpret_cast<const uint32_t*>(wsm) + lane * 17;
     uint32_t pk0[16], pk1[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const uint64_t d2 = f2_mul(f2_pack(wsm[lane * 33 + 2 * i], wsm[lane * 33 + 2 * i + 1]), mk2);
+      const uint32_t dw = drow[i];
+      const uint64_t d2 = f2_mul(f2_pack(bf16_lo(dw), bf16_hi(dw)), mk2);
       float h0, h1, a0, a1, b0, b1;
       f2_unpack(f2_mul(f2_pack(v1[2 * i], v1[2 * i + 1]), half2), h0, h1);
       const uint64_t t2 = f2_pack(tanh_fast(h0), tanh_fast(h1));
@@ -648,16 +658,20 @@ static int pack_weights(const float* p_in, const float* g_in, const float* p_out
   return TPF_OK;
 }
 
-template <int C, class Epi>
-static int proj_gemm(const bf16* zln, const bf16* W5, int64_t R, int n_cols, const typename Epi::Params& ep,
-                     int* status, cudaStream_t stream) {
+// BLOCKS: weight blocks of C rows (a_p, a_g, b_p, b_g and, forward, g).
+template <int C, int BLOCKS, class Epi, class EpiResident>
+static int proj_gemm(const bf16* zln, const bf16* W5, int64_t R, const typename Epi::Params& ep, int* status,
+                     cudaStream_t stream) {
   // The gated epilogues are latency-bound: at C = 128 and 96 (four, three 32-column chunk pairs per tile) 16
   // epilogue warps keep one chunk pair each in flight; narrower tiles have work for 8 only.
-  // The weight tile (2C rows x C) stays in shared memory while the CTA walks a contiguous range of row
-  // tiles; only the activations stream.  CTAs j, j + n/3, j + 2n/3 walk the same rows for the a, b and
-  // gate tiles at about the same time, so the activations come from DRAM once and from L2 twice.
+  // The weights (all of them, or a tile of 2C rows x C) stay in shared memory; only the activations stream.
+  const GemmShape sh{(int)R, BLOCKS * C, C, 1, 0};
+  if (resident_pays(R, (BLOCKS + 1) / 2)) {
+    using Cfg = GemmCfg<128, 2 * C, 128, false, 128, false, (C + 63) / 64, (C >= 96 ? 16 : 8), 3, (C + 63) / 64,
+                        BLOCKS * C, (C == 128 && BLOCKS == 5)>;
+    return launch_gemm<Cfg, EpiResident>(zln, C, 0, W5, C, 0, sh, ep, status, stream);
+  }
   using Cfg = GemmCfg<128, 2 * C, 128, false, 128, false, 4, (C >= 96 ? 16 : 8), 2, (C + 63) / 64>;
-  GemmShape sh{(int)R, n_cols, C, 1, 0};
   return launch_gemm<Cfg, Epi>(zln, C, 0, W5, C, 0, sh, ep, status, stream);
 }
 
@@ -677,12 +691,12 @@ static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPack
                   dim3(ln_fwd_blocks<C>(R)), dim3(256), 0, stream, z, t.w.norm_in_w, t.w.norm_in_b, zln, t.mean_in,
                   t.rstd_in, rows, pm, t.mask_grid, R);
     TPF_LAUNCH_OK();
-    EpiProjGate::Params ep{{}, {}, {}, (bf16*)t.a_cm, (bf16*)t.b_cm, (bf16*)t.gate, mask, C, NN};
+    ProjGateParams ep{{}, {}, {}, (bf16*)t.a_cm, (bf16*)t.b_cm, (bf16*)t.gate, mask, C, NN};
     if ((rc = make_store_tmap(&ep.map_a, t.a_cm, NN, C, NN, B, C * NN)) ||
         (rc = make_store_tmap(&ep.map_b, t.b_cm, NN, C, NN, B, C * NN)) ||
         (rc = make_store_tmap(&ep.map_gate, t.gate, C, R, C, 1, 0)))
       return rc;
-    if ((rc = proj_gemm<C, EpiProjGate>(zln, pk.W5, R, 5 * C, ep, status, stream))) return rc;
+    if ((rc = proj_gemm<C, 5, EpiProjGate<false>, EpiProjGate<C == 128>>(zln, pk.W5, R, ep, status, stream))) return rc;
   }
   if (stages & 2) {
     // k-contraction: batch = B*C problems of N x N x N
@@ -842,7 +856,7 @@ static int trimul_bwd_t(const TrimulCall& t, const TrimulGrads& g, const float* 
   {
     EpiGateSplitBwd::Params ep{{}, w.da_cm, w.db_cm, mask, w.d_proj5, C, NN};
     if ((rc = make_store_tmap(&ep.map_d, w.d_proj5, 5 * C, R, 5 * C, 1, 0))) return rc;
-    if ((rc = proj_gemm<C, EpiGateSplitBwd>(zln, pk.W5, R, 4 * C, ep, status, stream))) return rc;
+    if ((rc = proj_gemm<C, 4, EpiGateSplitBwd, EpiGateSplitBwd>(zln, pk.W5, R, ep, status, stream))) return rc;
   }
   // 6. d_zln = d_proj5 W5 ; dW5 = d_proj5^T zln
   bf16* d_zln = w.d_xln;

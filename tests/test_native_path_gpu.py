@@ -30,6 +30,23 @@ def test_trimul_any_length(N, direction):
         assert ao.rel_l2(w[k].grad.cpu(), ref["d_" + k]) <= 2.5e-2, k
 
 
+# Enough rows for the projections that keep all weights in shared memory (113 row tiles and more), with a ragged last
+# row tile; 145 tiles at N = 136, one round of 148 row tiles and a second one at N = 184.
+@pytest.mark.parametrize("N,C", [(119, 128), (136, 32), (136, 64), (120, 96), (184, 128)])
+def test_trimul_resident_weights(N, C):
+    t = trimul_inputs(1, N, C, seed=N, mask_mode="trailing10")
+    d_out = torch.randn(1, N, N, C, generator=torch.Generator().manual_seed(N)).bfloat16()
+    z = t["z"].cuda().requires_grad_(True)
+    w = {k: v.cuda().requires_grad_(True) for k, v in t["weights"].items()}
+    out = tk.turbo_trimul(z, "outgoing", t["mask"].cuda(), **w)
+    out.backward(d_out.cuda())
+    ref = to.trimul_forward_backward(t["z"], "outgoing", t["mask"], t["weights"], d_out)
+    assert ao.rel_l2(out.detach().cpu(), ref["out"]) <= 1e-2
+    assert ao.rel_l2(z.grad.cpu(), ref["dz"]) <= 2e-2
+    for k in ("p_in_weight", "g_in_weight", "g_out_weight", "norm_in_bias"):
+        assert ao.rel_l2(w[k].grad.cpu(), ref["d_" + k]) <= 2.5e-2, k
+
+
 @pytest.mark.parametrize("N,D,bias_type,mask_type", [(3, 16, torch.float32, torch.float16), (37, 32, torch.bfloat16, torch.bfloat16),
                                                      (66, 40, torch.float32, torch.float32), (64, 64, torch.bfloat16, torch.float32)])
 def test_attention_operand_types_and_strides(N, D, bias_type, mask_type):
@@ -53,7 +70,8 @@ def test_attention_operand_types_and_strides(N, D, bias_type, mask_type):
     assert torch.equal(q2.grad, q.grad)
 
 
-@pytest.mark.parametrize("N,C,H,D", [(1, 64, 4, 16), (9, 128, 4, 32), (65, 32, 2, 16), (130, 96, 3, 32), (40, 64, 8, 16)])
+@pytest.mark.parametrize("N,C,H,D", [(1, 64, 4, 16), (9, 128, 4, 32), (65, 32, 2, 16), (130, 96, 3, 32), (40, 64, 8, 16),
+                                     (119, 128, 4, 32)])
 def test_pair_block_any_length(N, C, H, D):
     from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
     from oracle.pair_block_oracle import block_params, pair_block_forward
