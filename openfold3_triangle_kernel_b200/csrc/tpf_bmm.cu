@@ -16,16 +16,53 @@ int bmm_status_fetch_and_clear(int* out) {
   return TPF_OK;
 }
 
+// Width of the output tiles.  A tile of 128 x BN moves (128 + BN) operand rows per k step through shared memory twice
+// (TMA writes them, the tensor pipe reads them) for 128 x BN products: at BN = 128 that is 256 bytes a clock at full
+// tensor rate where shared memory gives 128, so such tiles end at half the peak (1.16 of 2.3 PFLOP/s measured at
+// N = 1024), and wider ones at 0.6 (192) and 0.67 (256) of it.  The time of a tile is therefore taken as 128 + BN,
+// and the width with the shortest sequence of tiles per CTA is used; ragged widths and nearly empty last rounds count.
+// Wide tiles have fewer stages and a longer start and end, so they have to promise a tenth: at N = 384 (0.94 by this
+// count) 192 columns took 25 instead of 22 us.  128 channels, N = 520: 92 -> 68 us (192); N = 1024: 235 -> 208, N = 1536:
+// 742 -> 634 (256).
+static int tile_width(const GemmShape& sh) {
+  const int64_t mt = (int64_t)sh.batch * ((sh.M + 127) / 128), sms = sm_count();
+  int best = 128;
+  int64_t best_cost = INT64_MAX;
+  for (int bn = 128; bn <= 256; bn += 64) {
+    const int64_t tiles = mt * ((sh.N + bn - 1) / bn);
+    const int64_t cost = (tiles + sms - 1) / sms * (128 + bn) * (bn == 128 ? 9 : 10);
+    if (cost < best_cost) {
+      best = bn;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+template <int BN, int SWZ, bool A_MN, bool B_MN, typename OutT>
+int bmm_run(const void* A, int64_t lda, int64_t bsa, const void* B, int64_t ldb, int64_t bsb, void* D,
+            int64_t ldd, int64_t bsd, const GemmShape& sh, int* status, cudaStream_t stream) {
+  constexpr int kBK = (A_MN && B_MN) ? 64 : SWZ / 2;
+  constexpr int kBufs = BN == 256 ? 1 : 2;  // one staging tile per warp makes room for the fourth stage
+  constexpr int kFit = (BN == 128 ? 196608 : BN == 192 ? 163840 : 196608) / ((128 + BN) * kBK * 2);
+  using Cfg = GemmCfg<128, BN, SWZ, A_MN, SWZ, B_MN, (kFit > 8 ? 8 : kFit), (BN == 128 ? 8 : 16)>;
+  using Epi = EpiStore<OutT, kBufs>;
+  typename Epi::Params ep;
+  if (int rc = epi_store_params<OutT, kBufs>(&ep, reinterpret_cast<OutT*>(D), ldd, bsd, sh)) return rc;
+  return launch_gemm<Cfg, Epi>(A, lda, bsa, B, ldb, bsb, sh, ep, status, stream);
+}
+
 template <int SWZ, bool A_MN, bool B_MN, typename OutT>
 int bmm_dispatch(const void* A, int64_t lda, int64_t bsa, const void* B, int64_t ldb, int64_t bsb, void* D,
                  int64_t ldd, int64_t bsd, const GemmShape& sh, int* status, cudaStream_t stream) {
-  constexpr int kBK = (A_MN && B_MN) ? 64 : SWZ / 2;
-  constexpr int kStages = (196608 / (256 * kBK * 2)) > 8 ? 8 : (196608 / (256 * kBK * 2));
-  using Cfg = GemmCfg<128, 128, SWZ, A_MN, SWZ, B_MN, kStages>;
-  using Epi = EpiStore<OutT>;
-  typename Epi::Params ep;
-  if (int rc = epi_store_params<OutT>(&ep, reinterpret_cast<OutT*>(D), ldd, bsd, sh)) return rc;
-  return launch_gemm<Cfg, Epi>(A, lda, bsa, B, ldb, bsb, sh, ep, status, stream);
+  if constexpr (SWZ == 128 && sizeof(OutT) == 2) {  // the others (split K, narrow swizzles) are not tensor-bound
+    const int bn = tile_width(sh);
+    if (bn == 256)
+      return bmm_run<256, SWZ, A_MN, B_MN, OutT>(A, lda, bsa, B, ldb, bsb, D, ldd, bsd, sh, status, stream);
+    if (bn == 192)
+      return bmm_run<192, SWZ, A_MN, B_MN, OutT>(A, lda, bsa, B, ldb, bsb, D, ldd, bsd, sh, status, stream);
+  }
+  return bmm_run<128, SWZ, A_MN, B_MN, OutT>(A, lda, bsa, B, ldb, bsb, D, ldd, bsd, sh, status, stream);
 }
 
 int bmm_bf16(const void* A, int64_t lda, int64_t bsa, int a_mn, const void* B, int64_t ldb, int64_t bsb, int b_mn,

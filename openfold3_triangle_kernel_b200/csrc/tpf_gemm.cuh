@@ -204,7 +204,7 @@ constexpr int kTmaTiles = 4096;  // bytes of the two buffers
 
 // Plain stores.  OutT = __nv_bfloat16 or float; row-major D[b][m][n] with leading dimension ldd.  bf16 results leave by
 // TMA when the output has a tensor map (16-byte aligned rows), else from the registers.
-template <typename OutT>
+template <typename OutT, int BUFS = 2>
 struct EpiStore {
   struct Params {
     CUtensorMap map;
@@ -215,7 +215,7 @@ struct EpiStore {
   };
   static constexpr bool kPaired = false;
   static constexpr bool kStaged = false;
-  static constexpr int kSmemPerWarp = sizeof(OutT) == 2 ? kTmaTiles : 0;  // bytes of per-warp epilogue scratch
+  static constexpr int kSmemPerWarp = sizeof(OutT) == 2 ? 2048 * BUFS : 0;  // bytes of per-warp epilogue scratch
   // Global-memory operands of the epilogue, requested before the accumulator wait so that their
   // latency hides behind the UMMAs instead of stalling the (few) epilogue warps chunk by chunk.
   struct Pre {};
@@ -229,7 +229,7 @@ struct EpiStore {
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-        warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk, &p.map, n0, m - lane, b);
+        warp_tile_store_tma<BUFS>(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk, &p.map, n0, m - lane, b);
         return;
       }
     }

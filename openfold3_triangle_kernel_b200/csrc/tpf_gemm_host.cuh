@@ -31,8 +31,8 @@ inline int make_store_tmap(CUtensorMap* tm, const void* base, int64_t cols, int6
   return make_tmap_bf16(tm, base, 3, dims, strides, box, 64);
 }
 // Parameters of EpiStore; bf16 outputs with 16-byte aligned rows get a tensor map.
-template <typename OutT>
-inline int epi_store_params(typename EpiStore<OutT>::Params* ep, OutT* D, int64_t ldd, int64_t batch_stride,
+template <typename OutT, int BUFS = 2>
+inline int epi_store_params(typename EpiStore<OutT, BUFS>::Params* ep, OutT* D, int64_t ldd, int64_t batch_stride,
                             const GemmShape& sh) {
   *ep = {};
   ep->D = D;

@@ -97,3 +97,20 @@ def test_bmm_many_tiles_per_cta():
     torch.cuda.synchronize()
     assert C.device_status() == 0
     assert _rel(d.float(), torch.matmul(a.float(), b.float().transpose(1, 2))) < TOL_BF16
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (1, 1), (1, 0), (0, 1)])
+@pytest.mark.parametrize("N,K", [(136, 72), (192, 200), (200, 64), (256, 8)])
+def test_bmm_wide_tiles(a_mn, b_mn, N, K):
+    """Enough problems that one wide tile per problem (192 columns up to N = 192, 256 above) is the shortest schedule."""
+    M, batch = 104, 130
+    gen = torch.Generator(device="cuda").manual_seed(N + K)
+    a_buf, a, lda, bsa = _operand(M, K, batch, a_mn, gen)
+    b_buf, b, ldb, bsb = _operand(N, K, batch, b_mn, gen)
+    d = torch.full((batch + 1, M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    C.call("tpf_bmm_bf16", C.ptr(a_buf), lda, bsa, a_mn, C.ptr(b_buf), ldb, bsb, b_mn, C.ptr(d), N, M * N, 0,
+           M, N, K, batch, 0, 128, C.current_stream())
+    torch.cuda.synchronize()
+    assert C.device_status() == 0
+    assert _rel(d[:batch].float(), torch.matmul(a.float(), b.float().transpose(1, 2))) < TOL_BF16
+    assert torch.isnan(d[batch].float()).all()
