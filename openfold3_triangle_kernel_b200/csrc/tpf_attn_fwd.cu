@@ -250,9 +250,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         load_k();
         load_bv();
       }
-      if (tiles > 2) load_k();
+      if (tiles > 2 && KT > 1) load_k();
       issue_qk();
       if (tiles > 1) issue_qk();
+      if (tiles > 2 && KT == 1) {
+        // the third tile is the third item, whose Q goes where the first one's lies: not before that has been used
+        mbar_wait(&s_full[0], 0, wctx);
+        load_k();
+      }
       int j = 0;
       for (int t = 0; t < tiles; ++t) {
         const int buf = t & 1;

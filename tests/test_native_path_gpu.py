@@ -70,6 +70,20 @@ def test_attention_operand_types_and_strides(N, D, bias_type, mask_type):
     assert torch.equal(q2.grad, q.grad)
 
 
+# Ragged ends of the gradient tiles (32-row blocks, 128-row tiles, strips of 384 keys), and more planes per CTA than the
+# backward kernel keeps records of, or than the forward kernel has buffers for (900 and 1800 one-tile planes).
+@pytest.mark.parametrize("O,N,D", [(2, 31, 32), (2, 33, 16), (3, 96, 32), (2, 129, 64), (2, 385, 16), (2, 416, 32), (450, 20, 32),
+                                   (900, 50, 16)])
+def test_attention_gradient_tiles(O, N, D):
+    a = attention_inputs(1, O, 2, N, D, seed=N, mask_mode="trailing15")
+    q, k, v, bias = (a[n].cuda().requires_grad_(True) for n in ("q", "k", "v", "pair_bias"))
+    d_out = torch.randn(1, O, N, 2, D, generator=torch.Generator().manual_seed(N)).bfloat16()
+    tk.turbo_attention(q, k, v, pair_bias=bias, res_mask=a["res_mask"].cuda()).backward(d_out.cuda())
+    ref = ao.attention_forward_backward(a["q"], a["k"], a["v"], a["pair_bias"], a["res_mask"], d_out)
+    for name, got in (("dq", q.grad), ("dk", k.grad), ("dv", v.grad), ("dbias", bias.grad)):
+        assert ao.rel_l2(got.cpu(), ref[name]) <= 1e-2, name
+
+
 @pytest.mark.parametrize("N,C,H,D", [(1, 64, 4, 16), (9, 128, 4, 32), (65, 32, 2, 16), (130, 96, 3, 32), (40, 64, 8, 16),
                                      (119, 128, 4, 32)])
 def test_pair_block_any_length(N, C, H, D):
