@@ -172,6 +172,7 @@ __device__ __forceinline__ void tc_fence_after() {
 // ----------------------------------------------------------------------------
 // TMA tile loads (global -> this CTA's shared memory, completion on an mbarrier)
 // ----------------------------------------------------------------------------
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -223,6 +224,15 @@ __device__ __forceinline__ void tma_store_3d(uint32_t elected, const CUtensorMap
       "@q cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];\n\t"
       "@q cp.async.bulk.commit_group;\n\t}"
       ::"l"(map), "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(elected)
+      : "memory");
+}
+__device__ __forceinline__ void tma_store_5d(uint32_t elected, const CUtensorMap* map, const void* src, int c0, int c1,
+                                             int c2, int c3, int c4) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+      "@q cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];\n\t"
+      "@q cp.async.bulk.commit_group;\n\t}"
+      ::"l"(map), "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(elected)
       : "memory");
 }
 template <int N>
@@ -446,6 +456,13 @@ __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc, bo
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gsrc),
                "r"(valid ? 16 : 0)
                : "memory");
+}
+// 4 bytes; zeros when !ok.  cp_async_arrive: one arrival on `bar` once this thread's copies so far have landed.
+__device__ __forceinline__ void cp_async_4(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
