@@ -212,13 +212,15 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const bf16* __restrict__ d_
 //   weight gradients: out[r][c] = sum over splits of part[s][m][c], rows routed in blocks of C to up to five
 //                     destinations (W5 = [a_p; a_g; b_p; b_g; g]);
 //   norm gradients:   out[j] = sum over CTAs of partials[blk][j], j < 2C, the halves going to d_gamma and d_beta.
-// A CTA owns 32 output elements; warp g adds its contiguous range of terms in ascending order (a batch of 8 loads is in
-// flight before the first add), then the 8 range sums are added in range order: a fixed summation tree, no atomics.
+// A CTA owns 32 output elements (8 of a job with many terms); thread group g adds its contiguous range of terms in
+// ascending order (a batch of 8 loads is in flight before the first add), then the 8 (32) range sums are added in range
+// order: a fixed summation tree, no atomics.
 struct FoldJob {
   const float* part;
   int terms, width;   // width: distance between consecutive terms
   int used;           // outputs wanted (the columns beyond are padding)
   int C;              // elements per destination row block: C * C (weights) or C (norms)
+  int log_lanes;      // a CTA folds 1 << log_lanes outputs, with 256 >> log_lanes threads each
   float* dst[5];
 };
 struct FoldJobs {
@@ -228,33 +230,31 @@ struct FoldJobs {
 };
 static __global__ void __launch_bounds__(256) fold_kernel(const __grid_constant__ FoldJobs jobs) {
   griddep_wait();
-  __shared__ float red[8][32];
+  __shared__ float red[256];
   int n = 0;
   while (n + 1 < jobs.n_jobs && (int)blockIdx.x >= jobs.first[n + 1]) ++n;
   const FoldJob& jb = jobs.job[n];
-  const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i = (blockIdx.x - jobs.first[n]) * 32 + lane;
-  const int per = (jb.terms + 7) / 8;
+  const int lanes = 1 << jb.log_lanes, groups = 256 >> jb.log_lanes;
+  const int g = threadIdx.x >> jb.log_lanes, lane = threadIdx.x & (lanes - 1);
+  const int i = (blockIdx.x - jobs.first[n]) * lanes + lane;
+  const int per = (jb.terms + groups - 1) >> (8 - jb.log_lanes);
   const int k0 = g * per, k1 = min(jb.terms, k0 + per);
   float s = 0.f;
   if (i < jb.used) {
     const float* src = jb.part + i;
-    int k = k0;
-    for (; k + 8 <= k1; k += 8) {
+    for (int k = k0; k < k1; k += 8) {
       float v[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = src[(int64_t)(k + u) * jb.width];
+      for (int u = 0; u < 8; ++u) v[u] = k + u < k1 ? src[(int64_t)(k + u) * jb.width] : 0.f;
 #pragma unroll
       for (int u = 0; u < 8; ++u) s = __fadd_rn(s, v[u]);
     }
-    for (; k < k1; ++k) s = __fadd_rn(s, src[(int64_t)k * jb.width]);
   }
-  red[g][lane] = s;
+  red[threadIdx.x] = s;
   __syncthreads();
   if (g == 0 && i < jb.used) {
-    float t = red[0][lane];
-#pragma unroll
-    for (int w = 1; w < 8; ++w) t = __fadd_rn(t, red[w][lane]);
+    float t = red[lane];
+    for (int w = 1; w < groups; ++w) t = __fadd_rn(t, red[w * lanes + lane]);
     const int d = i / jb.C;
     jb.dst[d][i - d * jb.C] = t;
   }
@@ -265,8 +265,12 @@ struct FoldList {
   void add(const float* part, int terms, int width, int C, float* d0, float* d1 = nullptr, float* d2 = nullptr,
            float* d3 = nullptr, float* d4 = nullptr, int used = 0) {
     if (used == 0) used = width;
-    j.job[j.n_jobs] = FoldJob{part, terms, width, used, C, {d0, d1, d2, d3, d4}};
-    j.first[j.n_jobs + 1] = j.first[j.n_jobs] + (used + 31) / 32;
+    // Few outputs with many terms (the norms: 2 C outputs, a term per CTA of the backward pass) are a chain of load
+    // latencies: 8 outputs per CTA (a sector of each row) leave 32 threads for the terms of each, where 32 outputs left
+    // 8 threads with 148 terms each.
+    const int log_lanes = terms > 256 ? 3 : 5;
+    j.job[j.n_jobs] = FoldJob{part, terms, width, used, C, log_lanes, {d0, d1, d2, d3, d4}};
+    j.first[j.n_jobs + 1] = j.first[j.n_jobs] + ((used + (1 << log_lanes) - 1) >> log_lanes);
     ++j.n_jobs;
   }
   int launch(cudaStream_t stream) {
