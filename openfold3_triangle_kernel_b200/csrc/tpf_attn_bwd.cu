@@ -167,7 +167,11 @@ struct BwdWalk {
 // TMEM (S and dP), forms P and dS, and keeps the bf16 results packed in 32 registers; only the
 // shared-memory stores wait for the UMMAs of the previous tile to release the P / dS tiles, so
 // the arithmetic of tile t+1 overlaps the dV / dK / dQ UMMAs of tile t.
-template <class Cfg>
+//
+// RAGGED: a warp whose rows or keys of a tile all lie beyond the last one only stores zeros and keeps the barriers going;
+// the others have the arithmetic pipes to themselves.  At N = 257 that is half of the 32 x 32 blocks (D = 64: 263 -> 255 us),
+// at N = 400 a third (412 -> 397 us).  The test costs 2 % of a kernel that has no such warps.
+template <class Cfg, bool RAGGED>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -647,6 +651,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const bool general = tail || __any_sync(0xffffffffu, mask_row[lane] != 0.f);
 
       uint32_t ppk[16], dpk[16];  // bf16 pairs of P and dS of this thread's 32 keys
+      bool dead = false;
+      if constexpr (RAGGED) dead = qt * 128 + (int)lane_base >= p.N || kt * 128 + 32 * part >= p.N;
+      if (dead) {
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(sdp_free);
+          mbar_arrive(&b_empty[b_s]);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) ppk[i] = dpk[i] = 0u;
+      } else
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) {  // 16 keys per step
         uint32_t rs[16], rd[16];
@@ -1130,9 +1145,10 @@ int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
                     const CUtensorMap& tb, const CUtensorMap& tmk, const CUtensorMap& tdk, const CUtensorMap& tdv,
                     AttnBwdParams& p, int* status, int grid, cudaStream_t stream) {
   using Cfg = AttnBwdCfg<D>;
-  auto kern = attn_bwd_kernel<Cfg>;
-  static PerDeviceOnce once;  // per instantiation
-  if (int rc = ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, once)) return rc;
+  const bool ragged = p.N % 128 != 0 && p.N % 128 <= 96;  // some 32-row (32-key) block of the last tile is empty
+  auto kern = ragged ? attn_bwd_kernel<Cfg, true> : attn_bwd_kernel<Cfg, false>;
+  static PerDeviceOnce once[2];  // per instantiation
+  if (int rc = ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, once[ragged])) return rc;
   launch_kernel(kern, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, tq, tk, tv, tdo, tb, tmk, tdk, tdv, p, status);
   TPF_LAUNCH_OK();
   return TPF_OK;
