@@ -134,11 +134,14 @@ int64_t tpf_attn_bwd_static_scratch_capacity(void);
 
 /* tpf_attn_bwd for callers that cannot allocate device memory (code between stream-capture
  * begin/end, plugin or real-time hosts that get their memory once at start-up, runtimes that
- * own the device heap): same inputs, outputs and results as tpf_attn_bwd, but the scratch is a
+ * own the device heap): same inputs and outputs as tpf_attn_bwd, but the scratch is a
  * fixed 16 MiB array inside the library image instead of a caller workspace.  The call allocates
  * and frees nothing.  This entry point has no counterpart in the reference.
- *  - Shapes whose scratch need (tpf_attn_bwd_workspace_bytes) exceeds the capacity are rejected
- *    with TPF_ERR_WORKSPACE and a message; nothing is launched.
+ *  - Shapes whose tpf_attn_bwd_workspace_bytes fits the capacity give the bits of tpf_attn_bwd.  For larger ones
+ *    the outer rows of dbias are summed in fewer chunks (fp32, another fixed order; the other results are the same
+ *    bits), down to none: then the call needs only the dQ sums, min(SMs, B*O*H) * N * D * 4 bytes for more than
+ *    384 keys (D <= 32) or 128 keys (D = 64).  If those exceed the capacity the shape is rejected with
+ *    TPF_ERR_WORKSPACE and a message; nothing is launched.
  *  - The first call on each device looks up the array's device address (a synchronous runtime
  *    query); make that first call outside any stream capture.
  *  - All calls on a device share the one array and it keeps whatever the last call left there.

@@ -1289,13 +1289,15 @@ int launch_attn_dbias(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 // How the outer planes of one dBias tile are split into independent chunks: the split with the shortest schedule, i.e.
 // waves of CTAs (one per SM) times planes per CTA, plus about three planes' time for a CTA's start and its partial
 // plane.  With one chunk whenever there are more tiles than SMs (N = 1021: 256 tiles) the last wave left half the
-// machine idle.
-static void dbias_plan(int64_t B, int64_t O, int64_t H, int64_t N, int64_t G, int* n_chunks, int* chunk_len) {
+// machine idle.  Chunk planes take at most `max_bytes`; one chunk needs none.
+static void dbias_plan(int64_t B, int64_t O, int64_t H, int64_t N, int64_t G, double max_bytes, int* n_chunks,
+                       int* chunk_len) {
   const int64_t tiles = G * H * ((N + 127) / 128) * ((N + 127) / 128);
   const int64_t planes = (B / G) * O;
+  const double chunk_bytes = 4.0 * G * H * N * N;
   const int64_t sms = sm_count();
   int64_t best = 0, best_cost = 0;
-  for (int64_t c = 1; c <= planes && (c == 1 || tiles * c <= 8 * sms); ++c) {
+  for (int64_t c = 1; c <= planes && (c == 1 || (tiles * c <= 8 * sms && c * chunk_bytes <= max_bytes)); ++c) {
     const int64_t len = (planes + c - 1) / c;
     const int64_t cost = (tiles * c + sms - 1) / sms * (len + 3);
     if (best == 0 || cost < best_cost) {
@@ -1310,13 +1312,13 @@ static void dbias_plan(int64_t B, int64_t O, int64_t H, int64_t N, int64_t G, in
 
 int64_t attn_dbias_workspace_bytes(int64_t B, int64_t O, int64_t H, int64_t N, int64_t G) {
   int c, len;
-  dbias_plan(B, O, H, N, G, &c, &len);
+  dbias_plan(B, O, H, N, G, kNoByteLimit, &c, &len);
   return c > 1 ? (int64_t)c * G * H * N * N * 4 : 0;
 }
 
 int64_t attn_dbias_rows_workspace_bytes(int64_t B, int64_t O, int64_t H, int64_t N, int64_t G) {
   int c, len;
-  dbias_plan(B, O, H, N, G, &c, &len);
+  dbias_plan(B, O, H, N, G, kNoByteLimit, &c, &len);
   return (int64_t)c * G * H * N * N * 4;
 }
 
@@ -1324,7 +1326,7 @@ int attn_bwd_dbias(const void* q, const void* k, const void* v, const void* d_ou
                    const int64_t* k_strides, const int64_t* v_strides, const float* lse, const float* delta,
                    const float* mask, int64_t mask_pitch, const void* bias, int64_t bias_pitch, int64_t bias_batch,
                    float* dbias, void* workspace, int64_t workspace_bytes, int64_t B, int64_t O, int64_t H, int64_t N,
-                   int64_t D, float scale, cudaStream_t stream) {
+                   int64_t D, float scale, cudaStream_t stream, double dbias_limit) {
   TPF_REQUIRE(dbias != nullptr, TPF_ERR_INVALID_ARGUMENT, "attn_bwd: dbias is NULL");
   TPF_REQUIRE_ALIGNED16(dbias, "attn_bwd", "dbias");  // rows are written with float4 stores
   AttnCall c = {};
@@ -1343,16 +1345,16 @@ int attn_bwd_dbias(const void* q, const void* k, const void* v, const void* d_ou
   c.dos[0] = O * N * H * D; c.dos[1] = N * H * D; c.dos[2] = D; c.dos[3] = H * D;
   c.delta = const_cast<float*>(delta);
   c.dbias = dbias;
+  c.dbias_limit = dbias_limit;
   return attn_backward_bias(c, workspace, workspace_bytes, stream);
 }
 
 int attn_backward_bias(const AttnCall& c, void* workspace, int64_t workspace_bytes, cudaStream_t stream) {
   const int64_t B = c.B, O = c.O, H = c.H, N = c.N, D = c.D, G = c.G;
   int n_chunks, chunk_len;
-  dbias_plan(B, O, H, N, G, &n_chunks, &chunk_len);
+  dbias_plan(B, O, H, N, G, c.dbias_limit, &n_chunks, &chunk_len);
   const bool rows = c.dbias == nullptr;  // fp32 planes go to the workspace, bf16 rows come out
-  const int64_t need =
-      rows ? attn_dbias_rows_workspace_bytes(B, O, H, N, G) : attn_dbias_workspace_bytes(B, O, H, N, G);
+  const int64_t need = n_chunks > 1 || rows ? n_chunks * G * H * N * N * 4 : 0;
   TPF_REQUIRE(need == 0 || (workspace && workspace_bytes >= need), TPF_ERR_WORKSPACE,
               "attn_bwd: dBias workspace of %lld bytes required, %lld given", (long long)need,
               (long long)workspace_bytes);
@@ -1436,11 +1438,13 @@ int attn_bwd_static_scratch(const void* q, const void* k, const void* v, const v
   TPF_REQUIRE(D == 16 || D == 32 || D == 64, TPF_ERR_UNSUPPORTED,
               "attn_bwd (library scratch): head dim %lld not in {16,32,64}", (long long)D);
   const int64_t ws_a = (attn_bwd_workspace_bytes(B, O, H, N, D) + 255) / 256 * 256;
-  const int64_t ws_b = (attn_dbias_workspace_bytes(B, O, H, N, bias_batch) + 255) / 256 * 256;
-  TPF_REQUIRE(ws_a + ws_b <= kStaticScratchBytes, TPF_ERR_WORKSPACE,
+  // The dQ sums have to fit; dBias takes as many chunk planes as the rest of the array holds, down to one chunk, which
+  // needs none.  (Chunks planned without that limit took up to 8 * SMs tiles of 64 KiB: N = 640, H = 4 would need 74 MiB.)
+  TPF_REQUIRE(ws_a <= kStaticScratchBytes, TPF_ERR_WORKSPACE,
               "attn_bwd (library scratch): this shape needs %lld bytes of scratch, the built-in array holds %lld; "
               "use tpf_attn_bwd with a caller-provided workspace",
-              (long long)(ws_a + ws_b), (long long)kStaticScratchBytes);
+              (long long)ws_a, (long long)kStaticScratchBytes);
+  const int64_t ws_b = kStaticScratchBytes - ws_a;
   void* base = nullptr;
   int rc = static_scratch_address(&base);
   if (rc) return rc;
@@ -1451,7 +1455,7 @@ int attn_bwd_static_scratch(const void* q, const void* k, const void* v, const v
   if (rc) return rc;
   return attn_bwd_dbias(q, k, v, d_out, q_strides, k_strides, v_strides, lse, delta, mask, mask_pitch, bias,
                         bias_pitch, bias_batch, dbias, static_cast<char*>(base) + ws_a, ws_b, B, O, H, N, D, scale,
-                        stream);
+                        stream, (double)ws_b);
 }
 
 }  // namespace tpf

@@ -1,6 +1,7 @@
 // extern "C" surface of libtpf_b200.so (declarations: include/tpf_b200.h).
 #include "../../include/tpf_b200.h"
 #include "tpf_host.cuh"
+#include "tpf_internal.h"
 
 namespace tpf {
 
@@ -32,7 +33,7 @@ int attn_bwd_dbias(const void* q, const void* k, const void* v, const void* d_ou
                    const int64_t* k_strides, const int64_t* v_strides, const float* lse, const float* delta,
                    const float* mask, int64_t mask_pitch, const void* bias, int64_t bias_pitch, int64_t bias_batch,
                    float* dbias, void* workspace, int64_t workspace_bytes, int64_t B, int64_t O, int64_t H, int64_t N,
-                   int64_t D, float scale, cudaStream_t stream);
+                   int64_t D, float scale, cudaStream_t stream, double dbias_limit);
 
 int64_t attn_bwd_static_scratch_capacity();
 int attn_bwd_static_scratch(const void* q, const void* k, const void* v, const void* d_out, const int64_t* q_strides,
@@ -158,7 +159,7 @@ int tpf_attn_bwd_stages(const void* q, const void* k, const void* v, const void*
   if (!(stages & TPF_ATTN_BWD_STAGE_DBIAS)) return TPF_OK;
   return tpf::attn_bwd_dbias(q, k, v, d_out, q_strides, k_strides, v_strides, lse, delta, mask, mask_pitch, bias,
                              bias_pitch, bias_batch, dbias, static_cast<char*>(workspace) + ws_a, ws_b, B, O, H, N, D,
-                             scale, st);
+                             scale, st, tpf::kNoByteLimit);
 }
 
 int64_t tpf_attn_bwd_static_scratch_capacity(void) { return tpf::attn_bwd_static_scratch_capacity(); }

@@ -20,6 +20,8 @@ int attn_prep(const PrepSource& bias, int64_t G, int64_t H, void* bias_dst, int6
               int64_t B, int64_t O, float* mask_dst, int64_t mask_pitch, int64_t N, cudaStream_t stream,
               float mask_add = 0.f, float mask_mul = 1.f);
 
+constexpr double kNoByteLimit = 1e300;
+
 // One triangle-attention problem.  Strides are in elements, order (b, o, h, n); the last dimension is contiguous.
 struct AttnCall {
   int64_t B, O, H, N, D, G;  // G: bias batch, 1 or B
@@ -44,6 +46,7 @@ struct AttnCall {
   float* dbias;              // fp32 [G,H,N,N]; or nullptr with dbias_rows:
   void* dbias_rows;          // bf16, row (g, i, j) of pitch dbias_ld holds the H bias gradients of pair (i, j), then
   int64_t dbias_ld;          //   zeros up to a multiple of 8 columns
+  double dbias_limit = kNoByteLimit;  // most bytes of workspace that chunk planes of dbias may take
 };
 int attn_forward(const AttnCall& c, cudaStream_t stream);
 int attn_backward_qkv(const AttnCall& c, void* workspace, int64_t workspace_bytes, cudaStream_t stream);

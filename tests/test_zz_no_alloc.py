@@ -1,8 +1,8 @@
 """tpf_attn_bwd_static_scratch: the backward pass for hosts that cannot allocate device memory
 (code inside a stream capture, plugin hosts that receive their memory once, runtimes that own the
 device heap).  It must give exactly what tpf_attn_bwd gives with a caller workspace, on
-repeated calls that reuse the library's built-in scratch array, and must refuse shapes whose
-scratch would not fit.  Collected last so a failure here cannot hide other results."""
+repeated calls that reuse the library's built-in scratch array, as long as the workspace fits that array; for larger ones
+it sums dBias in fewer chunks, and it must refuse shapes whose dQ sums would not fit.  Collected last so a failure here cannot hide other results."""
 import math
 
 import pytest
@@ -69,6 +69,29 @@ def test_static_scratch_matches_workspace_entry_twice_in_a_row(shape):
             # same kernels, same summation order: identical bits
             assert torch.equal(got[n].view(torch.uint8), ref[n].view(torch.uint8)), n
             assert torch.isfinite(got[n].float()).all(), n
+
+
+# Shapes whose unlimited dBias plan does not fit the array: one and several key strips, several chunks and one chunk left.
+@pytest.mark.parametrize("shape", [(1, 400, 4, 400, 32), (1, 300, 4, 512, 16), (1, 40, 4, 800, 32), (1, 256, 8, 256, 32),
+                                   (1, 50, 4, 416, 64)])
+def test_static_scratch_limits_the_dbias_chunks(shape):
+    B, O, H, N, D = shape
+    lib = C.load()
+    need = lib.tpf_attn_bwd_workspace_bytes(B, O, H, N, D, 1)
+    assert need > lib.tpf_attn_bwd_static_scratch_capacity()
+    t = _buffers(B, O, H, N, D, 5)
+    ref, got = _grads(B, O, H, N, D), _grads(B, O, H, N, D)
+    ws = torch.empty(need, device="cuda", dtype=torch.uint8)
+    _call("tpf_attn_bwd", t, ref, shape, extra=(C.ptr(ws), need))
+    _call("tpf_attn_bwd_static_scratch", t, got, shape)
+    torch.cuda.synchronize()
+    assert C.device_status() == 0
+    for n in ("dq", "dk", "dv", "delta"):
+        assert torch.equal(got[n].view(torch.uint8), ref[n].view(torch.uint8)), n
+    # the same O fp32 terms added in another order: each sum is off by at most O * 2^-24 of the sum of its terms'
+    # magnitudes, which for terms of either sign is about sqrt(O) times the sum itself; two sums are compared
+    err = (got["dbias"] - ref["dbias"]).norm() / ref["dbias"].norm()
+    assert err <= 2 * O ** 1.5 * 2.0 ** -24, float(err)
 
 
 def test_static_scratch_rejects_shapes_that_do_not_fit():
