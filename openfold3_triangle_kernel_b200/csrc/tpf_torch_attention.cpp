@@ -93,10 +93,10 @@ Tensor pad_lane(const Tensor& t, int64_t lane) {
 }
 
 // The autograd node of the eager call.  It takes the caller's tensors in the caller's shapes, so that no view nodes
-// surround it.
+// surround it.  An absent mask is an empty optional: the node cannot take an undefined tensor as an input.
 struct AttentionFn : public torch::autograd::Function<AttentionFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& q_in, const Tensor& k_in, const Tensor& v_in,
-                               const Tensor& bias_in, const Tensor& mask_in, bool save) {
+                               const Tensor& bias_in, const std::optional<Tensor>& mask_in, bool save) {
     const auto qs = q_in.sizes();
     const int64_t nd = q_in.dim(), D = qs[nd - 1], lane = D <= 16 ? 16 : D <= 32 ? 32 : 64;
     Shape s{1, qs[nd - 4], qs[nd - 3], qs[nd - 2], lane, 1};
@@ -124,7 +124,7 @@ struct AttentionFn : public torch::autograd::Function<AttentionFn> {
     if (shared) bias = bias.dim() == 5 ? bias.select(0, 0) : bias.reshape({1, s.H, s.N, s.N});  // [1,H,N,N]
     else bias = expanded(bias, s.B).select(1, 0);                                              // [B,H,N,N]
     Tensor mask;
-    if (mask_in.defined()) mask = expanded(mask_in.detach(), s.B).select(3, 0).select(2, 0);   // [B,O,N]
+    if (mask_in) mask = expanded(mask_in->detach(), s.B).select(3, 0).select(2, 0);   // [B,O,N]
     else mask = at::zeros({s.B, s.O, s.N}, q.options().dtype(at::kFloat));
 
     const double scale = 1.0 / std::sqrt((double)D);
@@ -218,13 +218,13 @@ py::object py_attention(py::handle hq, py::handle hk, py::handle hv, py::handle 
     if (!THPVariable_Check(h.ptr())) return py::none();
   const Tensor &q = THPVariable_Unpack(hq.ptr()), &k = THPVariable_Unpack(hk.ptr()), &v = THPVariable_Unpack(hv.ptr()),
                &bias = THPVariable_Unpack(hb.ptr());
-  Tensor mask;
+  std::optional<Tensor> mask;
   if (!hm.is_none()) {
     if (!THPVariable_Check(hm.ptr())) return py::none();
     mask = THPVariable_Unpack(hm.ptr());
   }
   if (!plain_context() || !plain_cuda(q) || !plain_cuda(k) || !plain_cuda(v) || !plain_cuda(bias) ||
-      (mask.defined() && !plain_cuda(mask)) || !device_supported(q))
+      (mask && !plain_cuda(*mask)) || !device_supported(q))
     return py::none();
   const int64_t nd = q.dim();
   if (nd < 5 || nd > 20 || q.numel() == 0 || q.size(-1) > 64 || bias.dim() < 4) return py::none();
@@ -236,9 +236,9 @@ py::object py_attention(py::handle hq, py::handle hk, py::handle hv, py::handle 
       (bias.scalar_type() != at::kBFloat16 && bias.scalar_type() != at::kFloat))
     return py::none();
   if (k.device() != q.device() || v.device() != q.device() || bias.device() != q.device()) return py::none();
-  if (mask.defined()) {
-    if (mask.dim() < 4 || mask.size(-4) != O || mask.size(-3) != 1 || mask.size(-2) != 1 || mask.size(-1) != N ||
-        !prefix_ok(mask, q) || !float_mask(mask) || mask.requires_grad() || mask.device() != q.device())
+  if (mask) {
+    if (mask->dim() < 4 || mask->size(-4) != O || mask->size(-3) != 1 || mask->size(-2) != 1 || mask->size(-1) != N ||
+        !prefix_ok(*mask, q) || !float_mask(*mask) || mask->requires_grad() || mask->device() != q.device())
       return py::none();
   }
   const bool save = at::GradMode::is_enabled() &&

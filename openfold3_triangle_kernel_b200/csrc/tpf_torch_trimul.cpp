@@ -96,15 +96,15 @@ namespace {
 
 cudaStream_t cu_stream() { return static_cast<cudaStream_t>(stream()); }
 
-// inputs: z, mask, then p_in, g_in, p_out, g_out, norm_in_w, norm_in_b, norm_out_w, norm_out_b
+// inputs: z, mask (an absent one is an empty optional: the node cannot take an undefined tensor as an input), then p_in, g_in, p_out, g_out, norm_in_w, norm_in_b, norm_out_w, norm_out_b
 struct TrimulFn : public torch::autograd::Function<TrimulFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& z_in, const Tensor& mask_in, const Tensor& w0,
+  static Tensor forward(AutogradContext* ctx, const Tensor& z_in, const std::optional<Tensor>& mask_in, const Tensor& w0,
                         const Tensor& w1, const Tensor& w2, const Tensor& w3, const Tensor& w4, const Tensor& w5,
                         const Tensor& w6, const Tensor& w7, bool incoming, bool save) {
     const Tensor z = aligned_bf16(z_in.detach());
     std::vector<Tensor> w;
     for (const Tensor* t : {&w0, &w1, &w2, &w3, &w4, &w5, &w6, &w7}) w.push_back(f32c(*t));
-    const Tensor mask = flat_pair_mask(mask_in, z, z.numel() / (z.size(-1) * z.size(-2) * z.size(-2)));
+    const Tensor mask = flat_pair_mask(mask_in.value_or(Tensor()), z, z.numel() / (z.size(-1) * z.size(-2) * z.size(-2)));
     tpf::TrimulCall t = {};
     Tensor arena = trimul_bind(t, z, mask, w, incoming, save, Tensor());
     Tensor out = empty_bf16(z.sizes(), z);
@@ -197,15 +197,16 @@ py::object py_trimul(py::handle hz, bool incoming, py::handle hm, py::tuple weig
   }
   if (!plain_context() || !trimul_supported(z, mask, w)) return py::none();
   const bool save = grad && at::GradMode::is_enabled();
+  const std::optional<Tensor> opt_mask = mask.defined() ? std::optional<Tensor>(mask) : std::nullopt;
   Tensor out;
   {
     py::gil_scoped_release release;
     c10::cuda::CUDAGuard guard(z.device());
     if (save) {
-      out = TrimulFn::apply(z, mask, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], incoming, true);
+      out = TrimulFn::apply(z, opt_mask, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], incoming, true);
     } else {
       at::NoGradGuard no_grad;
-      out = TrimulFn::forward(nullptr, z, mask, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], incoming, false);
+      out = TrimulFn::forward(nullptr, z, opt_mask, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], incoming, false);
     }
   }
   return py::cast(out);

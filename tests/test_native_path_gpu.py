@@ -30,6 +30,33 @@ def test_trimul_any_length(N, direction):
         assert ao.rel_l2(w[k].grad.cpu(), ref["d_" + k]) <= 2.5e-2, k
 
 
+@pytest.mark.parametrize("N", [1, 24, 37])
+def test_absent_mask_equals_a_mask_that_keeps_everything(N):
+    a = attention_inputs(2, 3, 2, N, 32, seed=N, mask_mode="none")
+    t = trimul_inputs(1, N, 32, seed=N, mask_mode="none")
+    d_att = torch.randn(2, 3, N, 2, 32, generator=torch.Generator().manual_seed(N)).bfloat16().cuda()
+    d_tri = torch.randn(1, N, N, 32, generator=torch.Generator().manual_seed(N)).bfloat16().cuda()
+
+    def attention(mask):
+        x = [a[n].cuda().requires_grad_(True) for n in ("q", "k", "v", "pair_bias")]
+        out = tk.turbo_attention(*x[:3], pair_bias=x[3], res_mask=mask)
+        with torch.no_grad():
+            assert torch.equal(tk.turbo_attention(*x[:3], pair_bias=x[3], res_mask=mask), out)
+        return [out, *torch.autograd.grad(out, x, d_att)]
+
+    def trimul(mask):
+        z = t["z"].cuda().requires_grad_(True)
+        w = {k: v.cuda().requires_grad_(True) for k, v in t["weights"].items()}
+        out = tk.turbo_trimul(z, "outgoing", mask, **w)
+        with torch.no_grad():
+            assert torch.equal(tk.turbo_trimul(z, "outgoing", mask, **w), out)
+        return [out, *torch.autograd.grad(out, [z, *w.values()], d_tri)]
+
+    for fn, keep in ((attention, torch.zeros(2, 3, 1, 1, N, device="cuda")), (trimul, torch.ones(1, N, N, device="cuda"))):
+        for got, want in zip(fn(None), fn(keep)):
+            assert torch.equal(got, want)
+
+
 # Enough rows for the projections that keep all weights in shared memory (113 row tiles and more), with a ragged last
 # row tile; 145 tiles at N = 136, one round of 148 row tiles and a second one at N = 184.
 @pytest.mark.parametrize("N,C", [(119, 128), (136, 32), (136, 64), (120, 96), (184, 128)])
