@@ -2,6 +2,8 @@
 #include "tpf_torch.h"
 
 #include <c10/core/impl/LocalDispatchKeySet.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 
 #include <atomic>
 
@@ -33,6 +35,26 @@ bool device_supported(const Tensor& t) {
     table[dev].store(v, std::memory_order_relaxed);
   }
   return v == 2;
+}
+
+// The raising node leads to everything the gradients depend on: the operator's inputs (the edges of the node that is
+// running) and the incoming gradients.  Without those edges a second pass that asks for certain inputs only
+// (autograd.grad) would prune it and leave the term out.
+variable_list first_order(const variable_list& incoming, variable_list grads) {
+  namespace ag = torch::autograd;
+  if (!at::GradMode::is_enabled()) return grads;
+  ag::edge_list edges = ag::get_current_node()->next_edges();
+  for (const Tensor& t : incoming)
+    if (t.defined()) edges.push_back(ag::impl::gradient_edge(t));
+  auto node = std::make_shared<ag::Error>(
+      "the triangle operators are differentiable once: there is no second derivative (create_graph=True)",
+      std::move(edges));
+  for (Tensor& g : grads) {
+    if (!g.defined()) continue;
+    g = g.variable_data();
+    ag::set_history(g, node);
+  }
+  return grads;
 }
 
 }  // namespace tpf_torch

@@ -44,6 +44,10 @@ bool plain_context();
 // Compute capability 10.x, cached per device.
 bool device_supported(const Tensor& t);
 
+// Last step of every backward.  The gradients have no derivative of their own; when the engine records them
+// (create_graph=True) they get a node that raises if one is asked for, instead of counting as constants.
+variable_list first_order(const variable_list& incoming, variable_list grads);
+
 // Hands out 256-byte aligned pieces of one allocation: an operator call keeps a dozen intermediate tensors, and one
 // allocation is cheaper on the host than twelve.
 struct Arena {

@@ -153,6 +153,10 @@ struct AttentionFn : public torch::autograd::Function<AttentionFn> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return first_order(grads, gradients(ctx, grads));
+  }
+
+  static variable_list gradients(AutogradContext* ctx, const variable_list& grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &out = saved[5], &lse = saved[6];
     const auto q_sizes = ctx->saved_data["q"].toIntVector();

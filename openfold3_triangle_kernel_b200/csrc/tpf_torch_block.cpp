@@ -46,6 +46,10 @@ struct TrimulResidualFn : public torch::autograd::Function<TrimulResidualFn> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return first_order(grads, gradients(ctx, grads));
+  }
+
+  static variable_list gradients(AutogradContext* ctx, const variable_list& grads) {
     variable_list r(12);
     if (!grads[0].defined()) return r;
     const auto saved = ctx->get_saved_variables();
@@ -139,6 +143,10 @@ struct PairAttnFn : public torch::autograd::Function<PairAttnFn> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return first_order(grads, gradients(ctx, grads));
+  }
+
+  static variable_list gradients(AutogradContext* ctx, const variable_list& grads) {
     variable_list r(13);
     if (!grads[0].defined()) return r;
     const auto saved = ctx->get_saved_variables();

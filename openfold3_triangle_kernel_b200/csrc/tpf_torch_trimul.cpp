@@ -121,6 +121,10 @@ struct TrimulFn : public torch::autograd::Function<TrimulFn> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    return first_order(grads, gradients(ctx, grads));
+  }
+
+  static variable_list gradients(AutogradContext* ctx, const variable_list& grads) {
     variable_list r(12);
     if (!grads[0].defined()) return r;
     const auto saved = ctx->get_saved_variables();

@@ -57,6 +57,42 @@ def test_absent_mask_equals_a_mask_that_keeps_everything(N):
             assert torch.equal(got, want)
 
 
+def _entry_points():
+    """name -> (call, differentiable inputs) of the three entry points at a small size"""
+    from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
+    from oracle.pair_block_oracle import block_params
+    a = attention_inputs(1, 9, 2, 24, 32, seed=1)
+    x = [a[n].cuda().requires_grad_(True) for n in ("q", "k", "v", "pair_bias")]
+    t = trimul_inputs(1, 24, 64, seed=2)
+    z = t["z"].cuda().requires_grad_(True)
+    w = {k: v.cuda().requires_grad_(True) for k, v in t["weights"].items()}
+    blk = {k: {n: v.cuda().requires_grad_(True) for n, v in m.items()} for k, m in block_params(64, 4, 16, seed=3).items()}
+    mask = t["mask"].cuda()
+    return {"attention": (lambda: tk.turbo_attention(*x[:3], pair_bias=x[3], res_mask=a["res_mask"].cuda()), x),
+            "trimul": (lambda: tk.turbo_trimul(z, "incoming", mask, **w), [z, *w.values()]),
+            "block": (lambda: pair_stack_block(z, mask, blk, 4), [z, *(v for m in blk.values() for v in m.values())])}
+
+
+@pytest.mark.parametrize("name", ["attention", "trimul", "block"])
+def test_second_derivative_is_refused(name):
+    call, leaves = _entry_points()[name]
+    want = torch.autograd.grad(call().float().square().sum(), leaves)
+    out = call()
+    got = torch.autograd.grad(out.float().square().sum(), leaves, create_graph=True)   # allowed: first derivatives
+    for g, r in zip(got, want):
+        assert torch.equal(g, r)
+    for g in got:   # a penalty on any of them, alone or next to a term that has a derivative
+        with pytest.raises(RuntimeError, match="no second derivative"):
+            torch.autograd.grad(out.float().sum() + g.float().square().sum(), leaves[:1], retain_graph=True)
+        with pytest.raises(RuntimeError, match="no second derivative"):
+            g.float().square().sum().backward(retain_graph=True)
+    # the incoming gradient is an input of the backward as well
+    d_out = torch.ones_like(out).requires_grad_(True)
+    g, = torch.autograd.grad(call(), leaves[:1], d_out, create_graph=True)
+    with pytest.raises(RuntimeError, match="no second derivative"):
+        torch.autograd.grad(g.float().sum(), d_out)
+
+
 # Enough rows for the projections that keep all weights in shared memory (113 row tiles and more), with a ragged last
 # row tile; 145 tiles at N = 136, one round of 148 row tiles and a second one at N = 184.
 @pytest.mark.parametrize("N,C", [(119, 128), (136, 32), (136, 64), (120, 96), (184, 128)])
