@@ -323,8 +323,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const uint32_t gw[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            v[2 * i] *= sigmoid_fast(__uint_as_float(gw[i] << 16));
-            v[2 * i + 1] *= sigmoid_fast(__uint_as_float(gw[i] & 0xFFFF0000u));
+            v[2 * i] *= sigmoid_rel(__uint_as_float(gw[i] << 16));
+            v[2 * i + 1] *= sigmoid_rel(__uint_as_float(gw[i] & 0xFFFF0000u));
           }
         }
         if (f_ok) {

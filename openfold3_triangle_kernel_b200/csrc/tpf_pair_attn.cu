@@ -205,7 +205,7 @@ struct EpiGateBwd {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float d0 = v[8 * i + 2 * e], d1 = v[8 * i + 2 * e + 1];
-        const float s0 = sigmoid_fast(bf16_lo(gw[e])), s1 = sigmoid_fast(bf16_hi(gw[e]));
+        const float s0 = sigmoid_rel(bf16_lo(gw[e])), s1 = sigmoid_rel(bf16_hi(gw[e]));
         const float t0 = d0 * bf16_lo(ow[e]), t1 = d1 * bf16_hi(ow[e]);
         po[4 * i + e] = pack_bf16x2(d0 * s0, d1 * s1);
         pg[4 * i + e] = pack_bf16x2(t0 - t0 * s0, t1 - t1 * s1);

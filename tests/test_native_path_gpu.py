@@ -179,3 +179,37 @@ def test_pair_block_any_length(N, C, H, D):
             want = pr[k][n].grad
             if want.norm() > 1e-6 * N:   # N = 1: a softmax over one key has no gradient in q, k and the bias
                 assert ao.rel_l2(t.grad.cpu(), want) <= 4e-2, (k, n)
+
+
+# Gates of the attention modules that are nearly closed (logits -10 .. -16): the gate's own value counts, since the output
+# projection scales it back up.  One LayerNorm channel is constant and alone carries the gate logits, which bf16 holds
+# exactly.  A gate that is off by a factor scales the gradients that belong to its column of w_o and its rows of w_v and
+# w_g by that factor; what the bf16 intermediates leave of that measure (about 1 % here, open gates included) bounds it.
+@pytest.mark.parametrize("N,C,H,D", [(40, 64, 4, 16), (33, 128, 4, 32)])
+def test_pair_block_closed_gates(N, C, H, D):
+    from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
+    from oracle.pair_block_oracle import block_params, pair_block_forward
+    g = torch.Generator().manual_seed(N)
+    z = torch.randn(1, N, N, C, generator=g).bfloat16()
+    mask = torch.ones(1, N, N)
+    params = block_params(C, H, D, seed=N)
+    logits = (-10.0 - 6.0 * torch.rand(H * D, generator=g)).bfloat16().float()
+    nodes = ("tri_att_start", "tri_att_end")
+    for k in nodes:
+        p = params[k]
+        p["ln_w"][0], p["ln_b"][0] = 0.0, 1.0
+        p["w_g"].zero_()
+        p["w_g"][:, 0] = logits
+        p["w_o"].mul_(10 * torch.exp(-logits))
+    d_out = torch.randn(1, N, N, C, generator=g).bfloat16()
+    pr = {k: {n: t.double().requires_grad_(k in nodes) for n, t in v.items()} for k, v in params.items()}
+    pair_block_forward(z.double(), mask, pr, H, dtype=torch.float64).backward(d_out.double())
+    pd = {k: {n: t.cuda().requires_grad_(k in nodes) for n, t in v.items()} for k, v in params.items()}
+    pair_stack_block(z.cuda(), mask.cuda(), pd, H).backward(d_out.cuda())
+    for k in nodes:
+        for n in ("w_o", "w_v", "w_g"):
+            got, want = pd[k][n].grad.cpu().double(), pr[k][n].grad
+            if n == "w_o":
+                got, want = got.T, want.T
+            factor = (got * want).sum(1) / (want * want).sum(1)
+            assert (factor - 1).abs().max() <= 2.5e-2, (k, n, float((factor - 1).abs().max()))
