@@ -33,9 +33,15 @@ _INVOCATIONS = 0
 
 
 def invocation_count() -> int:
-    """Number of ``turbo_attention`` calls that reached the kernels (reference:
-    ``_INVOCATIONS``, turbopairformer_triangle_attention.py:57-66)."""
+    """Number of ``turbo_attention`` calls that reached the kernels, the two of a pair-stack block included
+    (reference: ``_INVOCATIONS``, turbopairformer_triangle_attention.py:57-66)."""
     return _INVOCATIONS
+
+
+def count_invocations(n):
+    """Attention calls that reached the kernels on another way than :func:`turbo_attention`."""
+    global _INVOCATIONS
+    _INVOCATIONS += n
 
 
 # --------------------------------------------------------------------------------------

@@ -24,7 +24,7 @@ import torch.nn.functional as F
 
 from . import _cabi as C
 from . import dap
-from .attention import turbo_attention
+from .attention import count_invocations, turbo_attention
 from .trimul import native_weight_order, turbo_trimul
 
 _attention_order = operator.itemgetter("ln_w", "ln_b", "w_z", "w_q", "w_k", "w_v", "w_g", "w_o")
@@ -106,6 +106,7 @@ def pair_stack_block(z, mask, params, heads, group=None, trimul_backend=None, at
                                     _attention_order(params["tri_att_start"]),
                                     _attention_order(params["tri_att_end"]), heads)
         if out is not None:
+            count_invocations(2)
             return out
     if group is None:
         z = z + turbo_trimul(z, "outgoing", mask, **params["tri_mul_out"])

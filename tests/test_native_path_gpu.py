@@ -181,6 +181,19 @@ def test_pair_block_any_length(N, C, H, D):
                 assert ao.rel_l2(t.grad.cpu(), want) <= 4e-2, (k, n)
 
 
+# D = 16 is the fused block, D = 64 its composition of the operators
+@pytest.mark.parametrize("D", [16, 64])
+def test_pair_block_counts_its_attention_calls(D):
+    from openfold3_triangle_kernel_b200.attention import invocation_count
+    from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
+    from oracle.pair_block_oracle import block_params
+    z = torch.zeros(1, 16, 16, 64, device="cuda", dtype=torch.bfloat16)
+    params = {k: {n: t.cuda() for n, t in v.items()} for k, v in block_params(64, 2, D, seed=1).items()}
+    before = invocation_count()
+    pair_stack_block(z, torch.ones(1, 16, 16, device="cuda"), params, 2)
+    assert invocation_count() == before + 2
+
+
 # Gates of the attention modules that are nearly closed (logits -10 .. -16): the gate's own value counts, since the output
 # projection scales it back up.  One LayerNorm channel is constant and alone carries the gate logits, which bf16 holds
 # exactly.  A gate that is off by a factor scales the gradients that belong to its column of w_o and its rows of w_v and
