@@ -116,9 +116,20 @@ inline int make_tmap(CUtensorMap* out, CUtensorMapDataType dtype, const void* ba
                   i + 1, (unsigned long long)s[i]);
     }
   }
-  CUresult r = fn(out, dtype, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, e,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_enum(swizzle_bytes), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return fn(out, dtype, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, e, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              swizzle_enum(swizzle_bytes), CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // A driver call wants a context that is current in this host thread.  A thread whose first use of CUDA is a call
+    // of this library (an autograd worker whose allocations came from a cache, say) has none until a runtime call
+    // makes the device's primary context current.
+    int dev = 0;
+    TPF_CUDA_OK(cudaGetDevice(&dev));
+    TPF_CUDA_OK(cudaSetDevice(dev));
+    r = encode();
+  }
   TPF_REQUIRE(r == CUDA_SUCCESS, TPF_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return TPF_OK;
 }

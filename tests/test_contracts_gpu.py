@@ -126,6 +126,33 @@ def test_two_host_threads_call_concurrently():
     assert all(_same(g, ref_t) for g in results["t"])
 
 
+def test_first_cuda_use_of_a_host_thread_is_a_library_call():
+    """A thread has no current CUDA context until a runtime call gives it one; encoding a tensor map needs it."""
+    a = torch.randn(1, 64, 64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)).bfloat16()
+    d = [torch.zeros(1, 64, 64, device="cuda") for _ in range(2)]
+    stream = C.current_stream()
+
+    def bmm(out):
+        C.call("tpf_bmm_bf16", C.ptr(a), 64, 4096, 0, C.ptr(a), 64, 4096, 0, C.ptr(out), 64, 4096, 1, 64, 64, 64, 1, 0,
+               128, stream)
+
+    bmm(d[0])   # per-device set-up is done: the thread below makes no runtime call before the map is encoded
+    errors = []
+
+    def work():
+        try:
+            bmm(d[1])
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    th = threading.Thread(target=work)
+    th.start()
+    th.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    assert torch.equal(d[0], d[1]) and d[0].abs().sum() > 0
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
 def test_second_device_after_the_first():
     """Launch attributes and symbol addresses are per device: a process that has used cuda:0 must be able
