@@ -50,7 +50,7 @@ struct GemmCfg {
   static constexpr bool RESIDENT = STAT == 3;
   static constexpr int B_ROWS = B_ROWS_, B_BOX = RESIDENT ? 32 : BN;  // resident B: capacity, rows per load
   static constexpr int MAX_NT = RESIDENT ? (B_ROWS + BN - 1) / BN : 1;
-  static constexpr bool TIGHT = TIGHT_;  // no room to align the shared memory base by hand
+  static constexpr bool TIGHT = TIGHT_;  // no room to align the shared memory base by hand: the launch checks it
   static constexpr int EPI_WARPS = EPI_WARPS_;          // 8 or 16: warps per TMEM lane quarter x 4
   static constexpr int EPI_PER_Q = EPI_WARPS / 4;       // warps sharing one lane quarter; they interleave 32-column chunks
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
@@ -264,7 +264,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                  const GemmShape sh, const __grid_constant__ typename Epi::Params ep, int* __restrict__ status) {
   griddep_wait();
   extern __shared__ __align__(1024) uint8_t smem_dyn[];
-  if (Cfg::TIGHT && (smem_u32(smem_dyn) & 1023u) != 0) {  // the declaration's alignment: not expected to be missed
+  if (Cfg::TIGHT && (smem_u32(smem_dyn) & 1023u) != 0) {  // the launch checks it: no write beyond the block's memory
     if (threadIdx.x == 0 && status != nullptr) *status = (int)kStatusWaitTimeout;
     return;
   }

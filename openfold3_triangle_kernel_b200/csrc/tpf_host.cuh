@@ -160,13 +160,24 @@ struct PerDeviceOnce {
   std::atomic<bool> done[kMaxDevices];
 };
 
-// cudaFuncAttributeMaxDynamicSharedMemorySize for `kern` on the current device, once per device.
+// cudaFuncAttributeMaxDynamicSharedMemorySize for `kern` on the current device, once per device.  `base_align`: what a
+// kernel without room to align its dynamic shared memory by hand relies on.  That memory starts behind the part of the
+// block's shared memory that the system keeps and the kernel's static variables (their padding included).
 template <class Kernel>
-inline int ensure_dynamic_smem(Kernel kern, int bytes, PerDeviceOnce& once) {
+inline int ensure_dynamic_smem(Kernel kern, int bytes, PerDeviceOnce& once, int base_align = 1) {
   int dev = 0;
   int rc = current_device(&dev);
   if (rc) return rc;
   if (once.done[dev].load(std::memory_order_acquire)) return TPF_OK;
+  if (base_align > 1) {
+    cudaFuncAttributes attr;
+    int reserved = 0;
+    TPF_CUDA_OK(cudaFuncGetAttributes(&attr, kern));
+    TPF_CUDA_OK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
+    TPF_REQUIRE((reserved + attr.sharedSizeBytes) % base_align == 0, TPF_ERR_UNSUPPORTED,
+                "dynamic shared memory starts at %d + %zu bytes on this device, the kernel needs a multiple of %d",
+                reserved, attr.sharedSizeBytes, base_align);
+  }
   TPF_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   once.done[dev].store(true, std::memory_order_release);
   return TPF_OK;
