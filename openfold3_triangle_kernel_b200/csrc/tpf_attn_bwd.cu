@@ -123,7 +123,7 @@ struct AttnBwdCfg {
   static constexpr int OFF_ITEM = OFF_ROW + (STAGED ? 1024 : 0);
   static constexpr int OFF_MASK = OFF_ITEM + (STAGED ? 128 : 0);  // [NKV] x 512
   static constexpr int OFF_BAR = OFF_MASK + NKV * 512;
-  static constexpr int N_BAR = 2 * NB + 2 * NQ + 2 * NKV + 7;
+  static constexpr int N_BAR = 2 * NB + 2 * NQ + 2 * NKV + 6;
   static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
   static constexpr int TM_S = 0, TM_DP = 128, TM_DQ = 256, TM_DK = 320, TM_DV = 320 + KS * D;
   static constexpr int TMEM_COLS = 512;
@@ -150,7 +150,6 @@ struct BwdWalk {
   __device__ bool first_kk() const { return kk == 0; }
   __device__ bool last_kk() const { return kk == strip_len() - 1; }
   __device__ bool first_qt() const { return qt == 0; }
-  __device__ bool last_qt() const { return qt == q_tiles - 1; }
   __device__ void next() {
     if (++kk < strip_len()) return;
     kk = 0;
@@ -196,9 +195,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* sdp_free = misc + 1;   // ... and have been read by all compute warps
   uint64_t* pds_ready = misc + 2;  // P and dS of a tile are in shared memory
   uint64_t* pds_free = misc + 3;   // ... and have been consumed by the dV / dK / dQ UMMAs
-  uint64_t* dkv_full = misc + 4;
-  uint64_t* dkv_free = misc + 5;
-  uint64_t* row_free = misc + 6;   // the compute warps have read the query rows' scalars
+  uint64_t* dkv_free = misc + 4;
+  uint64_t* row_free = misc + 5;   // the compute warps have read the query rows' scalars
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::N_BAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wctx{abort_flag, status};
@@ -223,7 +221,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(sdp_free, NCW);
     mbar_init(pds_ready, NCW);
     mbar_init(pds_free, 1);
-    mbar_init(dkv_full, 1);
     mbar_init(dkv_free, NCW);
     mbar_init(row_free, NCW);
     *abort_flag = 0;
@@ -415,13 +412,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         umma_commit(el, pds_free);
         umma_commit(el, &kv_empty[bkv_s]);
         if (++bkv_s == NKV) bkv_s = 0;
-        const bool last_kk = wb.last_kk();
-        const bool strip_done = last_kk && wb.last_qt();
-        if (last_kk) {
+        if (wb.last_kk()) {  // (the compute warps learn of a finished strip from pds_free of its last tile)
           umma_commit(el, &q_empty[bq_s]);
           if (++bq_s == NQ) bq_s = 0;
         }
-        (void)strip_done;  // the compute warps learn of a finished strip from pds_free of its last tile
         wb.next();
       }
     }
@@ -442,7 +436,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint64_t scale2 = f2_pack(scale, scale);
     const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
 
-    uint32_t sdpfull_ph = 0, pdsfree_ph = 1, kv_ph = 0, b_ph = 0, dkvfull_ph = 0;
+    uint32_t sdpfull_ph = 0, pdsfree_ph = 1, kv_ph = 0, b_ph = 0;
     int kv_s = 0, b_s = 0, q_s = 0;
     uint32_t q_ph = 0;
     bool have_prev_dq = false;     // a finished dQ tile waits in TMEM
