@@ -1284,6 +1284,16 @@ int launch_attn_dbias(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 // waves of CTAs (one per SM) times planes per CTA, plus about three planes' time for a CTA's start and its partial
 // plane.  With one chunk whenever there are more tiles than SMs (N = 1021: 256 tiles) the last wave left half the
 // machine idle.  Chunk planes take at most `max_bytes`; one chunk needs none.
+// dBias and its fold, us by number of chunks (H = 4, D = 32, O = N; * is what the rule takes, with its workspace):
+//   N =  384   1: 362   2: 194   4: 110*   8: 120            9 MiB
+//   N =  400   1: 471   2: 251   4: 234    9: 228*          22 MiB
+//   N =  512   1: 480   2: 256   9: 252*  16: 278           36 MiB
+//   N =  640   1: 592   4: 479   7: 474   10: 477*          62 MiB
+//   N =  768   1: 717*  2: 727   4: 744    8: 782            0
+//   N = 1024   1: 1863  2: 1889  4: 1698*                   64 MiB
+// The count leaves out the fold, which reads every chunk plane (N = 640: the time per count grows from 0.92 to 1.02 us
+// between 1 and 10 chunks); the steps between schedules are larger.  Where the rule misses: N = 704 (144 tiles, the last
+// ones half empty) takes 824 us with the one chunk of a full wave, 755 with five.
 static void dbias_plan(int64_t B, int64_t O, int64_t H, int64_t N, int64_t G, double max_bytes, int* n_chunks,
                        int* chunk_len) {
   const int64_t tiles = G * H * ((N + 127) / 128) * ((N + 127) / 128);

@@ -21,9 +21,15 @@ int bmm_status_fetch_and_clear(int* out) {
 // tensor rate where shared memory gives 128, so such tiles end at half the peak (1.16 of 2.3 PFLOP/s measured at
 // N = 1024), and wider ones at 0.6 (192) and 0.67 (256) of it.  The time of a tile is therefore taken as 128 + BN,
 // and the width with the shortest sequence of tiles per CTA is used; ragged widths and nearly empty last rounds count.
-// Wide tiles have fewer stages and a longer start and end, so they have to promise a tenth: at N = 384 (0.94 by this
-// count) 192 columns took 25 instead of 22 us.  128 channels, N = 520: 92 -> 68 us (192); N = 1024: 235 -> 208, N = 1536:
-// 742 -> 634 (256).
+// Wide tiles have fewer stages and a longer start and end, so they have to promise a tenth.  Alone, 128 channels, K-major,
+// us at 128 / 192 / 256 columns (* is what the rule takes; the count relative to 128 columns in brackets):
+//   N =  264   24.1*  25.8 (0.94)   30.9 (1.13)        N =  520   93.8   75.3* (0.74)   87.4 (0.89)
+//   N =  320   18.6*  19.5 (0.94)   21.6 (1.13)        N =  576   66.8   59.8* (0.74)   63.4 (0.89)
+//   N =  384   24.0*  26.7 (0.94)   28.4 (1.13)        N =  640   78.1   82.4  (1.02)   75.1* (0.89)
+//   N =  392   53.5   53.6 (0.98)   50.0* (0.75)       N =  896  195    191    (0.90)  183*   (0.87)
+//   N =  512   44.0   46.2 (0.98)   40.4* (0.75)       N = 1024  280    282    (0.94)  240*   (0.75)
+// At 64 channels N = 640 stays at 128 columns (46.1 us; 46.3 at 256, 0.955).  Over these and six more lengths, 64 and 128
+// channels, both operand majors, the choice is at most 2.5 % behind the best of the three.
 static int tile_width(const GemmShape& sh) {
   const int64_t mt = (int64_t)sh.batch * ((sh.M + 127) / 128), sms = sm_count();
   int best = 128;

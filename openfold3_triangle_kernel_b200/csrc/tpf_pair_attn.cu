@@ -358,7 +358,10 @@ int pair_attn_forward(const PairAttnCall& t, cudaStream_t stream) {
     if (t.D == 32 && (rc = make_store_tmap(&ep.map, t.qkvg, t.D, R, t.D, 4 * t.H, R * t.D))) return rc;
     GemmShape sh{(int)R, (int)P, (int)C, 1, 0};
     // 4 HD + H columns in as few, as full tiles as possible: 3 x 192 at H * D = 128, 3 x 96 at 64.  The weights, or as
-    // much of them as a tile needs, stay in shared memory while the rows stream past (see GemmCfg).
+    // much of them as a tile needs, stay in shared memory while the rows stream past (see GemmCfg).  All of them at
+    // H * D = 128 from 99 row tiles on: 13.4 -> 12.3 us at N = 192, 39.3 -> 34.9 at 384, 691 -> 482 at 1536, but
+    // 6.2 -> 7.9 at 72.  At H * D = 64 no variant with all weights resident is built; it would pay there as well (measured
+    // with 2 x 192 columns, C = 64: 32.2 -> 25.0 us at N = 384, 443 -> 326 at 1536).
     if (P > 272 && P <= 544 && resident_pays(R, 3)) {
       using Cfg = GemmCfg<128, 192, 128, false, 128, false, 3, 8, 3, 2, 544>;
       rc = launch_gemm<Cfg, EpiQkvg>(t.x, C, 0, pk.W, C, 0, sh, ep, status, stream);
