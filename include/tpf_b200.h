@@ -109,8 +109,8 @@ int64_t tpf_attn_bwd_workspace_bytes(int64_t B, int64_t O, int64_t H, int64_t N,
 #define TPF_ATTN_BWD_STAGE_DBIAS 4  /* dbias (reads delta) */
 #define TPF_ATTN_BWD_STAGE_ALL 7
 
-/* tpf_attn_bwd restricted to the stages in `stages` (bit mask above); used to time the
- * stages separately.  tpf_attn_bwd(...) is tpf_attn_bwd_stages(..., TPF_ATTN_BWD_STAGE_ALL). */
+/* tpf_attn_bwd restricted to the stages in `stages` (bit mask above): gradients that nobody wants are not
+ * computed, and their pointers (dq, dk, dv; dbias) may be NULL.  tpf_attn_bwd(...) is tpf_attn_bwd_stages(..., TPF_ATTN_BWD_STAGE_ALL). */
 int tpf_attn_bwd_stages(const void* q, const void* k, const void* v, const void* d_out,
                  const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
                  const void* out, const float* lse,

@@ -1164,8 +1164,8 @@ int attn_bwd_dqkv(const void* q, const void* k, const void* v, const void* d_out
                   const float* mask, int64_t mask_pitch, const void* bias, int64_t bias_pitch, int64_t bias_batch,
                   void* dq, void* dk, void* dv, float* delta, void* workspace, int64_t workspace_bytes, int64_t B,
                   int64_t O, int64_t H, int64_t N, int64_t D, float scale, int stages, cudaStream_t stream) {
-  TPF_REQUIRE(q && k && v && d_out && out && lse && mask && bias && dq && dk && dv && delta, TPF_ERR_INVALID_ARGUMENT,
-              "attn_bwd: null pointer");
+  TPF_REQUIRE(q && k && v && d_out && out && lse && mask && bias && delta && (!(stages & 2) || (dq && dk && dv)),
+              TPF_ERR_INVALID_ARGUMENT, "attn_bwd: null pointer");
   TPF_REQUIRE(B > 0 && O > 0 && H > 0 && N > 0, TPF_ERR_INVALID_ARGUMENT, "attn_bwd: B,O,H,N must be positive");
   TPF_REQUIRE(D == 16 || D == 32 || D == 64, TPF_ERR_UNSUPPORTED, "attn_bwd: head dim %lld not in {16,32,64}",
               (long long)D);

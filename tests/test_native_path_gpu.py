@@ -57,6 +57,23 @@ def test_absent_mask_equals_a_mask_that_keeps_everything(N):
             assert torch.equal(got, want)
 
 
+# every subset of the four inputs that can ask for a gradient: the kernels of the others are left out
+@pytest.mark.parametrize("wanted", range(1, 16))
+def test_attention_gradient_subsets(wanted):
+    a = attention_inputs(1, 5, 2, 40, 32, seed=8)
+    d_out = torch.randn(1, 5, 40, 2, 32, generator=torch.Generator().manual_seed(8)).bfloat16().cuda()
+
+    def grads(mask):
+        x = [a[n].cuda().requires_grad_(bool(mask >> i & 1)) for i, n in enumerate(("q", "k", "v", "pair_bias"))]
+        out = tk.turbo_attention(*x[:3], pair_bias=x[3], res_mask=a["res_mask"].cuda())
+        out.backward(d_out)
+        return [t.grad for t in x]
+
+    for i, (got, full) in enumerate(zip(grads(wanted), grads(15))):
+        assert (got is not None) == bool(wanted >> i & 1)
+        assert got is None or torch.equal(got, full)
+
+
 def _entry_points():
     """name -> (call, differentiable inputs) of the three entry points at a small size"""
     from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
