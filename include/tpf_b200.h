@@ -8,8 +8,8 @@
  *  - All pointers are device pointers unless stated otherwise.  Nothing here
  *    allocates device memory (except where a function says so) or synchronises;
  *    work is enqueued on `stream` (a cudaStream_t passed as void*).
- *  - bf16 tensors are 16-byte aligned, and so are the fp32 dbias output and every workspace
- *    (rows are written with 16-byte vector stores); other fp32 tensors are 4-byte aligned.
+ *  - bf16 tensors are 16-byte aligned, and so are the fp32 dbias output, the attention entries' mask (read
+ *    by TMA) and every workspace; other fp32 tensors are 4-byte aligned.
  *    A misaligned pointer is rejected with TPF_ERR_INVALID_ARGUMENT before anything is launched.
  *    Extents are int64_t.
  *  - Host threads may call concurrently and a process may use several GPUs: launch attributes,

@@ -219,7 +219,7 @@ py::object py_trimul(py::handle hz, bool incoming, py::handle hm, py::tuple weig
 // Launches behind the torch.library operators: z [B,N,N,C] with N a multiple of 8, mask fp32 [B,N,N].
 std::vector<Tensor> trimul_fwd(const Tensor& z_, const Tensor& mask_, std::vector<Tensor> w_, bool incoming) {
   c10::cuda::CUDAGuard guard(z_.device());
-  const Tensor z = z_.contiguous(), mask = mask_.to(at::kFloat).contiguous();
+  const Tensor z = aligned_bf16(z_), mask = mask_.to(at::kFloat).contiguous();
   const int64_t B = z.size(0), N = z.size(1), C = z.size(3), R = B * N * N;
   std::vector<Tensor> w;
   for (const Tensor& t : w_) w.push_back(f32c(t));
@@ -243,7 +243,7 @@ std::vector<Tensor> trimul_fwd(const Tensor& z_, const Tensor& mask_, std::vecto
 std::vector<Tensor> trimul_bwd(const Tensor& d_out_, const Tensor& z_, const Tensor& mask_, std::vector<Tensor> w_,
                                bool incoming, std::vector<Tensor> s) {
   c10::cuda::CUDAGuard guard(z_.device());
-  const Tensor z = z_.contiguous(), mask = mask_.to(at::kFloat).contiguous(), d_out = aligned_bf16(d_out_);
+  const Tensor z = aligned_bf16(z_), mask = mask_.to(at::kFloat).contiguous(), d_out = aligned_bf16(d_out_);
   const int64_t B = z.size(0), N = z.size(1), C = z.size(3);
   std::vector<Tensor> w;
   for (const Tensor& t : w_) w.push_back(f32c(t));

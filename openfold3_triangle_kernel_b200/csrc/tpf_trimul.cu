@@ -17,6 +17,9 @@
 // GEMM in both directions (K-major operands when outgoing, MN-major when incoming).
 #include <cuda_fp16.h>
 
+#include <initializer_list>
+#include <utility>
+
 #include "tpf_gemm_host.cuh"
 #include "tpf_internal.h"
 #include "tpf_norm.cuh"
@@ -94,13 +97,14 @@ __global__ void __launch_bounds__(256, 2) trimul_xnorm_fwd_kernel(const bf16* __
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k2 = 2 * (lane & 3);            // this lane's channel pair inside an 8-channel group
   const int rr = 8 * warp + (lane >> 2);    // this lane's pair row inside the tile
-  float2 g[NG][4], bt[NG][4];
+  float2 g[NG][4], bt[NG][4];  // read one by one, once per CTA: a parameter may start at any element of a flat buffer
 #pragma unroll
   for (int i = 0; i < NG; ++i)
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-      g[i][m] = *reinterpret_cast<const float2*>(gamma + 32 * i + 8 * m + k2);
-      bt[i][m] = *reinterpret_cast<const float2*>(beta + 32 * i + 8 * m + k2);
+      const int c = 32 * i + 8 * m + k2;
+      g[i][m] = make_float2(gamma[c], gamma[c + 1]);
+      bt[i][m] = make_float2(beta[c], beta[c + 1]);
     }
   // 16-byte copies: 8 consecutive pair rows of one channel (NN is a multiple of 8)
   auto fetch = [&](int tile, uint8_t* dst) {
@@ -511,7 +515,7 @@ __global__ void __launch_bounds__(256, 2) trimul_xnorm_bwd_kernel(const bf16* __
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k2 = 2 * (lane & 3);
   const int rr = 8 * warp + (lane >> 2);
-  if (threadIdx.x < C / 2) gsm[threadIdx.x] = *reinterpret_cast<const float2*>(gamma + 2 * threadIdx.x);
+  if (threadIdx.x < C / 2) gsm[threadIdx.x] = make_float2(gamma[2 * threadIdx.x], gamma[2 * threadIdx.x + 1]);
   float2 ag[NG][4], ab[NG][4];  // running sums of d * xhat and d for this lane's channels
 #pragma unroll
   for (int i = 0; i < NG; ++i)
@@ -919,10 +923,18 @@ static const float* grid_mask(const TrimulCall& t) {
   return t.mask_grid ? t.mask_grid : reinterpret_cast<const float*>(t.mask);
 }
 
+// The bf16 tensors are read and written 16 bytes at a time (masks, weights, statistics element by element).
+static int check_trimul_aligned(const char* who, std::initializer_list<std::pair<const char*, const void*>> tensors) {
+  for (const auto& t : tensors) TPF_REQUIRE_ALIGNED16(t.second, who, t.first);
+  return TPF_OK;
+}
+
 static int trimul_fwd_run(const TrimulCall& t, int64_t NN, int stages, bool with_pack, cudaStream_t stream) {
   int* status = nullptr;
-  int rc = trimul_status(&status);
-  if (rc) return rc;
+  int rc = check_trimul_aligned("trimul_fwd", {{"z", t.z}, {"out", t.out}, {"sum", t.sum}, {"zln", t.zln}, {"a_cm", t.a_cm},
+                                               {"b_cm", t.b_cm}, {"gate", t.gate}, {"x_cm", t.x_cm}, {"xln", t.xln},
+                                               {"workspace", t.packed}});
+  if (rc || (rc = trimul_status(&status))) return rc;
   const TrimulPacked pk = packed_at(t.packed, t.C);
   if (with_pack && (rc = pack_weights(t.w.p_in, t.w.g_in, t.w.p_out, t.w.g_out, pk, (int)t.C, stream))) return rc;
   switch (t.C) {
@@ -937,8 +949,11 @@ static int trimul_fwd_run(const TrimulCall& t, int64_t NN, int stages, bool with
 static int trimul_bwd_run(const TrimulCall& t, const TrimulGrads& g, int64_t NN, int stages, void* dx_io, void* da_io,
                           void* db_io, void* workspace, cudaStream_t stream) {
   int* status = nullptr;
-  int rc = trimul_status(&status);
-  if (rc) return rc;
+  int rc = check_trimul_aligned("trimul_bwd", {{"d_out", g.d_out}, {"d_res", g.d_res}, {"d_z", g.d_z}, {"z", t.z},
+                                               {"out", t.out}, {"zln", t.zln}, {"a_cm", t.a_cm}, {"b_cm", t.b_cm},
+                                               {"gate", t.gate}, {"x_cm", t.x_cm}, {"xln", t.xln}, {"dx_cm", dx_io},
+                                               {"da_cm", da_io}, {"db_cm", db_io}, {"packed weights", t.packed}});
+  if (rc || (rc = trimul_status(&status))) return rc;
   TrimulPacked pk = packed_at(t.packed, t.C);
   const TrimulPacked* packed = t.packed ? &pk : nullptr;
   bf16 *dx = (bf16*)dx_io, *da = (bf16*)da_io, *db = (bf16*)db_io;

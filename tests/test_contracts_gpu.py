@@ -97,6 +97,25 @@ def test_two_streams_at_once_give_the_serial_results():
     assert C.device_status() == 0
 
 
+@pytest.mark.parametrize("name", ["z", "out", "zln", "gate", "xln"])
+def test_misaligned_trimul_tensor_is_refused_before_any_launch(name):
+    N, Cc = 16, 32
+    R = N * N
+    bf = lambda n: torch.zeros(n + 8, device="cuda", dtype=torch.bfloat16)  # noqa: E731
+    f32 = lambda n: torch.zeros(n, device="cuda")  # noqa: E731
+    t = dict(z=bf(R * Cc), out=bf(R * Cc), zln=bf(R * Cc), a=bf(R * Cc), b=bf(R * Cc), gate=bf(R * Cc), x=bf(R * Cc),
+             xln=bf(R * Cc))
+    p = {k: ctypes.c_void_p(v.data_ptr() + (2 if k == name else 0)) for k, v in t.items()}
+    mask, w, stats = f32(R), [f32(2 * Cc * Cc) for _ in range(8)], [f32(R) for _ in range(4)]
+    ws = torch.empty(C.load().tpf_trimul_fwd_workspace_bytes(1, N, Cc), device="cuda", dtype=torch.uint8)
+    launches = C.load().tpf_launch_count()
+    with pytest.raises(ValueError, match=f"{name} must be 16-byte aligned"):
+        C.call("tpf_trimul_fwd", p["z"], C.ptr(mask), *(C.ptr(x) for x in w), 0, 1, N, Cc, p["out"], p["zln"],
+               C.ptr(stats[0]), C.ptr(stats[1]), p["a"], p["b"], p["gate"], p["x"], p["xln"], C.ptr(stats[2]),
+               C.ptr(stats[3]), C.ptr(ws), ws.numel(), C.current_stream())
+    assert C.load().tpf_launch_count() == launches
+
+
 def test_two_host_threads_call_concurrently():
     dev = torch.device("cuda", 0)
     a, d_a = _attention_case(dev, seed=9)

@@ -110,6 +110,44 @@ def test_second_derivative_is_refused(name):
         torch.autograd.grad(g.float().sum(), d_out)
 
 
+def _shifted(t):
+    """The same values one element behind a 16-byte boundary, as a parameter inside a flat buffer has them."""
+    flat = torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)
+    flat[1:].copy_(t.reshape(-1))
+    return flat[1:].view(t.shape)
+
+
+@pytest.mark.parametrize("N,C", [(16, 32), (17, 64), (24, 96), (33, 128)])
+def test_tensors_that_start_between_16_byte_boundaries(N, C):
+    from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
+    from oracle.pair_block_oracle import block_params
+    t = trimul_inputs(1, N, C, seed=N)
+    blk = block_params(C, 2, 16, seed=N)
+    d_out = torch.randn(1, N, N, C, generator=torch.Generator().manual_seed(N)).bfloat16()
+
+    def run(place):
+        z = place(t["z"].cuda()).requires_grad_(True)
+        mask = place(t["mask"].cuda())
+        w = {k: place(v.cuda()).requires_grad_(True) for k, v in t["weights"].items()}
+        b = {k: {n: place(v.cuda()).requires_grad_(True) for n, v in m.items()} for k, m in blk.items()}
+        out = tk.turbo_trimul(z, "outgoing", mask, **w)
+        res = [out, *torch.autograd.grad(out, [z, *w.values()], place(d_out.cuda()))]
+        out = pair_stack_block(z, mask, b, 2)
+        res += [out, *torch.autograd.grad(out, [z, *(v for m in b.values() for v in m.values())], place(d_out.cuda()))]
+        # the operators behind a traced graph
+        pad = (-N) % 8
+        zp = place(torch.nn.functional.pad(t["z"].cuda(), (0, 0, 0, pad, 0, pad))).requires_grad_(True)
+        mp = place(torch.nn.functional.pad(t["mask"].cuda(), (0, pad, 0, pad)))
+        order = ("p_in_weight", "g_in_weight", "p_out_weight", "g_out_weight", "norm_in_weight", "norm_in_bias",
+                 "norm_out_weight", "norm_out_bias")
+        op = torch.ops.tpf_b200.trimul_fwd(zp, mp, *(w[n] for n in order), False)[0]
+        res += [op, *torch.autograd.grad(op.float().square().sum(), [zp, *w.values()])]
+        return res
+
+    for got, want in zip(run(_shifted), run(lambda x: x.clone())):
+        assert torch.equal(got, want)
+
+
 # Enough rows for the projections that keep all weights in shared memory (113 row tiles and more), with a ragged last
 # row tile; 145 tiles at N = 136, one round of 148 row tiles and a second one at N = 184.
 @pytest.mark.parametrize("N,C", [(119, 128), (136, 32), (136, 64), (120, 96), (184, 128)])
