@@ -36,8 +36,10 @@ inline Tensor f32c(const Tensor& t) {
   return t.detach().to(at::kFloat).contiguous();
 }
 
-// A plain eager CUDA tensor: no subclass, no functorch wrapper, no lazy conjugation or negation.  Anything else (and
-// any active dispatch mode) takes the torch.library route, which every such mechanism sees.
+// A plain eager CUDA tensor: no functorch wrapper, no lazy conjugation or negation, no subclass that dispatches (those
+// that only override __torch_function__ are told by their Python type: THPVariable_CheckExact at the entry points, which
+// lets parameters pass).  Anything else (and any active dispatch mode) takes the torch.library route, which every such
+// mechanism sees.
 bool plain_cuda(const Tensor& t);
 bool plain_context();
 

@@ -110,6 +110,46 @@ def test_second_derivative_is_refused(name):
         torch.autograd.grad(g.float().sum(), d_out)
 
 
+class _Tagged(torch.Tensor):
+    """A subclass that sees what is called on it (default behaviour: results are of the subclass, too)."""
+    calls = []
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        cls.calls.append(str(func))
+        return super().__torch_function__(func, types, args, kwargs or {})
+
+
+@pytest.mark.parametrize("which", range(9))
+def test_tensor_subclasses_take_the_route_they_can_see(which):
+    from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
+    from oracle.pair_block_oracle import block_params
+    a = attention_inputs(1, 4, 2, 16, 32, seed=4)
+    t = trimul_inputs(1, 16, 64, seed=4)
+    blk = {k: {n: v.cuda() for n, v in m.items()} for k, m in block_params(64, 4, 16, seed=4).items()}
+    x = [a[n].cuda() for n in ("q", "pair_bias", "res_mask")] + [t["z"].cuda(), t["mask"].cuda(),
+         t["weights"]["g_out_weight"].cuda(), t["z"].cuda(), t["mask"].cuda(), blk["tri_att_end"]["w_q"]]
+    plain = list(x)
+    x[which] = x[which].as_subclass(_Tagged)
+
+    def call(x):
+        if which < 3:
+            return tk.turbo_attention(x[0], a["k"].cuda(), a["v"].cuda(), pair_bias=x[1], res_mask=x[2])
+        if which < 6:
+            w = {n: v.cuda() for n, v in t["weights"].items()}
+            return tk.turbo_trimul(x[3], "outgoing", x[4], **{**w, "g_out_weight": x[5]})
+        return pair_stack_block(x[6], x[7], {**blk, "tri_att_end": {**blk["tri_att_end"], "w_q": x[8]}}, 4)
+
+    _Tagged.calls.clear()
+    out = call(x)
+    assert type(out) is _Tagged and any("tpf_b200" in c for c in _Tagged.calls)
+    # (the block's subclass route is the composition of the operators, which rounds between its steps)
+    assert ao.rel_l2(out.as_subclass(torch.Tensor).cpu(), call(plain).cpu()) <= (1e-2 if which >= 6 else 0)
+    # parameters are tensors as far as the operators are concerned
+    assert type(call([torch.nn.Parameter(v) if v.is_floating_point() and i not in (2, 4, 7) else v
+                      for i, v in enumerate(plain)])) is torch.Tensor
+
+
 def _shifted(t):
     """The same values one element behind a 16-byte boundary, as a parameter inside a flat buffer has them."""
     flat = torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)
