@@ -21,7 +21,8 @@ bool plain_cuda(const Tensor& t) {
 bool plain_context() {
   using c10::DispatchKey;
   static const c10::DispatchKeySet special({DispatchKey::Python, DispatchKey::FuncTorchDynamicLayerFrontMode,
-                                            DispatchKey::FuncTorchDynamicLayerBackMode, DispatchKey::Functionalize});
+                                            DispatchKey::FuncTorchDynamicLayerBackMode, DispatchKey::Functionalize,
+                                            DispatchKey::Tracer});  // (torch.jit.trace)
   return !c10::impl::tls_local_dispatch_key_set().included_.has_any(special);
 }
 

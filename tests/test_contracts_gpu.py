@@ -302,6 +302,26 @@ def test_export_save_load_round_trip(tmp_path):
     assert torch.equal(torch.export.load(path).module()(*args), amod(*args))
 
 
+@pytest.mark.parametrize("name", ["attention", "trimul", "block"])
+def test_jit_trace_records_the_operators(name):
+    from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
+    from openfold3_triangle_kernel_b200.synthetic import block_params
+    a, t = attention_inputs(1, 4, 2, 16, 32, seed=6), trimul_inputs(1, 16, 64, seed=6)
+    w = {n: v.cuda() for n, v in t["weights"].items()}
+    blk = {k: {n: v.cuda() for n, v in m.items()} for k, m in block_params(64, 4, 16, 6).items()}
+    mask, res_mask = t["mask"].cuda(), a["res_mask"].cuda()
+    k, v, bias = (a[n].cuda() for n in ("k", "v", "pair_bias"))
+    fn, x = {"attention": (lambda q: tk.turbo_attention(q, k, v, pair_bias=bias, res_mask=res_mask), a["q"].cuda()),
+             "trimul": (lambda z: tk.turbo_trimul(z, "incoming", mask, **w), t["z"].cuda()),
+             "block": (lambda z: pair_stack_block(z, mask, blk, 4), t["z"].cuda())}[name]
+    traced = torch.jit.trace(fn, (x,), check_trace=False)
+    assert "tpf_b200" in str(traced.graph)
+    other = torch.randn(x.shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(6)).bfloat16()
+    got, want = traced(other), fn(other)
+    # the block's trace is the composition of the operators, which rounds between its steps
+    assert (got.float() - want.float()).norm() <= (1e-2 if name == "block" else 0) * want.float().norm()
+
+
 def test_lse_is_not_differentiable():
     dev = torch.device("cuda", 0)
     a, _ = _attention_case(dev, O=2, N=64)
