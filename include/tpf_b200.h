@@ -205,7 +205,8 @@ int tpf_trimul_bwd(const void* d_out, const void* z, const float* mask,
  *   forward : 1 = LayerNorm + projections + gating (z -> zln, a_cm, b_cm, gate, statistics)
  *             2 = k-contraction (whole pair tensors only; sharded callers run tpf_bmm_bf16 on their
  *                 channel shard between two all-to-alls instead)
- *             4 = output LayerNorm + projection + gate (x_cm, gate -> out, xln, statistics)
+ *             4 = output LayerNorm + projection + gate (x_cm, gate -> out, xln, statistics; at C = 64 and 128 the gate is
+ *                 computed again, from z, and written)
  *   backward: 1 = output gate / projection / LayerNorm backward (-> dx_cm, d_p_out, d_norm_out_*)
  *             2 = contraction backward (dx_cm, a_cm, b_cm -> da_cm, db_cm)
  *             4 = projection / input LayerNorm backward (da_cm, db_cm -> d_z, d_p_in, d_g_in, d_g_out, d_norm_in_*)

@@ -46,6 +46,7 @@ int selftest_status_fetch_and_clear(int* out);
 int selftest_bounded_wait(unsigned int* report, cudaStream_t stream);
 
 int trimul_status_fetch_and_clear(int* out);
+int trimul_fwd_status_fetch_and_clear(int* out);
 int64_t trimul_fwd_workspace_bytes(int64_t B, int64_t N, int64_t C);
 int64_t trimul_bwd_workspace_bytes(int64_t B, int64_t N, int64_t C);
 int trimul_fwd(const void* z, const float* mask, const float* p_in, const float* g_in, const float* p_out,
@@ -83,6 +84,8 @@ int tpf_device_status(int* status) {
   if ((rc = tpf::attn_bwd_status_fetch_and_clear(&v))) return rc;
   total |= v;
   if ((rc = tpf::trimul_status_fetch_and_clear(&v))) return rc;
+  total |= v;
+  if ((rc = tpf::trimul_fwd_status_fetch_and_clear(&v))) return rc;
   total |= v;
   if ((rc = tpf::pair_attn_status_fetch_and_clear(&v))) return rc;
   total |= v;

@@ -38,11 +38,10 @@ struct GemmShape {
 // blockIdx.x, + gridDim.x, ... and computes all their column tiles (the ragged last one first: its epilogue is the
 // short one) from one copy of the A tile.  A is read exactly once, and the CTAs work on neighbouring rows at any time.
 // With STAT_ 2 the CTAs of the different column tiles drift apart in the rows by a third of the problem; once that
-// distance exceeds L2 every one of them reads A from memory, next to output streams that are far apart.  Gated
-// projection of the multiplicative update, C = 128: 38.4 -> 36.6 us at N = 384, 313 -> 223 at 1024, 904 -> 620 at 1536;
-// joint attention projection: 143 -> 129 us at 768, 704 -> 492 at 1536.
+// distance exceeds L2 every one of them reads A from memory, next to output streams that are far apart.  Joint
+// attention projection: 143 -> 129 us at N = 768, 704 -> 492 at 1536.
 template <int BM_, int BN_, int SWZ_A_, bool A_MN_, int SWZ_B_, bool B_MN_, int STAGES_, int EPI_WARPS_ = 8,
-          int STAT_ = 0, int STAT_KB_ = 0, int B_ROWS_ = 0, bool TIGHT_ = false>
+          int STAT_ = 0, int STAT_KB_ = 0, int B_ROWS_ = 0>
 struct GemmCfg {
   static constexpr int BM = BM_, BN = BN_, SWZ_A = SWZ_A_, SWZ_B = SWZ_B_, STAGES = STAGES_;
   static constexpr bool A_MN = A_MN_, B_MN = B_MN_;
@@ -50,7 +49,6 @@ struct GemmCfg {
   static constexpr bool RESIDENT = STAT == 3;
   static constexpr int B_ROWS = B_ROWS_, B_BOX = RESIDENT ? 32 : BN;  // resident B: capacity, rows per load
   static constexpr int MAX_NT = RESIDENT ? (B_ROWS + BN - 1) / BN : 1;
-  static constexpr bool TIGHT = TIGHT_;  // no room to align the shared memory base by hand: the launch checks it
   static constexpr int EPI_WARPS = EPI_WARPS_;          // 8 or 16: warps per TMEM lane quarter x 4
   static constexpr int EPI_PER_Q = EPI_WARPS / 4;       // warps sharing one lane quarter; they interleave 32-column chunks
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
@@ -68,7 +66,7 @@ struct GemmCfg {
   static constexpr int STAGE_A = STAT == 1 ? 0 : A_BYTES;  // bytes of each operand in one ring stage
   static constexpr int STAGE_B = STAT >= 2 ? 0 : B_BYTES;
   static constexpr int STAGE_BYTES = STAGE_A + STAGE_B;
-  static constexpr int SMEM_BYTES = STAT_BYTES + STAGES * STAGE_BYTES + 1024 + (TIGHT ? 0 : 1024);  // + barriers + base alignment
+  static constexpr int SMEM_BYTES = STAT_BYTES + STAGES * STAGE_BYTES + 1024 + 1024;  // + barriers + base alignment
   static_assert(STAT >= 0 && STAT <= 3 && (STAT == 0 || STAT_KB > 0), "stationary operand");
   static_assert(!RESIDENT || (!B_MN && SWZ_B == 128 && B_ROWS % 32 == 0 && MAX_NT <= 4 && STAGES >= STAT_KB), "resident B");
   static_assert(EPI_WARPS == 8 || EPI_WARPS == 16, "epilogue warps");
@@ -247,27 +245,12 @@ struct EpiStore {
   }
 };
 
-// Distance between the scratch areas of two warps: all of kSmemPerWarp, unless the epilogue keeps a part of it behind
-// the last warp's area (kStagePitch).
-template <class Epi, class = void>
-struct EpiPitch {
-  static constexpr int value = Epi::kSmemPerWarp;
-};
-template <class Epi>
-struct EpiPitch<Epi, std::void_t<decltype(Epi::kStagePitch)>> {
-  static constexpr int value = Epi::kStagePitch;
-};
-
 template <class Cfg, class Epi>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const GemmShape sh, const __grid_constant__ typename Epi::Params ep, int* __restrict__ status) {
   griddep_wait();
   extern __shared__ __align__(1024) uint8_t smem_dyn[];
-  if (Cfg::TIGHT && (smem_u32(smem_dyn) & 1023u) != 0) {  // the launch checks it: no write beyond the block's memory
-    if (threadIdx.x == 0 && status != nullptr) *status = (int)kStatusWaitTimeout;
-    return;
-  }
   uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
   uint8_t* st_buf = smem;                      // stationary operand (STAT_BYTES, may be 0)
   uint8_t* ring = smem + Cfg::STAT_BYTES;      // STAGES x [A k-block | B k-block] (a stationary operand takes no room)
@@ -285,10 +268,6 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // A paired epilogue may ask for a tile with the operand roles exchanged (see the UMMA issuer).
-  constexpr bool kCanSwap = Epi::kPaired && Cfg::BN == 256 && Cfg::BM == 128 && !Cfg::A_MN && !Cfg::B_MN &&
-                            Cfg::SWZ_A == 128 && Cfg::SWZ_B == 128;
-
   const TileWalk<Cfg> walk(sh);
   const int k_len = sh.k_per_split > 0 ? sh.k_per_split : sh.K;
   const int kb_count = (k_len + Cfg::BK - 1) / Cfg::BK;
@@ -441,8 +420,6 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         mbar_wait(&tempty[acc], acc_ph, wctx);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_STRIDE;
-        bool swap = false;
-        if constexpr (kCanSwap) swap = Epi::swapped(ep, n0);
         const int s_tile = s;
         const uint32_t ph_tile = ph;
         for (int kb = 0; kb < kb_count; ++kb) {
@@ -456,25 +433,9 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const uint64_t bd0 = b_desc0 + (b_off >> 4);
           constexpr int A_STEP = Cfg::A_MN ? (16 * Cfg::SWZ_A >> 4) : 2;
           constexpr int B_STEP = Cfg::B_MN ? (16 * Cfg::SWZ_B >> 4) : 2;
-          bool swapped_now = false;
-          if constexpr (kCanSwap) swapped_now = swap;
-          if (swapped_now) {
-            // Operand roles exchanged: the two 128-row halves of the B tile are the M operands of two UMMAs
-            // that share the A tile as their N operand.  Accumulator lane = row of the B tile (an output
-            // column of the problem), accumulator column = row of the A tile; the first half's product sits
-            // in columns [0, BM), the second half's in [BN / 2, BN / 2 + BM).
-            constexpr uint32_t idesc_sw = make_idesc_bf16(128, Cfg::BM, false, false);
 #pragma unroll
-            for (int j = 0; j < Cfg::BK / 16; ++j) {
-              umma_ss(el, d_tmem, bd0 + j * B_STEP, ad0 + j * A_STEP, idesc_sw, (kb | j) != 0 ? 1u : 0u);
-              umma_ss(el, d_tmem + Cfg::BN / 2, bd0 + (128 * Cfg::SWZ_B >> 4) + j * B_STEP, ad0 + j * A_STEP, idesc_sw,
-                      (kb | j) != 0 ? 1u : 0u);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < Cfg::BK / 16; ++j)
-              umma_ss(el, d_tmem, ad0 + j * A_STEP, bd0 + j * B_STEP, id_n, (kb | j) != 0 ? 1u : 0u);
-          }
+          for (int j = 0; j < Cfg::BK / 16; ++j)
+            umma_ss(el, d_tmem, ad0 + j * A_STEP, bd0 + j * B_STEP, id_n, (kb | j) != 0 ? 1u : 0u);
           if (last_col) umma_commit(el, &empty[s]);
           if (++s == Cfg::STAGES) {
             s = 0;
@@ -504,7 +465,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // made only at the top of a tile would expose the whole DRAM latency once per tile).
     const int lane_base = 32 * (warp & 3);
     const int chunk_par = (warp - 2) >> 2;
-    float* wsm = reinterpret_cast<float*>(epi_smem + (warp - 2) * EpiPitch<Epi>::value);
+    float* wsm = reinterpret_cast<float*>(epi_smem + (warp - 2) * Epi::kSmemPerWarp);
     int acc = 0;
     uint32_t acc_ph = 0;
     constexpr int NCH = Epi::kPaired ? (Cfg::BN / 64 + Cfg::EPI_PER_Q - 1) / Cfg::EPI_PER_Q
@@ -518,9 +479,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if constexpr (!Epi::kPaired) {
           if (c < Cfg::BN && n0 + c < sh.N) Epi::prefetch(ep, sh, b, m, n0 + c, lane, pre[k]);
         } else {
-          bool swap = false;
-          if constexpr (kCanSwap) swap = Epi::swapped(ep, n0);
-          if (c < Cfg::BN / 2) Epi::prefetch2(ep, sh, b, m0, lane_base + lane, n0, c, lane, swap, pre[k]);
+          if (c < Cfg::BN / 2) Epi::prefetch2(ep, sh, b, m0, lane_base + lane, n0, c, lane, pre[k]);
         }
       }
     };
@@ -579,8 +538,6 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty[acc]);
-        bool swap = false;
-        if constexpr (kCanSwap) swap = Epi::swapped(ep, n0);
 #pragma unroll
         for (int k = 0; k < NCH; ++k) {
           const int c = 32 * (chunk_par + Cfg::EPI_PER_Q * k);
@@ -592,7 +549,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               v0[e] = __uint_as_float(raw0[k][e]);
               v1[e] = __uint_as_float(raw1[k][e]);
             }
-            Epi::apply2(ep, sh, b, m0, lane_base + lane, n0, c, v0, v1, wsm, lane, swap, pre[k], buf);
+            Epi::apply2(ep, sh, b, m0, lane_base + lane, n0, c, v0, v1, wsm, lane, pre[k], buf);
           }
         }
       }

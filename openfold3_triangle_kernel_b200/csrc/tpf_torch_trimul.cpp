@@ -40,6 +40,17 @@ Tensor trimul_bind(tpf::TrimulCall& t, const Tensor& z, const Tensor& mask, cons
   const int64_t R = t.B * t.Np * t.Np;
   Arena a;
   const int64_t packed = a.take(tpf::trimul_fwd_workspace_bytes(t.B, t.Np, C));
+  if (!keep && tpf::trimul_fused(C)) {
+    const int64_t x[3] = {a.take(R * C * 2), a.take(R * C * 2), a.take(R * C * 2)};
+    Tensor arena = arena_in.defined() ? arena_in : empty_bytes(a.off, z);
+    char* base = static_cast<char*>(arena.data_ptr());
+    t.packed = base + packed;
+    t.infer = true;
+    t.a_cm = base + x[0];
+    t.b_cm = base + x[1];
+    t.x_cm = base + x[2];
+    return arena;
+  }
   const int64_t zln = a.take(R * C * 2), acm = a.take(R * C * 2), bcm = a.take(R * C * 2), gate = a.take(R * C * 2);
   const int64_t xcm = keep ? a.take(R * C * 2) : zln;  // zln is dead once a, b and the gate exist,
   const int64_t xln = keep ? a.take(R * C * 2) : acm;  // a once x exists
@@ -214,6 +225,20 @@ py::object py_trimul(py::handle hz, bool incoming, py::handle hm, py::tuple weig
     }
   }
   return py::cast(out);
+}
+
+// The forward that keeps nothing, for the torch.library operators: z [B,N,N,C], any N, mask fp32 [B,N,N].
+Tensor trimul_infer(const Tensor& z_, const Tensor& mask_, std::vector<Tensor> w_, bool incoming) {
+  c10::cuda::CUDAGuard guard(z_.device());
+  const Tensor z = aligned_bf16(z_), mask = mask_.to(at::kFloat);
+  std::vector<Tensor> w;
+  for (const Tensor& t : w_) w.push_back(f32c(t));
+  tpf::TrimulCall t = {};
+  const Tensor arena = trimul_bind(t, z, mask, w, incoming, false, Tensor());
+  Tensor out = empty_bf16(z.sizes(), z);
+  t.out = out.data_ptr();
+  check(tpf::trimul_forward(t, cu_stream()), "tpf_trimul_fwd");
+  return out;
 }
 
 // Launches behind the torch.library operators: z [B,N,N,C] with N a multiple of 8, mask fp32 [B,N,N].

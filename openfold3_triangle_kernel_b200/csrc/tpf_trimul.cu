@@ -11,8 +11,9 @@
 // var = E[x^2] - mean^2 and eps = 1e-5, intermediates (zn, a, b, gate logits, x) are bf16,
 // weight gradients are fp32 sums folded in a fixed order.
 //
-// Every GEMM-shaped stage runs on the tcgen05 engine of tpf_gemm.cuh; gating, masking and the
-// channel-major re-layout that the k-contraction wants are fused into GEMM epilogues.  The
+// At C = 64 and 128 the forward's projections and output stage are the kernels of tpf_trimul_fwd.cu; every other
+// GEMM-shaped stage runs on the tcgen05 engine of tpf_gemm.cuh, with gating, masking and the
+// channel-major re-layout that the k-contraction wants fused into GEMM epilogues.  The
 // a / b / x tensors live channel-major ([B*C][N*N]) so that the k-contraction is a plain batched
 // GEMM in both directions (K-major operands when outgoing, MN-major when incoming).
 #include <cuda_fp16.h>
@@ -42,32 +43,58 @@ int bmm_bf16(const void* A, int64_t lda, int64_t bsa, int a_mn, const void* B, i
              int64_t k_per_split, int swizzle_bytes, cudaStream_t stream);
 
 // =============================================================================================
-// weight packing: fp32 masters -> bf16 W5 [5C,C] = [a_p; a_g; b_p; b_g; g], W5T [C,5C], Wz [C,C], WzT [C,C]
+// weight packing: fp32 masters -> bf16 W5 [5C,C] = [a_p; a_g; b_p; b_g; g], W5T [C,5C], Wz [C,C], WzT [C,C] (W5 null:
+// not wanted), and what the fused forward reads (TrimulFused; fw null: not wanted).  One warp a row.
 // =============================================================================================
-__global__ void trimul_pack_weights_kernel(const float* __restrict__ p_in, const float* __restrict__ g_in,
-                                           const float* __restrict__ p_out, const float* __restrict__ g_out,
-                                           bf16* __restrict__ W5, bf16* __restrict__ W5T, bf16* __restrict__ Wz,
-                                           bf16* __restrict__ WzT, int C) {
+__global__ void __launch_bounds__(64) trimul_pack_weights_kernel(const TrimulWeights w, bf16* __restrict__ W5,
+                                                                  bf16* __restrict__ W5T, bf16* __restrict__ Wz,
+                                                                  bf16* __restrict__ WzT, bf16* __restrict__ fw,
+                                                                  float2* __restrict__ st, int C) {
   griddep_wait();
-  const int n = 5 * C * C;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int row = i / C, col = i % C;
-    const int blk = row / C, r = row % C;
-    float v;
-    if (blk == 0) v = p_in[r * C + col];
-    else if (blk == 1) v = g_in[r * C + col];
-    else if (blk == 2) v = p_in[(C + r) * C + col];
-    else if (blk == 3) v = g_in[(C + r) * C + col];
-    else v = g_out[r * C + col];
-    const bf16 h = __float2bfloat16(v);
-    W5[i] = h;
-    W5T[col * 5 * C + row] = h;
-    if (i < C * C) {
-      const bf16 hz = __float2bfloat16(p_out[i]);
-      Wz[i] = hz;
-      WzT[col * C + row] = hz;
+  const int row = (int)((blockIdx.x * 64 + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  const int blk = row / C, r = row % C;
+  const float* src = blk == 0 ? w.p_in + r * C : blk == 1 ? w.g_in + r * C : blk == 2 ? w.p_in + (C + r) * C
+                     : blk == 3 ? w.g_in + (C + r) * C : blk == 4 ? w.g_out + r * C : w.p_out + r * C;
+  const float* gamma = blk == 5 ? w.norm_out_w : w.norm_in_w;
+  const float* beta = blk == 5 ? w.norm_out_b : w.norm_in_b;
+  float s = 0.f, t = 0.f, in[4], ga[4], be[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = lane + 32 * i;
+    const bool ok = k < C;
+    in[i] = ok ? src[k] : 0.f;
+    ga[i] = ok && fw != nullptr ? gamma[k] : 0.f;
+    be[i] = ok && fw != nullptr ? beta[k] : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int k = lane + 32 * i;
+    if (k >= C) break;
+    const float v = in[i];
+    if (W5 != nullptr) {
+      const bf16 h = __float2bfloat16(v);
+      if (blk < 5) {
+        W5[row * C + k] = h;
+        W5T[k * 5 * C + row] = h;
+      } else {
+        Wz[r * C + k] = h;
+        WzT[k * C + r] = h;
+      }
+    }
+    if (fw != nullptr) {
+      const bf16 h = __float2bfloat16(0.5f * ga[i] * v);
+      fw[row * C + k] = h;
+      s += __bfloat162float(h);
+      t += 0.5f * be[i] * v;
     }
   }
+  if (fw == nullptr) return;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, off);
+    t += __shfl_xor_sync(0xffffffffu, t, off);
+  }
+  if (lane == 0) st[row] = make_float2(s, t);
 }
 
 // =============================================================================================
@@ -180,7 +207,7 @@ __global__ void __launch_bounds__(256, 2) trimul_xnorm_fwd_kernel(const bf16* __
 // =============================================================================================
 // GEMM epilogues
 // =============================================================================================
-// Projection + gating.  GEMM N axis = [a_p | a_g] [b_p | b_g] [g | pad], one tile of width 2C each.
+// Projection + gating (C = 32 and 96; the others: tpf_trimul_fwd.cu).  GEMM N axis = [a_p | a_g] [b_p | b_g] [g | pad], one tile of width 2C each.
 // a and b are stored channel-major.  Each lane owns one row of the accumulator tile, which would
 // make 2-byte scattered stores; the 32x32 block is transposed through a per-warp smem tile so
 // that each lane writes 32 consecutive rows of ONE channel (4 x 16 bytes).
@@ -199,75 +226,30 @@ __device__ __forceinline__ void split_row(int row, int64_t NN, int M, int& bb, i
 }
 
 struct ProjGateParams {
-  CUtensorMap map_a, map_b, map_gate;  // stores: [B][C][NN], [R][C]
+  CUtensorMap map_gate;  // stores: [R][C]
   bf16* a_cm;        // [B*C][NN]
   bf16* b_cm;        // [B*C][NN]
-  bf16* gate;        // [R][C] raw gate logits
   const float* mask; // [R]
   int C;
   int64_t NN;
 };
-// COMPACT (C = 128 with 16 warps and all weights in shared memory): one staging tile per warp, the warps' mask rows
-// behind the last of them.
-template <bool COMPACT>
 struct EpiProjGate {
   using Params = ProjGateParams;
   static constexpr bool kPaired = true;
   static constexpr bool kStaged = false;
-  static constexpr int kSmemPerWarp = COMPACT ? 2048 + 128 : 4608;  // staging and a mask row, or one 32 x 33 float block
-  static constexpr int kStagePitch = COMPACT ? 2048 : 4608;         // from warp to warp
-  static constexpr int kBufs = COMPACT ? 1 : 2;
+  static constexpr int kSmemPerWarp = 4608;  // staging tiles, or one 32 x 33 float block
   struct Pre {
-    float mk;  // pair mask: of this lane's row, or (exchanged tile) of row `lane` of the warp's 32-row chunk
+    float mk;  // pair mask of this lane's row
   };
-  // At C = 128 the a and b tiles are computed with the operand roles exchanged: accumulator lane = channel,
-  // accumulator column = pair row, so a lane holds 32 consecutive pair rows of ONE channel, which is 64
-  // contiguous bytes of the channel-major output, and no transpose is needed.  The gate tile (row-major
-  // output) keeps lane = pair row.
-  __device__ static __forceinline__ bool swapped(const Params& p, int n0) { return n0 < 4 * p.C; }
   __device__ static __forceinline__ void prefetch2(const Params& p, const GemmShape& sh, int, int m0, int rit, int,
-                                                   int c0, int lane, bool swap, Pre& pre) {
-    const int m = swap ? m0 + c0 + lane : m0 + rit;
+                                                   int, int, Pre& pre) {
+    const int m = m0 + rit;
     pre.mk = (m < sh.M) ? p.mask[m] : 0.f;
   }
   __device__ static __forceinline__ void apply2(const Params& p, const GemmShape& sh, int, int m0, int rit, int n0,
                                                 int c0, const float (&v0)[32], const float (&v1)[32], float* wsm,
-                                                int lane, bool swap, const Pre& pre, int& buf) {
+                                                int lane, const Pre& pre, int& buf) {
     const int which = tile_kind(n0, p.C);
-    if (swap) {
-      // lane = channel `rit`; v0[i] / v1[i] = projection / gate logit of pair row m0 + c0 + i
-      const int ew = (threadIdx.x >> 5) - 2;
-      float* msm = COMPACT ? wsm + (16 - ew) * 512 + ew * 32 : wsm + kTmaTiles / 4;
-      msm[lane] = pre.mk;
-      __syncwarp();
-      const uint64_t half2 = f2_pack(0.5f, 0.5f);
-      uint32_t ow[16];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 mk = reinterpret_cast<const float4*>(msm)[q];  // same address in every lane: one broadcast
-        const float mks[4] = {mk.x, mk.y, mk.z, mk.w};
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = 4 * q + 2 * e;
-          float h0, h1, a0, a1;
-          f2_unpack(f2_mul(f2_pack(v1[i], v1[i + 1]), half2), h0, h1);
-          const uint64_t sg = f2_fma(f2_pack(tanh_fast(h0), tanh_fast(h1)), half2, half2);
-          const uint64_t pm = f2_mul(f2_pack(v0[i], v0[i + 1]), f2_pack(mks[2 * e], mks[2 * e + 1]));
-          f2_unpack(f2_mul(pm, sg), a0, a1);
-          ow[2 * q + e] = pack_bf16x2(a0, a1);
-        }
-      }
-      // Rows (and the sharded row count) are multiples of 64, so the 32-row chunk lies inside one batch entry
-      // and is inside M as a whole or not at all.
-      const int r0 = m0 + c0;
-      int bb, rr;
-      split_row(r0, p.NN, sh.M, bb, rr);
-      if (r0 < sh.M)
-        warp_tile_store_tma<kBufs>(reinterpret_cast<uint8_t*>(wsm), buf, lane, ow, which == 0 ? &p.map_a : &p.map_b, rr, rit - lane,
-                            bb);
-      __syncwarp();  // the mask row has been read
-      return;
-    }
     const int m = m0 + rit;
     const int m_base = m - lane;  // first row of this warp's 32-row block (a multiple of 32)
     if (which == 2) {
@@ -275,11 +257,10 @@ struct EpiProjGate {
 #pragma unroll
       for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(v0[2 * i], v0[2 * i + 1]);
       if (m_base < sh.M)
-        warp_tile_store_tma<kBufs>(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk, &p.map_gate, c0, m_base, 0);
+        warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk, &p.map_gate, c0, m_base, 0);
       return;
     }
-    if constexpr (COMPACT) return;  // C = 128: both other tiles are exchanged
-    // a / b tile with lane = pair row (C < 128): each lane owns one row of the accumulator tile, which would
+    // a / b tile: each lane owns one row of the accumulator tile, which would
     // make 2-byte scattered stores; the 32x32 block is transposed through a per-warp smem tile so that each
     // lane writes 8 consecutive rows of four channels (4 x 16 bytes).
     bulk_wait_read<0>();  // the block shares its memory with the gate tiles' staging buffers
@@ -377,9 +358,8 @@ struct EpiGateSplitBwd {
     uint4 d[4];  // incoming gradient, channel-major: d[g] = 8 consecutive rows of channel 8*g + lane/4
     float mk;    // pair mask of this lane's row
   };
-  __device__ static __forceinline__ bool swapped(const Params&, int) { return false; }
   __device__ static __forceinline__ void prefetch2(const Params& p, const GemmShape& sh, int, int m0, int rit, int n0,
-                                                   int c0, int lane, bool, Pre& pre) {
+                                                   int c0, int lane, Pre& pre) {
     const int which = tile_kind(n0, p.C);  // 0: a, 1: b
     const int m = m0 + rit;
     const int m_base = m - lane;
@@ -417,7 +397,7 @@ struct EpiGateSplitBwd {
   }
   __device__ static __forceinline__ void apply2(const Params& p, const GemmShape& sh, int, int m0, int rit, int n0,
                                                 int c0, const float (&v0)[32], const float (&v1)[32], float* wsm,
-                                                int lane, bool, const Pre& pre, int& buf) {
+                                                int lane, const Pre& pre, int& buf) {
     const int which = tile_kind(n0, p.C);  // 0: a, 1: b
     const int m = m0 + rit;
     // d = incoming gradient * mask; t = tanh(g / 2): sigmoid s = 0.5 + 0.5 t, s (1 - s) = 0.25 - 0.25 t^2.
@@ -654,16 +634,23 @@ static TrimulPacked packed_at(void* buf, int64_t C) {
   bf16* base = reinterpret_cast<bf16*>(buf);
   return TrimulPacked{base, base + 5 * C * C, base + 10 * C * C, base + 11 * C * C};
 }
-static int pack_weights(const float* p_in, const float* g_in, const float* p_out, const float* g_out,
-                        const TrimulPacked& pk, int C, cudaStream_t stream) {
-  launch_kernel(trimul_pack_weights_kernel, dim3((5 * C * C + 255) / 256), dim3(256), 0, stream, p_in, g_in, p_out,
-                g_out, pk.W5, pk.W5T, pk.Wz, pk.WzT, C);
+// behind them in the forward's workspace
+static TrimulFused fused_at(void* buf, int64_t C) {
+  bf16* w = reinterpret_cast<bf16*>(buf) + packed_weight_elems(C);
+  float* st = reinterpret_cast<float*>(w + 6 * C * C);
+  return TrimulFused{w, st, st + 12 * C};
+}
+static int pack_weights(const TrimulWeights& w, const TrimulPacked* pk, const TrimulFused* fused, int C, cudaStream_t stream) {
+  const TrimulPacked p = pk ? *pk : TrimulPacked{};
+  const TrimulFused f = fused ? *fused : TrimulFused{};
+  launch_kernel(trimul_pack_weights_kernel, dim3(6 * C / 2), dim3(64), 0, stream, w, p.W5, p.W5T, p.Wz, p.WzT,
+                (bf16*)const_cast<void*>(f.w), reinterpret_cast<float2*>(const_cast<float*>(f.st)), C);
   TPF_LAUNCH_OK();
   return TPF_OK;
 }
 
 // BLOCKS: weight blocks of C rows (a_p, a_g, b_p, b_g and, forward, g).
-template <int C, int BLOCKS, class Epi, class EpiResident>
+template <int C, int BLOCKS, class Epi>
 static int proj_gemm(const bf16* zln, const bf16* W5, int64_t R, const typename Epi::Params& ep, int* status,
                      cudaStream_t stream) {
   // The gated epilogues are latency-bound: at C = 128 and 96 (four, three 32-column chunk pairs per tile) 16
@@ -671,36 +658,47 @@ static int proj_gemm(const bf16* zln, const bf16* W5, int64_t R, const typename 
   // The weights (all of them, or a tile of 2C rows x C) stay in shared memory; only the activations stream.
   const GemmShape sh{(int)R, BLOCKS * C, C, 1, 0};
   if (resident_pays(R, (BLOCKS + 1) / 2)) {
-    using Cfg = GemmCfg<128, 2 * C, 128, false, 128, false, (C + 63) / 64, (C >= 96 ? 16 : 8), 3, (C + 63) / 64,
-                        BLOCKS * C, (C == 128 && BLOCKS == 5)>;
-    return launch_gemm<Cfg, EpiResident>(zln, C, 0, W5, C, 0, sh, ep, status, stream);
+    using Cfg = GemmCfg<128, 2 * C, 128, false, 128, false, (C + 63) / 64, (C >= 96 ? 16 : 8), 3, (C + 63) / 64, BLOCKS * C>;
+    return launch_gemm<Cfg, Epi>(zln, C, 0, W5, C, 0, sh, ep, status, stream);
   }
   using Cfg = GemmCfg<128, 2 * C, 128, false, 128, false, 4, (C >= 96 ? 16 : 8), 2, (C + 63) / 64>;
   return launch_gemm<Cfg, Epi>(zln, C, 0, W5, C, 0, sh, ep, status, stream);
 }
 
 template <int C>
-static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPacked& pk, int64_t NN, int stages,
-                        int* status, cudaStream_t stream) {
+static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPacked& pk, const TrimulFused& fused, int64_t NN,
+                        int stages, int* status, cudaStream_t stream) {
   // t.Np: internal extent (a multiple of 8); NN: internal rows per batch entry (Np * Np for a whole pair tensor,
   // N_local * N for a row shard).
   const int64_t B = t.B, N = t.Np, R = B * NN;
   const bf16* z = (const bf16*)t.z;
   bf16 *zln = (bf16*)t.zln, *xln = (bf16*)t.xln, *x_cm = (bf16*)t.x_cm;
   const PairRows rows = PairRows::make(t.N, t.Np, false);
+  constexpr bool kFused = C % 64 == 0;
   int rc = TPF_OK;
   if (stages & 1) {
-    const PairMask pm{t.mask, t.mask_type, t.mask_stride[0], t.mask_stride[1], t.mask_stride[2]};
-    launch_kernel(rows.identity && !t.mask_grid ? ln_fwd_kernel<C, false> : ln_fwd_kernel<C, true>,
-                  dim3(ln_fwd_blocks<C>(R)), dim3(256), 0, stream, z, t.w.norm_in_w, t.w.norm_in_b, zln, t.mean_in,
-                  t.rstd_in, rows, pm, t.mask_grid, R);
-    TPF_LAUNCH_OK();
-    ProjGateParams ep{{}, {}, {}, (bf16*)t.a_cm, (bf16*)t.b_cm, (bf16*)t.gate, mask, C, NN};
-    if ((rc = make_store_tmap(&ep.map_a, t.a_cm, NN, C, NN, B, C * NN)) ||
-        (rc = make_store_tmap(&ep.map_b, t.b_cm, NN, C, NN, B, C * NN)) ||
-        (rc = make_store_tmap(&ep.map_gate, t.gate, C, R, C, 1, 0)))
-      return rc;
-    if ((rc = proj_gemm<C, 5, EpiProjGate<false>, EpiProjGate<C == 128>>(zln, pk.W5, R, ep, status, stream))) return rc;
+    if (!t.infer) {
+      const PairMask pm{t.mask, t.mask_type, t.mask_stride[0], t.mask_stride[1], t.mask_stride[2]};
+      launch_kernel(rows.identity && !t.mask_grid ? ln_fwd_kernel<C, false> : ln_fwd_kernel<C, true>,
+                    dim3(ln_fwd_blocks<C>(R)), dim3(256), 0, stream, z, t.w.norm_in_w, t.w.norm_in_b, zln, t.mean_in,
+                    t.rstd_in, rows, pm, t.mask_grid, R);
+      TPF_LAUNCH_OK();
+    }
+    if constexpr (kFused) {
+      if ((rc = trimul_project(t, fused, t.infer ? nullptr : mask, NN, stream))) return rc;
+      if (!(stages & 4)) {
+        // The gate logits are a result of this stage; the output kernel, which computes its own, is part of another call.
+        using Cfg = GemmCfg<128, 128, 128, false, 128, false, 4>;
+        const GemmShape sh{(int)R, C, C, 1, 0};
+        typename EpiStore<bf16>::Params ep;
+        if ((rc = epi_store_params<bf16>(&ep, (bf16*)t.gate, C, 0, sh))) return rc;
+        if ((rc = launch_gemm<Cfg, EpiStore<bf16>>(zln, C, 0, pk.W5 + 4 * C * C, C, 0, sh, ep, status, stream))) return rc;
+      }
+    } else {
+      ProjGateParams ep{{}, (bf16*)t.a_cm, (bf16*)t.b_cm, mask, C, NN};
+      if ((rc = make_store_tmap(&ep.map_gate, t.gate, C, R, C, 1, 0))) return rc;
+      if ((rc = proj_gemm<C, 5, EpiProjGate>(zln, pk.W5, R, ep, status, stream))) return rc;
+    }
   }
   if (stages & 2) {
     // k-contraction: batch = B*C problems of N x N x N
@@ -708,24 +706,25 @@ static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPack
     if (rc) return rc;
   }
   if (stages & 4) {
-    const int tiles = (int)((NN + 63) / 64);
-    int grid = (int)(B * tiles);
-    if (grid > 2 * sm_count()) grid = 2 * sm_count();
-    {
+    if (!t.infer) {
+      const int tiles = (int)((NN + 63) / 64);
+      int grid = (int)(B * tiles);
+      if (grid > 2 * sm_count()) grid = 2 * sm_count();
       auto kern = trimul_xnorm_fwd_kernel<C>;
       constexpr int smem = 2 * C * (64 * 2 + 16) + 64 * (C * 2 + 16);
       static PerDeviceOnce once;  // per instantiation
       if ((rc = ensure_dynamic_smem(kern, smem, once))) return rc;
       launch_kernel(kern, dim3(grid), dim3(256), smem, stream, x_cm, t.w.norm_out_w, t.w.norm_out_b, xln, t.mean_out,
                     t.rstd_out, NN, tiles, (int)(B * tiles));
+      TPF_LAUNCH_OK();
     }
-    TPF_LAUNCH_OK();
+    if constexpr (kFused) return trimul_output(t, fused, (stages & 1) != 0, NN, stream);
     GemmShape sh{(int)R, C, C, 1, 0};
     if (t.sum) {
       // The residual doubles the operands the epilogue keeps in flight: narrow tiles, so that a warp has one 32-column
       // chunk and 165 registers for it (wider tiles with two chunks, or with 16 warps of 96 registers, spill).  The
       // activations are read once more per tile column, from L2.
-      using Cfg = GemmCfg<128, (C % 64 == 0 ? 64 : 32), 128, false, 128, false, 4>;
+      using Cfg = GemmCfg<128, 32, 128, false, 128, false, 4>;
       typename EpiOutGate<true>::Params ep{{}, (bf16*)t.out, (bf16*)t.sum, z, (const bf16*)t.gate, rows, C};
       rc = launch_gemm<Cfg, EpiOutGate<true>>(xln, C, 0, pk.Wz, C, 0, sh, ep, status, stream);
     } else {
@@ -804,7 +803,7 @@ static int trimul_bwd_t(const TrimulCall& t, const TrimulGrads& g, const float* 
   if (db_io) w.db_cm = db_io;
   TrimulPacked pk = packed ? *packed : packed_at(w.wpack, C);
   int rc;
-  if (!packed && (rc = pack_weights(t.w.p_in, t.w.g_in, t.w.p_out, t.w.g_out, pk, C, stream))) return rc;
+  if (!packed && (rc = pack_weights(t.w, &pk, nullptr, C, stream))) return rc;
   FoldList folds;
 
   if (stages & 1) {
@@ -860,7 +859,7 @@ static int trimul_bwd_t(const TrimulCall& t, const TrimulGrads& g, const float* 
   {
     EpiGateSplitBwd::Params ep{{}, w.da_cm, w.db_cm, mask, w.d_proj5, C, NN};
     if ((rc = make_store_tmap(&ep.map_d, w.d_proj5, 5 * C, R, 5 * C, 1, 0))) return rc;
-    if ((rc = proj_gemm<C, 4, EpiGateSplitBwd, EpiGateSplitBwd>(zln, pk.W5, R, ep, status, stream))) return rc;
+    if ((rc = proj_gemm<C, 4, EpiGateSplitBwd>(zln, pk.W5, R, ep, status, stream))) return rc;
   }
   // 6. d_zln = d_proj5 W5 ; dW5 = d_proj5^T zln
   bf16* d_zln = w.d_xln;
@@ -905,7 +904,9 @@ static int check_trimul_shape(const char* who, int64_t B, int64_t N, int64_t C) 
   return TPF_OK;
 }
 
-int64_t trimul_fwd_workspace_bytes(int64_t B, int64_t N, int64_t C) { return align256(packed_weight_elems(C) * 2); }
+int64_t trimul_fwd_workspace_bytes(int64_t B, int64_t N, int64_t C) {
+  return align256(packed_weight_elems(C) * 2 + (trimul_fused(C) ? 6 * C * C * 2 + 6 * C * 8 + B * N * N * 8 : 0));
+}
 
 int64_t trimul_bwd_workspace_bytes(int64_t B, int64_t NN, int64_t C) {
   TrimulBwdWorkspace w;
@@ -929,19 +930,20 @@ static int check_trimul_aligned(const char* who, std::initializer_list<std::pair
   return TPF_OK;
 }
 
-static int trimul_fwd_run(const TrimulCall& t, int64_t NN, int stages, bool with_pack, cudaStream_t stream) {
+static int trimul_fwd_run(const TrimulCall& t, int64_t NN, int stages, cudaStream_t stream) {
   int* status = nullptr;
   int rc = check_trimul_aligned("trimul_fwd", {{"z", t.z}, {"out", t.out}, {"sum", t.sum}, {"zln", t.zln}, {"a_cm", t.a_cm},
                                                {"b_cm", t.b_cm}, {"gate", t.gate}, {"x_cm", t.x_cm}, {"xln", t.xln},
                                                {"workspace", t.packed}});
   if (rc || (rc = trimul_status(&status))) return rc;
   const TrimulPacked pk = packed_at(t.packed, t.C);
-  if (with_pack && (rc = pack_weights(t.w.p_in, t.w.g_in, t.w.p_out, t.w.g_out, pk, (int)t.C, stream))) return rc;
+  const TrimulFused fused = fused_at(t.packed, t.C);
+  if ((rc = pack_weights(t.w, t.infer ? nullptr : &pk, trimul_fused(t.C) ? &fused : nullptr, (int)t.C, stream))) return rc;
   switch (t.C) {
-    case 32: return trimul_fwd_t<32>(t, grid_mask(t), pk, NN, stages, status, stream);
-    case 64: return trimul_fwd_t<64>(t, grid_mask(t), pk, NN, stages, status, stream);
-    case 96: return trimul_fwd_t<96>(t, grid_mask(t), pk, NN, stages, status, stream);
-    case 128: return trimul_fwd_t<128>(t, grid_mask(t), pk, NN, stages, status, stream);
+    case 32: return trimul_fwd_t<32>(t, grid_mask(t), pk, fused, NN, stages, status, stream);
+    case 64: return trimul_fwd_t<64>(t, grid_mask(t), pk, fused, NN, stages, status, stream);
+    case 96: return trimul_fwd_t<96>(t, grid_mask(t), pk, fused, NN, stages, status, stream);
+    case 128: return trimul_fwd_t<128>(t, grid_mask(t), pk, fused, NN, stages, status, stream);
   }
   return fail(TPF_ERR_UNSUPPORTED, "trimul_fwd: unsupported C");
 }
@@ -970,7 +972,7 @@ static int trimul_bwd_run(const TrimulCall& t, const TrimulGrads& g, int64_t NN,
 int trimul_forward(const TrimulCall& t, cudaStream_t stream) {
   int rc = check_trimul_shape("trimul_fwd", t.B, t.Np, t.C);
   if (rc) return rc;
-  return trimul_fwd_run(t, t.Np * t.Np, 7, true, stream);
+  return trimul_fwd_run(t, t.Np * t.Np, 7, stream);
 }
 
 int trimul_backward(const TrimulCall& t, const TrimulGrads& g, void* workspace, int64_t workspace_bytes,
@@ -1004,7 +1006,7 @@ int trimul_fwd(const void* z, const float* mask, const float* p_in, const float*
   t.packed = workspace;
   t.out = out; t.zln = zln; t.mean_in = mean_in; t.rstd_in = rstd_in; t.a_cm = a_cm; t.b_cm = b_cm; t.gate = gate;
   t.x_cm = x_cm; t.xln = xln; t.mean_out = mean_out; t.rstd_out = rstd_out;
-  return trimul_fwd_run(t, NN, stages, true, stream);
+  return trimul_fwd_run(t, NN, stages, stream);
 }
 
 int trimul_bwd(const void* d_out, const void* z, const float* mask, const float* p_in, const float* g_in,
