@@ -9,7 +9,8 @@
 //  1541-1809, 226-438 and turbopairformer_trimul.py:184-392).  Rounding points follow the
 // reference: fp32 master weights are rounded to bf16 once, LayerNorm statistics are fp32 with
 // var = E[x^2] - mean^2 and eps = 1e-5, intermediates (zn, a, b, gate logits, x) are bf16,
-// weight gradients are fp32 sums folded in a fixed order.
+// weight gradients are fp32 sums folded in a fixed order.  (The forward's kernels at C = 64 and 128 round gamma W instead
+// of zn and of the weights, and their own gate not at all.)
 //
 // At C = 64 and 128 the forward's projections and output stage are the kernels of tpf_trimul_fwd.cu; every other
 // GEMM-shaped stage runs on the tcgen05 engine of tpf_gemm.cuh, with gating, masking and the
