@@ -202,11 +202,11 @@ int tpf_trimul_bwd(const void* d_out, const void* z, const float* mask,
 /* Stage-wise TriMul for row-sharded (axially parallel) execution.  `rows_per_batch` is the number of
  * pair rows each batch entry holds on this rank (N_local * N; 0 means N * N; a multiple of 64) and
  * replaces N*N in every [B*N*N, C] / [B*C, N*N] extent above.  `stages` selects
- *   forward : 1 = LayerNorm + projections + gating (z -> zln, a_cm, b_cm, gate, statistics)
+ *   forward : 1 = LayerNorm + projections + gating (z -> zln, a_cm, b_cm, mean_in, rstd_in; gate at C = 32 and 96)
  *             2 = k-contraction (whole pair tensors only; sharded callers run tpf_bmm_bf16 on their
  *                 channel shard between two all-to-alls instead)
- *             4 = output LayerNorm + projection + gate (x_cm, gate -> out, xln, statistics; at C = 64 and 128 the gate is
- *                 computed again, from z, and written)
+ *             4 = output LayerNorm + projection + gate (x_cm -> out, xln, mean_out, rstd_out; reads the gate at C = 32 and
+ *                 96; at C = 64 and 128 reads z, mean_in and rstd_in of stage 1 and writes the gate)
  *   backward: 1 = output gate / projection / LayerNorm backward (-> dx_cm, d_p_out, d_norm_out_*)
  *             2 = contraction backward (dx_cm, a_cm, b_cm -> da_cm, db_cm)
  *             4 = projection / input LayerNorm backward (da_cm, db_cm -> d_z, d_p_in, d_g_in, d_g_out, d_norm_in_*)

@@ -41,7 +41,7 @@ Tensor trimul_bind(tpf::TrimulCall& t, const Tensor& z, const Tensor& mask, cons
   Arena a;
   const int64_t packed = a.take(tpf::trimul_fwd_workspace_bytes(t.B, t.Np, C));
   if (!keep && tpf::trimul_fused(C)) {
-    const int64_t x[3] = {a.take(R * C * 2), a.take(R * C * 2), a.take(R * C * 2)};
+    const int64_t x[3] = {a.take(R * C * 2), a.take(R * C * 2), a.take(R * C * 2)}, stats = a.take(2 * R * 4);
     Tensor arena = arena_in.defined() ? arena_in : empty_bytes(a.off, z);
     char* base = static_cast<char*>(arena.data_ptr());
     t.packed = base + packed;
@@ -49,6 +49,8 @@ Tensor trimul_bind(tpf::TrimulCall& t, const Tensor& z, const Tensor& mask, cons
     t.a_cm = base + x[0];
     t.b_cm = base + x[1];
     t.x_cm = base + x[2];
+    t.mean_in = reinterpret_cast<float*>(base + stats);
+    t.rstd_in = t.mean_in + R;
     return arena;
   }
   const int64_t zln = a.take(R * C * 2), acm = a.take(R * C * 2), bcm = a.take(R * C * 2), gate = a.take(R * C * 2);

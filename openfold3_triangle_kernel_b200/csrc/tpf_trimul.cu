@@ -638,8 +638,7 @@ static TrimulPacked packed_at(void* buf, int64_t C) {
 // behind them in the forward's workspace
 static TrimulFused fused_at(void* buf, int64_t C) {
   bf16* w = reinterpret_cast<bf16*>(buf) + packed_weight_elems(C);
-  float* st = reinterpret_cast<float*>(w + 6 * C * C);
-  return TrimulFused{w, st, st + 12 * C};
+  return TrimulFused{w, reinterpret_cast<float*>(w + 6 * C * C)};
 }
 static int pack_weights(const TrimulWeights& w, const TrimulPacked* pk, const TrimulFused* fused, int C, cudaStream_t stream) {
   const TrimulPacked p = pk ? *pk : TrimulPacked{};
@@ -681,20 +680,12 @@ static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPack
     if (!t.infer) {
       const PairMask pm{t.mask, t.mask_type, t.mask_stride[0], t.mask_stride[1], t.mask_stride[2]};
       launch_kernel(rows.identity && !t.mask_grid ? ln_fwd_kernel<C, false> : ln_fwd_kernel<C, true>,
-                    dim3(ln_fwd_blocks<C>(R)), dim3(256), 0, stream, z, t.w.norm_in_w, t.w.norm_in_b, zln, t.mean_in,
-                    t.rstd_in, rows, pm, t.mask_grid, R);
+                    dim3(ln_fwd_blocks<C>(R)), dim3(256), 0, stream, z, t.w.norm_in_w, t.w.norm_in_b, zln,
+                    kFused ? nullptr : t.mean_in, kFused ? nullptr : t.rstd_in, rows, pm, t.mask_grid, R);
       TPF_LAUNCH_OK();
     }
     if constexpr (kFused) {
       if ((rc = trimul_project(t, fused, t.infer ? nullptr : mask, NN, stream))) return rc;
-      if (!(stages & 4)) {
-        // The gate logits are a result of this stage; the output kernel, which computes its own, is part of another call.
-        using Cfg = GemmCfg<128, 128, 128, false, 128, false, 4>;
-        const GemmShape sh{(int)R, C, C, 1, 0};
-        typename EpiStore<bf16>::Params ep;
-        if ((rc = epi_store_params<bf16>(&ep, (bf16*)t.gate, C, 0, sh))) return rc;
-        if ((rc = launch_gemm<Cfg, EpiStore<bf16>>(zln, C, 0, pk.W5 + 4 * C * C, C, 0, sh, ep, status, stream))) return rc;
-      }
     } else {
       ProjGateParams ep{{}, (bf16*)t.a_cm, (bf16*)t.b_cm, mask, C, NN};
       if ((rc = make_store_tmap(&ep.map_gate, t.gate, C, R, C, 1, 0))) return rc;
@@ -719,7 +710,7 @@ static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPack
                     t.rstd_out, NN, tiles, (int)(B * tiles));
       TPF_LAUNCH_OK();
     }
-    if constexpr (kFused) return trimul_output(t, fused, (stages & 1) != 0, NN, stream);
+    if constexpr (kFused) return trimul_output(t, fused, NN, stream);
     GemmShape sh{(int)R, C, C, 1, 0};
     if (t.sum) {
       // The residual doubles the operands the epilogue keeps in flight: narrow tiles, so that a warp has one 32-column
@@ -906,7 +897,7 @@ static int check_trimul_shape(const char* who, int64_t B, int64_t N, int64_t C) 
 }
 
 int64_t trimul_fwd_workspace_bytes(int64_t B, int64_t N, int64_t C) {
-  return align256(packed_weight_elems(C) * 2 + (trimul_fused(C) ? 6 * C * C * 2 + 6 * C * 8 + B * N * N * 8 : 0));
+  return align256(packed_weight_elems(C) * 2 + (trimul_fused(C) ? 6 * C * C * 2 + 6 * C * 8 : 0));
 }
 
 int64_t trimul_bwd_workspace_bytes(int64_t B, int64_t NN, int64_t C) {

@@ -84,12 +84,13 @@ __device__ __forceinline__ void unpack_pairs(const uint4& u, uint64_t (&x)[4]) {
   x[2] = f2_pack(bf16_lo(u.z), bf16_hi(u.z));
   x[3] = f2_pack(bf16_lo(u.w), bf16_hi(u.w));
 }
-// What the epilogue needs of a row: rs and -rs mu.
+struct RowStats {
+  float mu, rs;
+};
 template <int C>
-__device__ __forceinline__ float2 row_stats(float s1, float s2) {
+__device__ __forceinline__ RowStats row_stats(float s1, float s2) {
   const float mu = s1 * (1.f / C);
-  const float rs = rsqrtf(fmaxf(s2 * (1.f / C) - mu * mu, 0.f) + 1e-5f);
-  return make_float2(rs, -rs * mu);
+  return RowStats{mu, rsqrtf(fmaxf(s2 * (1.f / C) - mu * mu, 0.f) + 1e-5f)};
 }
 
 // Sum and sum of squares of a lane's channels: eight of each 64.
@@ -139,23 +140,6 @@ __device__ __forceinline__ void stats_rows(const uint8_t* const (&kb)[C / 64], i
       for (int u = 0; u < U; ++u) store(row0 + r + 4 * u + (lane >> 3), row_stats<C>(s1[u], s2[u]));
     }
   }
-}
-
-// The same of rows in memory, for an output kernel that no projection of the same call precedes (the stages of a sharded
-// update): the same sums in the same order.
-template <int C>
-__global__ void __launch_bounds__(256) trimul_row_stats_kernel(const bf16* __restrict__ z, float2* __restrict__ stats, int R) {
-  griddep_wait();
-  const int row = (int)((blockIdx.x * 256 + threadIdx.x) >> 3), lane = threadIdx.x & 7;
-  const bf16* src = z + (int64_t)(row < R ? row : 0) * C + 8 * lane;
-  float s1, s2;
-  lane_sums<C>([&](int k) { return *reinterpret_cast<const uint4*>(src + 64 * k); }, s1, s2);
-#pragma unroll
-  for (int off = 4; off > 0; off >>= 1) {
-    s1 += __shfl_xor_sync(0xffffffffu, s1, off);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, off);
-  }
-  if (row < R && lane == 0) stats[row] = row_stats<C>(s1, s2);
 }
 
 // Sums of the 64 rows of an MN-major tile (C lines of 128 bytes, one a channel, 128-byte swizzle) by one warp: a lane
@@ -210,7 +194,7 @@ struct TrimulProjectParams {
   FastDiv per_entry;       // internal rows per batch entry
   PairMask mask;           // the caller's,
   const float* mask_grid;  // or, if not null, [R]
-  float2* z_stats;         // [R], for the output kernel
+  float *mean, *rstd;      // [R]: for the output kernel, and kept for a backward
   int R;                   // internal rows
 };
 
@@ -454,10 +438,13 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
           ph ^= 1;
         }
       }
-      stats_rows<C, 64>(kb, 64 * sw0, lane, [&](int row, float2 v) {
-        rs[row] = v.x;
-        rs[128 + row] = v.y;
-        if (tile * 128 + row < p.R) p.z_stats[tile * 128 + row] = v;
+      stats_rows<C, 64>(kb, 64 * sw0, lane, [&](int row, const RowStats& v) {
+        rs[row] = v.rs;
+        rs[128 + row] = -v.rs * v.mu;
+        if (tile * 128 + row < p.R) {
+          p.mean[tile * 128 + row] = v.mu;
+          p.rstd[tile * 128 + row] = v.rs;
+        }
       });
       rs[256 + 64 * sw0 + lane] = mk[0];
       rs[256 + 64 * sw0 + 32 + lane] = mk[1];
@@ -483,7 +470,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
 // =============================================================================================
 struct TrimulOutputParams {
   const float2 *st_x, *st_z;  // (S, T) of the rows of Wz and Wg
-  const float2* z_stats;      // (rs, -rs mu) of the rows of z
+  const float *z_mean, *z_rstd;  // [R], from the projection
   PairRows rows;
   FastDiv per_entry;
   bf16* gate;        // KEEP: [R, C]
@@ -628,13 +615,16 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++i) {
       const int s = i & 1;
       const int m_base = tile * 128 + 32 * quarter;
-      float2 zst = make_float2(0.f, 0.f);
-      if (m_base + lane < p.R) zst = p.z_stats[m_base + lane];
+      float z_mu = 0.f, z_rs = 0.f;
+      if (m_base + lane < p.R) {
+        z_mu = p.z_mean[m_base + lane];
+        z_rs = p.z_rstd[m_base + lane];
+      }
       mbar_wait2(&tfull[s], (i >> 1) & 1, &r_full[i & 3], (i >> 2) & 1, wctx);
       tc_fence_after();
       const float* row = reinterpret_cast<const float*>(smem + Cfg::OFF_ROW + (i & 3) * 1024) + 32 * quarter + lane;
       const uint64_t xr = f2_pack(row[0], row[0]), xm = f2_pack(row[128], row[128]);
-      const uint64_t zr = f2_pack(zst.x, zst.x), zm = f2_pack(zst.y, zst.y);
+      const uint64_t zr = f2_pack(z_rs, z_rs), zm = f2_pack(-z_rs * z_mu, -z_rs * z_mu);
 #pragma unroll
       for (int k = 0; k < C / 64; ++k) {
         const int n0 = 32 * (par + 2 * k);
@@ -721,9 +711,9 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       if (s != sw >> 1) continue;
       float* row = reinterpret_cast<float*>(smem + Cfg::OFF_ROW + (i & 3) * 1024);
       mbar_wait(&x_full[s], (i >> 1) & 1, wctx);
-      stats_lines<C>(smem + Cfg::OFF_X + s * Cfg::T_BYTES + h * C * 128, lane, [&](int q, float2 v) {
-        row[64 * h + q] = v.x;
-        row[128 + 64 * h + q] = v.y;
+      stats_lines<C>(smem + Cfg::OFF_X + s * Cfg::T_BYTES + h * C * 128, lane, [&](int q, const RowStats& v) {
+        row[64 * h + q] = v.rs;
+        row[128 + 64 * h + q] = -v.rs * v.mu;
       });
       __syncwarp();
       if (lane == 0) {
@@ -787,7 +777,8 @@ static int project(const TrimulCall& t, const TrimulFused& w, const float* mask_
   p.per_entry = FastDiv::make((uint32_t)NN);
   p.mask = PairMask{t.mask, t.mask_type, t.mask_stride[0], t.mask_stride[1], t.mask_stride[2]};
   p.mask_grid = mask_grid;
-  p.z_stats = reinterpret_cast<float2*>(w.z_stats);
+  p.mean = t.mean_in;
+  p.rstd = t.rstd_in;
   p.R = (int)R;
   CUtensorMap tz, tz8, tw, ta, tb;
   if ((rc = make_z_tmaps(&tz, &tz8, t, p.rows, R)) || (rc = make_operand_tmap(&tw, w.w, false, 4 * C, C, C, 1, 0, 128, 32, 64)) ||
@@ -811,7 +802,8 @@ static int output(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStr
   TrimulOutputParams p{};
   p.st_z = reinterpret_cast<const float2*>(w.st) + 4 * C;
   p.st_x = p.st_z + C;
-  p.z_stats = reinterpret_cast<const float2*>(w.z_stats);
+  p.z_mean = t.mean_in;
+  p.z_rstd = t.rstd_in;
   p.rows = PairRows::make(t.N, t.Np, false);
   p.per_entry = FastDiv::make((uint32_t)NN);
   p.gate = (bf16*)t.gate;
@@ -836,13 +828,7 @@ static int output(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStr
 }
 
 template <int C>
-static int output(const TrimulCall& t, const TrimulFused& w, bool projected, int64_t NN, cudaStream_t stream) {
-  if (!projected) {  // the caller's rows are the internal ones
-    const int64_t R = t.B * NN;
-    launch_kernel(trimul_row_stats_kernel<C>, dim3((unsigned)((R + 31) / 32)), dim3(256), 0, stream, (const bf16*)t.z,
-                  reinterpret_cast<float2*>(w.z_stats), (int)R);
-    TPF_LAUNCH_OK();
-  }
+static int output(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStream_t stream) {
   if (t.infer) return t.sum ? output<C, true, false>(t, w, NN, stream) : output<C, false, false>(t, w, NN, stream);
   return t.sum ? output<C, true, true>(t, w, NN, stream) : output<C, false, true>(t, w, NN, stream);
 }
@@ -853,9 +839,8 @@ bool trimul_fused(int64_t C) { return C == 64 || C == 128; }
 int trimul_project(const TrimulCall& t, const TrimulFused& w, const float* mask_grid, int64_t NN, cudaStream_t stream) {
   return t.C == 64 ? project<64>(t, w, mask_grid, NN, stream) : project<128>(t, w, mask_grid, NN, stream);
 }
-// projected: trimul_project has run before in the same call.
-int trimul_output(const TrimulCall& t, const TrimulFused& w, bool projected, int64_t NN, cudaStream_t stream) {
-  return t.C == 64 ? output<64>(t, w, projected, NN, stream) : output<128>(t, w, projected, NN, stream);
+int trimul_output(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStream_t stream) {
+  return t.C == 64 ? output<64>(t, w, NN, stream) : output<128>(t, w, NN, stream);
 }
 
 }  // namespace tpf
