@@ -74,9 +74,10 @@ struct TrimulCall {
   void* sum;          // bf16 [B,N,N,C] = z + out, or nullptr
   void *zln, *a_cm, *b_cm, *gate, *x_cm, *xln;            // bf16 [B*Np*Np, C]
   float *mean_in, *rstd_in, *mean_out, *rstd_out;         // fp32 [B*Np*Np]
-  // Nothing is kept for a backward (only where trimul_fused(C)): of the intermediates the forward then needs a_cm, b_cm, x_cm,
-  // mean_in and rstd_in alone, and no mask_grid.
+  // Nothing is kept for a backward (only where trimul_fused(C)): of the intermediates the forward then needs a_cm, b_cm and
+  // x_cm alone, z_stats in place of the input norm's statistics, and no mask_grid.
   bool infer;
+  float* z_stats;     // fp32 [B*Np*Np, 2]
 };
 // The forward's weights in kernel layout (tpf_trimul_fwd.cu): w = gamma W in bf16, rows [a_p; a_g; b_p; b_g; g] (input norm)
 // and z (output norm), all halved (which is exact: p sigmoid(g) = p / 2 + p / 2 tanh(g / 2)); st: (sum of w, sum of beta W)
@@ -86,8 +87,9 @@ struct TrimulFused {
   const float* st;  // fp32 [6C, 2]
 };
 bool trimul_fused(int64_t C);
-// NN: internal rows per batch entry.  The first writes mean_in and rstd_in, which the second reads.
-int trimul_project(const TrimulCall& t, const TrimulFused& w, const float* mask_grid, int64_t NN, cudaStream_t stream);
+// NN: internal rows per batch entry.  The first writes the statistics of z's rows (mean_in and rstd_in, or z_stats), which
+// the second reads.
+int trimul_project(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStream_t stream);
 int trimul_output(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStream_t stream);
 struct TrimulGrads {
   const void* d_out;  // bf16 [B,N,N,C]

@@ -49,8 +49,7 @@ Tensor trimul_bind(tpf::TrimulCall& t, const Tensor& z, const Tensor& mask, cons
     t.a_cm = base + x[0];
     t.b_cm = base + x[1];
     t.x_cm = base + x[2];
-    t.mean_in = reinterpret_cast<float*>(base + stats);
-    t.rstd_in = t.mean_in + R;
+    t.z_stats = reinterpret_cast<float*>(base + stats);
     return arena;
   }
   const int64_t zln = a.take(R * C * 2), acm = a.take(R * C * 2), bcm = a.take(R * C * 2), gate = a.take(R * C * 2);

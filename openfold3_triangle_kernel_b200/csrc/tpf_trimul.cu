@@ -677,16 +677,14 @@ static int trimul_fwd_t(const TrimulCall& t, const float* mask, const TrimulPack
   constexpr bool kFused = C % 64 == 0;
   int rc = TPF_OK;
   if (stages & 1) {
-    if (!t.infer) {
+    if constexpr (kFused) {
+      if ((rc = trimul_project(t, fused, NN, stream))) return rc;
+    } else {
       const PairMask pm{t.mask, t.mask_type, t.mask_stride[0], t.mask_stride[1], t.mask_stride[2]};
       launch_kernel(rows.identity && !t.mask_grid ? ln_fwd_kernel<C, false> : ln_fwd_kernel<C, true>,
-                    dim3(ln_fwd_blocks<C>(R)), dim3(256), 0, stream, z, t.w.norm_in_w, t.w.norm_in_b, zln,
-                    kFused ? nullptr : t.mean_in, kFused ? nullptr : t.rstd_in, rows, pm, t.mask_grid, R);
+                    dim3(ln_fwd_blocks<C>(R)), dim3(256), 0, stream, z, t.w.norm_in_w, t.w.norm_in_b, zln, t.mean_in,
+                    t.rstd_in, rows, pm, t.mask_grid, R);
       TPF_LAUNCH_OK();
-    }
-    if constexpr (kFused) {
-      if ((rc = trimul_project(t, fused, t.infer ? nullptr : mask, NN, stream))) return rc;
-    } else {
       ProjGateParams ep{{}, (bf16*)t.a_cm, (bf16*)t.b_cm, mask, C, NN};
       if ((rc = make_store_tmap(&ep.map_gate, t.gate, C, R, C, 1, 0))) return rc;
       if ((rc = proj_gemm<C, 5, EpiProjGate>(zln, pk.W5, R, ep, status, stream))) return rc;

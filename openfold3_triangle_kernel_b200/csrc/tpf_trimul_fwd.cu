@@ -13,19 +13,22 @@
 // and the epilogue applies a row's rs and mu.  S is summed from the rounded W', so the mean cancels up to fp32 rounding,
 // and of the two roundings of the other order (of the normalised rows and of W) one is left: 4.5e-3 from an fp64
 // evaluation instead of 5.5e-3.  Nor does the gate pass through memory: its logits are computed where they are used, from
-// z, which costs the read that the gate would have cost.  A forward with a backward behind it has its norms (kernels of
-// tpf_trimul.cu) write what that one reads, zln, xln and the statistics, and its output kernel the gate logits.
+// z, which costs the read that the gate would have cost.  Of what a backward reads, the projection writes zln, the statistics
+// and the mask of its rows, the output kernel the gate logits, and the output norm (a kernel of tpf_trimul.cu) xln.
 //
 // Both kernels are persistent and warp-specialised like the GEMM engine.  The weights stay in shared memory; a few warps
 // read each landed tile once more for the sums of its rows, in 16-byte accesses without bank conflicts (normalising the
-// tile in place instead, before the UMMAs, took 249 and 190 us where this takes 215 and 135).
+// tile in place instead, before the UMMAs, took 249 and 190 us where this took 215 and 135).
 //
-// Measured, C = 128, nothing kept: N = 1024 763 -> 565 us of kernels (norm 99 + projection 223 -> projection 215; norm 100
-// + output 126 -> output 135; contraction 210 either way), N = 517 248 -> 183 us.  The output kernel runs at the copy
+// Measured, C = 128, nothing kept: N = 1024 763 -> 550 us of kernels (norm 99 + projection 223 -> projection 207; norm 100
+// + output 126 -> output 133; contraction 210 either way), N = 517 248 -> 178 us.  The output kernel runs at the copy
 // rate (805 MB).  The projection does not (124 us): a tile takes an SM 7100 cycles, of which its 32 UMMAs of 128 x 128 x
 // 16 need all of the shared memory bandwidth for 2050, beside 16 epilogue warps that take about 1650 cycles of arithmetic
-// and 600 of staging and fence for 32 x 32 elements.  With a backward behind it: projection 36 -> 32, output 22 -> 29 us at
-// N = 384 (which then stores the gate that the projection stored before).
+// and 600 of staging and fence for 32 x 32 elements.  With a backward behind it, N = 384: norm 17 + projection 36 + output
+// 22 -> projection 38 + output 30 us (which then stores the gate that the projection stored before).  A kernel of its own
+// for zln read z a second time: 17 + 32 instead of 38 us.  Two warps for the rows, as without zln, take 52.
+#include <type_traits>
+
 #include "tpf_gemm_host.cuh"
 #include "tpf_internal.h"
 #include "tpf_norm.cuh"
@@ -115,9 +118,13 @@ __device__ __forceinline__ void lane_sums(Load load, float& s1, float& s2) {
 }
 
 // Sums of ROWS consecutive rows of a K-major tile (64-channel blocks kb[] of 128 rows x 128 bytes, 128-byte swizzle) by one
-// warp: eight lanes a row, 16 bytes of each block, four steps of four rows in flight.
-template <int C, int ROWS, class Store>
-__device__ __forceinline__ void stats_rows(const uint8_t* const (&kb)[C / 64], int row0, int lane, Store store) {
+// warp: eight lanes a row, 16 bytes of each block, four steps of four rows in flight.  `store` is called in one lane a row,
+// all four rows behind one branch (with a branch for each row the projection took 225 instead of 207 us at N = 1024: its
+// tiles wait for these warps); `each`, if there is one, in all lanes, with the place of the lane's 16 bytes.
+struct NoEach {};
+template <int C, int ROWS, class Store, class Each = NoEach>
+__device__ __forceinline__ void stats_rows(const uint8_t* const (&kb)[C / 64], int row0, int lane, Store store,
+                                           Each each = {}) {
   constexpr int U = 4;
 #pragma unroll 1
   for (int r = 0; r < ROWS; r += 4 * U) {
@@ -138,6 +145,13 @@ __device__ __forceinline__ void stats_rows(const uint8_t* const (&kb)[C / 64], i
     if ((lane & 7) == 0) {
 #pragma unroll
       for (int u = 0; u < U; ++u) store(row0 + r + 4 * u + (lane >> 3), row_stats<C>(s1[u], s2[u]));
+    }
+    if constexpr (!std::is_same<Each, NoEach>::value) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int row = row0 + r + 4 * u + (lane >> 3);
+        each(row, row * 128 + (((lane & 7) ^ (row & 7)) << 4), row_stats<C>(s1[u], s2[u]));
+      }
     }
   }
 }
@@ -194,18 +208,26 @@ struct TrimulProjectParams {
   FastDiv per_entry;       // internal rows per batch entry
   PairMask mask;           // the caller's,
   const float* mask_grid;  // or, if not null, [R]
-  float *mean, *rstd;      // [R]: for the output kernel, and kept for a backward
+  float2* z_stats;         // [R] for the output kernel; KEEP: in its place
+  float *mean, *rstd;      // [R]
+  const float *gamma, *beta;
+  bf16* zln;               // [R, C] normalised rows, zeros where the grid has no row of the caller
+  float* mask_out;         // [R], or null: the mask has the internal layout
   int R;                   // internal rows
 };
 
-template <int C_>
+// KEEP: what a backward reads of the norm and the mask is written.
+template <int C_, bool KEEP_>
 struct TrimulProjectCfg {
   static constexpr int C = C_;
+  static constexpr bool KEEP = KEEP_;
   static constexpr int NT = C / 64;              // accumulator tiles of 128 channels: the 2 C channels of [a, b]
   static constexpr int KB = C / 64;
   static constexpr int W_BYTES = 4 * C * C * 2;  // per 64 channels of k: projection rows [a, b], gate rows [a, b]
   static constexpr int NST = 3;                  // slots of 64 channels x 128 rows
-  static constexpr int NCW = 16, NSW = 2;        // epilogue warps, warps that sum rows (20 in all: 96 registers)
+  static constexpr int NCW = 16, NSW = KEEP ? 4 : 2;  // epilogue warps, warps that sum rows (96 or 80 registers)
+  static constexpr int SR = 128 / NSW;           // rows of a tile that one of the latter sums
+  static_assert(!KEEP || SR == 32, "one ballot tells which of its rows exist");
   static constexpr int THREADS = 32 * (2 + NCW + NSW);
   static constexpr int OFF_A = W_BYTES;
   // Tiles whose row scalars are kept: what is loaded ahead, two accumulators, and one being written.
@@ -410,21 +432,39 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     const int sw0 = warp - 2 - Cfg::NCW;
     int i = 0, s = 0;
     uint32_t ph = 0;
+    // KEEP: gamma and beta of this lane's channels, eight of each 64 (a parameter may start at any element: one by one)
+    uint64_t ga[KB][4], be[KB][4];
+    if constexpr (Cfg::KEEP) {
+#pragma unroll
+      for (int k = 0; k < KB; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = 64 * k + 8 * (lane & 7) + 2 * e;
+          ga[k][e] = f2_pack(p.gamma[c], p.gamma[c + 1]);
+          be[k][e] = f2_pack(p.beta[c], p.beta[c + 1]);
+        }
+    }
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++i) {
       float* rs = reinterpret_cast<float*>(smem + Cfg::OFF_ROW + (i % NRB) * 1536);
-      float mk[2];
+      constexpr int NH = Cfg::SR / 32;
+      float mk[NH];
+      uint32_t real[NH];  // KEEP: which of the rows exist in the caller's tensor
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {  // (the map costs two divisions: before the wait)
-        const int r = tile * 128 + 64 * sw0 + 32 * h + lane;
+      for (int h = 0; h < NH; ++h) {  // (the map costs two divisions: before the wait)
+        const int r = tile * 128 + Cfg::SR * sw0 + 32 * h + lane;
         mk[h] = 0.f;
-        if (r < p.R) {
+        bool there = r < p.R;
+        if (there) {
           if (p.mask_grid != nullptr) {
             mk[h] = p.mask_grid[r];
           } else {
             const PairPos pos = p.rows.split((uint32_t)r);
-            if (pos.src >= 0) mk[h] = p.mask.load(pos);
+            there = pos.src >= 0;
+            if (there) mk[h] = p.mask.load(pos);
+            if (Cfg::KEEP) p.mask_out[r] = mk[h];
           }
         }
+        if constexpr (Cfg::KEEP) real[h] = __ballot_sync(0xffffffffu, there);
       }
       const uint8_t* kb[KB];
       int slot[KB];
@@ -438,16 +478,45 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
           ph ^= 1;
         }
       }
-      stats_rows<C, 64>(kb, 64 * sw0, lane, [&](int row, const RowStats& v) {
+      auto store = [&](int row, const RowStats& v) {
+        const int m = tile * 128 + row;
         rs[row] = v.rs;
         rs[128 + row] = -v.rs * v.mu;
-        if (tile * 128 + row < p.R) {
-          p.mean[tile * 128 + row] = v.mu;
-          p.rstd[tile * 128 + row] = v.rs;
+        if (m < p.R) {
+          if constexpr (Cfg::KEEP) {
+            p.mean[m] = v.mu;
+            p.rstd[m] = v.rs;
+          } else {
+            p.z_stats[m] = make_float2(v.rs, -v.rs * v.mu);
+          }
         }
-      });
-      rs[256 + 64 * sw0 + lane] = mk[0];
-      rs[256 + 64 * sw0 + 32 + lane] = mk[1];
+      };
+      if constexpr (Cfg::KEEP) {
+        // the normalised row, 128 bytes by eight lanes
+        stats_rows<C, Cfg::SR>(kb, Cfg::SR * sw0, lane, store, [&](int row, int off, const RowStats& v) {
+          const int m = tile * 128 + row;
+          const bool there = (real[0] >> (row & 31)) & 1;
+          const uint64_t r2 = f2_pack(v.rs, v.rs), m2 = f2_pack(-v.mu, -v.mu);
+#pragma unroll
+          for (int k = 0; k < KB; ++k) {
+            uint64_t x[4];
+            unpack_pairs(*reinterpret_cast<const uint4*>(kb[k] + off), x);
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              float lo, hi;
+              f2_unpack(f2_fma(f2_mul(f2_add(x[e], m2), r2), ga[k][e], be[k][e]), lo, hi);
+              o[e] = there ? pack_bf16x2(lo, hi) : 0u;
+            }
+            if (m < p.R)
+              *reinterpret_cast<uint4*>(p.zln + (int64_t)m * C + 64 * k + 8 * (lane & 7)) = make_uint4(o[0], o[1], o[2], o[3]);
+          }
+        });
+      } else {
+        stats_rows<C, Cfg::SR>(kb, Cfg::SR * sw0, lane, store);
+      }
+#pragma unroll
+      for (int h = 0; h < NH; ++h) rs[256 + Cfg::SR * sw0 + 32 * h + lane] = mk[h];
       __syncwarp();
       if (lane == 0) {
 #pragma unroll
@@ -470,7 +539,8 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
 // =============================================================================================
 struct TrimulOutputParams {
   const float2 *st_x, *st_z;  // (S, T) of the rows of Wz and Wg
-  const float *z_mean, *z_rstd;  // [R], from the projection
+  const float2* z_stats;      // (rs, -rs mu) of the rows of z; KEEP: their mean and rs in two arrays
+  const float *z_mean, *z_rstd;
   PairRows rows;
   FastDiv per_entry;
   bf16* gate;        // KEEP: [R, C]
@@ -615,16 +685,20 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++i) {
       const int s = i & 1;
       const int m_base = tile * 128 + 32 * quarter;
-      float z_mu = 0.f, z_rs = 0.f;
+      float2 zst = make_float2(0.f, 0.f);
       if (m_base + lane < p.R) {
-        z_mu = p.z_mean[m_base + lane];
-        z_rs = p.z_rstd[m_base + lane];
+        if constexpr (Cfg::KEEP) {
+          const float mu = p.z_mean[m_base + lane], rs = p.z_rstd[m_base + lane];
+          zst = make_float2(rs, -rs * mu);
+        } else {
+          zst = p.z_stats[m_base + lane];
+        }
       }
       mbar_wait2(&tfull[s], (i >> 1) & 1, &r_full[i & 3], (i >> 2) & 1, wctx);
       tc_fence_after();
       const float* row = reinterpret_cast<const float*>(smem + Cfg::OFF_ROW + (i & 3) * 1024) + 32 * quarter + lane;
       const uint64_t xr = f2_pack(row[0], row[0]), xm = f2_pack(row[128], row[128]);
-      const uint64_t zr = f2_pack(z_rs, z_rs), zm = f2_pack(-z_rs * z_mu, -z_rs * z_mu);
+      const uint64_t zr = f2_pack(zst.x, zst.x), zm = f2_pack(zst.y, zst.y);
 #pragma unroll
       for (int k = 0; k < C / 64; ++k) {
         const int n0 = 32 * (par + 2 * k);
@@ -764,9 +838,9 @@ static int row_tile_grid(int64_t R) {
   return (int)(tiles < sm_count() ? tiles : sm_count());
 }
 
-template <int C>
-static int project(const TrimulCall& t, const TrimulFused& w, const float* mask_grid, int64_t NN, cudaStream_t stream) {
-  using Cfg = TrimulProjectCfg<C>;
+template <int C, bool KEEP>
+static int project(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStream_t stream) {
+  using Cfg = TrimulProjectCfg<C, KEEP>;
   const int64_t R = t.B * NN;
   int* status = nullptr;
   int rc = fwd_status(&status);
@@ -776,9 +850,17 @@ static int project(const TrimulCall& t, const TrimulFused& w, const float* mask_
   p.rows = PairRows::make(t.N, t.Np, false);
   p.per_entry = FastDiv::make((uint32_t)NN);
   p.mask = PairMask{t.mask, t.mask_type, t.mask_stride[0], t.mask_stride[1], t.mask_stride[2]};
-  p.mask_grid = mask_grid;
-  p.mean = t.mean_in;
-  p.rstd = t.rstd_in;
+  // A mask without a copy of its own, of a forward that keeps what it makes, has the internal layout.
+  p.mask_grid = KEEP && t.mask_grid == nullptr ? reinterpret_cast<const float*>(t.mask) : nullptr;
+  p.z_stats = reinterpret_cast<float2*>(t.z_stats);
+  if (KEEP) {
+    p.mean = t.mean_in;
+    p.rstd = t.rstd_in;
+    p.gamma = t.w.norm_in_w;
+    p.beta = t.w.norm_in_b;
+    p.zln = (bf16*)t.zln;
+    p.mask_out = t.mask_grid;
+  }
   p.R = (int)R;
   CUtensorMap tz, tz8, tw, ta, tb;
   if ((rc = make_z_tmaps(&tz, &tz8, t, p.rows, R)) || (rc = make_operand_tmap(&tw, w.w, false, 4 * C, C, C, 1, 0, 128, 32, 64)) ||
@@ -802,6 +884,7 @@ static int output(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStr
   TrimulOutputParams p{};
   p.st_z = reinterpret_cast<const float2*>(w.st) + 4 * C;
   p.st_x = p.st_z + C;
+  p.z_stats = reinterpret_cast<const float2*>(t.z_stats);
   p.z_mean = t.mean_in;
   p.z_rstd = t.rstd_in;
   p.rows = PairRows::make(t.N, t.Np, false);
@@ -836,8 +919,9 @@ static int output(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStr
 bool trimul_fused(int64_t C) { return C == 64 || C == 128; }
 
 // NN: internal rows per batch entry.
-int trimul_project(const TrimulCall& t, const TrimulFused& w, const float* mask_grid, int64_t NN, cudaStream_t stream) {
-  return t.C == 64 ? project<64>(t, w, mask_grid, NN, stream) : project<128>(t, w, mask_grid, NN, stream);
+int trimul_project(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStream_t stream) {
+  if (t.infer) return t.C == 64 ? project<64, false>(t, w, NN, stream) : project<128, false>(t, w, NN, stream);
+  return t.C == 64 ? project<64, true>(t, w, NN, stream) : project<128, true>(t, w, NN, stream);
 }
 int trimul_output(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStream_t stream) {
   return t.C == 64 ? output<64>(t, w, NN, stream) : output<128>(t, w, NN, stream);

@@ -32,8 +32,8 @@ def test_stages_of_two_shards(channels, direction):
         rows = slice(r * N // P, (r + 1) * N // P)
         n0 = launches()
         shards.append(be.proj_fwd(z[:, rows].contiguous(), mask[:, rows].contiguous(), w, incoming))
-        # the weights' layouts, the norm where it is a kernel, the projection
-        assert launches() - n0 <= 3
+        # the weights' layouts, the norm where it is a kernel of its own, the projection
+        assert launches() - n0 <= (2 if channels % 64 == 0 else 3)
     cat = lambda name: torch.cat([s[name] for s in shards], 2)  # noqa: E731
     x = be.contract(cat("a_cm"), cat("b_cm"), incoming)
     for r in range(P):
