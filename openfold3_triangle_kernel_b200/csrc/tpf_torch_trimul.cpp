@@ -228,20 +228,6 @@ py::object py_trimul(py::handle hz, bool incoming, py::handle hm, py::tuple weig
   return py::cast(out);
 }
 
-// The forward that keeps nothing, for the torch.library operators: z [B,N,N,C], any N, mask fp32 [B,N,N].
-Tensor trimul_infer(const Tensor& z_, const Tensor& mask_, std::vector<Tensor> w_, bool incoming) {
-  c10::cuda::CUDAGuard guard(z_.device());
-  const Tensor z = aligned_bf16(z_), mask = mask_.to(at::kFloat);
-  std::vector<Tensor> w;
-  for (const Tensor& t : w_) w.push_back(f32c(t));
-  tpf::TrimulCall t = {};
-  const Tensor arena = trimul_bind(t, z, mask, w, incoming, false, Tensor());
-  Tensor out = empty_bf16(z.sizes(), z);
-  t.out = out.data_ptr();
-  check(tpf::trimul_forward(t, cu_stream()), "tpf_trimul_fwd");
-  return out;
-}
-
 // Launches behind the torch.library operators: z [B,N,N,C] with N a multiple of 8, mask fp32 [B,N,N].
 std::vector<Tensor> trimul_fwd(const Tensor& z_, const Tensor& mask_, std::vector<Tensor> w_, bool incoming) {
   c10::cuda::CUDAGuard guard(z_.device());
