@@ -18,6 +18,14 @@ bool plain_cuda(const Tensor& t) {
   return t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has_any(special);
 }
 
+// Parameter carries torch's marker for "no __torch_function__", and a subclass inherits it unless it defines one.
+bool plain_type(py::handle h) {
+  if (THPVariable_CheckExact(h.ptr())) return true;
+  if (!THPVariable_Check(h.ptr())) return false;
+  return py::getattr(py::type::handle_of(h), "__torch_function__", py::none())
+      .is(py::module_::import("torch._C").attr("_disabled_torch_function_impl"));
+}
+
 bool plain_context() {
   using c10::DispatchKey;
   static const c10::DispatchKeySet special({DispatchKey::Python, DispatchKey::FuncTorchDynamicLayerFrontMode,

@@ -36,11 +36,12 @@ inline Tensor f32c(const Tensor& t) {
   return t.detach().to(at::kFloat).contiguous();
 }
 
-// A plain eager CUDA tensor: no functorch wrapper, no lazy conjugation or negation, no subclass that dispatches (those
-// that only override __torch_function__ are told by their Python type: THPVariable_CheckExact at the entry points, which
-// lets parameters pass).  Anything else (and any active dispatch mode) takes the torch.library route, which every such
-// mechanism sees.
+// A plain eager CUDA tensor: no functorch wrapper, no lazy conjugation or negation, no subclass that dispatches.  Anything
+// else (and any active dispatch mode) takes the torch.library route, which every such mechanism sees.
 bool plain_cuda(const Tensor& t);
+// ... and no subclass whose __torch_function__ wants to see the call, which the Python object tells: tensors, parameters and
+// subclasses of Parameter without one of their own pass.
+bool plain_type(py::handle h);
 bool plain_context();
 
 // Compute capability 10.x, cached per device.

@@ -219,12 +219,12 @@ bool prefix_ok(const Tensor& t, const Tensor& q) {
 // with its reason), a tensor subclass, an active dispatch mode.
 py::object py_attention(py::handle hq, py::handle hk, py::handle hv, py::handle hb, py::handle hm, bool return_lse) {
   for (py::handle h : {hq, hk, hv, hb})
-    if (!THPVariable_CheckExact(h.ptr())) return py::none();
+    if (!plain_type(h)) return py::none();
   const Tensor &q = THPVariable_Unpack(hq.ptr()), &k = THPVariable_Unpack(hk.ptr()), &v = THPVariable_Unpack(hv.ptr()),
                &bias = THPVariable_Unpack(hb.ptr());
   std::optional<Tensor> mask;
   if (!hm.is_none()) {
-    if (!THPVariable_CheckExact(hm.ptr())) return py::none();
+    if (!plain_type(hm)) return py::none();
     mask = THPVariable_Unpack(hm.ptr());
   }
   if (!plain_context() || !plain_cuda(q) || !plain_cuda(k) || !plain_cuda(v) || !plain_cuda(bias) ||

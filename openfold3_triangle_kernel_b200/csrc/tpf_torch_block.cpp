@@ -192,7 +192,7 @@ bool attn_weights_ok(const std::vector<Tensor>& w, const Tensor& z, int64_t head
 bool unpack(const py::tuple& p, std::vector<Tensor>& w, bool& grad) {
   if (p.size() != 8) return false;
   for (py::handle h : p) {
-    if (!THPVariable_CheckExact(h.ptr())) return false;
+    if (!plain_type(h)) return false;
     w.push_back(THPVariable_Unpack(h.ptr()));
     grad = grad || w.back().requires_grad();
   }
@@ -205,7 +205,7 @@ bool unpack(const py::tuple& p, std::vector<Tensor>& w, bool& grad) {
 // w_v, w_g, w_o.  Returns None when the arguments need the Python route.
 py::object py_pair_block(py::handle hz, py::handle hm, py::tuple tri_out, py::tuple tri_in, py::tuple start,
                          py::tuple end, int64_t heads) {
-  if (!THPVariable_CheckExact(hz.ptr()) || !THPVariable_CheckExact(hm.ptr())) return py::none();
+  if (!plain_type(hz) || !plain_type(hm)) return py::none();
   const Tensor &z = THPVariable_Unpack(hz.ptr()), &mask = THPVariable_Unpack(hm.ptr());
   std::vector<Tensor> w[4];
   bool grad = z.requires_grad();

@@ -196,18 +196,18 @@ bool trimul_supported(const Tensor& z, const Tensor& mask, const std::vector<Ten
 
 // The eager call.  Returns None when the arguments need the Python route (see py_attention).
 py::object py_trimul(py::handle hz, bool incoming, py::handle hm, py::tuple weights) {
-  if (!THPVariable_CheckExact(hz.ptr()) || weights.size() != 8) return py::none();
+  if (!plain_type(hz) || weights.size() != 8) return py::none();
   const Tensor& z = THPVariable_Unpack(hz.ptr());
   Tensor mask;
   if (!hm.is_none()) {
-    if (!THPVariable_CheckExact(hm.ptr())) return py::none();
+    if (!plain_type(hm)) return py::none();
     mask = THPVariable_Unpack(hm.ptr());
   }
   std::vector<Tensor> w;
   bool grad = z.requires_grad();
   for (int i = 0; i < 8; ++i) {
     py::handle h = weights[i];
-    if (!THPVariable_CheckExact(h.ptr())) return py::none();
+    if (!plain_type(h)) return py::none();
     w.push_back(THPVariable_Unpack(h.ptr()));
     grad = grad || w.back().requires_grad();
   }

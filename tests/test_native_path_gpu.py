@@ -150,6 +150,44 @@ def test_tensor_subclasses_take_the_route_they_can_see(which):
                       for i, v in enumerate(plain)])) is torch.Tensor
 
 
+class _Named(torch.nn.Parameter):
+    """A parameter class that carries something of its own and overrides nothing."""
+
+
+class _Watched(torch.nn.Parameter):
+    calls = []
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        cls.calls.append(str(func))
+        with torch._C.DisableTorchFunctionSubclass():
+            return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("cls,native", [(torch.nn.Parameter, True), (_Named, True), (_Watched, False)])
+def test_parameter_classes_take_the_native_route_unless_they_watch(cls, native):
+    from openfold3_triangle_kernel_b200 import _cabi
+    from oracle.pair_block_oracle import block_params
+    own = lambda t: cls(t.cuda())  # noqa: E731
+    lib = _cabi.native()
+    a = attention_inputs(1, 4, 2, 16, 32, seed=4)
+    t = trimul_inputs(1, 16, 64, seed=4)
+    order = ("p_in_weight", "g_in_weight", "p_out_weight", "g_out_weight", "norm_in_weight", "norm_in_bias",
+             "norm_out_weight", "norm_out_bias")
+    weights = tuple(own(t["weights"][n]) for n in order)
+    z, mask = t["z"].cuda(), t["mask"].cuda()
+    blk = block_params(64, 4, 16, seed=4)
+    parts = [tuple(own(blk[m][n]) for n in order) for m in ("tri_mul_out", "tri_mul_in")]
+    parts += [tuple(own(blk[m][n]) for n in ("ln_w", "ln_b", "w_z", "w_q", "w_k", "w_v", "w_g", "w_o"))
+              for m in ("tri_att_start", "tri_att_end")]
+    for out in (lib.attention(a["q"].cuda(), a["k"].cuda(), a["v"].cuda(), own(a["pair_bias"]), a["res_mask"].cuda(), False),
+                lib.trimul(z, False, mask, weights), lib.pair_block(z, mask, *parts, 4)):
+        assert (out is not None) == native
+    got = tk.turbo_trimul(z, "outgoing", mask, **dict(zip(order, weights)))
+    assert torch.equal(got, tk.turbo_trimul(z, "outgoing", mask, **{n: w.detach().as_subclass(torch.Tensor)
+                                                                    for n, w in zip(order, weights)}))
+
+
 def _shifted(t):
     """The same values one element behind a 16-byte boundary, as a parameter inside a flat buffer has them."""
     flat = torch.empty(t.numel() + 1, device="cuda", dtype=t.dtype)
