@@ -25,8 +25,8 @@ pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not torch.cuda.is_available(),
     (3, 33, 128, "incoming", "bool", 0.0),
     (1, 64, 128, "outgoing", "none", 0.0),     # the caller's rows as they are
     (2, 72, 64, "incoming", "pair", 0.0),
-    (1, 131, 128, "outgoing", "pair", 0.0),    # 64-row copies and lines that end inside one; a second tile for some CTAs
-    (2, 259, 64, "outgoing", "pair", 0.0),     # more tiles of a CTA than it keeps row sums of
+    (1, 131, 128, "outgoing", "pair", 0.0),    # 64-row copies and lines that end inside one
+    (2, 259, 64, "outgoing", "pair", 0.0),     # seven or eight tiles a CTA
     (1, 40, 128, "incoming", "pair", 40.0),    # rows whose mean is forty times their spread
 ])
 def test_forward_at_tile_edges(B, N, channels, direction, mask, shift):
@@ -46,6 +46,48 @@ def test_forward_at_tile_edges(B, N, channels, direction, mask, shift):
     ref = to.trimul_forward_backward(z, direction, torch.ones(B, N, N) if m is None else m.float(), w,
                                      torch.zeros_like(z))["out"]
     assert rel_l2(got.cpu(), ref) <= 5.5e-3
+
+
+# A CTA keeps the row sums of four tiles at C = 128 and of eight at C = 64, on 148 SMs: 800 tiles are five or six a CTA, 841
+# the same with padded lines, 1250 and 1301 are eight or nine.
+@pytest.mark.parametrize("N,channels,direction,mask", [
+    (320, 128, "outgoing", "pair"), (325, 128, "incoming", "bool"), (400, 64, "incoming", "pair"),
+    (403, 64, "outgoing", "none")])
+def test_forward_with_rings_used_again(N, channels, direction, mask):
+    t = trimul_inputs(1, N, channels, seed=N)
+    g = torch.Generator().manual_seed(N)
+    w = {n: x + 0.2 * torch.randn(x.shape, generator=g) if x.ndim == 1 else x for n, x in t["weights"].items()}
+    m = {"pair": t["mask"], "bool": t["mask"].bool(), "none": None}[mask]
+    dm = None if m is None else m.cuda()
+    z = t["z"].cuda()
+    with torch.no_grad():
+        got = tk.turbo_trimul(z, direction, dm, **{n: x.cuda() for n, x in w.items()})
+    kept = tk.turbo_trimul(z, direction, dm, **{n: x.cuda().requires_grad_(True) for n, x in w.items()}).detach()
+    torch.cuda.synchronize()
+    assert C.device_status() == 0
+    assert torch.equal(got, kept)
+    ref = to.trimul_forward(t["z"], direction, torch.ones(1, N, N) if m is None else m.float(), w)
+    assert rel_l2(got.cpu(), ref) <= 5.5e-3
+
+
+def test_passes_over_different_inputs_do_not_leak_into_one_another():
+    """The block at C = 64 with more row tiles than CTAs: its residual is the z tile in shared memory, whose slot the next
+    tile's copy takes.  Read after that copy had begun, it gave other values in some passes, and only where the
+    passes before had left other data."""
+    from openfold3_triangle_kernel_b200.pair_block import pair_stack_block
+    from oracle.pair_block_oracle import block_params
+    N = 400
+    params = {k: {n: v.cuda() for n, v in m.items()} for k, m in block_params(64, 4, 16, seed=5).items()}
+    mask = torch.ones(1, N, N, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    zs = [torch.randn(1, N, N, 64, generator=g, device="cuda").bfloat16() for _ in range(5)]
+    first = None
+    with torch.no_grad():
+        for _ in range(10):
+            outs = [pair_stack_block(z, mask, params, 4) for z in zs]
+            first = first or outs
+            assert all(torch.equal(a, b) for a, b in zip(outs, first))
+    assert C.device_status() == 0
 
 
 @pytest.mark.parametrize("B,N,channels,shift", [
