@@ -428,7 +428,9 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           // descriptors = a base descriptor + (byte offset >> 4) in the start-address field (no carry out of it:
           // shared memory is far smaller than the field's range)
           const uint32_t a_off = Cfg::STAT == 1 ? kb * Cfg::A_BYTES : Cfg::STAT_BYTES + s * Cfg::STAGE_BYTES;
-          const uint32_t b_off = Cfg::RESIDENT ? (kb * Cfg::B_ROWS + n0) * Cfg::SWZ_B : Cfg::STAT == 2 ? kb * Cfg::B_BYTES : Cfg::STAT_BYTES + s * Cfg::STAGE_BYTES + Cfg::STAGE_A;
+          const uint32_t b_off = Cfg::RESIDENT    ? (kb * Cfg::B_ROWS + n0) * Cfg::SWZ_B
+                                 : Cfg::STAT == 2 ? kb * Cfg::B_BYTES
+                                                  : Cfg::STAT_BYTES + s * Cfg::STAGE_BYTES + Cfg::STAGE_A;
           const uint64_t ad0 = a_desc0 + (a_off >> 4);
           const uint64_t bd0 = b_desc0 + (b_off >> 4);
           constexpr int A_STEP = Cfg::A_MN ? (16 * Cfg::SWZ_A >> 4) : 2;

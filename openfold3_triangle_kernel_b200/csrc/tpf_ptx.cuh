@@ -377,8 +377,9 @@ __device__ __forceinline__ float sigmoid_fast(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * x));
   return fmaf(t, 0.5f, 0.5f);
 }
-// The same to 1e-6 of its own value, closed gates included (two MUFU ops): the gates of the attention modules, where it
-// made no measurable difference in time (block training at N = 768: 12.30 and 12.26 ms).
+// The same with an error relative to its own value (two MUFU ops): 8e-7 down to -16, 3.4e-6 down to -87 (measured over all
+// bf16 logits; __expf's bound grows with its argument), 0 below, where it is 1e-38.  The gates of the attention modules,
+// where it made no measurable difference in time (block training at N = 768: 12.30 and 12.26 ms).
 __device__ __forceinline__ float sigmoid_rel(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 // Packed fp32 pairs (sm_100 executes two fp32 FMAs / adds per instruction) and 3-input max.
 __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {

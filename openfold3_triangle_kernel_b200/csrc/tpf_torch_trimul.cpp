@@ -108,7 +108,8 @@ namespace {
 
 cudaStream_t cu_stream() { return static_cast<cudaStream_t>(stream()); }
 
-// inputs: z, mask (an absent one is an empty optional: the node cannot take an undefined tensor as an input), then p_in, g_in, p_out, g_out, norm_in_w, norm_in_b, norm_out_w, norm_out_b
+// inputs: z, mask (an absent one is an empty optional: the node cannot take an undefined tensor as an input), then p_in,
+// g_in, p_out, g_out, norm_in_w, norm_in_b, norm_out_w, norm_out_b
 struct TrimulFn : public torch::autograd::Function<TrimulFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& z_in, const std::optional<Tensor>& mask_in, const Tensor& w0,
                         const Tensor& w1, const Tensor& w2, const Tensor& w3, const Tensor& w4, const Tensor& w5,

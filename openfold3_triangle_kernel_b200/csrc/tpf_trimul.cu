@@ -208,10 +208,10 @@ __global__ void __launch_bounds__(256, 2) trimul_xnorm_fwd_kernel(const bf16* __
 // =============================================================================================
 // GEMM epilogues
 // =============================================================================================
-// Projection + gating (C = 32 and 96; the others: tpf_trimul_fwd.cu).  GEMM N axis = [a_p | a_g] [b_p | b_g] [g | pad], one tile of width 2C each.
-// a and b are stored channel-major.  Each lane owns one row of the accumulator tile, which would
-// make 2-byte scattered stores; the 32x32 block is transposed through a per-warp smem tile so
-// that each lane writes 32 consecutive rows of ONE channel (4 x 16 bytes).
+// Projection + gating (C = 32 and 96; the others: tpf_trimul_fwd.cu).  GEMM N axis = [a_p | a_g] [b_p | b_g] [g | pad],
+// one tile of width 2C each.  a and b are stored channel-major.  Each lane owns one row of the accumulator tile, which
+// would make 2-byte scattered stores; the 32x32 block is transposed through a per-warp smem tile so that each lane writes
+// 32 consecutive rows of ONE channel (4 x 16 bytes).
 // Integer divisions by run-time values cost a lone epilogue warp 300-600 cycles each (a chain of conversions and
 // a reciprocal on the XU pipe), once per tile and on its critical path, so the epilogues avoid them: the tile
 // kind comes from comparisons, and the batch entry of a row is found by division only when there is more than one.

@@ -242,9 +242,8 @@ struct TrimulProjectCfg {
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmZ8,
-                            const __grid_constant__ CUtensorMap tmW,
-                            const __grid_constant__ CUtensorMap tmAB0, const __grid_constant__ CUtensorMap tmAB1,
-                            const TrimulProjectParams p, int* __restrict__ status) {
+                      const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmAB0,
+                      const __grid_constant__ CUtensorMap tmAB1, const TrimulProjectParams p, int* __restrict__ status) {
   griddep_wait();
   constexpr int C = Cfg::C, NT = Cfg::NT, KB = Cfg::KB, NST = Cfg::NST, NRB = Cfg::NRB;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -509,7 +508,8 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
               o[e] = there ? pack_bf16x2(lo, hi) : 0u;
             }
             if (m < p.R)
-              *reinterpret_cast<uint4*>(p.zln + (int64_t)m * C + 64 * k + 8 * (lane & 7)) = make_uint4(o[0], o[1], o[2], o[3]);
+              *reinterpret_cast<uint4*>(p.zln + (int64_t)m * C + 64 * k + 8 * (lane & 7)) =
+                  make_uint4(o[0], o[1], o[2], o[3]);
           }
         });
       } else {
@@ -572,9 +572,9 @@ struct TrimulOutputCfg {
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmZ,
-                           const __grid_constant__ CUtensorMap tmZ8,
-                           const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ CUtensorMap tmGate,
-                           const TrimulOutputParams p, int* __restrict__ status) {
+                     const __grid_constant__ CUtensorMap tmZ8, const __grid_constant__ CUtensorMap tmW,
+                     const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ CUtensorMap tmGate,
+                     const TrimulOutputParams p, int* __restrict__ status) {
   griddep_wait();
   constexpr int C = Cfg::C, KB = Cfg::KB;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -638,10 +638,12 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       for (int h = 0; h < 2; ++h) {  // 64 rows lie inside one batch entry
         const uint32_t r = (uint32_t)(tile * 128 + 64 * h);
         const int b = (int)p.per_entry.div(r);
-        tma_load_3d(el, smem + Cfg::OFF_X + s * Cfg::T_BYTES + h * C * 128, &tmX, &x_full[s], (int)(r - b * p.per_entry.d), 0, b);
+        tma_load_3d(el, smem + Cfg::OFF_X + s * Cfg::T_BYTES + h * C * 128, &tmX, &x_full[s],
+                    (int)(r - b * p.per_entry.d), 0, b);
       }
       for (int kb = 0; kb < KB; ++kb)
-        load_z_block(el, smem + Cfg::OFF_Z + s * Cfg::T_BYTES + kb * 16384, &tmZ, &tmZ8, &z_full[s], p.rows, 64 * kb, tile * 128);
+        load_z_block(el, smem + Cfg::OFF_Z + s * Cfg::T_BYTES + kb * 16384, &tmZ, &tmZ8, &z_full[s], p.rows, 64 * kb,
+                     tile * 128);
       if (i == 0) {
         mbar_expect_tx(el, w_full, Cfg::W_BYTES);
         for (int kb = 0; kb < KB; ++kb) {
@@ -863,8 +865,10 @@ static int project(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaSt
   }
   p.R = (int)R;
   CUtensorMap tz, tz8, tw, ta, tb;
-  if ((rc = make_z_tmaps(&tz, &tz8, t, p.rows, R)) || (rc = make_operand_tmap(&tw, w.w, false, 4 * C, C, C, 1, 0, 128, 32, 64)) ||
-      (rc = make_store_tmap(&ta, t.a_cm, NN, C, NN, t.B, C * NN)) || (rc = make_store_tmap(&tb, t.b_cm, NN, C, NN, t.B, C * NN)))
+  if ((rc = make_z_tmaps(&tz, &tz8, t, p.rows, R)) ||
+      (rc = make_operand_tmap(&tw, w.w, false, 4 * C, C, C, 1, 0, 128, 32, 64)) ||
+      (rc = make_store_tmap(&ta, t.a_cm, NN, C, NN, t.B, C * NN)) ||
+      (rc = make_store_tmap(&tb, t.b_cm, NN, C, NN, t.B, C * NN)))
     return rc;
   auto kern = trimul_project_kernel<Cfg>;
   static PerDeviceOnce once;  // per instantiation
@@ -905,7 +909,8 @@ static int output(const TrimulCall& t, const TrimulFused& w, int64_t NN, cudaStr
   auto kern = trimul_output_kernel<Cfg>;
   static PerDeviceOnce once;  // per instantiation
   if ((rc = ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, once, 1024))) return rc;
-  launch_kernel(kern, dim3(row_tile_grid(R)), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, tx, tz, tz8, tw, to, tg, p, status);
+  launch_kernel(kern, dim3(row_tile_grid(R)), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, tx, tz, tz8, tw, to, tg, p,
+                status);
   TPF_LAUNCH_OK();
   return TPF_OK;
 }

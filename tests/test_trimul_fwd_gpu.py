@@ -98,7 +98,8 @@ def test_passes_over_different_inputs_do_not_leak_into_one_another():
 ])
 def test_rows_kept_for_the_backward(B, N, channels, shift):
     """The normalised rows and their statistics, which the projection kernel writes beside a and b.  A value is rounded
-    to bf16 once (half of a unit in the eighth bit: 2^-8 of it at most); fp32 sums of squares leave (shift / spread)^2 2^-24 times a few in the variance, 1e-4."""
+    to bf16 once (half of a unit in the eighth bit: 2^-8 of it at most); fp32 sums of squares leave (shift / spread)^2 2^-24
+    times a few in the variance, 1e-4."""
     t = trimul_inputs(B, N, channels, seed=N)
     z = (t["z"].float() + shift).bfloat16().cuda()
     g = torch.Generator().manual_seed(N)
