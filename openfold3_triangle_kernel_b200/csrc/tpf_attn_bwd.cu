@@ -201,7 +201,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wctx{abort_flag, status};
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -831,7 +831,7 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::N_BAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wctx{abort_flag, status};
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   uint8_t* bias_stage = smem + Cfg::OFF_BSTG;  // bf16 tile as TMA delivers it
 

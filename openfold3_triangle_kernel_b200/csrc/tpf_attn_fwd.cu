@@ -107,7 +107,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
   const WaitCtx wctx{abort_flag, status};
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const bf16* __restrict__ d_
   griddep_wait();
   using L = RowLanes<C>;
   __shared__ float red[8][2][C];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int sub = lane / L::LS, part = lane % L::LS;
   const bool on = part < L::LPR;
   const int64_t row_begin = (int64_t)blockIdx.x * rows_per_block;

@@ -74,6 +74,12 @@ __device__ __forceinline__ uint32_t elect_one() {
   return p;
 }
 
+// The warp's index in its block.  Read from lane 0, because threadIdx.x / 32 is a per-lane value to the compiler: every branch
+// on it (roles, warps without rows) and every loop inside is then compiled as one that lanes may leave separately, and what
+// depends on it lives in vector registers.  Measured, threadIdx.x / 32 -> this: attention dQ / dK / dV at N = 384 204 -> 188 us,
+// TriMul projection 39 -> 34, k-contraction 21.4 -> 19.8, attention forward at N = 1021 1842 -> 1790 us.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // Per-CTA abort state: `flag` lives in shared memory, `status` in global memory.
 struct WaitCtx {
   volatile int* flag;

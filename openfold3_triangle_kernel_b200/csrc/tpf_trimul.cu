@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256, 2) trimul_xnorm_fwd_kernel(const bf16* __
   extern __shared__ __align__(16) uint8_t xnorm_smem[];
   uint8_t* xs0 = xnorm_smem;                       // two input tiles: the next one is fetched (cp.async)
   uint8_t* ys = xnorm_smem + 2 * C * IN_PITCH;     // while the current one is processed
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int k2 = 2 * (lane & 3);            // this lane's channel pair inside an 8-channel group
   const int rr = 8 * warp + (lane >> 2);    // this lane's pair row inside the tile
   float2 g[NG][4], bt[NG][4];  // read one by one, once per CTA: a parameter may start at any element of a flat buffer
@@ -430,6 +430,8 @@ struct EpiGateSplitBwd {
     warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk1, &p.map_d, col + p.C, m_base, 0);
   }
 };
+template <>
+constexpr bool kPerLaneWarpIndex<EpiGateSplitBwd> = true;
 
 // =============================================================================================
 // backward elementwise stages
@@ -493,7 +495,7 @@ __global__ void __launch_bounds__(256, 2) trimul_xnorm_bwd_kernel(const bf16* __
   uint8_t* xs0 = xnorm_smem;                          // x, later d_x: [channel][pair row]
   uint8_t* ds0 = xnorm_smem + 2 * C * IN_PITCH;       // d_xln: [pair row][channel]
   __shared__ float2 gsm[C / 2];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int k2 = 2 * (lane & 3);
   const int rr = 8 * warp + (lane >> 2);
   if (threadIdx.x < C / 2) gsm[threadIdx.x] = make_float2(gamma[2 * threadIdx.x], gamma[2 * threadIdx.x + 1]);

@@ -261,7 +261,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wctx{abort_flag, status};
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tiles = (p.R + 127) / 128;
 
   if (threadIdx.x == 0) {
@@ -593,7 +593,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wctx{abort_flag, status};
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tiles = (p.R + 127) / 128;
   float* col = reinterpret_cast<float*>(smem + Cfg::OFF_COL);
 
