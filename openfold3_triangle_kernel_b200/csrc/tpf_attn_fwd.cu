@@ -24,10 +24,12 @@
 //  * Items are numbered with the query tile fastest: CTAs running at the same time share K and V of an outer row (and
 //    each bias strip stays in L2 anyway).  With the outer row fastest K and V came from DRAM once per query tile.
 //  * A tile whose mask row is all zero and that has no ragged key tail (the common case) skips the mask add; warps
-//    whose 32 query rows lie beyond N, and the second half of a key tile with at most 32 keys, are skipped.
+//    whose 32 query rows lie beyond N, the second half of a key tile with at most 32 keys, and the exponentials of a tile
+//    whose keys are all masked, are skipped.
 //
-// Measured (B200, H = 4, D = 32, cold L2): N = 384 119 us (142 us before: four CTAs of six warps, 16 logits at a time,
-// roles issued by one lane), N = 768 789 us (977), N = 1021 1.82 ms (2.27); D = 64, N = 257 86 us (127).
+// Measured (B200, H = 4, D = 32, cold L2, 5 % of the keys masked): N = 384 102 us, N = 768 711, N = 1021 1.66 ms;
+// D = 64, N = 257 74 us.  Before the tiles with a mask got code of their own and one store path for an item's rows: 109, 765,
+// 1.78 and 78.
 #include "tpf_host.cuh"
 #include "tpf_internal.h"
 #include "tpf_ptx.cuh"
@@ -85,6 +87,11 @@ struct AttnFwdCfg {
   static_assert((S_COLS + O_COLS) * CTAS_PER_SM <= 512, "TMEM budget");
   static_assert((SMEM_BYTES + 1024) * CTAS_PER_SM <= 233472, "shared memory budget");
   static_assert(KV_TILE % 1024 == 0 && Q_TILE % 1024 == 0, "tile buffers keep 1024-byte alignment");
+};
+
+template <bool B>
+struct BoolTag {
+  static constexpr bool value = B;
 };
 
 template <class Cfg>
@@ -350,107 +357,110 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // arrives on the same barrier have landed
         mbar_wait2(&s_full[buf], ph, &b_full[buf], ph, wctx);
         tc_fence_after();
-        if (!live) {
-          if (++m_s == NS) m_s = 0;
-          if (pend) {
-            finish_item();
-            pend = false;
-            tc_fence_before();
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&p_ready[buf]);
-          continue;
-        }
-        uint32_t raw[64];  // this row's logits
-        tmem_ld32(t_s + 64 * buf, *reinterpret_cast<uint32_t(*)[32]>(raw));
-        tmem_ld32(t_s + 64 * buf + 32, *reinterpret_cast<uint32_t(*)[32]>(raw + 32));
-        const float* mask_row = reinterpret_cast<const float*>(smem + Cfg::OFF_MASK + m_s * 256);
+        float* mask_row = reinterpret_cast<float*>(smem + Cfg::OFF_MASK + m_s * 256);
+        if (++m_s == NS) m_s = 0;
         const int n_keys = p.N - j * KEYS;
         const float2 mprobe = *reinterpret_cast<const float2*>(mask_row + 2 * lane);
         const bool general = n_keys < KEYS || __any_sync(0xffffffffu, (mprobe.x != 0.f) || (mprobe.y != 0.f));
         const uint8_t* bias_row = smem + Cfg::OFF_BIAS + buf * Cfg::BIAS_STAGE + row * 128;
-        tmem_ld_wait();
-        if (++m_s == NS) m_s = 0;
-        float cm0 = -INFINITY, cm1 = -INFINITY;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          if (u == 4 && n_keys <= 32) break;
-          const uint4 bv = *reinterpret_cast<const uint4*>(bias_row + ((u ^ (row & 7)) << 4));
-          const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = 8 * u + 2 * e;
-            float v0, v1;
-            f2_unpack(f2_fma(f2_pack_bits(raw[i], raw[i + 1]), scale2, f2_pack_bits(bw[e] << 16, bw[e] & 0xFFFF0000u)), v0, v1);
-            raw[i] = __float_as_uint(v0);
-            raw[i + 1] = __float_as_uint(v1);
+        // A tile from its logits to its probabilities.  GENERAL: with a mask or a ragged tail.  Two copies, because as a
+        // branch between the bias and the maximum it cost every tile: the 64 logits had to be in the same registers on
+        // both ways, and the stages before and after it could not be interleaved.
+        auto tile = [&](auto general_tag) {
+          constexpr bool GENERAL = decltype(general_tag)::value;
+          if (GENERAL && n_keys < KEYS) {
+            // no keys there: every warp writes the same values over the zeros that the copy filled in
+            if (lane >= n_keys) mask_row[lane] = -INFINITY;
+            if (lane + 32 >= n_keys) mask_row[lane + 32] = -INFINITY;
+            fence_async_smem();  // the next copy into this slot comes after these stores
+            __syncwarp();
           }
-        }
-        if (general) {
+          uint32_t raw[64];  // this row's logits
+          tmem_ld32(t_s + 64 * buf, *reinterpret_cast<uint32_t(*)[32]>(raw));
+          tmem_ld32(t_s + 64 * buf + 32, *reinterpret_cast<uint32_t(*)[32]>(raw + 32));
+          tmem_ld_wait();
+          float cm0 = -INFINITY, cm1 = -INFINITY;
 #pragma unroll
-          for (int u = 0; u < 16; ++u) {
-            if (u == 8 && n_keys <= 32) break;
-            const float4 mk = *reinterpret_cast<const float4*>(mask_row + 4 * u);
-            const float m4[4] = {mk.x, mk.y, mk.z, mk.w};
+          for (int u = 0; u < 8; ++u) {
+            if (GENERAL && u == 4 && n_keys <= 32) break;
+            const uint4 bv = *reinterpret_cast<const uint4*>(bias_row + ((u ^ (row & 7)) << 4));
+            const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+            float4 mk[2];
+            if (GENERAL) {
+              mk[0] = *reinterpret_cast<const float4*>(mask_row + 8 * u);
+              mk[1] = *reinterpret_cast<const float4*>(mask_row + 8 * u + 4);
+            }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const float v = __uint_as_float(raw[4 * u + e]) + m4[e];
-              raw[4 * u + e] = __float_as_uint(4 * u + e < n_keys ? v : -INFINITY);
+              const int i = 8 * u + 2 * e;
+              uint64_t v = f2_fma(f2_pack_bits(raw[i], raw[i + 1]), scale2, f2_pack_bits(bw[e] << 16, bw[e] & 0xFFFF0000u));
+              if (GENERAL) v = f2_add(v, e & 1 ? f2_pack(mk[e >> 1].z, mk[e >> 1].w) : f2_pack(mk[e >> 1].x, mk[e >> 1].y));
+              float v0, v1;
+              f2_unpack(v, v0, v1);
+              raw[i] = __float_as_uint(v0);
+              raw[i + 1] = __float_as_uint(v1);
+              float& cm = e & 1 ? cm1 : cm0;
+              cm = GENERAL ? max3_nan(cm, v0, v1) : max3(cm, v0, v1);
             }
           }
-        }
-#pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          if (i == 32 && n_keys <= 32) break;
-          cm0 = max3(cm0, __uint_as_float(raw[i]), __uint_as_float(raw[i + 1]));
-          cm1 = max3(cm1, __uint_as_float(raw[i + 2]), __uint_as_float(raw[i + 3]));
-        }
-        const float cmax = fmaxf(cm0, cm1);
-        if (__any_sync(0xffffffffu, cmax > m_use + kGap)) {
-          // Raise the reference maximum of the rows that need it (f = 1 for the others) and rescale what
-          // those rows have accumulated.  Runs for the first finite tile of every row and then only
-          // when the logits of a row grow by more than kGap.
-          const bool grow = cmax > m_use + kGap;
-          const float f = grow ? ex2_approx((m_use - cmax) * kLog2e) : 1.f;  // m_use = -inf gives 0; nothing accumulated then
-          if (grow) m_use = cmax;
-          l_run *= f;
-          if (j > 0) {
-            mbar_wait(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, wctx);
-            tc_fence_after();
+          const float cmax = GENERAL ? max3_nan(cm0, cm1, cm1) : fmaxf(cm0, cm1);
+          if (__any_sync(0xffffffffu, cmax > m_use + kGap)) {
+            // Raise the reference maximum of the rows that need it (f = 1 for the others) and rescale what
+            // those rows have accumulated.  Runs for the first finite tile of every row and then only
+            // when the logits of a row grow by more than kGap.
+            const bool grow = cmax > m_use + kGap;
+            const float f = grow ? ex2_approx((m_use - cmax) * kLog2e) : 1.f;  // m_use = -inf gives 0; nothing accumulated then
+            if (grow) m_use = cmax;
+            l_run *= f;
+            if (j > 0) {
+              mbar_wait(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, wctx);
+              tc_fence_after();
 #pragma unroll 1
-            for (int cc = 0; cc < D; cc += 8) {
-              uint32_t ro[8];
-              tmem_ld8(t_o + cc, ro);
-              tmem_ld_wait();
+              for (int cc = 0; cc < D; cc += 8) {
+                uint32_t ro[8];
+                tmem_ld8(t_o + cc, ro);
+                tmem_ld_wait();
 #pragma unroll
-              for (int i = 0; i < 8; ++i) ro[i] = __float_as_uint(__uint_as_float(ro[i]) * f);
-              tmem_st8(t_o + cc, ro);
+                for (int i = 0; i < 8; ++i) ro[i] = __float_as_uint(__uint_as_float(ro[i]) * f);
+                tmem_st8(t_o + cc, ro);
+              }
             }
           }
-        }
-        const float neg_m = (m_use == -INFINITY) ? 0.f : -m_use * kLog2e;
-        const uint64_t neg_m2 = f2_pack(neg_m, neg_m);
-        uint64_t rs2a = 0ull, rs2b = 0ull;  // packed partial row sums of this tile
+          if (GENERAL && !__any_sync(0xffffffffu, !(cmax < m_use - 104.f))) {
+            // masked keys only: every probability is below the smallest fp32 number (no NaN among the logits either)
+            const uint32_t zero[8] = {};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (c == 2 && n_keys <= 32) break;
-          uint32_t pk[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            float a0, a1;
-            f2_unpack(f2_fma(f2_pack_bits(raw[16 * c + 2 * e], raw[16 * c + 2 * e + 1]), log2e2, neg_m2), a0, a1);
-            const float e0 = ex2_approx(a0), e1 = ex2_approx(a1);
-            if (e & 1) rs2b = f2_add(rs2b, f2_pack(e0, e1));
-            else rs2a = f2_add(rs2a, f2_pack(e0, e1));
-            pk[e] = pack_bf16x2(e0, e1);
+            for (int c = 0; c < 4; ++c) tmem_st8(t_s + 64 * buf + 8 * c, zero);
+            return;
           }
-          tmem_st8(t_s + 64 * buf + 8 * c, pk);
-        }
-        float r0, r1;
-        f2_unpack(f2_add(rs2a, rs2b), r0, r1);
-        l_run += r0 + r1;
+          const float neg_m = (m_use == -INFINITY) ? 0.f : -m_use * kLog2e;
+          const uint64_t neg_m2 = f2_pack(neg_m, neg_m);
+          uint64_t rs2a = 0ull, rs2b = 0ull;  // packed partial row sums of this tile
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (GENERAL && c == 2 && n_keys <= 32) break;
+            uint32_t pk[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              float a0, a1;
+              f2_unpack(f2_fma(f2_pack_bits(raw[16 * c + 2 * e], raw[16 * c + 2 * e + 1]), log2e2, neg_m2), a0, a1);
+              const float e0 = ex2_approx(a0), e1 = ex2_approx(a1);
+              if (e & 1) rs2b = f2_add(rs2b, f2_pack(e0, e1));
+              else rs2a = f2_add(rs2a, f2_pack(e0, e1));
+              pk[e] = pack_bf16x2(e0, e1);
+            }
+            tmem_st8(t_s + 64 * buf + 8 * c, pk);
+          }
+          float r0, r1;
+          f2_unpack(f2_add(rs2a, rs2b), r0, r1);
+          l_run += r0 + r1;
+        };
+        if (!live) {
+        } else if (general) tile(BoolTag<true>{});
+        else tile(BoolTag<false>{});
         // the previous item's row leaves before this item's first P V overwrites the accumulator
         if (j == 0 && pend) finish_item();
+        if (j == 0) pend = false;
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();

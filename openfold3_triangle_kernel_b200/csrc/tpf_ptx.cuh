@@ -422,6 +422,13 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
+// The same, NaN if one of them is.
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 // 16-byte asynchronous copy global -> shared (no registers in between); `valid` false writes zeros.
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gsrc),

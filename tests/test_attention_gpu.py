@@ -204,6 +204,41 @@ def test_large_finite_mask_value_behaves_like_minus_inf():
         assert ao.rel_l2(got_big[n], got_inf[n]) <= 1e-6, n
 
 
+@pytest.mark.parametrize("value", [-1e9, -float("inf")])
+@pytest.mark.parametrize("N,D", [(33, 32), (64, 16), (65, 32), (97, 64), (160, 32), (321, 32)])
+def test_masks_over_whole_key_tiles(N, D, value):
+    """Key tiles (64 keys) that are masked as a whole, at the end, at the start (a row's reference maximum is then first that of
+    masked logits) and in the middle, beside unmasked and partly masked ones and a ragged tail."""
+    O, H = 3, 4
+    gen = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn(1, O, H, N, D, generator=gen).bfloat16() for _ in range(3))
+    bias = torch.randn(1, 1, H, N, N, generator=gen).bfloat16()
+    mask = torch.zeros(1, O, 1, 1, N)
+    mask[0, 0, ..., N // 3:] = value
+    mask[0, 1, ..., : N - N // 3] = value
+    mask[0, 2, ..., 20:N - 5] = value
+    out, lse = tk.turbo_attention(q.cuda(), k.cuda(), v.cuda(), pair_bias=bias.cuda(), res_mask=mask.cuda(), return_lse=True)
+    ref, ref_lse = ao.attention_forward(q, k, v, bias, mask)
+    assert torch.isfinite(out).all()
+    for o in range(O):
+        assert ao.rel_l2(out[:, o].cpu(), ref[:, o]) <= REL_TOL, o
+    assert (lse.cpu().double() - ref_lse).abs().max().item() <= LSE_TOL * max(1.0, ref_lse.abs().max().item())
+
+
+def test_nan_under_a_mask_reaches_the_output():
+    """A NaN logit stays a NaN whatever is added to it: the tile of masked keys that holds it is not passed over."""
+    N, D, H = 192, 32, 4
+    gen = torch.Generator().manual_seed(3)
+    q, k, v = (torch.randn(1, 1, H, N, D, generator=gen).bfloat16() for _ in range(3))
+    bias = torch.zeros(1, 1, H, N, N).bfloat16()
+    bias[0, 0, 1, 40, 170] = float("nan")
+    mask = torch.zeros(1, 1, 1, 1, N)
+    mask[..., 100:] = -1e9
+    out = tk.turbo_attention(q.cuda(), k.cuda(), v.cuda(), pair_bias=bias.cuda(), res_mask=mask.cuda()).cpu()
+    assert torch.isnan(out[0, 0, 40, 1]).all()
+    assert torch.isnan(out).sum().item() == D
+
+
 def test_no_python_fallback_native_library_is_loaded():
     with open("/proc/self/maps") as f:
         assert "libtpf_b200.so" in f.read()
