@@ -766,6 +766,38 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
 }
 
+// The additive mask of a tile's keys as an operand of S: row = key (32 bytes, as a D = 16 tile), its first three columns hold
+// value / scale split into bf16 parts, which an A operand of ones adds up again (24 bits: what fp32 has); S then gets the mask
+// with the scale like any logit.  Keys from n_keys on are masked.  Called by the issuing warp; returns whether there is anything
+// to add.  A lane makes the rows of four keys.
+// A row whose log-sum-exp is below this has masked keys only (by -inf or by a large finite value such as -1e9): its logits and
+// the log-sum-exp differ by nothing but rounding, of more than one unit.  It gets no gradient, with either value.
+constexpr float kMaskedLse = -1e8f;
+__device__ __forceinline__ bool mask_operand(uint8_t* dst, const float* mask_row, int n_keys, int lane, float inv_scale) {
+  const float4 m = reinterpret_cast<const float4*>(mask_row)[lane];
+  float v[4] = {m.x, m.y, m.z, m.w};
+  bool any = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (4 * lane + i >= n_keys) v[i] = -INFINITY;
+    any |= v[i] != 0.f;
+  }
+  if (!__any_sync(0xffffffffu, any)) return false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int key = 4 * lane + i;
+    const float x = v[i] * inv_scale;
+    const float hi = __bfloat162float(__float2bfloat16_rn(x));
+    const bool inf = hi - hi != 0.f;  // (NaN too: one part carries it)
+    const float r = inf ? 0.f : x - hi;
+    const float mid = __bfloat162float(__float2bfloat16_rn(r));
+    *reinterpret_cast<uint2*>(dst + key * 32 + ((key >> 2) & 1) * 16) = make_uint2(pack_bf16x2(hi, mid), pack_bf16x2(r - mid, 0.f));
+  }
+  fence_async_smem();
+  __syncwarp();
+  return true;
+}
+
 // =============================================================================================
 // kernel 2: dBias partial planes.  One CTA = one (group, h, query tile, key tile) and a chunk of
 // outer planes; dS summed over the chunk in ascending plane order, fp32, in registers.
@@ -796,7 +828,10 @@ struct AttnDbiasCfg {
   // producer waits for the conversion before it first fills that buffer), else in a region of its own
   static constexpr bool STAGE_HOLDS_BIAS = STAGE >= 32768 + 1024;
   static constexpr int OFF_BSTG = STAGE_HOLDS_BIAS ? OFF_ST + (NST - 1) * STAGE : OFF_ST + NST * STAGE;
-  static constexpr int OFF_BAR = OFF_ST + NST * STAGE + (STAGE_HOLDS_BIAS ? 0 : 32768);
+  // the mask as an operand (see mask_operand): ones [128][16], and the mask of each S buffer [128][16]
+  static constexpr int OFF_ONES = OFF_ST + NST * STAGE + (STAGE_HOLDS_BIAS ? 0 : 32768);
+  static constexpr int OFF_MOP = OFF_ONES + 4096;
+  static constexpr int OFF_BAR = OFF_MOP + 2 * 4096;
   static constexpr int N_BAR = 2 * NST + 4 + 2;
   static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
   static constexpr int TMEM_COLS = 512;
@@ -806,8 +841,10 @@ struct AttnDbiasCfg {
 // 16 compute warps: four threads share one query row (TMEM lane) and take 32 of the 128 keys of the
 // tile each.  The bias tile of a CTA never changes, so it is converted once to fp32 (already
 // multiplied by log2 e) and read back with conflict-free 16-byte loads; per logit the inner loop is
-// three packed fp32x2 operations, one ex2 and (only for planes whose mask row is not all zero in
-// this key range, or for a ragged key tail) the mask add.
+// four packed fp32x2 operations per pair and one ex2.  The mask is no business of these warps: where a plane has one in this key
+// range, the issuing warp adds it to S by one more UMMA (K = 16).  As an add in the loop, behind a vote, it cost every plane
+// and made the CTAs of the masked keys the last to finish.  Measured, N = 384 with 5 % of the keys masked: 115 -> 85 us, N = 768
+// 844 -> 603.  Columns beyond N are computed with the zeros that TMA fills in and never stored.
 template <class Cfg>
 __global__ void __launch_bounds__(32 * (Cfg::NCW + 2), 1)
 attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -849,7 +886,7 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1 + NCW);
+      mbar_init(&empty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&sdp_full[s], 1);
@@ -866,6 +903,9 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     tma_prefetch_desc(&tmBias);
     tma_prefetch_desc(&tmMask);
   }
+  for (int i = threadIdx.x; i < 3 * 1024; i += blockDim.x)
+    reinterpret_cast<uint32_t*>(smem + Cfg::OFF_ONES)[i] = i < 1024 ? 0x3F803F80u : 0u;
+  fence_async_smem();
   if (warp == WARP_MMA) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
@@ -905,6 +945,9 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const uint32_t el = elect_one();
       constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, false);
       constexpr uint32_t swz = swizzle_mode_for_bytes(Cfg::SWZ);
+      const uint64_t ones_desc = make_smem_desc(smem_u32(smem + Cfg::OFF_ONES), 16, 256, swizzle_mode_for_bytes(32));
+      const uint64_t mop_desc = make_smem_desc(smem_u32(smem + Cfg::OFF_MOP), 16, 256, swizzle_mode_for_bytes(32));
+      const float inv_scale = 1.f / p.scale;
       int s = 0, buf = 0;
       uint32_t ph = 0, free_ph[2] = {1, 1};
       for (int pl = pl0; pl < pl1; ++pl) {
@@ -916,6 +959,10 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         for (int ks = 0; ks < D / 16; ++ks)
           umma_ss(el, tmem_base + buf * 256, make_smem_desc(st + ks * 32, 16, 8 * Cfg::SWZ, swz),
                   make_smem_desc(st + 2 * Cfg::TILE + ks * 32, 16, 8 * Cfg::SWZ, swz), idesc, ks != 0);
+        // (S of this buffer has been read, so the UMMA that used its mask operand is done)
+        if (mask_operand(smem + Cfg::OFF_MOP + buf * 4096, reinterpret_cast<const float*>(smem + Cfg::OFF_ST + s * Cfg::STAGE + 4 * Cfg::TILE),
+                         128, lane, inv_scale))
+          umma_ss(el, tmem_base + buf * 256, ones_desc, mop_desc + (uint64_t)(buf * (4096 >> 4)), idesc, 1u);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
           umma_ss(el, tmem_base + buf * 256 + 128, make_smem_desc(st + Cfg::TILE + ks * 32, 16, 8 * Cfg::SWZ, swz),
@@ -936,9 +983,7 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     constexpr float kLog2e = 1.4426950408889634f;
     const float c1 = p.scale * kLog2e;
     const uint64_t c2 = f2_pack(c1, c1);
-    const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
     const int q = qt * 128 + row;
-    const bool tail = (kt + 1) * 128 > p.N;
 
     // ---- bias tile -> fp32 * log2(e), laid out [part][16-column half][4-column group][row][4] so that
     //      the 32 lanes of a warp read 32 consecutive 16-byte pieces
@@ -980,33 +1025,29 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
     };
 
-    int s = 0, buf = 0;
-    uint32_t ph = 0, full_ph[2] = {0, 0};
+    int buf = 0;
+    uint32_t full_ph[2] = {0, 0};
     // row scalars travel two planes ahead of their use (they come from HBM on first touch)
     float l_n1, dl_n1, l_n2, dl_n2;
     load_row_scalars(pl0, l_n1, dl_n1);
     load_row_scalars(pl0 + 1, l_n2, dl_n2);
     for (int pl = pl0; pl < pl1; ++pl) {
-      // exp2(t - lse log2e) with lse = -inf (fully masked row) must give 0, not NaN: use -inf there
-      const float nl = (l_n1 == -INFINITY || l_n1 == INFINITY) ? -INFINITY : -l_n1 * kLog2e;
+      // exp2(t - lse log2e) of a fully masked row must give 0, not NaN or infinity
+      const float nl = (l_n1 < kMaskedLse || l_n1 == INFINITY) ? -INFINITY : -l_n1 * kLog2e;
       const uint64_t nl2 = f2_pack(nl, nl);
       const uint64_t nd2 = f2_pack(-dl_n1, -dl_n1);
       l_n1 = l_n2;
       dl_n1 = dl_n2;
       load_row_scalars(pl + 2, l_n2, dl_n2);
-      mbar_wait2(&sdp_full[buf], full_ph[buf], &full[s], ph, wctx);
+      mbar_wait(&sdp_full[buf], full_ph[buf], wctx);
       full_ph[buf] ^= 1;
       tc_fence_after();
-      const float* mask_row =
-          reinterpret_cast<const float*>(smem + Cfg::OFF_ST + s * Cfg::STAGE + 4 * Cfg::TILE) + CPT * part;
       const uint32_t t_s = tmem_addr(tmem_base, lane_base, buf * 256 + CPT * part);
       const uint32_t t_dp = tmem_addr(tmem_base, lane_base, buf * 256 + 128 + CPT * part);
       // 8 columns per step; the TMEM loads of step c+1 are in flight while step c is computed
       uint32_t rs[2][8], rd[2][8];
       tmem_ld8(t_s, rs[0]);
       tmem_ld8(t_dp, rd[0]);
-      // the mask probe (shared-memory load + vote) runs under the latency of the first TMEM loads
-      const bool general = tail || __any_sync(0xffffffffu, mask_row[lane] != 0.f);
 #pragma unroll
       for (int c = 0; c < CPT / 8; ++c) {
         const float4 bb0 = bias32[((part * 2 + (c >> 1)) * 4 + 2 * (c & 1)) * 128 + row];
@@ -1028,20 +1069,6 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         t2[1] = f2_fma(f2_pack_bits(s8[2], s8[3]), c2, f2_pack(bb0.z, bb0.w));
         t2[2] = f2_fma(f2_pack_bits(s8[4], s8[5]), c2, f2_pack(bb1.x, bb1.y));
         t2[3] = f2_fma(f2_pack_bits(s8[6], s8[7]), c2, f2_pack(bb1.z, bb1.w));
-        if (general) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float2 mk = *reinterpret_cast<const float2*>(mask_row + 8 * c + 2 * i);
-            float v0, v1;
-            f2_unpack(f2_fma(f2_pack(mk.x, mk.y), log2e2, t2[i]), v0, v1);
-            if (tail) {
-              const int k0 = kt * 128 + CPT * part + 8 * c + 2 * i;
-              if (k0 >= p.N) v0 = -INFINITY;
-              if (k0 + 1 >= p.N) v1 = -INFINITY;
-            }
-            t2[i] = f2_pack(v0, v1);
-          }
-        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           float a0, a1;
@@ -1051,13 +1078,7 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           acc[4 * c + i] = f2_fma(pr, gd, acc[4 * c + i]);
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
       buf ^= 1;
-      if (++s == NST) {
-        s = 0;
-        ph ^= 1;
-      }
     }
 
     if (q < p.N) {

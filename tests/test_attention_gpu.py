@@ -239,6 +239,35 @@ def test_nan_under_a_mask_reaches_the_output():
     assert torch.isnan(out).sum().item() == D
 
 
+@pytest.mark.parametrize("N,D", [(20, 32), (128, 16), (129, 32), (150, 64), (300, 32)])
+def test_gradients_under_masks_of_any_value(N, D):
+    """Masks that are not just 0 and a large value (they enter S as a sum of bf16 parts), single masked keys, masked key
+    tiles, and a plane whose keys are all masked by a large finite value: its gradients are finite, and zero where d_out is."""
+    O, H = 6, 4
+    gen = torch.Generator().manual_seed(N + D)
+    inp = dict(zip(("q", "k", "v"), (torch.randn(1, O, H, N, D, generator=gen) for _ in range(3))))
+    inp["pair_bias"] = torch.randn(1, 1, H, N, N, generator=gen)
+    mask = torch.zeros(1, O, 1, 1, N)
+    mask[0, 0] = torch.randn(N, generator=gen)
+    mask[0, 1] = 30 * torch.randn(N, generator=gen)
+    mask[0, 2, ..., N // 2:] = -1e9
+    mask[0, 3, ..., ::3] = -float("inf")
+    mask[0, 4, ..., : N // 2] = -1e4
+    mask[0, 5] = -1e9
+    inp["res_mask"] = mask
+    d_out = torch.randn(1, O, N, H, D, generator=gen).bfloat16()
+    d_out[0, 5] = 0
+    got, _ = _run(inp, d_out)
+    ref = _oracle(inp, d_out)
+    for n in ("dq", "dk", "dv"):
+        assert torch.equal(got[n][0, 5], torch.zeros_like(got[n][0, 5])), n
+        assert ao.rel_l2(got[n][:, :5], ref[n][:, :5]) <= REL_TOL, n
+    assert ao.rel_l2(got["dbias"], ref["dbias"]) <= REL_TOL
+    d_out[0, 5] = 1
+    got, _ = _run(inp, d_out)
+    assert torch.isfinite(got["dbias"]).all()
+
+
 def test_no_python_fallback_native_library_is_loaded():
     with open("/proc/self/maps") as f:
         assert "libtpf_b200.so" in f.read()
