@@ -20,6 +20,7 @@
 //    S and dP (two cheap K = D GEMMs) and summing dS in fp32 registers in ascending o.
 //    A few independent o-chunks per tile fill the machine; their partial planes are folded
 //    in fixed order by a tiny kernel.
+#include <math.h>
 #include <stdlib.h>
 
 #include "tpf_host.cuh"
@@ -86,54 +87,78 @@ struct AttnBwdParams {
   int64_t gb, go, gh, gn;       // their element strides
   const float* lse;             // [B,O,H,N]
   const float* delta;           // [B,O,H,N]
+  const float* mask;            // [B,O,mask_pitch]
+  int64_t mask_pitch;
   float* dq_scratch;            // per-CTA [N][D] fp32 when the key axis needs several strips
   int B, O, H, N;
   int q_tiles, k_tiles, n_strips;
   int bias_broadcast;
   float scale;
+  float logit_scale;            // scale, kept away from zero: what the added operands are divided by
   int n_items;
   FastDiv div_h, div_o;
 };
+
+// Numbers that are added to every logit of a row or of a column enter S and dP by one more UMMA of K = 16: an fp32 value is
+// three bf16 parts in three K columns (24 bits, as many as fp32 has), met by ones on the other side.  A tile of such rows has
+// 32 bytes per row, as a D = 16 operand tile; rows hold their values in the first 16 bytes, the second half is zero.
+struct Bf16x3 {
+  uint32_t hi, mid, lo;  // bf16 bits
+};
+__device__ __forceinline__ Bf16x3 split_bf16x3(float x) {
+  const float hi = __bfloat162float(__float2bfloat16_rn(x));
+  const float r = hi - hi != 0.f ? 0.f : x - hi;  // infinity or NaN: one part carries it
+  const float mid = __bfloat162float(__float2bfloat16_rn(r));
+  return {__float_as_uint(hi) >> 16, __float_as_uint(mid) >> 16, pack_bf16x2(r - mid, 0.f)};
+}
+__device__ __forceinline__ void store_added(uint8_t* tile, int row, uint4 v) {
+  *reinterpret_cast<uint4*>(tile + row * 32 + ((row >> 2) & 1) * 16) = v;  // (the 32-byte swizzle)
+}
+constexpr uint32_t kOnesBf16x2 = 0x3F803F80u;
+// A row whose log-sum-exp is below this has masked keys only (by -inf or by a large finite value such as -1e9): its logits and
+// the log-sum-exp differ by nothing but rounding, of more than one unit.  It gets no gradient, with either value.
+constexpr float kMaskedLse = -1e8f;
 
 template <int D_>
 struct AttnBwdCfg {
   static constexpr int D = D_;
   static constexpr int KS = D <= 32 ? 3 : 1;   // key tiles whose dK/dV stay in TMEM together
-  static constexpr int NKV = 2, NQ = 2;
+  // With one key tile per strip K and V stay for the strip; else they are loaded for every tile, and K, which dQ reads last,
+  // three tiles deep (with two the loads of the next tile came late: 800 cycles of a tile of 3250).
+  static constexpr bool KV_STAYS = KS == 1;
+  static constexpr int NK = KV_STAYS ? 2 : 3, NV = 2, NQ = 2;
   static constexpr int NB = D <= 32 ? 2 : 1;   // bias stages
-  static constexpr int NCW = 16;               // compute warps: four threads per query row, 32 keys each
-  static constexpr int THREADS = 32 * (NCW + 2);
-  static constexpr int WARP_TMA = NCW, WARP_MMA = NCW + 1;
+  static constexpr int NCW = 16;               // compute warps: two groups of eight, 64 queries each
+  static constexpr int THREADS = 32 * (NCW + 6);
+  static constexpr int WARP_TMA = NCW, WARP_MMA = NCW + 1;  // then four that store finished gradients
   static constexpr int SWZ = 2 * D;
   static constexpr int TILE = 128 * D * 2;
-  static constexpr int BIAS_STAGE = 32768, PD_BYTES = 32768;
+  static constexpr int ADD_TILE = 128 * 32;
+  static constexpr int BIAS_STAGE = 32768, DS_BYTES = 32768;
   static constexpr int OFF_BIAS = 0;
-  static constexpr int OFF_P = OFF_BIAS + NB * BIAS_STAGE;
-  static constexpr int OFF_DS = OFF_P + PD_BYTES;
-  static constexpr int OFF_Q = OFF_DS + PD_BYTES;        // [NQ]
+  static constexpr int OFF_DS = OFF_BIAS + NB * BIAS_STAGE;
+  static constexpr int OFF_Q = OFF_DS + DS_BYTES;        // [NQ]
   static constexpr int OFF_DO = OFF_Q + NQ * TILE;       // [NQ]
-  static constexpr int OFF_K = OFF_DO + NQ * TILE;       // [NKV]
-  static constexpr int OFF_V = OFF_K + NKV * TILE;       // [NKV]
-  // D <= 32: per compute warp a 32-row block of a finished dK / dV tile on its way out (at D = 64 there is no room)
+  static constexpr int OFF_K = OFF_DO + NQ * TILE;       // [NK]
+  static constexpr int OFF_V = OFF_K + NK * TILE;        // [NV]
+  // added operands: -lse and a row of ones with Q, -delta with dO, ones and the mask (with V's stages), ones with V
+  static constexpr int OFF_QADD = OFF_V + NV * TILE;         // [NQ]
+  static constexpr int OFF_DOADD = OFF_QADD + NQ * ADD_TILE;  // [NQ]
+  static constexpr int OFF_KADD = OFF_DOADD + NQ * ADD_TILE;  // [NV]
+  static constexpr int OFF_VADD = OFF_KADD + NV * ADD_TILE;
+  static constexpr int ADD_BYTES = (2 * NQ + NV + 1) * ADD_TILE;
+  // D <= 32: per storing warp two 32-row blocks of a finished tile on their way out (at D = 64 there is no room)
   static constexpr bool STAGED = D <= 32;
   static constexpr int STG_BYTES = 32 * D * 2;
-  static constexpr int OFF_STG = OFF_V + NKV * TILE;
-  // and what the compute warps need beside the tiles: lse and delta of a query tile's rows, and four AttnBwdItem records
-  static constexpr int OFF_ROW = OFF_STG + (STAGED ? 12 * STG_BYTES : 0);
-  static constexpr int OFF_ITEM = OFF_ROW + (STAGED ? 1024 : 0);
-  static constexpr int OFF_MASK = OFF_ITEM + (STAGED ? 128 : 0);  // [NKV] x 512
-  static constexpr int OFF_BAR = OFF_MASK + NKV * 512;
-  static constexpr int N_BAR = 2 * NB + 2 * NQ + 2 * NKV + 6;
+  static constexpr int OFF_STG = OFF_VADD + ADD_TILE;
+  static constexpr int OFF_BAR = OFF_STG + (STAGED ? 8 * STG_BYTES : 0);
+  static constexpr int N_BAR = 2 * NB + 2 * NQ + 2 * NK + 2 * NV + 8 + 2 * KS;
   static constexpr int SMEM_BYTES = OFF_BAR + N_BAR * 8 + 16 + 1024;
+  // S^T and dP^T of the two groups (64 queries each); P^T and dS^T, bf16, take their place
   static constexpr int TM_S = 0, TM_DP = 128, TM_DQ = 256, TM_DK = 320, TM_DV = 320 + KS * D;
   static constexpr int TMEM_COLS = 512;
   static_assert(TM_DV + KS * D <= 512, "TMEM budget");
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
-};
-
-struct AttnBwdItem {
-  int b, o, h, pad;
-  int64_t off, pad2;  // of the plane in dq / dk / dv
 };
 
 // Walks the (item, strip, query tile, key tile) sequence of one CTA.
@@ -150,6 +175,7 @@ struct BwdWalk {
   __device__ bool first_kk() const { return kk == 0; }
   __device__ bool last_kk() const { return kk == strip_len() - 1; }
   __device__ bool first_qt() const { return qt == 0; }
+  __device__ bool last_qt() const { return qt == q_tiles - 1; }
   __device__ void next() {
     if (++kk < strip_len()) return;
     kk = 0;
@@ -161,26 +187,30 @@ struct BwdWalk {
   }
 };
 
-// Sixteen compute warps: thread (row, part) owns query row `row` (= TMEM lane) and the 32 keys
-// [32 part, 32 part + 32) of a 128 x 128 tile.  It walks them 16 columns at a time straight from
-// TMEM (S and dP), forms P and dS, and keeps the bf16 results packed in 32 registers; only the
-// shared-memory stores wait for the UMMAs of the previous tile to release the P / dS tiles, so
-// the arithmetic of tile t+1 overlaps the dV / dK / dQ UMMAs of tile t.
+// S and dP are computed transposed (S^T = K Q^T, TMEM lane = key, column = query), so that bf16 P^T and dS^T, written over them,
+// are the A operands of dV += P^T dO and dK += dS^T Q straight from TMEM; only dS goes through shared memory, for dQ += dS K.
+// The log-sum-exp, the mask and delta are in S and dP already (see Bf16x3): what is left per logit is the bias, an ex2 and a
+// product.
+// The sixteen compute warps are two groups, each with the 64 queries of one half of a 128 x 128 tile and S / dP columns of its
+// own: while one group's UMMAs run, the other one computes.  A thread has the 32 queries of one key.
 //
-// RAGGED: a warp whose rows or keys of a tile all lie beyond the last one only stores zeros and keeps the barriers going;
-// the others have the arithmetic pipes to themselves.  At N = 257 that is half of the 32 x 32 blocks (D = 64: 263 -> 255 us),
-// at N = 400 a third (412 -> 397 us).  The test costs 2 % of a kernel that has no such warps.
+// What bounds it: the chain of a half tile, 1200 cycles of arithmetic and 1000 between P being written and the next S being
+// there (hand-shakes, 14 UMMAs, completion), of which the other group hides most; the ex2 pipe alone needs 1024 cycles a tile.
+// Before, with a thread per query row, P and dS went through shared memory for three products of 128 x 128 tiles, whose operand
+// traffic kept it busy for 2400 cycles a tile, and one S / dP pair left all warps waiting together.  Measured, H = 4, us:
+// N = 384, D = 32 188 -> 133; N = 768 1523 -> 1010; N = 257, D = 64 233 -> 162; N = 128, D = 16, B = 4 35.4 -> 33.9.
+// Waiting for S and dP apart was slower (136 us at N = 384), so was a warp of its own for dQ's UMMAs (137).
+//
+// RAGGED: a warp whose rows or keys of a tile all lie beyond the last one only keeps the barriers going, and the UMMAs leave its
+// part of their K extent out; the others have the pipes to themselves.
 template <class Cfg, bool RAGGED>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                const __grid_constant__ CUtensorMap tmBias, const __grid_constant__ CUtensorMap tmMask,
-                const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV,
-                const AttnBwdParams p, int* __restrict__ status) {
+                const __grid_constant__ CUtensorMap tmBias, const __grid_constant__ CUtensorMap tmDQ,
+                const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV, const AttnBwdParams p, int* __restrict__ status) {
   griddep_wait();
-  constexpr int D = Cfg::D, KS = Cfg::KS, NKV = Cfg::NKV, NQ = Cfg::NQ, NB = Cfg::NB, NCW = Cfg::NCW;
-  // (Declared 1024-byte aligned, every address below becomes a constant, and this kernel and the forward one get 4 %
-  // slower, the dBias kernel 4 % faster.)
+  constexpr int D = Cfg::D, KS = Cfg::KS, NK = Cfg::NK, NV = Cfg::NV, NQ = Cfg::NQ, NB = Cfg::NB, NCW = Cfg::NCW;
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
@@ -188,15 +218,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* b_empty = b_full + NB;
   uint64_t* q_full = b_empty + NB;
   uint64_t* q_empty = q_full + NQ;
-  uint64_t* kv_full = q_empty + NQ;
-  uint64_t* kv_empty = kv_full + NKV;
-  uint64_t* misc = kv_empty + NKV;
-  uint64_t* sdp_full = misc + 0;   // S and dP of a tile are in TMEM
-  uint64_t* sdp_free = misc + 1;   // ... and have been read by all compute warps
-  uint64_t* pds_ready = misc + 2;  // P and dS of a tile are in shared memory
-  uint64_t* pds_free = misc + 3;   // ... and have been consumed by the dV / dK / dQ UMMAs
-  uint64_t* dkv_free = misc + 4;
-  uint64_t* row_free = misc + 5;   // the compute warps have read the query rows' scalars
+  uint64_t* k_full = q_empty + NQ;
+  uint64_t* k_empty = k_full + NK;
+  uint64_t* v_full = k_empty + NK;  // V and the added operand of the keys
+  uint64_t* v_empty = v_full + NV;
+  uint64_t* misc = v_empty + NV;
+  uint64_t* sdp_full = misc + 0;   // [2] S and dP of a group's half tile are in TMEM
+  uint64_t* pds_ready = misc + 2;  // [2] ... and P and dS have taken their place
+  uint64_t* ds_ready = misc + 4;   // dS of a tile is in shared memory
+  uint64_t* ds_free = misc + 5;    // ... and has been consumed; so have P and dS in TMEM
+  uint64_t* dq_full = misc + 6;    // dQ of a query tile is complete
+  uint64_t* dq_free = misc + 7;    // ... and has been read
+  uint64_t* dkv_full = misc + 8;   // [KS] dK and dV of a key tile are complete
+  uint64_t* dkv_free = dkv_full + KS;  // ... and have been read
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::N_BAR);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx wctx{abort_flag, status};
@@ -210,19 +244,29 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&b_empty[s], NCW);
     }
     for (int s = 0; s < NQ; ++s) {
-      mbar_init(&q_full[s], Cfg::STAGED ? 1 + 32 : 1);  // the loading thread, and the warp's copies of the row scalars
+      mbar_init(&q_full[s], 1);
       mbar_init(&q_empty[s], 1);
     }
-    for (int s = 0; s < NKV; ++s) {
-      mbar_init(&kv_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
+    for (int s = 0; s < NK; ++s) {
+      mbar_init(&k_full[s], 1);
+      mbar_init(&k_empty[s], 1);
     }
-    mbar_init(sdp_full, 1);
-    mbar_init(sdp_free, NCW);
-    mbar_init(pds_ready, NCW);
-    mbar_init(pds_free, 1);
-    mbar_init(dkv_free, NCW);
-    mbar_init(row_free, NCW);
+    for (int s = 0; s < NV; ++s) {
+      mbar_init(&v_full[s], 1);
+      mbar_init(&v_empty[s], 1);
+    }
+    for (int g = 0; g < 2; ++g) {
+      mbar_init(&sdp_full[g], 1);
+      mbar_init(&pds_ready[g], NCW / 2);
+    }
+    mbar_init(ds_ready, NCW);
+    mbar_init(ds_free, 1);
+    mbar_init(dq_full, 1);
+    mbar_init(dq_free, 4);
+    for (int s = 0; s < KS; ++s) {
+      mbar_init(&dkv_full[s], 1);
+      mbar_init(&dkv_free[s], 8);
+    }
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
@@ -230,8 +274,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmDO);
     tma_prefetch_desc(&tmBias);
-    tma_prefetch_desc(&tmMask);
   }
+  for (int i = threadIdx.x; i < Cfg::ADD_BYTES / 4; i += blockDim.x)
+    reinterpret_cast<uint32_t*>(smem + Cfg::OFF_QADD)[i] = i >= (Cfg::OFF_VADD - Cfg::OFF_QADD) / 4 ? kOnesBf16x2 : 0u;
+  fence_async_smem();
   if (warp == Cfg::WARP_MMA) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish();
@@ -249,513 +295,466 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   };
 
   if (warp == Cfg::WARP_TMA) {
-    // ------------------------------------------------------------------ TMA producer
-    {
-      const uint32_t el = elect_one();
-      int q_s = 0, kv_s = 0, b_s = 0;
-      uint32_t q_ph = 1, kv_ph = 1, b_ph = 1, row_ph = 1;
-      BwdWalk w;
-      w.init(blockIdx.x, gridDim.x, p.n_items, p.q_tiles, p.k_tiles, KS, p.n_strips);
-      int b = 0, o = 0, h = 0, cur = -1, n_item = 0;
-      for (; w.valid(); w.next()) {
-        if (w.item != cur) {
-          cur = w.item;
-          decode(cur, b, o, h);
-        }
-        if (w.first_kk()) {
-          mbar_wait(&q_empty[q_s], q_ph, wctx);
-          if constexpr (Cfg::STAGED) {
-            // This warp prepares what the compute warps would otherwise wait for at the ends of a query tile, all at the
-            // same time: the rows' scalars (from memory: 600 to 1500 cycles) and the plane's coordinates and offset (1000).
-            // It is at most two query tiles ahead of them: four item records are enough.
-            if (w.first_qt() && w.strip == 0) {
-              AttnBwdItem* rec = reinterpret_cast<AttnBwdItem*>(smem + Cfg::OFF_ITEM) + (n_item++ & 3);
-              if (el) {
-                rec->b = b;
-                rec->o = o;
-                rec->h = h;
-                rec->off = b * p.gb + o * p.go + h * p.gh;
-              }
-            }
-            mbar_wait(row_free, row_ph, wctx);
-            row_ph ^= 1;
-            float* rows = reinterpret_cast<float*>(smem + Cfg::OFF_ROW);
+    // ------------------------------------------------------------------ TMA producer, and the added operands
+    const uint32_t el = elect_one();
+    int q_s = 0, k_s = 0, v_s = 0, b_s = 0;
+    uint32_t q_ph = 1, k_ph = 1, v_ph = 1, b_ph = 1;
+    BwdWalk w;
+    w.init(blockIdx.x, gridDim.x, p.n_items, p.q_tiles, p.k_tiles, KS, p.n_strips);
+    const float inv = 1.f / p.logit_scale;
+    const float no_row = copysignf(1e30f, -p.logit_scale);  // makes exp2 zero, and no NaN with masked keys
+    // What a step adds to its logits and the coordinates of its plane.  The next step's are requested before this step's waits:
+    // requested after them, their latency made this warp the slowest part of the pipeline.
+    struct Step {
+      int b, o, h;
+      float4 mask;
+      float l[4], d[4];
+    } cur, nxt;
+    auto request = [&](const BwdWalk& at, Step& s) {
+      decode(at.item, s.b, s.o, s.h);
+      const int k0 = at.kt() * 128 + 4 * lane;
+      if (k0 < p.mask_pitch)
+        s.mask = __ldg(reinterpret_cast<const float4*>(p.mask + ((int64_t)s.b * p.O + s.o) * p.mask_pitch + k0));
+      if (at.first_kk()) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int q = w.qt * 128 + 32 * i + lane;
-              const bool ok = q < p.N;
-              const int64_t idx = (int64_t)cur * p.N + (ok ? q : 0);  // items are numbered as their planes lie in memory
-              cp_async_4(rows + 32 * i + lane, p.lse + idx, ok);
-              cp_async_4(rows + 128 + 32 * i + lane, p.delta + idx, ok);
-            }
-            cp_async_arrive(&q_full[q_s]);
+        for (int i = 0; i < 4; ++i) {
+          const int q = at.qt * 128 + 32 * i + lane;
+          if (q < p.N) {
+            const int64_t idx = (int64_t)at.item * p.N + q;  // items are numbered as their planes lie in memory
+            s.l[i] = __ldg(p.lse + idx);
+            s.d[i] = __ldg(p.delta + idx);
           }
-          mbar_expect_tx(el, &q_full[q_s], 2 * Cfg::TILE);
-          tma_load_5d(el, smem + Cfg::OFF_Q + q_s * Cfg::TILE, &tmQ, &q_full[q_s], 0, w.qt * 128, h, o, b);
-          tma_load_5d(el, smem + Cfg::OFF_DO + q_s * Cfg::TILE, &tmDO, &q_full[q_s], 0, w.qt * 128, h, o, b);
-          if (++q_s == NQ) {
-            q_s = 0;
-            q_ph ^= 1;
-          }
-        }
-        const int kt = w.kt();
-        mbar_wait(&kv_empty[kv_s], kv_ph, wctx);
-        mbar_expect_tx(el, &kv_full[kv_s], 2 * Cfg::TILE + 512);
-        tma_load_5d(el, smem + Cfg::OFF_K + kv_s * Cfg::TILE, &tmK, &kv_full[kv_s], 0, kt * 128, h, o, b);
-        tma_load_5d(el, smem + Cfg::OFF_V + kv_s * Cfg::TILE, &tmV, &kv_full[kv_s], 0, kt * 128, h, o, b);
-        tma_load_3d(el, smem + Cfg::OFF_MASK + kv_s * 512, &tmMask, &kv_full[kv_s], kt * 128, o, b);
-        if (++kv_s == NKV) {
-          kv_s = 0;
-          kv_ph ^= 1;
-        }
-        const int bb = p.bias_broadcast ? 0 : b;
-        mbar_wait(&b_empty[b_s], b_ph, wctx);
-        mbar_expect_tx(el, &b_full[b_s], Cfg::BIAS_STAGE);
-        tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], kt * 128, w.qt * 128, h, bb);
-        tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE + 16384, &tmBias, &b_full[b_s], kt * 128 + 64,
-                    w.qt * 128, h, bb);
-        if (++b_s == NB) {
-          b_s = 0;
-          b_ph ^= 1;
-        }
-      }
-    }
-  } else if (warp == Cfg::WARP_MMA) {
-    // ------------------------------------------------------------------ UMMA issuer
-    {
-      const uint32_t el = elect_one();
-      constexpr uint32_t idesc_sd = make_idesc_bf16(128, 128, false, false);  // S, dP
-      constexpr uint32_t idesc_kv = make_idesc_bf16(128, D, true, true);      // dV, dK
-      constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, false, true);     // dQ
-      constexpr uint32_t swz = swizzle_mode_for_bytes(Cfg::SWZ);
-      constexpr uint32_t swz128 = swizzle_mode_for_bytes(128);
-      // Descriptors of stage 0 of every operand; a stage or a k-step only changes the start-address
-      // field (bits 0-13, 16-byte units), so the per-UMMA work is one 64-bit add.
-      const uint64_t dq_k = make_smem_desc(smem_u32(smem + Cfg::OFF_Q), 16, 8 * Cfg::SWZ, swz);     // Q, K-major (S)
-      const uint64_t dk_k = make_smem_desc(smem_u32(smem + Cfg::OFF_K), 16, 8 * Cfg::SWZ, swz);     // K, K-major (S)
-      const uint64_t ddo_k = make_smem_desc(smem_u32(smem + Cfg::OFF_DO), 16, 8 * Cfg::SWZ, swz);   // dO, K-major (dP)
-      const uint64_t dv_k = make_smem_desc(smem_u32(smem + Cfg::OFF_V), 16, 8 * Cfg::SWZ, swz);     // V, K-major (dP)
-      const uint64_t dp_mn = make_smem_desc(smem_u32(smem + Cfg::OFF_P), 16384, 1024, swz128);      // P^T as A (dV)
-      const uint64_t dds_mn = make_smem_desc(smem_u32(smem + Cfg::OFF_DS), 16384, 1024, swz128);    // dS^T as A (dK)
-      const uint64_t dds_k = make_smem_desc(smem_u32(smem + Cfg::OFF_DS), 16, 1024, swz128);        // dS as A (dQ)
-      const uint64_t ddo_mn = make_smem_desc(smem_u32(smem + Cfg::OFF_DO), 128 * Cfg::SWZ, 8 * Cfg::SWZ, swz);  // dO as B (dV)
-      const uint64_t dq_mn = make_smem_desc(smem_u32(smem + Cfg::OFF_Q), 128 * Cfg::SWZ, 8 * Cfg::SWZ, swz);    // Q as B (dK)
-      const uint64_t dk_mn = make_smem_desc(smem_u32(smem + Cfg::OFF_K), 128 * Cfg::SWZ, 8 * Cfg::SWZ, swz);    // K as B (dQ)
-      constexpr uint64_t kTile16 = Cfg::TILE >> 4;
-
-      // stage trackers for the "ahead" stream (S, dP) and the "behind" stream (dV, dK, dQ)
-      int aq_s = 0, akv_s = 0;
-      uint32_t aq_ph = 0, akv_ph = 0;
-      int bq_s = 0, bkv_s = 0;
-      uint32_t sdpfree_ph = 1, pdsready_ph = 0, dkvfree_ph = 1;
-
-      BwdWalk wa, wb;  // ahead / behind
-      wa.init(blockIdx.x, gridDim.x, p.n_items, p.q_tiles, p.k_tiles, KS, p.n_strips);
-      wb = wa;
-
-      auto issue_sdp = [&]() {  // S and dP of tile wa, then advance wa
-        if (wa.first_kk()) mbar_wait3(&q_full[aq_s], aq_ph, &kv_full[akv_s], akv_ph, sdp_free, sdpfree_ph, wctx);
-        else mbar_wait2(&kv_full[akv_s], akv_ph, sdp_free, sdpfree_ph, wctx);
-        sdpfree_ph ^= 1;
-        tc_fence_after();
-        const uint64_t qo = aq_s * kTile16, ko = akv_s * kTile16;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          umma_ss(el, tmem_base + Cfg::TM_S, dq_k + qo + 2 * ks, dk_k + ko + 2 * ks, idesc_sd, ks != 0);
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          umma_ss(el, tmem_base + Cfg::TM_DP, ddo_k + qo + 2 * ks, dv_k + ko + 2 * ks, idesc_sd, ks != 0);
-        umma_commit(el, sdp_full);
-        if (++akv_s == NKV) {
-          akv_s = 0;
-          akv_ph ^= 1;
-        }
-        const bool last_kk = wa.last_kk();
-        wa.next();
-        if (last_kk) {
-          if (++aq_s == NQ) {
-            aq_s = 0;
-            aq_ph ^= 1;
-          }
-        }
-      };
-
-      if (wa.valid()) issue_sdp();
-      for (; wb.valid();) {
-        // S and dP of the next tile as soon as the current pair has been read out of TMEM
-        if (wa.valid()) issue_sdp();
-        mbar_wait(pds_ready, pdsready_ph, wctx);
-        pdsready_ph ^= 1;
-        if (wb.first_qt() && wb.first_kk()) {
-          // first accumulation of a strip overwrites dK/dV: the previous strip must have been read out
-          mbar_wait(dkv_free, dkvfree_ph, wctx);
-          dkvfree_ph ^= 1;
-        }
-        tc_fence_after();
-        const uint64_t qo = bq_s * kTile16, ko = bkv_s * kTile16;
-        const uint32_t acc_kv = wb.first_qt() ? 0u : 1u;
-        // dV(kt) (+)= P^T dO ; dK(kt) (+)= dS^T Q   (16 queries per step)
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          umma_ss(el, tmem_base + Cfg::TM_DV + wb.kk * D, dp_mn + (uint64_t)(ks * 128), ddo_mn + qo + (uint64_t)(ks * Cfg::SWZ),
-                  idesc_kv, (ks != 0) ? 1u : acc_kv);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          umma_ss(el, tmem_base + Cfg::TM_DK + wb.kk * D, dds_mn + (uint64_t)(ks * 128), dq_mn + qo + (uint64_t)(ks * Cfg::SWZ),
-                  idesc_kv, (ks != 0) ? 1u : acc_kv);
-        // dQ(qt) (+)= dS K   (16 keys per step)
-        const uint32_t acc_q = wb.first_kk() ? 0u : 1u;
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          umma_ss(el, tmem_base + Cfg::TM_DQ, dds_k + (uint64_t)((ks >> 2) * 1024 + (ks & 3) * 2),
-                  dk_mn + ko + (uint64_t)(ks * Cfg::SWZ), idesc_dq, (ks != 0) ? 1u : acc_q);
-        umma_commit(el, pds_free);
-        umma_commit(el, &kv_empty[bkv_s]);
-        if (++bkv_s == NKV) bkv_s = 0;
-        if (wb.last_kk()) {  // (the compute warps learn of a finished strip from pds_free of its last tile)
-          umma_commit(el, &q_empty[bq_s]);
-          if (++bq_s == NQ) bq_s = 0;
-        }
-        wb.next();
-      }
-    }
-  } else {
-    // ------------------------------------------------------------------ compute warps
-    const int part = warp >> 2;                 // which 32-key slice of the tile
-    const int row = 32 * (warp & 3) + lane;     // query row in the tile == TMEM lane
-    const uint32_t lane_base = 32 * (warp & 3);
-    const uint32_t t_s = tmem_addr(tmem_base, lane_base, Cfg::TM_S + 32 * part);
-    const uint32_t t_dp = tmem_addr(tmem_base, lane_base, Cfg::TM_DP + 32 * part);
-    constexpr int DQ = D / 4;                   // output columns per thread
-    const uint32_t t_dq = tmem_addr(tmem_base, lane_base, Cfg::TM_DQ + DQ * part);
-    // the thread's 32 keys are four 16-byte pieces of a 128-byte row of one 64-key half tile
-    const int half_off = (part >> 1) * 16384 + row * 128;
-    const int piece0 = (part & 1) * 4;
-    constexpr float kLog2e = 1.4426950408889634f;
-    const float scale = p.scale;
-    const uint64_t scale2 = f2_pack(scale, scale);
-    const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
-
-    uint32_t sdpfull_ph = 0, pdsfree_ph = 1, kv_ph = 0, b_ph = 0;
-    int kv_s = 0, b_s = 0, q_s = 0;
-    uint32_t q_ph = 0;
-    bool have_prev_dq = false;     // a finished dQ tile waits in TMEM
-    bool have_prev_strip = false;  // the dK / dV accumulators of a finished strip wait in TMEM
-    __nv_bfloat16* dq_dst = nullptr;  // this thread's piece of that dQ tile's row; null beyond the last row
-    int item_no = 0, prev_no = 0, prev_q0 = 0, prev_strip = 0;
-
-    // read DQ consecutive accumulator columns of this thread's row
-    auto ld_cols = [&](uint32_t taddr, float (&v)[DQ]) {
-      if constexpr (DQ == 4) {
-        uint32_t r[4];
-        tmem_ld4(taddr, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < DQ; c += 8) {
-          uint32_t r[8];
-          tmem_ld8(taddr + c, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[c + i] = __uint_as_float(r[i]);
         }
       }
     };
-    // dQ tiles leave straight from registers, 16 bytes (8 at D = 16) of a row per thread: the stores are not waited for.
-    // A dQ tile, which is finished most often, is only packed before the hand-over of P / dS and stored after it.
-    constexpr int PQ = DQ / 2;  // packed words per thread
-    auto pack_cols = [&](const float (&v)[DQ], float mul, uint32_t (&w)[PQ]) {
+    cur.mask = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < 4; ++i) cur.l[i] = cur.d[i] = 0.f;
+    if (w.valid()) request(w, cur);
+    nxt = cur;
+    BwdWalk next = w;
+    while (w.valid()) {
+      next.next();
+      if (next.valid()) request(next, nxt);
+      const int b = cur.b, o = cur.o, h = cur.h;
+      if (w.first_kk()) {
+        warp_wait(&q_empty[q_s], q_ph, wctx);
 #pragma unroll
-      for (int i = 0; i < PQ; ++i) w[i] = pack_bf16x2(v[2 * i] * mul, v[2 * i + 1] * mul);
-    };
-    auto store_packed = [&](__nv_bfloat16* dst, const uint32_t (&w)[PQ]) {
-      if constexpr (PQ == 2) {
-        *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < PQ; i += 4) *reinterpret_cast<uint4*>(dst + 2 * i) = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
-      }
-    };
-    uint32_t dqw[PQ];
-    bool out_dq = false;  // a packed dQ tile waits in registers
-
-    // a finished dQ tile that has been read out of TMEM: packed, or folded into the per-CTA running sum
-    auto take_dq = [&](float (&v)[DQ]) {
-      if (p.n_strips > 1) {
-        const int q = prev_q0 + row;
-        if (q < p.N) {
-          float* sc = p.dq_scratch + ((int64_t)blockIdx.x * p.N + q) * D + DQ * part;
-          if (prev_strip > 0) {
-#pragma unroll
-            for (int c = 0; c < DQ; c += 4) {
-              const float4 o4 = *reinterpret_cast<const float4*>(sc + c);
-              v[c] += o4.x; v[c + 1] += o4.y; v[c + 2] += o4.z; v[c + 3] += o4.w;
-            }
-          }
-          if (prev_strip + 1 < p.n_strips) {
-#pragma unroll
-            for (int c = 0; c < DQ; c += 4) *reinterpret_cast<float4*>(sc + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
-          }
+        for (int i = 0; i < 4; ++i) {
+          const int row = 32 * i + lane;
+          const bool ok = w.qt * 128 + row < p.N;
+          const Bf16x3 l = split_bf16x3(ok && !(cur.l[i] < kMaskedLse) ? -cur.l[i] * inv : no_row);
+          const Bf16x3 d = split_bf16x3(ok ? -cur.d[i] : 0.f);
+          store_added(smem + Cfg::OFF_QADD + q_s * Cfg::ADD_TILE, row,
+                      make_uint4(l.hi | l.mid << 16, l.lo | 0x3F800000u, kOnesBf16x2, 0u));
+          store_added(smem + Cfg::OFF_DOADD + q_s * Cfg::ADD_TILE, row, make_uint4(d.hi | d.mid << 16, d.lo, 0u, 0u));
         }
-      }
-      out_dq = prev_strip + 1 == p.n_strips;
-      pack_cols(v, scale, dqw);
-    };
-
-    // D = 64: the same by the threads themselves, requested one query tile ahead: into L1, not into registers, which this
-    // kernel has none to spare of (kept there they were spilled, and the spill waited for the load).
-    auto request_row_scalars = [&](int item, int q) {
-      if (item < p.n_items && q < p.N) {
-        const int64_t idx = (int64_t)item * p.N + q;
-        prefetch_l1(p.lse + idx);
-        prefetch_l1(p.delta + idx);
-      }
-    };
-    const AttnBwdItem* items = reinterpret_cast<const AttnBwdItem*>(smem + Cfg::OFF_ITEM);
-
-    // Reads finished accumulators out of TMEM: the dQ tile of a finished query tile and, after the last tile of a
-    // strip, the strip's dK / dV tiles, which are stored at once (then the UMMA issuer may start the next strip in those
-    // columns).  Called by all compute warps once the UMMAs of the previous tile are done.
-    // The dK / dV tiles of a strip are dealt out whole to three of the four warps of a TMEM lane quarter; a warp packs its 32 rows
-    // into shared memory and stores them by one TMA.  (Every thread storing its 8 columns of every tile as 16-byte
-    // pieces took 3400 cycles of the 37000 of a plane at N = 384.)
-    auto take_finished = [&]() {
-      if (have_prev_dq) {
-        float dqv[DQ];
-        ld_cols(t_dq, dqv);
-        have_prev_dq = false;
-        take_dq(dqv);
-      }
-      if (have_prev_strip) {
-        have_prev_strip = false;
-        const int tiles = min(KS, p.k_tiles - prev_strip * KS);
-        if constexpr (Cfg::STAGED) {
-          const int4 pos = *reinterpret_cast<const int4*>(items + (prev_no & 3));
-          uint8_t* stg = smem + Cfg::OFF_STG + warp * Cfg::STG_BYTES;
-          const int sw = D == 32 ? (lane >> 1) & 3 : (lane >> 2) & 1;  // the maps' 64- / 32-byte swizzle
-          for (int a = part < 3 ? part : 2 * KS; a < 2 * tiles; a += 3) {
-            const bool is_v = a >= tiles;
-            const int kk = is_v ? a - tiles : a;
-            const uint32_t src = tmem_addr(tmem_base, lane_base, (is_v ? Cfg::TM_DV : Cfg::TM_DK) + kk * D);
-            const float mul = is_v ? 1.f : scale;
-            bulk_wait_read<0>();
-            __syncwarp();
-#pragma unroll
-            for (int c = 0; c < D; c += 16) {
-              uint32_t r[16], w[8];
-              tmem_ld16(src + c, r);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 8; ++i)
-                w[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * mul, __uint_as_float(r[2 * i + 1]) * mul);
-#pragma unroll
-              for (int i = 0; i < 2; ++i)
-                *reinterpret_cast<uint4*>(stg + lane * (2 * D) + (((c >> 3) + i) ^ sw) * 16) =
-                    make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-            }
-            fence_async_smem();
-            __syncwarp();
-            const int n0 = (prev_strip * KS + kk) * 128 + (int)lane_base;
-            if (n0 < p.N) tma_store_5d(lane == 0, is_v ? &tmDV : &tmDK, stg, 0, n0, pos.z, pos.y, pos.x);
-          }
-        } else {
-          int b, o, h;
-          decode(prev_no, b, o, h);
-          __nv_bfloat16* dk = p.dk + b * p.gb + o * p.go + h * p.gh + (prev_strip * KS * 128 + row) * p.gn + DQ * part;
-          __nv_bfloat16* dv = p.dv + (dk - p.dk);
-#pragma unroll
-          for (int kk = 0; kk < KS; ++kk) {
-            if (kk < tiles) {
-              float vk[DQ], vv[DQ];
-              ld_cols(tmem_addr(tmem_base, lane_base, Cfg::TM_DK + kk * D + DQ * part), vk);
-              ld_cols(tmem_addr(tmem_base, lane_base, Cfg::TM_DV + kk * D + DQ * part), vv);
-              if ((prev_strip * KS + kk) * 128 + row < p.N) {
-                uint32_t w[PQ];
-                pack_cols(vk, scale, w);
-                store_packed(dk + kk * 128 * p.gn, w);
-                pack_cols(vv, 1.f, w);
-                store_packed(dv + kk * 128 * p.gn, w);
-              }
-            }
-          }
-        }
-        tc_fence_before();
+        fence_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(dkv_free);
-      } else {
-        tc_fence_before();
-      }
-    };
-    auto store_finished = [&]() {
-      if (out_dq) {
-        out_dq = false;
-        if (dq_dst != nullptr) store_packed(dq_dst, dqw);
-      }
-    };
-
-    // The (item, strip, query tile, key tile) sequence as plain loops: the scalar part of a step is on the path between
-    // two UMMA batches.
-    for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++item_no) {
-      [[maybe_unused]] __nv_bfloat16* dq_row = nullptr;
-      if constexpr (!Cfg::STAGED) {
-        int b, o, h;
-        decode(item, b, o, h);
-        dq_row = p.dq + b * p.gb + o * p.go + h * p.gh + row * p.gn + DQ * part;
-      }
-    for (int strip = 0; strip < p.n_strips; ++strip) {
-      const int tiles_k = min(KS, p.k_tiles - strip * KS);
-    for (int qt = 0; qt < p.q_tiles; ++qt) {
-      float neg_lse2 = -INFINITY, delta = 0.f;
-      if constexpr (Cfg::STAGED) {
-        mbar_wait(&q_full[q_s], q_ph, wctx);
-        if (qt * 128 + row < p.N) {
-          const float* rows = reinterpret_cast<const float*>(smem + Cfg::OFF_ROW) + row;
-          if (rows[0] != -INFINITY) neg_lse2 = -rows[0] * kLog2e;
-          delta = rows[128];
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(row_free);
+        mbar_expect_tx(el, &q_full[q_s], 2 * Cfg::TILE);
+        tma_load_5d(el, smem + Cfg::OFF_Q + q_s * Cfg::TILE, &tmQ, &q_full[q_s], 0, w.qt * 128, h, o, b);
+        tma_load_5d(el, smem + Cfg::OFF_DO + q_s * Cfg::TILE, &tmDO, &q_full[q_s], 0, w.qt * 128, h, o, b);
         if (++q_s == NQ) {
           q_s = 0;
           q_ph ^= 1;
         }
-      } else {
-        if (qt * 128 + row < p.N) {
-          const int64_t idx = (int64_t)item * p.N + qt * 128 + row;
-          const float l = __ldg(p.lse + idx);
-          delta = __ldg(p.delta + idx);
-          if (l != -INFINITY) neg_lse2 = -l * kLog2e;
-        }
-        if (qt + 1 < p.q_tiles) request_row_scalars(item, (qt + 1) * 128 + row);
-        else request_row_scalars(strip + 1 < p.n_strips ? item : item + (int)gridDim.x, row);
       }
-    for (int kk = 0; kk < tiles_k; ++kk) {
-      const int kt = strip * KS + kk;
-      const uint64_t nlse2 = f2_pack(neg_lse2, neg_lse2);
-      const uint64_t ndel2 = f2_pack(-delta, -delta);
-
-      mbar_wait3(sdp_full, sdpfull_ph, &kv_full[kv_s], kv_ph, &b_full[b_s], b_ph, wctx);
-      sdpfull_ph ^= 1;
-      tc_fence_after();
-      const uint8_t* bias_row = smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE + half_off;
-      const float* mask_row = reinterpret_cast<const float*>(smem + Cfg::OFF_MASK + kv_s * 512) + 32 * part;
-      const bool tail = (kt + 1) * 128 > p.N;
-      const bool general = tail || __any_sync(0xffffffffu, mask_row[lane] != 0.f);
-
-      uint32_t ppk[16], dpk[16];  // bf16 pairs of P and dS of this thread's 32 keys
-      bool dead = false;
-      if constexpr (RAGGED) dead = qt * 128 + (int)lane_base >= p.N || kt * 128 + 32 * part >= p.N;
-      if (dead) {
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(sdp_free);
-          mbar_arrive(&b_empty[b_s]);
+      const int kt = w.kt();
+      if (!Cfg::KV_STAYS || w.first_qt()) {
+        warp_wait(&v_empty[v_s], v_ph, wctx);
+        const float mv[4] = {cur.mask.x, cur.mask.y, cur.mask.z, cur.mask.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int key = 4 * lane + i;
+          const Bf16x3 m = split_bf16x3(kt * 128 + key < p.N ? mv[i] * inv : copysignf(INFINITY, -p.logit_scale));
+          store_added(smem + Cfg::OFF_KADD + v_s * Cfg::ADD_TILE, key,
+                      make_uint4(kOnesBf16x2, 0x3F80u | m.hi << 16, m.mid | m.lo << 16, 0u));
         }
+        fence_async_smem();
+        __syncwarp();
+        mbar_expect_tx(el, &v_full[v_s], Cfg::TILE);
+        tma_load_5d(el, smem + Cfg::OFF_V + v_s * Cfg::TILE, &tmV, &v_full[v_s], 0, kt * 128, h, o, b);
+        if (++v_s == NV) {
+          v_s = 0;
+          v_ph ^= 1;
+        }
+        warp_wait(&k_empty[k_s], k_ph, wctx);
+        mbar_expect_tx(el, &k_full[k_s], Cfg::TILE);
+        tma_load_5d(el, smem + Cfg::OFF_K + k_s * Cfg::TILE, &tmK, &k_full[k_s], 0, kt * 128, h, o, b);
+        if (++k_s == NK) {
+          k_s = 0;
+          k_ph ^= 1;
+        }
+      }
+      warp_wait(&b_empty[b_s], b_ph, wctx);
+      mbar_expect_tx(el, &b_full[b_s], Cfg::BIAS_STAGE);
+      tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], kt * 128, w.qt * 128, h,
+                  p.bias_broadcast ? 0 : b);
+      if (++b_s == NB) {
+        b_s = 0;
+        b_ph ^= 1;
+      }
+      w = next;
+      cur = nxt;
+    }
+  } else if (warp == Cfg::WARP_MMA) {
+    // ------------------------------------------------------------------ UMMA issuer
+    const uint32_t el = elect_one();
+    constexpr uint32_t idesc_sd = make_idesc_bf16(128, 64, false, false);  // S^T, dP^T
+    constexpr uint32_t idesc_kv = make_idesc_bf16(128, D, false, true);    // dV, dK
+    constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, true, true);     // dQ
+    constexpr uint32_t swz = swizzle_mode_for_bytes(Cfg::SWZ);
+    // Lower descriptor words of stage 0 of every operand; a stage, a half or a k-step only changes the start-address
+    // field (bits 0-13, 16-byte units).
+    constexpr uint32_t hi = smem_desc_hi(8 * Cfg::SWZ, swz);                       // q, k, v, dO tiles, K-major and MN-major
+    constexpr uint32_t hi_ds = smem_desc_hi(1024, swizzle_mode_for_bytes(128));
+    constexpr uint32_t hi_add = smem_desc_hi(256, swizzle_mode_for_bytes(32));
+    constexpr uint32_t kMn = (128 * Cfg::SWZ - 16) >> 4 << 16;                     // from a tile's K-major word to its MN-major one
+    const uint32_t d_q = smem_desc_lo(smem_u32(smem + Cfg::OFF_Q), 16);
+    const uint32_t d_k = smem_desc_lo(smem_u32(smem + Cfg::OFF_K), 16);
+    const uint32_t d_do = smem_desc_lo(smem_u32(smem + Cfg::OFF_DO), 16);
+    const uint32_t d_v = smem_desc_lo(smem_u32(smem + Cfg::OFF_V), 16);
+    const uint32_t d_ds = smem_desc_lo(smem_u32(smem + Cfg::OFF_DS), 16384);
+    const uint32_t d_qadd = smem_desc_lo(smem_u32(smem + Cfg::OFF_QADD), 16);
+    const uint32_t d_doadd = smem_desc_lo(smem_u32(smem + Cfg::OFF_DOADD), 16);
+    const uint32_t d_kadd = smem_desc_lo(smem_u32(smem + Cfg::OFF_KADD), 16);
+    const uint32_t d_vadd = smem_desc_lo(smem_u32(smem + Cfg::OFF_VADD), 16);
+    constexpr uint32_t kTile16 = Cfg::TILE >> 4, kAdd16 = Cfg::ADD_TILE >> 4;
+
+    // stage trackers for the "ahead" stream (S, dP) and the "behind" stream (dV, dK, dQ)
+    int aq_s = 0, ak_s = 0, av_s = 0;
+    uint32_t aq_ph = 0, ak_ph = 0, av_ph = 0;
+    int bq_s = 0, bk_s = 0;
+    uint32_t pds_ph[2] = {0, 0}, dsready_ph = 0, dqfree_ph = 1, dkvfree_ph = ~0u;  // (dkvfree_ph: a bit per key tile of a strip)
+
+    BwdWalk wa, wb;  // ahead / behind
+    wa.init(blockIdx.x, gridDim.x, p.n_items, p.q_tiles, p.k_tiles, KS, p.n_strips);
+    wb = wa;
+
+    // whether the second half of a query tile has rows
+    auto two_halves = [&](int qt) { return !RAGGED || qt * 128 + 64 < p.N; };
+    auto wait_sdp = [&]() {  // for the operands of tile wa
+      if (Cfg::KV_STAYS && !wa.first_qt()) warp_wait(&q_full[aq_s], aq_ph, wctx);
+      else if (wa.first_kk()) warp_wait3(&q_full[aq_s], aq_ph, &k_full[ak_s], ak_ph, &v_full[av_s], av_ph, wctx);
+      else warp_wait2(&k_full[ak_s], ak_ph, &v_full[av_s], av_ph, wctx);
+      tc_fence_after();
+    };
+    auto issue_sdp = [&](int g) {  // S^T and dP^T of half g of tile wa
+      const uint32_t qo = aq_s * kTile16 + g * 4 * Cfg::SWZ, ko = ak_s * kTile16, vo = av_s * kTile16;
+      const uint32_t qa = aq_s * kAdd16 + g * 128;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) ppk[i] = dpk[i] = 0u;
-      } else
+      for (int ks = 0; ks < D / 16; ++ks)
+        umma_ss_w<hi, hi, idesc_sd>(el, tmem_base + Cfg::TM_S + 64 * g, d_k + ko + 2 * ks, d_q + qo + 2 * ks, ks != 0);
+      umma_ss_w<hi_add, hi_add, idesc_sd>(el, tmem_base + Cfg::TM_S + 64 * g, d_kadd + av_s * kAdd16, d_qadd + qa, 1u);
 #pragma unroll
-      for (int ch = 0; ch < 2; ++ch) {  // 16 keys per step
-        uint32_t rs[16], rd[16];
-        tmem_ld16(t_s + 16 * ch, rs);
-        tmem_ld16(t_dp + 16 * ch, rd);
-        const uint4 bv0 = *reinterpret_cast<const uint4*>(bias_row + (((piece0 + 2 * ch) ^ (row & 7)) << 4));
-        const uint4 bv1 = *reinterpret_cast<const uint4*>(bias_row + (((piece0 + 2 * ch + 1) ^ (row & 7)) << 4));
+      for (int ks = 0; ks < D / 16; ++ks)
+        umma_ss_w<hi, hi, idesc_sd>(el, tmem_base + Cfg::TM_DP + 64 * g, d_v + vo + 2 * ks, d_do + qo + 2 * ks, ks != 0);
+      umma_ss_w<hi_add, hi_add, idesc_sd>(el, tmem_base + Cfg::TM_DP + 64 * g, d_vadd, d_doadd + qa, 1u);
+      umma_commit(el, &sdp_full[g]);
+    };
+    auto next_sdp = [&]() {
+      if (!Cfg::KV_STAYS || wa.last_qt()) {
+        umma_commit(el, &v_empty[av_s]);
+        if (++av_s == NV) {
+          av_s = 0;
+          av_ph ^= 1;
+        }
+        if (++ak_s == NK) {
+          ak_s = 0;
+          ak_ph ^= 1;
+        }
+      }
+      const bool last_kk = wa.last_kk();
+      wa.next();
+      if (last_kk) {
+        if (++aq_s == NQ) {
+          aq_s = 0;
+          aq_ph ^= 1;
+        }
+      }
+    };
+
+    if (wa.valid()) {
+      wait_sdp();
+      issue_sdp(0);
+      if (two_halves(wa.qt)) issue_sdp(1);
+      next_sdp();
+    }
+    while (wb.valid()) {
+      const uint32_t qo = bq_s * kTile16, ko = bk_s * kTile16;
+      const uint32_t acc_kv = wb.first_qt() ? 0u : 1u;
+      const int q_left = p.N - wb.qt * 128, k_left = p.N - wb.kt() * 128;
+      const bool ahead = wa.valid();
+      if (ahead) wait_sdp();  // (here the answer of the probe is not waited for in the chain of a tile)
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        if (g == 0 || two_halves(wb.qt)) {
+          warp_wait(&pds_ready[g], pds_ph[g], wctx);
+          pds_ph[g] ^= 1;
+          if (g == 0 && wb.first_qt()) {
+            // the first accumulation overwrites dK/dV: those of the previous strip must have been read out
+            warp_wait(&dkv_free[wb.kk], (dkvfree_ph >> wb.kk) & 1u, wctx);
+            dkvfree_ph ^= 1u << wb.kk;
+          }
+          tc_fence_after();
+          // dV(kt) (+)= P^T dO ; dK(kt) (+)= dS^T Q   (16 queries per step; a warp's 32 queries start at its own 32 columns)
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            if (!RAGGED || 64 * g + 32 * (ks >> 1) < q_left)
+              umma_ts_w<hi, idesc_kv>(el, tmem_base + Cfg::TM_DV + wb.kk * D, tmem_base + Cfg::TM_S + 64 * g + (ks >> 1) * 32 + (ks & 1) * 8,
+                                      d_do + kMn + qo + (4 * g + ks) * Cfg::SWZ, (g | ks) != 0 ? 1u : acc_kv);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            if (!RAGGED || 64 * g + 32 * (ks >> 1) < q_left)
+              umma_ts_w<hi, idesc_kv>(el, tmem_base + Cfg::TM_DK + wb.kk * D, tmem_base + Cfg::TM_DP + 64 * g + (ks >> 1) * 32 + (ks & 1) * 8,
+                                      d_q + kMn + qo + (4 * g + ks) * Cfg::SWZ, (g | ks) != 0 ? 1u : acc_kv);
+        }
+        if (g == 1 && wb.last_qt()) umma_commit(el, &dkv_full[wb.kk]);
+        if (g == 1 && wb.last_kk()) {
+          umma_commit(el, &q_empty[bq_s]);
+          if (++bq_s == NQ) bq_s = 0;
+        }
+        // S and dP of the next tile's half: P and dS there have been read once these UMMAs start, which run in order
+        if (ahead) {
+          if (g == 0 || two_halves(wa.qt)) issue_sdp(g);
+          if (g == 1) next_sdp();
+        }
+      }
+      // dQ(qt) (+)= dS K   (16 keys per step)
+      warp_wait(ds_ready, dsready_ph, wctx);
+      dsready_ph ^= 1;
+      if (wb.first_kk()) {  // overwrites dQ
+        warp_wait(dq_free, dqfree_ph, wctx);
+        dqfree_ph ^= 1;
+      }
+      tc_fence_after();
+      const uint32_t acc_q = wb.first_kk() ? 0u : 1u;
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks)
+        if (!RAGGED || 32 * (ks >> 1) < k_left)
+          umma_ss_w<hi_ds, hi, idesc_dq>(el, tmem_base + Cfg::TM_DQ, d_ds + ks * 128, d_k + kMn + ko + ks * Cfg::SWZ,
+                                         (ks != 0) ? 1u : acc_q);
+      umma_commit(el, ds_free);
+      if (wb.last_kk()) umma_commit(el, dq_full);
+      if (!Cfg::KV_STAYS || wb.last_qt()) {
+        umma_commit(el, &k_empty[bk_s]);
+        if (++bk_s == NK) bk_s = 0;
+      }
+      wb.next();
+    }
+  } else if (warp > Cfg::WARP_MMA) {
+    // ------------------------------------------------------------------ finished gradients
+    // Four warps, one per TMEM lane quarter, read dQ after the last key tile of a query tile, and dK and dV of every key tile of
+    // a strip after the last query tile, as they are finished: 32 rows go through shared memory and leave by one TMA (D = 64:
+    // from registers).  With several strips dQ is summed in the CTA's scratch, in the order of the strips.
+    // (By the compute warps between two tiles this was 450 cycles of a tile's 2550.)
+    const int lane_base = 32 * (warp & 3);
+    const float scale = p.scale;
+    uint32_t dqfull_ph = 0, dkvfull_ph = 0;
+    [[maybe_unused]] int stg_buf = 0;
+    // tile rows n0 .. n0 + 127 in TMEM columns col ..; part: the tile is a part of the sum, `strip` of n_strips
+    auto drain = [&](uint32_t col, float mul, const CUtensorMap* map, __nv_bfloat16* plane, int n0, uint64_t* free_bar, bool part,
+                     int strip, int b, int o, int h) {
+      const int r0 = n0 + lane_base, row = r0 + lane;
+      const uint32_t src = tmem_addr(tmem_base, lane_base, col);
+      const bool out = !part || strip + 1 == p.n_strips;
+      if (r0 >= p.N) {
+        if (lane == 0) mbar_arrive(free_bar);
+        return;
+      }
+      // scratch of 32 rows (fewer at the end): 4 columns of every row, the next 4 ..., so that a warp's accesses are contiguous
+      const int rows = min(32, p.N - r0);
+      float4* const sums = reinterpret_cast<float4*>(p.dq_scratch + ((int64_t)blockIdx.x * p.N + r0) * D) + lane;
+      uint8_t* const stg = smem + Cfg::OFF_STG + ((warp & 3) * 2 + stg_buf) * Cfg::STG_BYTES;
+      if constexpr (Cfg::STAGED) {
+        if (out) {  // every use of a buffer is followed by its store: all stores but the newest have left the other one
+          stg_buf ^= 1;
+          bulk_wait_read<1>();
+          __syncwarp();
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < D; c += 16) {
+        uint32_t r[16];
+        tmem_ld16(src + c, r);
         tmem_ld_wait();
-        if (ch == 1) {
-          // S, dP and the bias tile have been read: the next pair of UMMAs / the next bias load may overwrite them
+        if (c + 16 == D) {
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) {
-            mbar_arrive(sdp_free);
-            mbar_arrive(&b_empty[b_s]);
+          if (lane == 0) mbar_arrive(free_bar);
+        }
+        if (part && row < p.N) {
+          if (strip > 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 a = sums[(c / 4 + i) * rows];
+              r[4 * i] = __float_as_uint(__uint_as_float(r[4 * i]) + a.x);
+              r[4 * i + 1] = __float_as_uint(__uint_as_float(r[4 * i + 1]) + a.y);
+              r[4 * i + 2] = __float_as_uint(__uint_as_float(r[4 * i + 2]) + a.z);
+              r[4 * i + 3] = __float_as_uint(__uint_as_float(r[4 * i + 3]) + a.w);
+            }
+          }
+          if (!out) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              sums[(c / 4 + i) * rows] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
+                                                     __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
           }
         }
-        const uint32_t bw[8] = {bv0.x, bv0.y, bv0.z, bv0.w, bv1.x, bv1.y, bv1.z, bv1.w};
-        uint64_t vv[8];
+        if (!out) continue;
+        uint4 w[2];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          vv[e] = f2_fma(f2_pack_bits(rs[2 * e], rs[2 * e + 1]), scale2, f2_pack_bits(bw[e] << 16, bw[e] & 0xFFFF0000u));
-        if (general) {
+        for (int i = 0; i < 2; ++i) {
+          float v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * i + e]) * mul;
+          w[i] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+        }
+        if constexpr (Cfg::STAGED) {
+          const int sw = D == 32 ? (lane >> 1) & 3 : (lane >> 2) & 1;  // the maps' 64- / 32-byte swizzle
+#pragma unroll
+          for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(stg + lane * (2 * D) + (((c >> 3) + i) ^ sw) * 16) = w[i];
+        } else if (row < p.N) {
+          uint4* dst = reinterpret_cast<uint4*>(plane + row * p.gn + c);
+          dst[0] = w[0];
+          dst[1] = w[1];
+        }
+      }
+      if constexpr (Cfg::STAGED) {
+        fence_async_smem();
+        __syncwarp();
+        if (out) tma_store_5d(lane == 0, map, stg, 0, r0, h, o, b);
+      }
+    };
+    for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
+      int b, o, h;
+      decode(item, b, o, h);
+      const int64_t off = b * p.gb + o * p.go + h * p.gh;
+      for (int strip = 0; strip < p.n_strips; ++strip) {
+        const int tiles_k = min(KS, p.k_tiles - strip * KS);
+        for (int qt = 0; qt < p.q_tiles; ++qt) {
+          if (qt == p.q_tiles - 1) {
+            for (int kk = 0; kk < tiles_k; ++kk) {
+              warp_wait(&dkv_full[kk], (dkvfull_ph >> kk) & 1u, wctx);
+              dkvfull_ph ^= 1u << kk;
+              tc_fence_after();
+              const int n0 = (strip * KS + kk) * 128;
+              // (each of the two reads arrives: dkv_free counts eight)
+              drain(Cfg::TM_DK + kk * D, scale, &tmDK, p.dk + off, n0, &dkv_free[kk], false, 0, b, o, h);
+              drain(Cfg::TM_DV + kk * D, 1.f, &tmDV, p.dv + off, n0, &dkv_free[kk], false, 0, b, o, h);
+            }
+          }
+          warp_wait(dq_full, dqfull_ph, wctx);
+          dqfull_ph ^= 1;
+          tc_fence_after();
+          drain(Cfg::TM_DQ, scale, &tmDQ, p.dq + off, qt * 128, dq_free, p.n_strips > 1, strip, b, o, h);
+        }
+      }
+    }
+    if constexpr (Cfg::STAGED) bulk_wait_all();
+  } else {
+    // ------------------------------------------------------------------ compute warps
+    const int part = warp >> 2;                 // which 32 queries of the tile
+    const int g = part >> 1;                    // group
+    const int lane_base = 32 * (warp & 3);
+    const int row = lane_base + lane;           // key in the tile == TMEM lane
+    const uint32_t t_s = tmem_addr(tmem_base, lane_base, Cfg::TM_S + 32 * part);
+    const uint32_t t_dp = tmem_addr(tmem_base, lane_base, Cfg::TM_DP + 32 * part);
+    // dS^T tile: a row per key, 128 bytes = the 64 queries of a group; the thread's 32 queries are four 16-byte pieces
+    uint8_t* const ds_row = smem + Cfg::OFF_DS + g * 16384 + row * 128;
+    const int piece0 = (part & 1) * 4;
+    // bias tile: a row per query, 256 bytes = 128 keys, not swizzled: the lanes of a warp read 64 consecutive bytes
+    const uint8_t* const bias_col = smem + Cfg::OFF_BIAS + part * (32 * 256) + row * 2;
+    constexpr float kLog2e = 1.4426950408889634f;
+    const uint64_t c1 = f2_pack(p.logit_scale * kLog2e, p.logit_scale * kLog2e);
+    const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
+
+    uint32_t sdpfull_ph = 0, dsfree_ph = 1, b_ph = 0;
+    int b_s = 0;
+    // The (item, strip, query tile, key tile) sequence as plain loops: the scalar part of a step is on the path between
+    // two UMMA batches.
+    for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
+    for (int strip = 0; strip < p.n_strips; ++strip) {
+      const int tiles_k = min(KS, p.k_tiles - strip * KS);
+    for (int qt = 0; qt < p.q_tiles; ++qt) {
+      bool no_half = false, no_rows = false;  // the group's / this warp's queries all lie beyond the last one
+      if constexpr (RAGGED) {
+        no_half = qt * 128 + 64 * g >= p.N;
+        no_rows = qt * 128 + 32 * part >= p.N;
+      }
+    for (int kk = 0; kk < tiles_k; ++kk) {
+      uint32_t dpk[16];  // bf16 pairs of dS of this thread's 32 queries
+      bool dead = false;
+      if constexpr (RAGGED) dead = no_rows || (strip * KS + kk) * 128 + lane_base >= p.N;
+      if (RAGGED && no_half) {
+        warp_wait(&b_full[b_s], b_ph, wctx);
+      } else {
+        warp_wait2(&sdp_full[g], sdpfull_ph, &b_full[b_s], b_ph, wctx);
+        sdpfull_ph ^= 1;
+      }
+      tc_fence_after();
+      const uint8_t* bias = bias_col + b_s * Cfg::BIAS_STAGE;
+      if (dead) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&b_empty[b_s]);
+      } else {
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {  // 16 queries per step
+          uint32_t rs[16], rd[16], bu[16];
+          tmem_ld16(t_s + 16 * ch, rs);
+          tmem_ld16(t_dp + 16 * ch, rd);
+#pragma unroll
+          for (int e = 0; e < 16; ++e) bu[e] = *reinterpret_cast<const uint16_t*>(bias + (16 * ch + e) * 256);
+          tmem_ld_wait();
+          uint32_t ppk[8], dtm[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const float2 mk = *reinterpret_cast<const float2*>(mask_row + 16 * ch + 2 * e);
-            float v0, v1;
-            f2_unpack(f2_add(vv[e], f2_pack(mk.x, mk.y)), v0, v1);
-            if (tail) {
-              const int k0 = kt * 128 + 32 * part + 16 * ch + 2 * e;
-              if (k0 >= p.N) v0 = -INFINITY;
-              if (k0 + 1 >= p.N) v1 = -INFINITY;
-            }
-            vv[e] = f2_pack(v0, v1);
+            const uint64_t bl = f2_mul(f2_pack_bits(bu[2 * e] << 16, bu[2 * e + 1] << 16), log2e2);
+            float a0, a1;
+            f2_unpack(f2_fma(f2_pack_bits(rs[2 * e], rs[2 * e + 1]), c1, bl), a0, a1);
+            const float p0 = ex2_approx(a0), p1 = ex2_approx(a1);
+            float d0, d1;
+            f2_unpack(f2_mul(f2_pack(p0, p1), f2_pack_bits(rd[2 * e], rd[2 * e + 1])), d0, d1);
+            ppk[e] = pack_bf16x2(p0, p1);
+            dtm[e] = dpk[8 * ch + e] = pack_bf16x2(d0, d1);
           }
+          if (ch == 1) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&b_empty[b_s]);
+          }
+          tmem_st8(t_s + 8 * ch, ppk);
+          tmem_st8(t_dp + 8 * ch, dtm);
         }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const uint64_t v2 = vv[e];
-          float a0, a1;
-          f2_unpack(f2_fma(v2, log2e2, nlse2), a0, a1);
-          const float p0 = ex2_approx(a0), p1 = ex2_approx(a1);
-          float d0, d1;
-          f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack_bits(rd[2 * e], rd[2 * e + 1]), ndel2)), d0, d1);
-          ppk[8 * ch + e] = pack_bf16x2(p0, p1);
-          dpk[8 * ch + e] = pack_bf16x2(d0, d1);
-        }
+        tmem_st_wait();
+      }
+      if (!(RAGGED && no_half)) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&pds_ready[g]);
       }
       if (++b_s == NB) {
         b_s = 0;
         b_ph ^= 1;
       }
-      if (++kv_s == NKV) {
-        kv_s = 0;
-        kv_ph ^= 1;
-      }
 
-      // the dV / dK / dQ UMMAs of the previous tile are done: the P and dS tiles are free and a finished dQ can be read
-      mbar_wait(pds_free, pdsfree_ph, wctx);
-      pdsfree_ph ^= 1;
-      tc_fence_after();
-      // the same completion covers the last tile of a strip: its dQ and the strip's dK / dV are read out now,
-      // before this tile's P / dS release the UMMAs that would overwrite them
-      take_finished();
-      {
-        uint8_t* p_row = smem + Cfg::OFF_P + half_off;
-        uint8_t* ds_row = smem + Cfg::OFF_DS + half_off;
+      // the dQ UMMAs of the previous tile are done: the dS tile is free
+      warp_wait(ds_free, dsfree_ph, wctx);
+      dsfree_ph ^= 1;
+      if (!dead) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int off = ((piece0 + u) ^ (row & 7)) << 4;
-          *reinterpret_cast<uint4*>(p_row + off) = make_uint4(ppk[4 * u], ppk[4 * u + 1], ppk[4 * u + 2], ppk[4 * u + 3]);
-          *reinterpret_cast<uint4*>(ds_row + off) = make_uint4(dpk[4 * u], dpk[4 * u + 1], dpk[4 * u + 2], dpk[4 * u + 3]);
-        }
+        for (int u = 0; u < 4; ++u)
+          *reinterpret_cast<uint4*>(ds_row + (((piece0 + u) ^ (row & 7)) << 4)) =
+              make_uint4(dpk[4 * u], dpk[4 * u + 1], dpk[4 * u + 2], dpk[4 * u + 3]);
       }
       fence_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(pds_ready);
-      store_finished();
-
+      if (lane == 0) mbar_arrive(ds_ready);
     }  // key tiles
-      have_prev_dq = true;
-      prev_q0 = qt * 128;
-      prev_strip = strip;
-      dq_dst = nullptr;
-      if (prev_q0 + row < p.N)
-        dq_dst = Cfg::STAGED ? p.dq + items[item_no & 3].off + (prev_q0 + row) * p.gn + DQ * part : dq_row + prev_q0 * p.gn;
     }  // query tiles
-      have_prev_strip = true;
-      prev_no = Cfg::STAGED ? item_no : item;
     }
     }
-    // the last tile of this CTA: wait for its UMMAs, then the same drain
-    if (have_prev_dq || have_prev_strip) {
-      mbar_wait(pds_free, pdsfree_ph, wctx);
-      pdsfree_ph ^= 1;
-      tc_fence_after();
-      take_finished();
-      store_finished();
-    }
-    if constexpr (Cfg::STAGED) bulk_wait_all();
+    // the UMMAs of this CTA's last tile have to be over before it ends
+    warp_wait(ds_free, dsfree_ph, wctx);
+    tc_fence_after();
   }
 
   tc_fence_before();
@@ -766,13 +765,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
 }
 
-// The additive mask of a tile's keys as an operand of S: row = key (32 bytes, as a D = 16 tile), its first three columns hold
-// value / scale split into bf16 parts, which an A operand of ones adds up again (24 bits: what fp32 has); S then gets the mask
-// with the scale like any logit.  Keys from n_keys on are masked.  Called by the issuing warp; returns whether there is anything
-// to add.  A lane makes the rows of four keys.
-// A row whose log-sum-exp is below this has masked keys only (by -inf or by a large finite value such as -1e9): its logits and
-// the log-sum-exp differ by nothing but rounding, of more than one unit.  It gets no gradient, with either value.
-constexpr float kMaskedLse = -1e8f;
+// The additive mask of a tile's keys as an operand of S (see Bf16x3; the A operand is ones).  Keys from n_keys on are masked.
+// Called by the issuing warp; returns whether there is anything to add.  A lane makes the rows of four keys.
 __device__ __forceinline__ bool mask_operand(uint8_t* dst, const float* mask_row, int n_keys, int lane, float inv_scale) {
   const float4 m = reinterpret_cast<const float4*>(mask_row)[lane];
   float v[4] = {m.x, m.y, m.z, m.w};
@@ -785,13 +779,8 @@ __device__ __forceinline__ bool mask_operand(uint8_t* dst, const float* mask_row
   if (!__any_sync(0xffffffffu, any)) return false;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int key = 4 * lane + i;
-    const float x = v[i] * inv_scale;
-    const float hi = __bfloat162float(__float2bfloat16_rn(x));
-    const bool inf = hi - hi != 0.f;  // (NaN too: one part carries it)
-    const float r = inf ? 0.f : x - hi;
-    const float mid = __bfloat162float(__float2bfloat16_rn(r));
-    *reinterpret_cast<uint2*>(dst + key * 32 + ((key >> 2) & 1) * 16) = make_uint2(pack_bf16x2(hi, mid), pack_bf16x2(r - mid, 0.f));
+    const Bf16x3 x = split_bf16x3(v[i] * inv_scale);
+    store_added(dst, 4 * lane + i, make_uint4(x.hi | x.mid << 16, x.lo, 0u, 0u));
   }
   fence_async_smem();
   __syncwarp();
@@ -1151,20 +1140,25 @@ __global__ void __launch_bounds__(256) attn_dbias_rows_kernel(const float* __res
 int make_qkv_tmap(CUtensorMap* tm, const void* base, int64_t B, int64_t O, int64_t H, int64_t N, int64_t D,
                   const int64_t* st, int swz);
 int make_bias_tmap(CUtensorMap* tm, const void* base, int64_t Bb, int64_t H, int64_t N, int64_t pitch);
+int make_bias_tmap_plain(CUtensorMap* tm, const void* base, int64_t Bb, int64_t H, int64_t N, int64_t pitch);
 int make_mask_tmap(CUtensorMap* tm, const void* base, int64_t B, int64_t O, int64_t N, int64_t pitch);
 int make_qkv_tmap_rows(CUtensorMap* tm, const void* base, int64_t B, int64_t O, int64_t H, int64_t N, int64_t D,
                        const int64_t* st, int swz, int rows);
 
+// What is added to the logits by UMMAs is divided by the softmax scale first.  A scale of zero (or nearly) leaves the logits
+// themselves out of fp32 sums with these quotients, which is what it asks for.
+static float logit_scale(float scale) { return fabsf(scale) < 1e-20f ? copysignf(1e-20f, scale) : scale; }
+
 template <int D>
 int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                    const CUtensorMap& tb, const CUtensorMap& tmk, const CUtensorMap& tdk, const CUtensorMap& tdv,
+                    const CUtensorMap& tb, const CUtensorMap& tdq, const CUtensorMap& tdk, const CUtensorMap& tdv,
                     AttnBwdParams& p, int* status, int grid, cudaStream_t stream) {
   using Cfg = AttnBwdCfg<D>;
   const bool ragged = p.N % 128 != 0 && p.N % 128 <= 96;  // some 32-row (32-key) block of the last tile is empty
   auto kern = ragged ? attn_bwd_kernel<Cfg, true> : attn_bwd_kernel<Cfg, false>;
   static PerDeviceOnce once[2];  // per instantiation
   if (int rc = ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, once[ragged])) return rc;
-  launch_kernel(kern, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, tq, tk, tv, tdo, tb, tmk, tdk, tdv, p, status);
+  launch_kernel(kern, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, tq, tk, tv, tdo, tb, tdq, tdk, tdv, p, status);
   TPF_LAUNCH_OK();
   return TPF_OK;
 }
@@ -1248,17 +1242,17 @@ int attn_backward_qkv(const AttnCall& c, void* workspace, int64_t workspace_byte
   const int64_t B = c.B, O = c.O, H = c.H, N = c.N, D = c.D;
   const int64_t need = attn_bwd_workspace_bytes(B, O, H, N, D);
   TPF_REQUIRE(need == 0 || (workspace && workspace_bytes >= need), TPF_ERR_WORKSPACE, "attn_bwd: workspace too small");
+  TPF_REQUIRE_ALIGNED16(c.mask, "attn_bwd", "mask");  // rows are read with 16-byte loads
   const int swz = 2 * (int)D;
-  CUtensorMap tq, tk, tv, tdo, tb, tm, tdk = {}, tdv = {};
+  CUtensorMap tq, tk, tv, tdo, tb, tdq = {}, tdk = {}, tdv = {};
   int rc;
   if ((rc = make_qkv_tmap(&tq, c.q, B, O, H, N, D, c.qs, swz))) return rc;
   if ((rc = make_qkv_tmap(&tk, c.k, B, O, H, N, D, c.ks, swz))) return rc;
   if ((rc = make_qkv_tmap(&tv, c.v, B, O, H, N, D, c.vs, swz))) return rc;
   if ((rc = make_qkv_tmap(&tdo, c.d_out, B, O, H, N, D, c.dos, swz))) return rc;
-  if ((rc = make_bias_tmap(&tb, c.bias, c.G, H, N, c.bias_pitch))) return rc;
-  if ((rc = make_mask_tmap(&tm, c.mask, B, O, N, c.mask_pitch))) return rc;
-
-  if (D <= 32 && ((rc = make_qkv_tmap_rows(&tdk, c.dk, B, O, H, N, D, c.ds, swz, 32)) ||
+  if ((rc = make_bias_tmap_plain(&tb, c.bias, c.G, H, N, c.bias_pitch))) return rc;
+  if (D <= 32 && ((rc = make_qkv_tmap_rows(&tdq, c.dq, B, O, H, N, D, c.ds, swz, 32)) ||
+                  (rc = make_qkv_tmap_rows(&tdk, c.dk, B, O, H, N, D, c.ds, swz, 32)) ||
                   (rc = make_qkv_tmap_rows(&tdv, c.dv, B, O, H, N, D, c.ds, swz, 32))))
     return rc;
   AttnBwdParams p;
@@ -1268,6 +1262,8 @@ int attn_backward_qkv(const AttnCall& c, void* workspace, int64_t workspace_byte
   p.gb = c.ds[0]; p.go = c.ds[1]; p.gh = c.ds[2]; p.gn = c.ds[3];
   p.lse = c.lse;
   p.delta = c.delta;
+  p.mask = c.mask;
+  p.mask_pitch = c.mask_pitch;
   p.dq_scratch = reinterpret_cast<float*>(workspace);
   p.B = (int)B; p.O = (int)O; p.H = (int)H; p.N = (int)N;
   p.q_tiles = (int)((N + 127) / 128);
@@ -1276,6 +1272,7 @@ int attn_backward_qkv(const AttnCall& c, void* workspace, int64_t workspace_byte
   p.n_strips = (p.k_tiles + ks - 1) / ks;
   p.bias_broadcast = c.G == 1 && B > 1 ? 1 : 0;
   p.scale = c.scale;
+  p.logit_scale = logit_scale(c.scale);
   p.n_items = (int)(B * O * H);
   p.div_h = FastDiv::make((uint32_t)H);
   p.div_o = FastDiv::make((uint32_t)O);
@@ -1283,9 +1280,9 @@ int attn_backward_qkv(const AttnCall& c, void* workspace, int64_t workspace_byte
   if (grid > p.n_items) grid = p.n_items;
   int* status = nullptr;
   if ((rc = attn_bwd_status_address(&status))) return rc;
-  if (D == 16) return launch_attn_bwd<16>(tq, tk, tv, tdo, tb, tm, tdk, tdv, p, status, grid, stream);
-  if (D == 32) return launch_attn_bwd<32>(tq, tk, tv, tdo, tb, tm, tdk, tdv, p, status, grid, stream);
-  return launch_attn_bwd<64>(tq, tk, tv, tdo, tb, tm, tdk, tdv, p, status, grid, stream);
+  if (D == 16) return launch_attn_bwd<16>(tq, tk, tv, tdo, tb, tdq, tdk, tdv, p, status, grid, stream);
+  if (D == 32) return launch_attn_bwd<32>(tq, tk, tv, tdo, tb, tdq, tdk, tdv, p, status, grid, stream);
+  return launch_attn_bwd<64>(tq, tk, tv, tdo, tb, tdq, tdk, tdv, p, status, grid, stream);
 }
 
 template <int D>
@@ -1405,7 +1402,7 @@ int attn_backward_bias(const AttnCall& c, void* workspace, int64_t workspace_byt
   p.chunk_len = chunk_len;
   p.q_tiles = (int)((N + 127) / 128);
   p.k_tiles = p.q_tiles;
-  p.scale = c.scale;
+  p.scale = logit_scale(c.scale);
   const int64_t grid = (int64_t)G * H * p.q_tiles * p.k_tiles * n_chunks;
   TPF_REQUIRE(grid < (1ll << 31), TPF_ERR_INVALID_ARGUMENT, "attn_bwd: dBias grid too large");
   int* status = nullptr;

@@ -509,6 +509,14 @@ int make_bias_tmap(CUtensorMap* tm, const void* base, int64_t Bb, int64_t H, int
   return make_tmap_bf16(tm, base, 4, dims, strides, box, 128);
 }
 
+// The same with boxes of 128 x 128, not swizzled.
+int make_bias_tmap_plain(CUtensorMap* tm, const void* base, int64_t Bb, int64_t H, int64_t N, int64_t pitch) {
+  uint64_t dims[4] = {(uint64_t)N, (uint64_t)N, (uint64_t)H, (uint64_t)Bb};
+  uint64_t strides[3] = {(uint64_t)pitch * 2, (uint64_t)pitch * N * 2, (uint64_t)pitch * N * H * 2};
+  uint32_t box[4] = {128, 128, 1, 1};
+  return make_tmap_bf16(tm, base, 4, dims, strides, box, 0);
+}
+
 // 3-D map over the fp32 additive mask [B,O,N] whose rows are `pitch` elements apart.
 int make_mask_tmap_cols(CUtensorMap* tm, const void* base, int64_t B, int64_t O, int64_t N, int64_t pitch, int cols) {
   uint64_t dims[3] = {(uint64_t)N, (uint64_t)O, (uint64_t)B};

@@ -144,6 +144,24 @@ __device__ __forceinline__ void mbar_wait3(uint64_t* a, uint32_t pa, uint64_t* b
   mbar_wait(c, pc, ctx);
 }
 
+// The same for a whole warp that goes on together: UMMAs, commits and TMA copies by an elected lane, TMEM loads and stores.  The
+// lanes may leave a wait one by one, and nothing but a barrier brings them together again for certain.  Left apart, two parts of
+// an issuing warp run through the same uniform registers: the dQ / dK / dV kernel issued UMMAs with descriptors whose upper word
+// was another operand's, on its first tile only, where the waits are long.
+__device__ __forceinline__ void warp_wait(uint64_t* bar, uint32_t parity, const WaitCtx& ctx) {
+  mbar_wait(bar, parity, ctx);
+  __syncwarp();
+}
+__device__ __forceinline__ void warp_wait2(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, const WaitCtx& ctx) {
+  mbar_wait2(a, pa, b, pb, ctx);
+  __syncwarp();
+}
+__device__ __forceinline__ void warp_wait3(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, uint64_t* c, uint32_t pc,
+                                           const WaitCtx& ctx) {
+  mbar_wait3(a, pa, b, pb, c, pc, ctx);
+  __syncwarp();
+}
+
 // ----------------------------------------------------------------------------
 // Proxy / tcgen05 fences
 // ----------------------------------------------------------------------------
@@ -282,6 +300,34 @@ __device__ __forceinline__ void umma_ts(uint32_t elected, uint32_t d_tmem, uint3
       "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected)
+      : "memory");
+}
+// The same with descriptors as two words, of which the upper one (stride, version, swizzle: smem_desc_hi) is a constant: a kernel
+// with many operands then keeps one register for each.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
+  return ((saddr & 0x3FFFFu) >> 4) | ((lbo_bytes >> 4) & 0x3FFFu) << 16;
+}
+__host__ __device__ constexpr uint32_t smem_desc_hi(uint32_t sbo_bytes, uint32_t swizzle_mode) {
+  return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | (swizzle_mode << 29);
+}
+template <uint32_t AHI, uint32_t BHI, uint32_t IDESC>
+__device__ __forceinline__ void umma_ss_w(uint32_t elected, uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t.reg .b32 i;\n\t"
+      "mov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %4};\n\tmov.b32 i, %5;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, i, p;\n\t}"
+      ::"r"(d_tmem), "r"(alo), "r"(blo), "n"(AHI), "n"(BHI), "n"(IDESC), "r"(accumulate), "r"(elected)
+      : "memory");
+}
+template <uint32_t BHI, uint32_t IDESC>
+__device__ __forceinline__ void umma_ts_w(uint32_t elected, uint32_t d_tmem, uint32_t a_tmem, uint32_t blo, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\t.reg .b32 i;\n\t"
+      "mov.b64 b, {%2, %3};\n\tmov.b32 i, %4;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, i, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(blo), "n"(BHI), "n"(IDESC), "r"(accumulate), "r"(elected)
       : "memory");
 }
 // Arrive on `bar` once every UMMA issued so far by the elected lane has completed.

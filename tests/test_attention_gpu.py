@@ -268,6 +268,50 @@ def test_gradients_under_masks_of_any_value(N, D):
     assert torch.isfinite(got["dbias"]).all()
 
 
+@pytest.mark.parametrize("N,D", [(33, 16), (64, 64), (65, 32), (97, 16), (128, 32), (130, 32), (161, 64), (257, 64), (400, 32),
+                                 (416, 16)])
+def test_equal_planes_get_equal_gradients(N, D):
+    """More planes than CTAs, all alike: every plane's gradients are the first one's bits, whatever the plane before left in
+    shared memory, TMEM or (poisoned here) device memory; the first plane's are the oracle's."""
+    O, H = 170, 2
+    gen = torch.Generator().manual_seed(N + D)
+    one = {n: torch.randn(1, 1, H, N, D, generator=gen).bfloat16() for n in ("q", "k", "v")}
+    bias = torch.randn(1, 1, H, N, N, generator=gen).bfloat16()
+    mask = torch.zeros(1, 1, 1, 1, N)
+    mask[..., N - N // 9:] = -1e9
+    d_one = torch.randn(1, 1, N, H, D, generator=gen).bfloat16()
+    poison = [torch.full((1 << 25,), float("nan"), device="cuda") for _ in range(4)]
+    del poison
+    planes = lambda t: t.cuda().expand(1, O, *t.shape[2:]).contiguous()  # noqa: E731
+    q, k, v = (planes(one[n]).requires_grad_(True) for n in ("q", "k", "v"))
+    out = tk.turbo_attention(q, k, v, pair_bias=bias.cuda(), res_mask=planes(mask))
+    grads = dict(zip(("dq", "dk", "dv"), torch.autograd.grad(out, (q, k, v), planes(d_one))))
+    ref = ao.attention_forward_backward(one["q"], one["k"], one["v"], bias, mask, d_one, dtype=torch.float64)
+    for n, g in grads.items():
+        assert ao.rel_l2(g[:, :1].cpu(), ref[n]) <= REL_TOL, n
+        assert torch.equal(g, g[:, :1].expand_as(g)), n
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.3, 1.5])
+def test_softmax_scale_of_any_value(scale):
+    """The log-sum-exp, the mask and delta enter the backward's products divided by the scale."""
+    O, H, N, D = 3, 2, 150, 32
+    gen = torch.Generator().manual_seed(7)
+    q, k, v = (torch.randn(1, O, H, N, D, generator=gen).bfloat16().cuda() for _ in range(3))
+    bias = torch.randn(1, H, N, N, generator=gen).bfloat16().cuda()
+    mask = torch.zeros(1, O, N, device="cuda")
+    mask[0, 1] = 3 * torch.randn(N, generator=gen)
+    mask[0, 2, 100:] = -1e9
+    d_out = torch.randn(1, O, N, H, D, generator=gen).bfloat16().cuda()
+    out, lse = torch.ops.tpf_b200.attn_fwd(q, k, v, mask, bias, scale)
+    got = torch.ops.tpf_b200.attn_bwd(q, k, v, d_out, out, lse, mask, bias, scale)
+    leaves = [t.double().requires_grad_(True) for t in (q, k, v, bias)]
+    logits = leaves[0] @ leaves[1].transpose(-1, -2) * scale + leaves[3] + mask[:, :, None, None, :]
+    ref_out = (logits.softmax(-1) @ leaves[2]).transpose(2, 3)
+    for n, g, r in zip(("dq", "dk", "dv", "dbias"), got, torch.autograd.grad(ref_out, leaves, d_out.double())):
+        assert (g.double() - r).norm() <= REL_TOL * r.norm(), n
+
+
 def test_no_python_fallback_native_library_is_loaded():
     with open("/proc/self/maps") as f:
         assert "libtpf_b200.so" in f.read()
