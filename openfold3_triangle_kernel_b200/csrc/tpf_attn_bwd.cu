@@ -914,8 +914,8 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       uint32_t ph = 1;
       for (int pl = pl0; pl < pl1; ++pl) {
         const int b = g * b_per_g + pl / p.O, o = pl % p.O;
-        if (pl - pl0 == NST - 1) mbar_wait(bias_done, 0, wctx);  // first use of the buffer the bias was staged in
-        mbar_wait(&empty[s], ph, wctx);
+        if (pl - pl0 == NST - 1) warp_wait(bias_done, 0, wctx);  // first use of the buffer the bias was staged in
+        warp_wait(&empty[s], ph, wctx);
         mbar_expect_tx(el, &full[s], 4 * Cfg::TILE + 512);
         uint8_t* st = smem + Cfg::OFF_ST + s * Cfg::STAGE;
         tma_load_5d(el, st, &tmQ, &full[s], 0, qt * 128, h, o, b);
@@ -940,7 +940,7 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       int s = 0, buf = 0;
       uint32_t ph = 0, free_ph[2] = {1, 1};
       for (int pl = pl0; pl < pl1; ++pl) {
-        mbar_wait2(&full[s], ph, &sdp_free[buf], free_ph[buf], wctx);
+        warp_wait2(&full[s], ph, &sdp_free[buf], free_ph[buf], wctx);
         free_ph[buf] ^= 1;
         tc_fence_after();
         const uint32_t st = smem_u32(smem + Cfg::OFF_ST + s * Cfg::STAGE);
@@ -977,7 +977,7 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     // ---- bias tile -> fp32 * log2(e), laid out [part][16-column half][4-column group][row][4] so that
     //      the 32 lanes of a warp read 32 consecutive 16-byte pieces
     float4* bias32 = reinterpret_cast<float4*>(smem + Cfg::OFF_BIAS32);
-    mbar_wait(bias_full, 0, wctx);
+    warp_wait(bias_full, 0, wctx);
     {
       const int col0 = CPT * part;
       const uint8_t* brow = bias_stage + (col0 >> 6) * 16384 + row * 128;
@@ -1028,7 +1028,7 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       l_n1 = l_n2;
       dl_n1 = dl_n2;
       load_row_scalars(pl + 2, l_n2, dl_n2);
-      mbar_wait(&sdp_full[buf], full_ph[buf], wctx);
+      warp_wait(&sdp_full[buf], full_ph[buf], wctx);
       full_ph[buf] ^= 1;
       tc_fence_after();
       const uint32_t t_s = tmem_addr(tmem_base, lane_base, buf * 256 + CPT * part);

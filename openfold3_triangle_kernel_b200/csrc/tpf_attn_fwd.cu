@@ -231,8 +231,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       int qj = 0, q_s = 0, qk_s = 0, qk_buf = 0;
       uint32_t q_ph = 0, qk_ph = 0;
       auto issue_qk = [&]() {
-        if (qj == 0) mbar_wait2(&q_full[q_s], q_ph, &k_full[qk_s], qk_ph, wctx);
-        else mbar_wait(&k_full[qk_s], qk_ph, wctx);
+        if (qj == 0) warp_wait2(&q_full[q_s], q_ph, &k_full[qk_s], qk_ph, wctx);
+        else warp_wait(&k_full[qk_s], qk_ph, wctx);
         const uint64_t qd = q_desc0 + (uint64_t)((q_s * Cfg::Q_TILE) >> 4);
         const uint64_t kd = k_desc0 + (uint64_t)((qk_s * Cfg::KV_TILE) >> 4);
 #pragma unroll
@@ -262,14 +262,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (tiles > 1) issue_qk();
       if (tiles > 2 && KT == 1) {
         // the third tile is the third item, whose Q goes where the first one's lies: not before that has been used
-        mbar_wait(&s_full[0], 0, wctx);
+        warp_wait(&s_full[0], 0, wctx);
         load_k();
       }
       int j = 0;
       for (int t = 0; t < tiles; ++t) {
         const int buf = t & 1;
         const uint32_t ph = (t >> 1) & 1;
-        mbar_wait(&p_ready[buf], ph, wctx);
+        warp_wait(&p_ready[buf], ph, wctx);
         tc_fence_after();
         const uint64_t vd = v_desc0 + (uint64_t)((buf * Cfg::KV_TILE) >> 4);
         // 16 keys per step; A = P from TMEM (8 columns of bf16 pairs).  A tail of at most 32 keys has no P beyond them.
@@ -281,7 +281,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         umma_commit(el, &pv_done[buf]);
         if (++j == KT) j = 0;
         if (t + 2 < tiles) {
-          mbar_wait(&pv_done[buf], ph, wctx);
+          warp_wait(&pv_done[buf], ph, wctx);
           tc_fence_after();
           issue_qk();
           load_bv();
@@ -307,7 +307,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float f_m = 0.f, f_l = 0.f;
     // normalise, gate and store the output row of the item whose last P V was tile t - 1
     auto finish_item = [&]() {
-      mbar_wait(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, wctx);
+      warp_wait(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, wctx);
       tc_fence_after();
       const float inv = f_l > 0.f ? __fdividef(1.f, f_l) : 0.f;
       const bool f_ok = f_q < p.N;
@@ -355,7 +355,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint32_t ph = (t >> 1) & 1;
         // s_full completes after Q K^T of this tile, hence after the K tile and the mask row that
         // arrives on the same barrier have landed
-        mbar_wait2(&s_full[buf], ph, &b_full[buf], ph, wctx);
+        warp_wait2(&s_full[buf], ph, &b_full[buf], ph, wctx);
         tc_fence_after();
         float* mask_row = reinterpret_cast<float*>(smem + Cfg::OFF_MASK + m_s * 256);
         if (++m_s == NS) m_s = 0;
@@ -413,7 +413,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (grow) m_use = cmax;
             l_run *= f;
             if (j > 0) {
-              mbar_wait(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, wctx);
+              warp_wait(&pv_done[(t - 1) & 1], ((t - 1) >> 1) & 1, wctx);
               tc_fence_after();
 #pragma unroll 1
               for (int cc = 0; cc < D; cc += 8) {

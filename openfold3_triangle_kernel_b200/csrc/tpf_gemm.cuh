@@ -336,7 +336,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if constexpr (Cfg::RESIDENT) {
           if (w.d0 == 0) {
             for (int kb = 0; kb < kb_count; ++kb) {
-              mbar_wait(&empty[s], ph, wctx);
+              warp_wait(&empty[s], ph, wctx);
               mbar_expect_tx(el, &full[s], Cfg::STAGE_BYTES);
               load_a(ring + s * Cfg::STAGE_BYTES, &full[s], kb * Cfg::BK, m0, 0);
               if (++s == Cfg::STAGES) {
@@ -361,7 +361,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if constexpr (Cfg::STAT != 0) {
           if (key != cur_key) {
             if (cur_key != -1) {  // the buffer is still being read by the previous run's UMMAs
-              mbar_wait(st_free, free_ph, wctx);
+              warp_wait(st_free, free_ph, wctx);
               free_ph ^= 1;
             }
             cur_key = key;
@@ -373,7 +373,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
         }
         for (int kb = 0; kb < kb_count; ++kb) {
-          mbar_wait(&empty[s], ph, wctx);
+          warp_wait(&empty[s], ph, wctx);
           mbar_expect_tx(el, &full[s], Cfg::STAGE_BYTES);
           const int k0 = kbase + kb * Cfg::BK;
           uint8_t* stage = ring + s * Cfg::STAGE_BYTES;
@@ -412,23 +412,23 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if constexpr (Cfg::RESIDENT) {
           first_col = w.d0 == 0;
           last_col = w.d0 == w.r0 - 1;
-          if (i < w.r0) mbar_wait(&st_full[i], 0, wctx);
+          if (i < w.r0) warp_wait(&st_full[i], 0, wctx);
           if (first_col && n0 + Cfg::BN > sh.N)
             id_n = make_idesc_bf16(Cfg::BM, (sh.N - n0 + 31) & ~31, Cfg::A_MN, Cfg::B_MN);
         } else if constexpr (Cfg::STAT != 0) {
           if (key != cur_key) {
-            mbar_wait(st_full, stat_ph, wctx);
+            warp_wait(st_full, stat_ph, wctx);
             stat_ph ^= 1;
             cur_key = key;
           }
         }
-        mbar_wait(&tempty[acc], acc_ph, wctx);
+        warp_wait(&tempty[acc], acc_ph, wctx);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_STRIDE;
         const int s_tile = s;
         const uint32_t ph_tile = ph;
         for (int kb = 0; kb < kb_count; ++kb) {
-          if (first_col) mbar_wait(&full[s], ph, wctx);
+          if (first_col) warp_wait(&full[s], ph, wctx);
           tc_fence_after();
           // descriptors = a base descriptor + (byte offset >> 4) in the start-address field (no carry out of it:
           // shared memory is far smaller than the field's range)

@@ -296,7 +296,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     uint32_t ph = 1;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
       for (int kb = 0; kb < KB; ++kb) {
-        mbar_wait(&a_empty[s], ph, wctx);
+        warp_wait(&a_empty[s], ph, wctx);
         load_z_block(el, smem + Cfg::OFF_A + s * 16384, &tmZ, &tmZ8, &a_full[s], p.rows, 64 * kb, tile * 128);
         if (++s == NST) {
           s = 0;
@@ -323,7 +323,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     const uint64_t a_desc = make_smem_desc(smem_u32(smem + Cfg::OFF_A), 16, 1024, sw);
     int s = 0, acc = 0;
     uint32_t ph = 0, acc_ph = 1;
-    mbar_wait(w_full, 0, wctx);
+    warp_wait(w_full, 0, wctx);
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
       const int s_tile = s;
       const uint32_t ph_tile = ph;
@@ -331,10 +331,10 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
       for (int n = 0; n < NT; ++n) {
         s = s_tile;
         ph = ph_tile;
-        mbar_wait(&tempty[acc], acc_ph, wctx);
+        warp_wait(&tempty[acc], acc_ph, wctx);
         const uint32_t d = tmem_base + 256 * acc;
         for (int kb = 0; kb < KB; ++kb) {
-          if (n == 0) mbar_wait(&a_full[s], ph, wctx);
+          if (n == 0) warp_wait(&a_full[s], ph, wctx);
           tc_fence_after();
           const uint64_t ad = a_desc + ((s * 16384) >> 4), wd = w_desc + ((kb * 4 * C * 128 + n * 16384) >> 4);
 #pragma unroll
@@ -632,7 +632,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     int i = 0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++i) {
       const int s = i & 1;
-      mbar_wait(&a_empty[s], ((i >> 1) & 1) ^ 1, wctx);
+      warp_wait(&a_empty[s], ((i >> 1) & 1) ^ 1, wctx);
       mbar_expect_tx(el, &x_full[s], Cfg::T_BYTES);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {  // 64 rows lie inside one batch entry
@@ -665,8 +665,8 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++i) {
       const int s = i & 1;
       const uint32_t ph = (i >> 1) & 1;
-      mbar_wait3(&tempty[s], ph ^ 1, &x_full[s], ph, &z_full[s], ph, wctx);
-      if (i == 0) mbar_wait(w_full, 0, wctx);
+      warp_wait3(&tempty[s], ph ^ 1, &x_full[s], ph, &z_full[s], ph, wctx);
+      if (i == 0) warp_wait(w_full, 0, wctx);
       tc_fence_after();
       const uint32_t d = tmem_base + Cfg::ACC * s;
 #pragma unroll
