@@ -129,8 +129,8 @@ struct AttnBwdCfg {
   static constexpr int NK = KV_STAYS ? 2 : 3, NV = 2, NQ = 2;
   static constexpr int NB = D <= 32 ? 2 : 1;   // bias stages
   static constexpr int NCW = 16;               // compute warps: two groups of eight, 64 queries each
-  static constexpr int THREADS = 32 * (NCW + 6);
-  static constexpr int WARP_TMA = NCW, WARP_MMA = NCW + 1;  // then four that store finished gradients
+  static constexpr int THREADS = 32 * (NCW + 7);
+  static constexpr int WARP_TMA = NCW, WARP_MMA = NCW + 1, WARP_ADD = NCW + 2;  // then four that store finished gradients
   static constexpr int SWZ = 2 * D;
   static constexpr int TILE = 128 * D * 2;
   static constexpr int ADD_TILE = 128 * 32;
@@ -198,7 +198,7 @@ struct BwdWalk {
 // there (hand-shakes, 14 UMMAs, completion), of which the other group hides most; the ex2 pipe alone needs 1024 cycles a tile.
 // Before, with a thread per query row, P and dS went through shared memory for three products of 128 x 128 tiles, whose operand
 // traffic kept it busy for 2400 cycles a tile, and one S / dP pair left all warps waiting together.  Measured, H = 4, us:
-// N = 384, D = 32 188 -> 133; N = 768 1523 -> 1010; N = 257, D = 64 233 -> 162; N = 128, D = 16, B = 4 35.4 -> 33.9.
+// N = 384, D = 32 188 -> 133; N = 768 1523 -> 1010; N = 257, D = 64 233 -> 156; N = 128, D = 16, B = 4 35.4 -> 30.4.
 // Waiting for S and dP apart was slower (136 us at N = 384), so was a warp of its own for dQ's UMMAs (137).
 //
 // RAGGED: a warp whose rows or keys of a tile all lie beyond the last one only keeps the barriers going, and the UMMAs leave its
@@ -244,7 +244,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&b_empty[s], NCW);
     }
     for (int s = 0; s < NQ; ++s) {
-      mbar_init(&q_full[s], 1);
+      mbar_init(&q_full[s], 2);  // the copies, the added operands
       mbar_init(&q_empty[s], 1);
     }
     for (int s = 0; s < NK; ++s) {
@@ -252,7 +252,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(&k_empty[s], 1);
     }
     for (int s = 0; s < NV; ++s) {
-      mbar_init(&v_full[s], 1);
+      mbar_init(&v_full[s], 2);
       mbar_init(&v_empty[s], 1);
     }
     for (int g = 0; g < 2; ++g) {
@@ -295,26 +295,73 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   };
 
   if (warp == Cfg::WARP_TMA) {
-    // ------------------------------------------------------------------ TMA producer, and the added operands
+    // ------------------------------------------------------------------ TMA producer
     const uint32_t el = elect_one();
     int q_s = 0, k_s = 0, v_s = 0, b_s = 0;
     uint32_t q_ph = 1, k_ph = 1, v_ph = 1, b_ph = 1;
+    int b = 0, o = 0, h = 0, cur = -1;
+    BwdWalk w;
+    for (w.init(blockIdx.x, gridDim.x, p.n_items, p.q_tiles, p.k_tiles, KS, p.n_strips); w.valid(); w.next()) {
+      if (w.item != cur) {
+        cur = w.item;
+        decode(cur, b, o, h);
+      }
+      if (w.first_kk()) {
+        warp_wait(&q_empty[q_s], q_ph, wctx);
+        mbar_expect_tx(el, &q_full[q_s], 2 * Cfg::TILE);
+        tma_load_5d(el, smem + Cfg::OFF_Q + q_s * Cfg::TILE, &tmQ, &q_full[q_s], 0, w.qt * 128, h, o, b);
+        tma_load_5d(el, smem + Cfg::OFF_DO + q_s * Cfg::TILE, &tmDO, &q_full[q_s], 0, w.qt * 128, h, o, b);
+        if (++q_s == NQ) {
+          q_s = 0;
+          q_ph ^= 1;
+        }
+      }
+      const int kt = w.kt();
+      if (!Cfg::KV_STAYS || w.first_qt()) {
+        warp_wait2(&v_empty[v_s], v_ph, &k_empty[k_s], k_ph, wctx);
+        mbar_expect_tx(el, &v_full[v_s], Cfg::TILE);
+        tma_load_5d(el, smem + Cfg::OFF_V + v_s * Cfg::TILE, &tmV, &v_full[v_s], 0, kt * 128, h, o, b);
+        mbar_expect_tx(el, &k_full[k_s], Cfg::TILE);
+        tma_load_5d(el, smem + Cfg::OFF_K + k_s * Cfg::TILE, &tmK, &k_full[k_s], 0, kt * 128, h, o, b);
+        if (++v_s == NV) {
+          v_s = 0;
+          v_ph ^= 1;
+        }
+        if (++k_s == NK) {
+          k_s = 0;
+          k_ph ^= 1;
+        }
+      }
+      warp_wait(&b_empty[b_s], b_ph, wctx);
+      mbar_expect_tx(el, &b_full[b_s], Cfg::BIAS_STAGE);
+      tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], kt * 128, w.qt * 128, h,
+                  p.bias_broadcast ? 0 : b);
+      if (++b_s == NB) {
+        b_s = 0;
+        b_ph ^= 1;
+      }
+    }
+  } else if (warp == Cfg::WARP_ADD) {
+    // ------------------------------------------------------------------ the added operands
+    // (By the loading warp between its copies they made the loads late.  Kernel, us: N = 128, D = 16, B = 4 33.9 -> 30.4,
+    // N = 257, D = 64 162 -> 156; N = 384 and 768, D = 32 no change.)
+    int q_s = 0, v_s = 0;
+    uint32_t q_ph = 1, v_ph = 1;
     BwdWalk w;
     w.init(blockIdx.x, gridDim.x, p.n_items, p.q_tiles, p.k_tiles, KS, p.n_strips);
     const float inv = 1.f / p.logit_scale;
     const float no_row = copysignf(1e30f, -p.logit_scale);  // makes exp2 zero, and no NaN with masked keys
-    // What a step adds to its logits and the coordinates of its plane.  The next step's are requested before this step's waits:
-    // requested after them, their latency made this warp the slowest part of the pipeline.
+    // The next step's values are requested before this step's waits.
     struct Step {
-      int b, o, h;
       float4 mask;
       float l[4], d[4];
     } cur, nxt;
     auto request = [&](const BwdWalk& at, Step& s) {
-      decode(at.item, s.b, s.o, s.h);
       const int k0 = at.kt() * 128 + 4 * lane;
-      if (k0 < p.mask_pitch)
-        s.mask = __ldg(reinterpret_cast<const float4*>(p.mask + ((int64_t)s.b * p.O + s.o) * p.mask_pitch + k0));
+      if (k0 < p.mask_pitch && (!Cfg::KV_STAYS || at.first_qt())) {
+        const int64_t bo = p.div_h.div((uint32_t)at.item);
+        s.mask = __ldg(reinterpret_cast<const float4*>(p.mask + bo * p.mask_pitch + k0));
+      }
       if (at.first_kk()) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -328,6 +375,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     };
     cur.mask = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
     for (int i = 0; i < 4; ++i) cur.l[i] = cur.d[i] = 0.f;
     if (w.valid()) request(w, cur);
     nxt = cur;
@@ -335,7 +383,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     while (w.valid()) {
       next.next();
       if (next.valid()) request(next, nxt);
-      const int b = cur.b, o = cur.o, h = cur.h;
       if (w.first_kk()) {
         warp_wait(&q_empty[q_s], q_ph, wctx);
 #pragma unroll
@@ -350,16 +397,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         fence_async_smem();
         __syncwarp();
-        mbar_expect_tx(el, &q_full[q_s], 2 * Cfg::TILE);
-        tma_load_5d(el, smem + Cfg::OFF_Q + q_s * Cfg::TILE, &tmQ, &q_full[q_s], 0, w.qt * 128, h, o, b);
-        tma_load_5d(el, smem + Cfg::OFF_DO + q_s * Cfg::TILE, &tmDO, &q_full[q_s], 0, w.qt * 128, h, o, b);
+        if (lane == 0) mbar_arrive(&q_full[q_s]);
         if (++q_s == NQ) {
           q_s = 0;
           q_ph ^= 1;
         }
       }
-      const int kt = w.kt();
       if (!Cfg::KV_STAYS || w.first_qt()) {
+        const int kt = w.kt();
         warp_wait(&v_empty[v_s], v_ph, wctx);
         const float mv[4] = {cur.mask.x, cur.mask.y, cur.mask.z, cur.mask.w};
 #pragma unroll
@@ -371,27 +416,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         fence_async_smem();
         __syncwarp();
-        mbar_expect_tx(el, &v_full[v_s], Cfg::TILE);
-        tma_load_5d(el, smem + Cfg::OFF_V + v_s * Cfg::TILE, &tmV, &v_full[v_s], 0, kt * 128, h, o, b);
+        if (lane == 0) mbar_arrive(&v_full[v_s]);
         if (++v_s == NV) {
           v_s = 0;
           v_ph ^= 1;
         }
-        warp_wait(&k_empty[k_s], k_ph, wctx);
-        mbar_expect_tx(el, &k_full[k_s], Cfg::TILE);
-        tma_load_5d(el, smem + Cfg::OFF_K + k_s * Cfg::TILE, &tmK, &k_full[k_s], 0, kt * 128, h, o, b);
-        if (++k_s == NK) {
-          k_s = 0;
-          k_ph ^= 1;
-        }
-      }
-      warp_wait(&b_empty[b_s], b_ph, wctx);
-      mbar_expect_tx(el, &b_full[b_s], Cfg::BIAS_STAGE);
-      tma_load_4d(el, smem + Cfg::OFF_BIAS + b_s * Cfg::BIAS_STAGE, &tmBias, &b_full[b_s], kt * 128, w.qt * 128, h,
-                  p.bias_broadcast ? 0 : b);
-      if (++b_s == NB) {
-        b_s = 0;
-        b_ph ^= 1;
       }
       w = next;
       cur = nxt;
@@ -541,7 +570,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       wb.next();
     }
-  } else if (warp > Cfg::WARP_MMA) {
+  } else if (warp > Cfg::WARP_ADD) {
     // ------------------------------------------------------------------ finished gradients
     // Four warps, one per TMEM lane quarter, read dQ after the last key tile of a query tile, and dK and dV of every key tile of
     // a strip after the last query tile, as they are finished: 32 rows go through shared memory and leave by one TMA (D = 64:
