@@ -358,9 +358,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     } cur, nxt;
     auto request = [&](const BwdWalk& at, Step& s) {
       const int k0 = at.kt() * 128 + 4 * lane;
-      if (k0 < p.mask_pitch && (!Cfg::KV_STAYS || at.first_qt())) {
-        const int64_t bo = p.div_h.div((uint32_t)at.item);
-        s.mask = __ldg(reinterpret_cast<const float4*>(p.mask + bo * p.mask_pitch + k0));
+      if (k0 < p.N && (!Cfg::KV_STAYS || at.first_qt())) {
+        const float* m = p.mask + (int64_t)p.div_h.div((uint32_t)at.item) * p.mask_pitch + k0;
+        if (k0 + 3 < p.N) s.mask = __ldg(reinterpret_cast<const float4*>(m));
+        else s.mask = make_float4(__ldg(m), k0 + 1 < p.N ? __ldg(m + 1) : 0.f, k0 + 2 < p.N ? __ldg(m + 2) : 0.f, 0.f);
       }
       if (at.first_kk()) {
 #pragma unroll
