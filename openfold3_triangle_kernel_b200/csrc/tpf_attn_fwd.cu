@@ -379,6 +379,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tmem_ld32(t_s + 64 * buf, *reinterpret_cast<uint32_t(*)[32]>(raw));
           tmem_ld32(t_s + 64 * buf + 32, *reinterpret_cast<uint32_t(*)[32]>(raw + 32));
           tmem_ld_wait();
+          // Keys that are not there (key 63 is one in a tail tile) are zeros, and an infinite query times zero is a NaN, which
+          // -inf does not mask.
+          if (GENERAL && n_keys < KEYS && __any_sync(0xffffffffu, __uint_as_float(raw[63]) != 0.f)) {
+#pragma unroll
+            for (int i = 0; i < 64; ++i)
+              if (i >= n_keys) raw[i] = 0u;
+          }
           float cm0 = -INFINITY, cm1 = -INFINITY;
 #pragma unroll
           for (int u = 0; u < 8; ++u) {

@@ -239,6 +239,33 @@ def test_nan_under_a_mask_reaches_the_output():
     assert torch.isnan(out).sum().item() == D
 
 
+def _row_of_minus_infinities(N, D):
+    """Query 5 of head 1, plane 1 is infinite where every key of that plane is positive: all its logits are -inf."""
+    O, H = 3, 2
+    gen = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn(1, O, H, N, D, generator=gen).bfloat16() for _ in range(3))
+    q[0, 1, 1, 5, 3] = -float("inf")
+    k[0, 1, 1, :, 3] = k[0, 1, 1, :, 3].abs() + 0.5
+    bias = torch.randn(1, 1, H, N, N, generator=gen).bfloat16()
+    return dict(q=q, k=k, v=v, pair_bias=bias, res_mask=torch.zeros(1, O, 1, 1, N))
+
+
+@pytest.mark.parametrize("N,D", [(6, 16), (32, 32), (33, 32), (63, 64), (64, 32), (97, 16), (120, 32), (257, 64)])
+def test_row_of_minus_infinities_is_a_masked_row(N, D):
+    """Its output is zero at every length: keys beyond the last one, which are read as zeros, add nothing (infinity times zero
+    is a NaN).  The other rows are those of a finite query there, bit for bit."""
+    inp = {n: t.cuda() for n, t in _row_of_minus_infinities(N, D).items()}
+    call = lambda: tk.turbo_attention(**inp, return_lse=True)  # noqa: E731
+    out, lse = call()
+    assert out[0, 1, 5, 1].abs().max().item() == 0.0
+    assert torch.isneginf(lse[0, 1, 1, 5])
+    inp["q"][0, 1, 1, 5] = 1.0
+    ref, ref_lse = call()
+    ref[0, 1, 5, 1] = 0
+    ref_lse[0, 1, 1, 5] = -float("inf")
+    assert torch.equal(out, ref) and torch.equal(lse, ref_lse)
+
+
 @pytest.mark.parametrize("N,D", [(20, 32), (128, 16), (129, 32), (150, 64), (300, 32)])
 def test_gradients_under_masks_of_any_value(N, D):
     """Masks that are not just 0 and a large value (they enter S as a sum of bf16 parts), single masked keys, masked key
