@@ -201,9 +201,14 @@ struct BwdWalk {
 // N = 384, D = 32 188 -> 133; N = 768 1523 -> 1010; N = 257, D = 64 233 -> 156; N = 128, D = 16, B = 4 35.4 -> 30.4.
 // Waiting for S and dP apart was slower (136 us at N = 384), so was a warp of its own for dQ's UMMAs (137).
 //
+// TAIL: the last tile has rows beyond the last key.  They are zeros, and an infinite query times zero is a NaN, which the added -inf
+// does not mask; their dS is written over with zeros, so that dQ of a query whose logits are all -inf is zero, as at any other
+// length.  (dK and dV of such rows are not stored.)  Without -> with that, us: N = 400 250 -> 252,
+// N = 517 455 -> 457, N = 510 320 -> 319; as a select of the registers in one kernel for every length N = 384 140 -> 144, N = 517 474.
+//
 // RAGGED: a warp whose rows or keys of a tile all lie beyond the last one only keeps the barriers going, and the UMMAs leave its
 // part of their K extent out; the others have the pipes to themselves.
-template <class Cfg, bool RAGGED>
+template <class Cfg, bool TAIL, bool RAGGED>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -697,6 +702,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     constexpr float kLog2e = 1.4426950408889634f;
     const uint64_t c1 = f2_pack(p.logit_scale * kLog2e, p.logit_scale * kLog2e);
     const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
+    [[maybe_unused]] const int tail_keys = p.N - (p.k_tiles - 1) * 128;  // of the last key tile
+    [[maybe_unused]] const bool tail_warp = lane_base + 32 > tail_keys;
 
     uint32_t sdpfull_ph = 0, dsfree_ph = 1, b_ph = 0;
     int b_s = 0;
@@ -774,6 +781,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int u = 0; u < 4; ++u)
           *reinterpret_cast<uint4*>(ds_row + (((piece0 + u) ^ (row & 7)) << 4)) =
               make_uint4(dpk[4 * u], dpk[4 * u + 1], dpk[4 * u + 2], dpk[4 * u + 3]);
+        if (TAIL && tail_warp && strip * KS + kk == p.k_tiles - 1 && row >= tail_keys) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            *reinterpret_cast<uint4*>(ds_row + (((piece0 + u) ^ (row & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+        }
       }
       fence_async_smem();
       __syncwarp();
@@ -1185,9 +1197,12 @@ int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
                     AttnBwdParams& p, int* status, int grid, cudaStream_t stream) {
   using Cfg = AttnBwdCfg<D>;
   const bool ragged = p.N % 128 != 0 && p.N % 128 <= 96;  // some 32-row (32-key) block of the last tile is empty
-  auto kern = ragged ? attn_bwd_kernel<Cfg, true> : attn_bwd_kernel<Cfg, false>;
-  static PerDeviceOnce once[2];  // per instantiation
-  if (int rc = ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, once[ragged])) return rc;
+  const int form = p.N % 128 == 0 ? 0 : ragged ? 2 : 1;
+  auto kern = form == 0   ? attn_bwd_kernel<Cfg, false, false>
+              : form == 1 ? attn_bwd_kernel<Cfg, true, false>
+                          : attn_bwd_kernel<Cfg, true, true>;
+  static PerDeviceOnce once[3];  // per instantiation
+  if (int rc = ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, once[form])) return rc;
   launch_kernel(kern, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, tq, tk, tv, tdo, tb, tdq, tdk, tdv, p, status);
   TPF_LAUNCH_OK();
   return TPF_OK;

@@ -266,6 +266,24 @@ def test_row_of_minus_infinities_is_a_masked_row(N, D):
     assert torch.equal(out, ref) and torch.equal(lse, ref_lse)
 
 
+@pytest.mark.parametrize("N,D", [(6, 16), (33, 32), (64, 64), (97, 16), (120, 32), (128, 32), (130, 64), (257, 64), (400, 32)])
+def test_row_of_minus_infinities_has_no_gradient(N, D):
+    """dQ of that query is zero at every length.  Without a gradient of its output the others are those of a finite query there,
+    bit for bit, but for the channel of dK that zero probabilities times the infinite query make NaN."""
+    inp = _row_of_minus_infinities(N, D)
+    gen = torch.Generator().manual_seed(N + D)
+    d_out = torch.randn(1, 3, N, 2, D, generator=gen).bfloat16()
+    assert _run(inp, d_out)[0]["dq"][0, 1, 1, 5].abs().max().item() == 0.0
+    d_out[0, 1, 5, 1] = 0
+    got, _ = _run(inp, d_out)
+    inp["q"][0, 1, 1, 5] = 1.0
+    ref, _ = _run(inp, d_out)
+    assert torch.isnan(got["dk"][0, 1, 1, :, 3]).all()
+    got["dk"][0, 1, 1, :, 3] = ref["dk"][0, 1, 1, :, 3]
+    for n in ("dq", "dk", "dv", "dbias"):
+        assert torch.equal(got[n], ref[n]), n
+
+
 @pytest.mark.parametrize("N,D", [(20, 32), (128, 16), (129, 32), (150, 64), (300, 32)])
 def test_gradients_under_masks_of_any_value(N, D):
     """Masks that are not just 0 and a large value (they enter S as a sum of bf16 parts), single masked keys, masked key
