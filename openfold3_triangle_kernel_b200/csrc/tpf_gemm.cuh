@@ -499,7 +499,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       w.next();  // w now names the next tile (its operands are requested below)
       const uint32_t t_acc = tmem_addr(tmem_base, lane_base, acc * Cfg::ACC_STRIDE);
       typename Epi::Pre nxt[NCH];
-      mbar_wait(&tfull[acc], acc_ph, wctx);
+      warp_wait(&tfull[acc], acc_ph, wctx);
       tc_fence_after();
       if constexpr (!Epi::kPaired) {
         const int m = m0 + lane_base + lane;

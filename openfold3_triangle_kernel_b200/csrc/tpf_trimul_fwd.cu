@@ -372,7 +372,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     const CUtensorMap* map = ch0 < C ? &tmAB0 : &tmAB1;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++i) {
       if (NT == 1 && (i & 1) != acc) continue;
-      mbar_wait2(&tfull[acc], acc_ph, &r_full[i % NRB], (i / NRB) & 1, wctx);
+      warp_wait2(&tfull[acc], acc_ph, &r_full[i % NRB], (i / NRB) & 1, wctx);
       acc_ph ^= 1;
       tc_fence_after();
 #pragma unroll 1
@@ -469,7 +469,7 @@ trimul_project_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
       int slot[KB];
 #pragma unroll
       for (int k = 0; k < KB; ++k) {
-        mbar_wait(&a_full[s], ph, wctx);
+        warp_wait(&a_full[s], ph, wctx);
         kb[k] = smem + Cfg::OFF_A + s * 16384;
         slot[k] = s;
         if (++s == NST) {
@@ -696,7 +696,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
           zst = p.z_stats[m_base + lane];
         }
       }
-      mbar_wait2(&tfull[s], (i >> 1) & 1, &r_full[i & 3], (i >> 2) & 1, wctx);
+      warp_wait2(&tfull[s], (i >> 1) & 1, &r_full[i & 3], (i >> 2) & 1, wctx);
       tc_fence_after();
       const float* row = reinterpret_cast<const float*>(smem + Cfg::OFF_ROW + (i & 3) * 1024) + 32 * quarter + lane;
       const uint64_t xr = f2_pack(row[0], row[0]), xm = f2_pack(row[128], row[128]);
@@ -786,7 +786,7 @@ trimul_output_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       const int s = i & 1;
       if (s != sw >> 1) continue;
       float* row = reinterpret_cast<float*>(smem + Cfg::OFF_ROW + (i & 3) * 1024);
-      mbar_wait(&x_full[s], (i >> 1) & 1, wctx);
+      warp_wait(&x_full[s], (i >> 1) & 1, wctx);
       stats_lines<C>(smem + Cfg::OFF_X + s * Cfg::T_BYTES + h * C * 128, lane, [&](int q, const RowStats& v) {
         row[64 * h + q] = v.rs;
         row[128 + 64 * h + q] = -v.rs * v.mu;

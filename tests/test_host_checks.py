@@ -1,5 +1,6 @@
 """Host-side checks of the launch helpers, compiled with the host compiler against a fake of the CUDA runtime."""
 import os
+import re
 import shutil
 import subprocess
 
@@ -57,3 +58,14 @@ def test_unaligned_shared_memory_base_is_an_error_before_the_launch(tmp_path):
     lines = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split("\n")
     # TPF_ERR_UNSUPPORTED (2) before any attribute is set, and again on the next call
     assert lines[:5] == ["0 1 0", "0 1 0", "2 0 2", "2 0 2", "0 1 0"]
+
+
+def test_a_warp_comes_together_again_after_every_wait():
+    """Kernels wait by warp_wait*, which end in a warp barrier: what follows (TMEM loads and stores, UMMAs, copies) is for whole
+    warps, and lanes may leave a bare mbar_wait one by one.  The bounded-wait self-test waits with one thread."""
+    csrc = os.path.join(ROOT, "openfold3_triangle_kernel_b200", "csrc")
+    bare = []
+    for name in sorted(set(os.listdir(csrc)) - {"tpf_ptx.cuh", "tpf_selftest.cu"}):
+        with open(os.path.join(csrc, name)) as f:
+            bare += [f"{name}:{i}" for i, line in enumerate(f, 1) if re.search(r"\bmbar_(try_)?wait\d?\s*\(", line)]
+    assert bare == []
