@@ -297,6 +297,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     constexpr float kLog2e = 1.4426950408889634f;
     constexpr float kLn2 = 0.6931471805599453f;
     constexpr float kGap = 12.0f;  // largest exponent (natural units) a probability may have relative to m
+    // A maximum below this belongs to a row that has met masked keys only, by a large finite value.  From 2^31 on m log2(e) is
+    // rounded by up to 2^7: the exponentials, made with one fma, would be infinite or zero.  Such a row subtracts m first.
+    constexpr float kFar = -1.4e9f;
     const uint64_t scale2 = f2_pack(p.scale, p.scale);
     const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
 
@@ -411,10 +414,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             }
           }
           const float cmax = GENERAL ? max3_nan(cm0, cm1, cm1) : fmaxf(cm0, cm1);
-          if (__any_sync(0xffffffffu, cmax > m_use + kGap)) {
+          if (__any_sync(0xffffffffu, cmax > (m_use < kFar ? -INFINITY : m_use + kGap))) {
             // Raise the reference maximum of the rows that need it (f = 1 for the others) and rescale what
             // those rows have accumulated.  Runs for the first finite tile of every row and then only
-            // when the logits of a row grow by more than kGap.
+            // when the logits of a row grow by more than kGap, or while a row has nothing but keys far below zero.
             const bool grow = cmax > m_use + kGap;
             const float f = grow ? ex2_approx((m_use - cmax) * kLog2e) : 1.f;  // m_use = -inf gives 0; nothing accumulated then
             if (grow) m_use = cmax;
@@ -432,6 +435,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 tmem_st8(t_o + cc, ro);
               }
             }
+            const float shift = m_use < kFar && m_use != -INFINITY ? m_use : 0.f;
+            if (__any_sync(0xffffffffu, shift != 0.f)) {
+#pragma unroll
+              for (int i = 0; i < 64; ++i) raw[i] = __float_as_uint(__uint_as_float(raw[i]) - shift);
+            }
           }
           if (GENERAL && !__any_sync(0xffffffffu, !(cmax < m_use - 104.f))) {
             // masked keys only: every probability is below the smallest fp32 number (no NaN among the logits either)
@@ -440,7 +448,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             for (int c = 0; c < 4; ++c) tmem_st8(t_s + 64 * buf + 8 * c, zero);
             return;
           }
-          const float neg_m = (m_use == -INFINITY) ? 0.f : -m_use * kLog2e;
+          const float neg_m = m_use < kFar ? 0.f : -m_use * kLog2e;
           const uint64_t neg_m2 = f2_pack(neg_m, neg_m);
           uint64_t rs2a = 0ull, rs2b = 0ull;  // packed partial row sums of this tile
 #pragma unroll

@@ -239,6 +239,35 @@ def test_nan_under_a_mask_reaches_the_output():
     assert torch.isnan(out).sum().item() == D
 
 
+@pytest.mark.parametrize("value", [-1e9, -1e10, -1e12, torch.finfo(torch.bfloat16).min, torch.finfo(torch.float32).min])
+@pytest.mark.parametrize("N,D", [(20, 32), (64, 16), (150, 64), (300, 32)])
+def test_masked_keys_by_large_finite_values(N, D, value):
+    """Whole key tiles that come first, single keys and whole planes, by the mask and by the bias.  The row maximum of such a tile
+    times log2(e) is rounded by more than an exponential bears."""
+    O, H = 5, 2
+    gen = torch.Generator().manual_seed(N + D)
+    inp = dict(zip(("q", "k", "v"), (torch.randn(1, O, H, N, D, generator=gen) for _ in range(3))))
+    inp["pair_bias"] = torch.randn(1, 1, H, N, N, generator=gen)
+    if value > torch.finfo(torch.float32).min:
+        inp["pair_bias"][..., 0, 1, 7, : N - 5] = value  # (as bf16 finfo.min of fp32 is an infinity)
+    mask = torch.zeros(1, O, 1, 1, N)
+    mask[0, 1, ..., : N - 3] = value
+    mask[0, 2, ..., ::3] = value
+    mask[0, 3, ..., N // 2: N - 5] = value
+    mask[0, 4] = value
+    inp["res_mask"] = mask
+    d_out = torch.randn(1, O, N, H, D, generator=gen).bfloat16()
+    d_out[0, 4] = 0
+    got, _ = _run(inp, d_out)
+    ref = _oracle(inp, d_out)
+    for n in ("out", "dq", "dk", "dv"):
+        assert ao.rel_l2(got[n][:, :4], ref[n][:, :4]) <= REL_TOL, n
+    assert ao.rel_l2(got["dbias"], ref["dbias"]) <= REL_TOL
+    rows = torch.arange(N) != 7  # (the bias there is added to the mask)
+    mean = inp["v"].bfloat16().double().mean(-2)[0, 4, None].expand(N, H, D)
+    assert ao.rel_l2(got["out"][0, 4][rows], mean[rows]) <= REL_TOL
+
+
 def _row_of_minus_infinities(N, D):
     """Query 5 of head 1, plane 1 is infinite where every key of that plane is positive: all its logits are -inf."""
     O, H = 3, 2
