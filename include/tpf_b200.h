@@ -99,6 +99,9 @@ int64_t tpf_attn_bwd_workspace_bytes(int64_t B, int64_t O, int64_t H, int64_t N,
  *   d_out, out   bf16 [B,O,N,H,D] contiguous (gradient of / the forward output)
  *   lse          fp32 [B,O,H,N] from tpf_attn_fwd
  *   workspace    at least tpf_attn_bwd_workspace_bytes(...) bytes, 256-byte aligned (may be NULL when 0)
+ * A row with lse < -2^24, i.e. one whose keys are all masked, by -inf or by a large finite value such as -1e9, has no
+ * gradient: dq of it is zero, and it adds nothing to dk, dv and dbias.  (Its output is zero with -inf; with a finite value
+ * fp32 logits hold little but the mask, and the output is a mean of v that is meant to be unused.)
  * Other arguments as in tpf_attn_fwd.  Deterministic: fixed summation orders, no atomics.
  * Replaces turbopairformer_triangle_delta_out + turbopairformer_triangle_sr_backward_out
  * (openfold3/core/kernels/turbopairformer/turbopairformer_triangle_delta.cu:343-414,

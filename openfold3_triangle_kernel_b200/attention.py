@@ -12,6 +12,9 @@ and README.md:84-115):
 * ``pair_bias``: required, bf16 or fp32 ``[*B, 1, H, N, N]`` (prefix broadcastable).
 * ``res_mask``: optional additive floating mask ``[*B, O, 1, 1, N]`` (0 keeps,
   ``-inf`` or a large negative drops); no boolean masks; never differentiated.
+  A row without any kept key has no gradient: its log-sum-exp is ``-inf`` or, with a
+  large finite mask such as -1e9, below -2**24.  Its output is zero in the first case
+  and a mean of v in the second.
 * returns bf16 ``[*B, O, N, H, D]``; autograd for q, k, v and pair_bias
   (the bias gradient has pair_bias's shape and dtype).
 

@@ -5,7 +5,7 @@
 // turbopairformer_triangle_sr_backward_out
 // (openfold3/core/kernels/turbopairformer/turbopairformer_triangle_delta.cu:343-414,
 //  openfold3/core/kernels/turbopairformer/turbopairformer_triangle_dq_dbias.cu:2526-2648).
-// Same math: P = exp(S - lse) (0 where lse = -inf), dP = dO V^T, dS = P (dP - delta),
+// Same math: P = exp(S - lse) (0 where lse < -2^24, -inf among it: no key is kept), dP = dO V^T, dS = P (dP - delta),
 // dV = P^T dO, dK = scale dS^T Q, dQ = scale dS K, dBias = sum over outer rows of dS; P and dS
 // are rounded to bf16 only as UMMA operands, all accumulation is fp32, no atomics anywhere.
 //
@@ -115,9 +115,10 @@ __device__ __forceinline__ void store_added(uint8_t* tile, int row, uint4 v) {
   *reinterpret_cast<uint4*>(tile + row * 32 + ((row >> 2) & 1) * 16) = v;  // (the 32-byte swizzle)
 }
 constexpr uint32_t kOnesBf16x2 = 0x3F803F80u;
-// A row whose log-sum-exp is below this has masked keys only (by -inf or by a large finite value such as -1e9): its logits and
-// the log-sum-exp differ by nothing but rounding, of more than one unit.  It gets no gradient, with either value.
-constexpr float kMaskedLse = -1e8f;
+// A row whose log-sum-exp is below -2^24 has masked keys only (by -inf or by a large finite value such as -1e9).  fp32 numbers are
+// two or more apart there, so what its logits and its log-sum-exp differ by is rounding, and exp of that is any number
+// (probabilities of 3e5 under a mask of -1e9, of 3.6 under -1e8).  It gets no gradient.
+constexpr float kMaskedLse = -16777216.f;
 
 template <int D_>
 struct AttnBwdCfg {

@@ -342,6 +342,29 @@ def test_gradients_under_masks_of_any_value(N, D):
     assert torch.isfinite(got["dbias"]).all()
 
 
+@pytest.mark.parametrize("N,D", [(20, 32), (128, 16), (150, 64), (300, 32)])
+def test_rows_masked_by_large_finite_values_have_no_gradient(N, D):
+    """Where all keys are masked by less than -2^24 the gradients are those of a mask of -inf, bit for bit: zero, and nothing added
+    to dbias, whatever d_out is.  The output stays the mean that it is (of v, where the mask rounds the logits away)."""
+    O, H = 6, 2
+    gen = torch.Generator().manual_seed(N + D)
+    inp = dict(zip(("q", "k", "v"), (torch.randn(1, O, H, N, D, generator=gen) for _ in range(3))))
+    inp["pair_bias"] = torch.randn(1, 1, H, N, N, generator=gen)
+    inp["res_mask"] = torch.zeros(1, O, 1, 1, N)
+    for o, value in enumerate((-2e7, -5e7, -1e8, -1e9, -1e12), 1):
+        inp["res_mask"][0, o] = value
+    d_out = torch.randn(1, O, N, H, D, generator=gen).bfloat16()
+    got, _ = _run(inp, d_out)
+    inp["res_mask"][0, 1:] = -float("inf")
+    ref, _ = _run(inp, d_out)
+    for n in ("dq", "dk", "dv"):
+        assert got[n][0, 1:].abs().max().item() == 0.0, n
+    for n in ("dq", "dk", "dv", "dbias"):
+        assert torch.equal(got[n], ref[n]), n
+    mean = inp["v"].bfloat16().double().mean(-2)[0, 4:, None].expand(2, N, H, D)  # planes of -1e9 and -1e12
+    assert ao.rel_l2(got["out"][0, 4:], mean) <= REL_TOL
+
+
 @pytest.mark.parametrize("N,D", [(33, 16), (64, 64), (65, 32), (97, 16), (128, 32), (130, 32), (161, 64), (257, 64), (400, 32),
                                  (416, 16)])
 def test_equal_planes_get_equal_gradients(N, D):
