@@ -245,9 +245,9 @@ struct EpiStore {
   }
 };
 
-// An epilogue without registers to spare: with a uniform warp index the compiler requests the next tile's operands above the
-// arithmetic of the present one (EpiGateSplitBwd, 96 registers: 300 bytes of spills, 103 instead of 62 us at N = 384).
-template <class Epi>
+// An epilogue without registers to spare at this tile width: with a uniform warp index the compiler requests the next tile's
+// operands above the arithmetic of the present one.
+template <class Epi, int BN>
 constexpr bool kPerLaneWarpIndex = false;
 
 template <class Cfg, class Epi>
@@ -271,7 +271,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // per-warp epilogue scratch (only when the epilogue asks for it) sits behind the barrier block, 1024-byte aligned
   uint8_t* epi_smem = ring + Cfg::STAGES * Cfg::STAGE_BYTES + 1024;
 
-  const int warp = kPerLaneWarpIndex<Epi> ? (int)(threadIdx.x >> 5) : warp_index();
+  const int warp = kPerLaneWarpIndex<Epi, Cfg::BN> ? (int)(threadIdx.x >> 5) : warp_index();
   const int lane = threadIdx.x & 31;
   const TileWalk<Cfg> walk(sh);
   const int k_len = sh.k_per_split > 0 ? sh.k_per_split : sh.K;

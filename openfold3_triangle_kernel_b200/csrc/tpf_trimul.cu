@@ -430,8 +430,10 @@ struct EpiGateSplitBwd {
     warp_tile_store_tma(reinterpret_cast<uint8_t*>(wsm), buf, lane, pk1, &p.map_d, col + p.C, m_base, 0);
   }
 };
+// (300 bytes of spills instead of 40.  Per lane -> uniform, us at N = 384: C = 128, 256 columns 65.5 -> 104; C = 96, 192 columns, where
+// the per-lane one spills 500 bytes, 96.5 -> 77; C = 64 31.4 -> 30.5; C = 32 22.6 -> 20.5.)
 template <>
-constexpr bool kPerLaneWarpIndex<EpiGateSplitBwd> = true;
+constexpr bool kPerLaneWarpIndex<EpiGateSplitBwd, 256> = true;
 
 // =============================================================================================
 // backward elementwise stages
