@@ -808,17 +808,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
 }
 
-// The additive mask of a tile's keys as an operand of S (see Bf16x3; the A operand is ones).  Keys from n_keys on are masked.
-// Called by the issuing warp; returns whether there is anything to add.  A lane makes the rows of four keys.
-__device__ __forceinline__ bool mask_operand(uint8_t* dst, const float* mask_row, int n_keys, int lane, float inv_scale) {
+// The additive mask of a tile's 128 keys as an operand of S (see Bf16x3; the A operand is ones).  Called by the issuing warp;
+// returns whether there is anything to add.  A lane makes the rows of four keys.
+__device__ __forceinline__ bool mask_operand(uint8_t* dst, const float* mask_row, int lane, float inv_scale) {
   const float4 m = reinterpret_cast<const float4*>(mask_row)[lane];
   float v[4] = {m.x, m.y, m.z, m.w};
   bool any = false;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (4 * lane + i >= n_keys) v[i] = -INFINITY;
-    any |= v[i] != 0.f;
-  }
+  for (int i = 0; i < 4; ++i) any |= v[i] != 0.f;
   if (!__any_sync(0xffffffffu, any)) return false;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -993,7 +990,7 @@ attn_dbias_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                   make_smem_desc(st + 2 * Cfg::TILE + ks * 32, 16, 8 * Cfg::SWZ, swz), idesc, ks != 0);
         // (S of this buffer has been read, so the UMMA that used its mask operand is done)
         if (mask_operand(smem + Cfg::OFF_MOP + buf * 4096, reinterpret_cast<const float*>(smem + Cfg::OFF_ST + s * Cfg::STAGE + 4 * Cfg::TILE),
-                         128, lane, inv_scale))
+                         lane, inv_scale))
           umma_ss(el, tmem_base + buf * 256, ones_desc, mop_desc + (uint64_t)(buf * (4096 >> 4)), idesc, 1u);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks)
