@@ -549,7 +549,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           umma_commit(el, &q_empty[bq_s]);
           if (++bq_s == NQ) bq_s = 0;
         }
-        // S and dP of the next tile's half: P and dS there have been read once these UMMAs start, which run in order
+        // S and dP of the next tile's half, over P and dS, which the UMMAs just issued still have to read.  PTX states the order
+        // of UMMAs for one accumulator and shape only, and these have others.  What this rests on is that the UMMAs of one
+        // issuing thread go through the CTA's one tensor pipe in the order of issue, which attention kernels that keep P in
+        // the columns of S are commonly built on; tests compare the bits of 170 equal planes.  A completion in between would
+        // put a commit and a probe (500 cycles) into the chain of every half tile.
         if (ahead) {
           if (g == 0 || two_halves(wa.qt)) issue_sdp(g);
           if (g == 1) next_sdp();
@@ -1346,15 +1350,16 @@ int launch_attn_dbias(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 // plane.  With one chunk whenever there are more tiles than SMs (N = 1021: 256 tiles) the last wave left half the
 // machine idle.  Chunk planes take at most `max_bytes`; one chunk needs none.
 // dBias and its fold, us by number of chunks (H = 4, D = 32, O = N; * is what the rule takes, with its workspace):
-//   N =  384   1: 362   2: 194   4: 110*   8: 120            9 MiB
-//   N =  400   1: 471   2: 251   4: 234    9: 228*          22 MiB
-//   N =  512   1: 480   2: 256   9: 252*  16: 278           36 MiB
-//   N =  640   1: 592   4: 479   7: 474   10: 477*          62 MiB
-//   N =  768   1: 717*  2: 727   4: 744    8: 782            0
-//   N = 1024   1: 1863  2: 1889  4: 1698*                   64 MiB
-// The count leaves out the fold, which reads every chunk plane (N = 640: the time per count grows from 0.92 to 1.02 us
-// between 1 and 10 chunks); the steps between schedules are larger.  Where the rule misses: N = 704 (144 tiles, the last
-// ones half empty) takes 824 us with the one chunk of a full wave, 755 with five.
+//   N =  384   1: 312   2: 167   4: 97*    8: 110            9 MiB
+//   N =  400   1: 322   2: 174   4: 183    9: 179*          22 MiB
+//   N =  512   1: 407   2: 220   9: 226*  16: 257           36 MiB
+//   N =  640   1: 509   4: 415   7: 419   10: 425*          62 MiB
+//   N =  704   1: 560*  5: 593                               0
+//   N =  768   1: 619*  2: 626   4: 648    8: 726            0
+//   N = 1024   1: 1688  2: 1761  4: 1585*                   64 MiB
+// The count leaves out the fold, which reads every chunk plane; the steps between schedules are larger.  Where the rule misses,
+// by 2 to 3 % (N = 400, 512, 640): planes have become a quarter cheaper than when the three were fitted, a CTA's start has not;
+// ten planes' time for it would take 2, 2 and 4 chunks there.
 static void dbias_plan(int64_t B, int64_t O, int64_t H, int64_t N, int64_t G, double max_bytes, int* n_chunks,
                        int* chunk_len) {
   const int64_t tiles = G * H * ((N + 127) / 128) * ((N + 127) / 128);
